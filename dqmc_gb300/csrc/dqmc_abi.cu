@@ -51,12 +51,12 @@ struct dqmc_handle {
   double *D1 = nullptr, *d2 = nullptr;
   int* ord1 = nullptr;
   QRWork qr{};
-  // mixed form: split-BF16 GEMM scratch and slicing
+  // split-BF16 GEMM scratch and slicing
   void* oz_scratch = nullptr;
   size_t oz_bytes = 0;
   unsigned long long* oz_acc = nullptr;   // split-K integer sums, zero between products
   size_t oz_acc_bytes = 0;
-  int oz_target = 40;   // mantissa bits kept per operand
+  int oz_target = 40;   // mantissa bits kept per operand of the mixed form's products
   // local updates
   double* delta_d = nullptr;
   double* unif_d = nullptr;
@@ -96,7 +96,7 @@ struct dqmc_handle {
   // the default: at n = 1024 both took about 0.3 ms per panel (the cluster's
   // FP64 work on 16 SMs offsets its cheaper barriers) and 141 ms of LU per sweep
   int lu_cluster = 0;
-  cplx* wy_v = nullptr;       // mixed form: (n x kWyMax) reflector block
+  cplx* wy_v = nullptr;       // (n x kWyMax) reflector block
   cplx* wy_s = nullptr;       // (kWyMax^2) Vb^H Vb
   cplx* wy_z = nullptr;       // (kWyMax x n) T Vb^H W
   cplx* wy_t = nullptr;       // (kWyMax) tau of the block
@@ -303,17 +303,32 @@ int wrap_greens(dqmc_handle* h, cplx* gf, int slice, int direction) {
 }
 
 // ---- dense kernels with their work models ----------------------------------
+// Every product goes through the split-BF16 GEMM: oz_target bits per operand
+// in the mixed form, 56 in the FP64 form.  56 bits leave no more error against
+// the exact product than FP64 FMA chains do (the slices are truncated at 2^-57
+// of a row's or column's largest entry and summed exactly, where an FMA chain
+// rounds K times at 2^-53) and take GB300's FP64 pipe, 1/1500 of its BF16 rate,
+// out of the product: n = 1024 8.3 -> 0.50 ms, n = 400 1.64 -> 0.09 ms, n = 64
+// 0.27 -> 0.04 ms (a 64 x 64 FMA tile is one SM's work), flush at n = 400 116 ->
+// 18 us.  allow_split = false keeps the FMA kernel (dqmc_gemm_check).
 // tensor flops of one split-BF16 complex GEMM: S(S+1)/2 slice pairs x 2 real GEMMs with K' = 2K
 double ozaki_tensor_flops(double m, double nn, double k, int S) {
   const double kp = 2.0 * std::ceil(k / 16.0) * 16.0;
   return S * (S + 1) / 2.0 * 2.0 * 2.0 * m * nn * kp;
 }
+// slices of a product of this handle: by K and the target in the mixed form
+bool oz_plan(const dqmc_handle* h, int k, int* S, int* bits) {
+  if (h->p.precision == DQMC_PREC_MIXED) return ozaki_plan(k, h->oz_target, S, bits);
+  *S = OZ_FP64_S;
+  *bits = OZ_FP64_BITS;
+  return true;
+}
 int zgemm_general(dqmc_handle* h, int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                   const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rs, const double* cs,
                   bool allow_split, int kind = -1, const int* active = nullptr, bool presliced = false) {
-  if (allow_split && h->p.precision == DQMC_PREC_MIXED) {
+  if (allow_split) {
     int S = 0, bits = 0;
-    if (!ozaki_plan(k, h->oz_target, &S, &bits)) return set_err(h, DQMC_ERR_ARG, "no exact slicing for this K");
+    if (!oz_plan(h, k, &S, &bits)) return set_err(h, DQMC_ERR_ARG, "no exact slicing for this K");
     // few output tiles and a long K: split K over more CTAs (exact integer partial sums)
     const int tiles = ((m + 63) / 64) * ((nn + 63) / 64);
     int splitk = 1;
@@ -321,12 +336,12 @@ int zgemm_general(dqmc_handle* h, int m, int nn, int k, char opA, char opB, cplx
       splitk = (h->sm_count + tiles - 1) / tiles;
       if (splitk > k / 64) splitk = k / 64;
     }
-    int kernels = 3;
+    int kernels = 2;
     LAUNCH(kind >= 0 ? kind : DQMC_K_OZGEMM, ozaki_tensor_flops(m, nn, k, S), gemm_bytes(m, nn, k),
            launch_ozaki_zgemm(m, nn, k, opA, opB, alpha, A, lda, B, ldb, beta, C, ldc, rs, cs, S, bits,
                               h->oz_scratch, h->oz_bytes, h->oz_acc, h->oz_acc_bytes, h->st, active, splitk,
                               &kernels, h->err_d, h->coop_cap == 0, presliced));
-    h->launches += kernels - 1;   // slicing kernels and the split-K finaliser
+    h->launches += kernels - 1;   // the slicing kernel and the split-K finaliser
     return DQMC_OK;
   }
   LAUNCH(kind >= 0 ? kind : DQMC_K_GEMM, gemm_flops(m, nn, k), gemm_bytes(m, nn, k),
@@ -394,10 +409,7 @@ int form_q_wy(dqmc_handle* h, cplx* W) {
 // decompose_udt! (src/linalg.jl:20-39) of A (destroyed): U (explicit), D, T.
 int decompose_udt(dqmc_handle* h, cplx* A, cplx* U, double* D, cplx* T) {
   CHK(qrp(h, A, T, D));
-  if (h->p.precision == DQMC_PREC_MIXED) return form_q_wy(h, U);
-  CHK(set_identity(h, U));
-  CHK(apply_q(h, U));
-  return DQMC_OK;
+  return form_q_wy(h, U);
 }
 
 // add_slice_sequence_left (src/stack.jl:278-293); idx 1-based.
@@ -546,14 +558,8 @@ int calculate_greens_scales(dqmc_handle* h, cplx* out) {
   LAUNCH(DQMC_K_MISC, 0.0, 32.0 * n2(h), launch_scale(h->W4, n, n, s, false, nullptr, false, h->st));
   CHK(permute(h, h->W4, h->W3, h->lu.perm, true, false));
   // U^-1 L^-1 (.), then diag(1/Drmax)
-  if (h->p.precision == DQMC_PREC_MIXED) {
-    CHK(trsm_blocked(h, Lm, nullptr, h->W3, true));
-    CHK(trsm_blocked(h, h->W1, h->lu.rdiag, h->W3, false));
-  } else {
-    LAUNCH(DQMC_K_TRSM, 4.0 * n3(h), 40.0 * n2(h), launch_trsm_left_lower_unit(Lm, h->W3, n, n, h->st));
-    LAUNCH(DQMC_K_TRSM, 4.0 * n3(h), 40.0 * n2(h), launch_trsm_left_upper(h->W1, nullptr, h->lu.rdiag, h->W3, n, n,
-                                                                           h->st));
-  }
+  CHK(trsm_blocked(h, Lm, nullptr, h->W3, true));
+  CHK(trsm_blocked(h, h->W1, h->lu.rdiag, h->W3, false));
   LAUNCH(DQMC_K_MISC, 0.0, 32.0 * n2(h), launch_scale(h->W3, n, n, s + 2 * n, false, nullptr, false, h->st));
   // G = Ur (.)
   CHK(gemm(h, 'N', 'N', h->Ur, h->W3, out));
@@ -880,15 +886,10 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
   }
   const int n = h->n, k = h->delay;
   DelayedArgs d{h->Xd, h->Yd, h->dstate, k, h->prep, h->blk, h->pub, {}};
-  // mixed form: the delayed kernel cuts the flush's slices at the round's end
-  bool presliced = false;
-  if (h->p.precision == DQMC_PREC_MIXED) {
-    int S = 0, bits = 0;
-    if (ozaki_plan(4 * k, h->oz_target, &S, &bits) && ozaki_scratch_bytes(n, n, 4 * k, S) <= h->oz_bytes) {
-      d.sl = ozaki_slices(h->oz_scratch, n, n, 4 * k, S, bits);
-      presliced = true;
-    }
-  }
+  // the delayed kernel cuts the flush's slices at the round's end
+  int S = 0, bits = 0;
+  const bool presliced = oz_plan(h, 4 * k, &S, &bits) && ozaki_scratch_bytes(n, n, 4 * k, S) <= h->oz_bytes;
+  if (presliced) d.sl = ozaki_slices(h->oz_scratch, n, n, 4 * k, S, bits);
   LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_prepare(a, h->prep, h->dstate, h->st));
   const int rounds = (h->N + k - 1) / k + 1;
   auto round = [&]() -> int {
@@ -991,13 +992,8 @@ int solve_left(dqmc_handle* h, const cplx* A, cplx* X, cplx* wa, cplx* wb) {
   const cplx* Lm = nullptr;
   CHK(lu_blocked(h, wa, &Lm));
   CHK(permute(h, X, wb, h->lu.perm, true, false));
-  if (h->p.precision == DQMC_PREC_MIXED) {
-    CHK(trsm_blocked(h, Lm, nullptr, wb, true));
-    CHK(trsm_blocked(h, wa, h->lu.rdiag, wb, false));
-  } else {
-    LAUNCH(DQMC_K_TRSM, 4.0 * n3(h), 40.0 * n2(h), launch_trsm_left_lower_unit(Lm, wb, n, n, h->st));
-    LAUNCH(DQMC_K_TRSM, 4.0 * n3(h), 40.0 * n2(h), launch_trsm_left_upper(wa, nullptr, h->lu.rdiag, wb, n, n, h->st));
-  }
+  CHK(trsm_blocked(h, Lm, nullptr, wb, true));
+  CHK(trsm_blocked(h, wa, h->lu.rdiag, wb, false));
   return copy_nn(h, X, wb);
 }
 
@@ -1319,25 +1315,22 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
     A((void**)&h->blk, (size_t)16 * h->N * sizeof(cplx));
     A((void**)&h->pub, (size_t)h->N * sizeof(int));
   }
-  if (p->precision == DQMC_PREC_MIXED) {
-    A((void**)&h->wy_v, (size_t)n * kWyMax * sizeof(cplx));
-    A((void**)&h->wy_s, (size_t)kWyMax * kWyMax * sizeof(cplx));
-    A((void**)&h->wy_z, (size_t)kWyMax * n * sizeof(cplx));
-    A((void**)&h->wy_t, (size_t)kWyMax * sizeof(cplx));
+  A((void**)&h->wy_v, (size_t)n * kWyMax * sizeof(cplx));
+  A((void**)&h->wy_s, (size_t)kWyMax * kWyMax * sizeof(cplx));
+  A((void**)&h->wy_z, (size_t)kWyMax * n * sizeof(cplx));
+  A((void**)&h->wy_t, (size_t)kWyMax * sizeof(cplx));
+  {
     h->oz_target = p->ozaki_bits > 0 ? p->ozaki_bits : 40;
-    // the largest products are n x n x n; the flush (K = 4k) needs fewer slices
+    // the largest products are n x n x n, or the flush (K = 4k)
     int S = 0, bits = 0;
-    if (!ozaki_plan((int)n, h->oz_target, &S, &bits)) return fail(DQMC_ERR_ARG);
-    size_t need = ozaki_scratch_bytes((int)n, (int)n, (int)n, S);
-    if (h->delay > 1 && ozaki_plan(4 * h->delay, h->oz_target, &S, &bits)) {
-      size_t f = ozaki_scratch_bytes((int)n, (int)n, 4 * h->delay, S);
-      if (f > need) need = f;
-    }
-    h->oz_bytes = need;
+    if (!oz_plan(h, (int)n, &S, &bits)) return fail(DQMC_ERR_ARG);
+    h->oz_bytes = ozaki_scratch_bytes((int)n, (int)n, (int)n, S);
+    if (h->delay > 1 && oz_plan(h, 4 * h->delay, &S, &bits))
+      h->oz_bytes = std::max(h->oz_bytes, ozaki_scratch_bytes((int)n, (int)n, 4 * h->delay, S));
     A(&h->oz_scratch, h->oz_bytes);
-    // split K is taken for fewer than sm_count / 2 output tiles of 64 x 64
+    // split K is taken for fewer than sm_count / 2 output tiles of 64 x 64; two words per real sum above 42 bits
     const size_t tiles = (size_t)(h->sm_count / 2 + 1);
-    h->oz_acc_bytes = std::min((size_t)n * n, tiles * 64 * 64) * 2 * sizeof(unsigned long long);
+    h->oz_acc_bytes = std::min((size_t)n * n, tiles * 64 * 64) * 4 * sizeof(unsigned long long);
     A((void**)&h->oz_acc, h->oz_acc_bytes);
   }
   if (!ok) return fail(DQMC_ERR_CUDA);

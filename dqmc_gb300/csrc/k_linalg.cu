@@ -1082,30 +1082,6 @@ __global__ void __launch_bounds__(128) k_trsm_left_upper(const cplx* __restrict_
   for (int r = lane; r < n; r += 32) yg[r] = y[r];
 }
 
-// Y <- L^-1 Y with L unit lower triangular (strictly lower part of Lc,
-// column-major), one warp per column of Y (column staged in shared memory).
-__global__ void __launch_bounds__(128) k_trsm_left_lower_unit(const cplx* __restrict__ Lc, cplx* __restrict__ Y, int n,
-                                                             int m) {
-  extern __shared__ double smem_t[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int col = blockIdx.x * (blockDim.x / 32) + wid;
-  if (col >= m) return;
-  cplx* y = reinterpret_cast<cplx*>(smem_t) + (size_t)wid * n;
-  cplx* yg = Y + (size_t)col * n;
-  for (int r = lane; r < n; r += 32) y[r] = yg[r];
-  __syncwarp();
-  for (int q = 0; q < n - 1; ++q) {
-    const cplx* lq = Lc + (size_t)q * n;
-    const cplx yq = y[q];
-    for (int r = q + 1 + lane; r < n; r += 32) {
-      const cplx t = __ldg(&lq[r]);
-      y[r] = cmake(fma(-yq.x, t.x, fma(yq.y, t.y, y[r].x)), fma(-yq.x, t.y, fma(-yq.y, t.x, y[r].y)));
-    }
-    __syncwarp();
-  }
-  for (int r = lane; r < n; r += 32) yg[r] = y[r];
-}
-
 // Diagonal-block solve of a blocked triangular solve: the b x b block of T
 // at (j0, j0) (leading dimension ldT) applied to rows j0..j0+b of the m
 // columns of Y (leading dimension ldY).  lower: unit lower triangular,
@@ -1382,14 +1358,6 @@ cudaError_t launch_trsm_diag_block(const cplx* T, int ldT, const cplx* rdiag, cp
   if (cudaError_t ea = smem_limit.raise((const void*)k_trsm_diag_block, kMaxTdb); ea != cudaSuccess) return ea;
   k_trsm_diag_block<<<(m + TRSM_DB_WARPS - 1) / TRSM_DB_WARPS, 32 * TRSM_DB_WARPS, smem, st>>>(
       T, ldT, rdiag, Y, ldY, j0, b, m, lower ? 1 : 0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_trsm_left_lower_unit(const cplx* Lc, cplx* Y, int n, int m, cudaStream_t st) {
-  size_t smem = (size_t)4 * n * sizeof(cplx);
-  static SmemLimit smem_limit;
-  if (cudaError_t ea = smem_limit.raise((const void*)k_trsm_left_lower_unit, 200 * 1024); ea != cudaSuccess) return ea;
-  k_trsm_left_lower_unit<<<(m + 3) / 4, 128, smem, st>>>(Lc, Y, n, m);
   return cudaGetLastError();
 }
 

@@ -6,22 +6,25 @@
 // form computes the dense products of the UDT stabilisation and of the
 // delayed local-update flush as sums of exact BF16 x BF16 -> FP32 products:
 //
-//  * every row i of op(A) gets a power-of-two scale sigma_i >= max_k |op(A)_ik|
+//  * every row i of op(A) gets a power-of-two scale sigma_i > max_k |op(A)_ik|
 //    (real and imaginary parts together), every column j of op(B) a scale
-//    tau_j; the scaled entries lie in [-1, 1];
-//  * each scaled entry x is cut into S slices of B_BITS bits,
-//    x ~ sum_p 2^{-B_BITS p} a_p with integers |a_p| <= 2^B_BITS, which BF16
-//    holds exactly;
+//    tau_j; the scaled entries lie in (-1, 1);
+//  * each scaled entry x is cut into S slices of B bits, x ~ sum_p 2^{-B p} a_p
+//    with integers |a_1| <= 2^B, |a_p| <= 2^(B-1), which BF16 holds exactly;
 //  * the complex product is two real GEMMs with K' = 2K on stacked operands,
 //    A' = [Re A, Im A] and B'_re = [Re B; -Im B], B'_im = [Im B; Re B];
 //  * slice pairs (p, q) with p + q = t <= S + 1 are accumulated into one FP32
-//    accumulator per t; with K' * S * 2^{2 B_BITS} <= 2^24 every partial sum is
-//    an integer below 2^24, so the FP32 accumulation is exact; the group sums
-//    are combined exactly in 64-bit integers (Horner in 2^B_BITS) and the
-//    result converted once with its power-of-two weight and the scales.
-// The only error is the truncation of the slice expansion (~2^{-B_BITS S}
-// relative to sigma_i tau_j K).
-//
+//    accumulator per t, over chunks of K' short enough that
+//    chunk (S + 2) 2^{2B - 2} <= 2^24 (the digit bounds above, summed over the
+//    pairs of a group): every partial sum is an integer of at most 24 bits, so
+//    the FP32 accumulation is exact whatever K is (S = 8 slices of 7 bits, the
+//    FP64 form's products: chunks of 384);
+//  * the group sums of a chunk are combined exactly in 64-bit integers (one for
+//    up to 61 bits, else a high and a low one) and the result rounded once to
+//    double with its power-of-two weight and the scales.
+// The only errors are the truncation of the slice expansion (2^{-B S - 1}
+// relative to sigma_i and tau_j), the dropped pairs p + q > S + 1 of the same
+// size, and one FP64 rounding per chunk.
 // The tensor-core products run on tcgen05.mma (kind::f16, BF16 in, FP32
 // accumulators in tensor memory), with every operand tile staged by TMA
 // (cp.async.bulk.tensor) onto mbarriers; see the engine section below.
@@ -32,7 +35,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include <type_traits>
+#include <algorithm>
 #include "common.cuh"
 #include "kernels.h"
 #include "oz_slice.cuh"
@@ -42,141 +45,73 @@ namespace {
 // ---------------------------------------------------------------------------
 // split: slices of op(X) scaled per row ("row" side = A) or per column (B side)
 // ---------------------------------------------------------------------------
-// element (r, c) of op(X) where X is column-major with leading dimension ld
-__device__ __forceinline__ cplx op_elem(const cplx* X, int ld, int r, int c, char op) {
-  if (op == 'N') return X[(size_t)c * ld + r];
-  cplx v = X[(size_t)r * ld + c];
-  return op == 'C' ? cconj(v) : v;
-}
+// (the digit helpers are in oz_slice.cuh)
 
-// (the digit helpers expo_field, fixed62 and next_digit are in oz_slice.cuh)
-__device__ __forceinline__ int block_max_int(int v, int* red) {
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int t = 0;
-  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t = max(t, red[q]);
-  return t;
-}
-
-// A side: op(A) is rows x K; writes S slices of A' (rows x Kp, row-major,
-// Kp = 2 * Kpad): row i = [Re op(A)_i,:  Im op(A)_i,:], zero padded.
-__global__ void k_oz_split_rows(const cplx* __restrict__ X, int ld, char op, int rows, int K, int Kpad, int S,
-                                int bits, __nv_bfloat16* __restrict__ out, double* __restrict__ scale,
-                                const int* __restrict__ active) {
-  const int i = blockIdx.x;
-  if (i >= rows) return;
-  if (active) {   // only the first 4p inner indices are live (delayed-update flush)
-    const int kk = 4 * *active;
-    if (kk == 0) return;
-    if (kk < K) K = kk;
-  }
-  __shared__ int red[32];
-  int me = 0;
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
-    const cplx v = op_elem(X, ld, i, k, op);
-    me = max(me, max(expo_field(v.x), expo_field(v.y)));
-  }
-  me = block_max_int(me, red);
-  const int E = me > 0 ? me - 1022 : 0;   // 2^E > max |.| (frexp exponent)
-  if (threadIdx.x == 0) scale[i] = ldexp(1.0, E);
-  const size_t Kp = 2 * (size_t)Kpad;
-  for (int k = threadIdx.x; k < Kpad; k += blockDim.x) {
-    const cplx v = k < K ? op_elem(X, ld, i, k, op) : cmake(0.0, 0.0);
-    long long xr = fixed62(v.x, E), xi = fixed62(v.y, E);
-    for (int p = 0; p < S; ++p) {
-      const int sft = 62 - (p + 1) * bits;
-      const int ar = next_digit(xr, sft), ai = next_digit(xi, sft);
-      __nv_bfloat16* o = out + (size_t)p * rows * Kp + (size_t)i * Kp;
-      o[k] = __float2bfloat16_rn((float)ar);
-      o[Kpad + k] = __float2bfloat16_rn((float)ai);
-    }
-  }
-}
-
-// B side: op(B) is K x cols; writes S slices of B'_re and B'_im (cols x Kp,
-// K contiguous per column): column j of B'_re = [Re op(B)_:,j ; -Im op(B)_:,j],
-// of B'_im = [Im op(B)_:,j ; Re op(B)_:,j].
-__global__ void k_oz_split_cols(const cplx* __restrict__ X, int ld, char op, int K, int cols, int Kpad, int S,
-                                int bits, __nv_bfloat16* __restrict__ out_re, __nv_bfloat16* __restrict__ out_im,
-                                double* __restrict__ scale, const int* __restrict__ active) {
-  const int j = blockIdx.x;
-  if (j >= cols) return;
-  if (active) {
-    const int kk = 4 * *active;
-    if (kk == 0) return;
-    if (kk < K) K = kk;
-  }
-  __shared__ int red[32];
-  int me = 0;
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
-    const cplx v = op_elem(X, ld, k, j, op);
-    me = max(me, max(expo_field(v.x), expo_field(v.y)));
-  }
-  me = block_max_int(me, red);
-  const int E = me > 0 ? me - 1022 : 0;
-  if (threadIdx.x == 0) scale[j] = ldexp(1.0, E);
-  const size_t Kp = 2 * (size_t)Kpad;
-  for (int k = threadIdx.x; k < Kpad; k += blockDim.x) {
-    const cplx v = k < K ? op_elem(X, ld, k, j, op) : cmake(0.0, 0.0);
-    long long xr = fixed62(v.x, E), xi = fixed62(v.y, E);
-    for (int p = 0; p < S; ++p) {
-      const int sft = 62 - (p + 1) * bits;
-      const int ar = next_digit(xr, sft), ai = next_digit(xi, sft);
-      const size_t base = (size_t)p * cols * Kp + (size_t)j * Kp;
-      out_re[base + k] = __float2bfloat16_rn((float)ar);
-      out_re[base + Kpad + k] = __float2bfloat16_rn((float)-ai);
-      out_im[base + k] = __float2bfloat16_rn((float)ai);
-      out_im[base + Kpad + k] = __float2bfloat16_rn((float)ar);
-    }
-  }
-}
-
-// Both sides in one launch when each operand vector is contiguous across
-// vectors (op(A) = A 'N': element k of row i at A[k lda + i]; op(B) = B^T
-// 'T': element k of column j at B[k ldb + j]) and Kpad <= 64, the shape of
-// the delayed-update flush: 8 vectors x Kpad elements are loaded with
-// coalesced reads into shared memory, then one warp per vector finds its
-// scale and cuts its digits (the same digits as k_oz_split_rows/cols).
-// blockIdx.y = 0: rows of A; 1: columns of B.
-constexpr int OZ_TILED_KMAX = 64;
-constexpr int OZ_TILED_V = 8;      // vectors per block: one warp each
-__global__ void __launch_bounds__(256) k_oz_split_tiled(const cplx* __restrict__ A, int lda, int m,
-                                                        const cplx* __restrict__ B, int ldb, int nn, int K, int Kpad,
-                                                        int S, int bits, __nv_bfloat16* __restrict__ As,
-                                                        __nv_bfloat16* __restrict__ Bre, __nv_bfloat16* __restrict__ Bim,
-                                                        double* __restrict__ sA, double* __restrict__ sB,
-                                                        const int* __restrict__ active) {
-  __shared__ cplx tile[OZ_TILED_KMAX][OZ_TILED_V + 1];
+// Slices of both operands in one launch: blockIdx.y = 0 rows of op(A), 1
+// columns of op(B), SPLIT_V vectors per CTA, two warps per vector.  The
+// vectors are read from global memory once, into shared memory, along the
+// direction in which X is contiguous (op(A) = A and op(B) = B^T, B^C: across
+// the vectors; otherwise along a vector); the scales and the digits are then
+// cut from shared memory, two entries per lane so that every store of a warp
+// is 128 contiguous bytes.  At 1024 x 1024 the two one-vector-per-CTA kernels
+// this replaces read X twice, with one 16-byte word per 16 KB stride on the
+// strided side.
+constexpr int SPLIT_V = 4;
+__global__ void __launch_bounds__(64 * SPLIT_V) k_oz_split(const cplx* __restrict__ A, int lda, char opA,
+                                                           const cplx* __restrict__ B, int ldb, char opB, int K,
+                                                           OzSlices o, const int* __restrict__ active) {
+  extern __shared__ double4_16a smem_split[];
+  cplx* tile = reinterpret_cast<cplx*>(smem_split);   // (SPLIT_V, K + 1)
+  __shared__ int s_me[2 * SPLIT_V];
   const int side = blockIdx.y;
   const cplx* X = side ? B : A;
-  const int ld = side ? ldb : lda, cnt = side ? nn : m;
-  const int v0 = blockIdx.x * OZ_TILED_V;
+  const int ld = side ? ldb : lda, cnt = side ? o.n : o.m;
+  const char op = side ? opB : opA;
+  const int v0 = blockIdx.x * SPLIT_V;
   if (v0 >= cnt) return;
   if (active) {   // only the first 4p inner indices are live (delayed-update flush)
     const int kk = 4 * *active;
     if (kk == 0) return;
     if (kk < K) K = kk;
   }
-  for (int idx = threadIdx.x; idx < Kpad * OZ_TILED_V; idx += blockDim.x) {
-    const int k = idx / OZ_TILED_V, v = idx % OZ_TILED_V;
-    tile[k][v] = (k < K && v0 + v < cnt) ? X[(size_t)k * ld + v0 + v] : cmake(0.0, 0.0);
+  const int ldt = K + 1;
+  const bool across = side ? op != 'N' : op == 'N';   // X contiguous across the vectors
+  const bool conj = op == 'C';
+  if (across) {
+    for (int e = threadIdx.x; e < K * SPLIT_V; e += blockDim.x) {
+      const int k = e / SPLIT_V, v = e % SPLIT_V;
+      cplx x = v0 + v < cnt ? X[(size_t)k * ld + v0 + v] : cmake(0.0, 0.0);
+      tile[v * ldt + k] = conj ? cconj(x) : x;
+    }
+  } else {
+    for (int v = 0; v < SPLIT_V && v0 + v < cnt; ++v)
+      for (int k = threadIdx.x; k < K; k += blockDim.x) {
+        const cplx x = X[(size_t)(v0 + v) * ld + k];
+        tile[v * ldt + k] = conj ? cconj(x) : x;
+      }
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const OzSlices o{As, Bre, Bim, sA, sB, m, nn, Kpad, S, bits};
-  for (int v = wid; v < OZ_TILED_V; v += blockDim.x >> 5) {
-    const int vec = v0 + v;
-    if (vec >= cnt) break;
-    oz_slice_vec(o, side, vec, K, [&](int k) { return tile[k][v]; }, lane);
-  }
+  const int v = wid >> 1, half = wid & 1;
+  const bool live = v0 + v < cnt;
+  const cplx* x = tile + v * ldt;
+  int me = 0;
+  if (live)
+    for (int k = 32 * half + lane; k < K; k += 64) me = max(me, max(expo_field(x[k].x), expo_field(x[k].y)));
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) me = max(me, __shfl_xor_sync(0xffffffffu, me, s));
+  if (lane == 0) s_me[wid] = me;
+  __syncthreads();
+  if (!live) return;
+  me = max(s_me[2 * v], s_me[2 * v + 1]);
+  if (half == 0 && lane == 0) (side ? o.sB : o.sA)[v0 + v] = oz_scale_value(me);
+  const int E = oz_scale_expo(me);
+  for (int k = 64 * half + 2 * lane; k < o.Kpad; k += 128)
+    oz_store_pair(o, side, v0 + v, k, k < K ? x[k] : cmake(0.0, 0.0), k + 1 < K ? x[k + 1] : cmake(0.0, 0.0), E);
 }
 
 struct OzArgs {
-  const __nv_bfloat16* As;   // S x (m x Kp), row-major
-  const __nv_bfloat16* Bre;  // S x (n x Kp), K contiguous per column
-  const __nv_bfloat16* Bim;
-  const double* sA;          // (m) row scales
+  const double* sA;          // (m) row scales 2^(E-1)
   const double* sB;          // (n) column scales
   int m, n, Kp, S, bits;
   cplx alpha, beta;
@@ -185,43 +120,23 @@ struct OzArgs {
   const double* rs;          // optional extra row scaling
   const double* cs;          // optional extra column scaling
   const int* active;         // optional: nothing to do when *active == 0
-  int int_combine;           // group sums combined exactly in 64-bit integers
-  int kchunk;                // split K: K steps per CTA layer (blockIdx.z); 0 = all
-  unsigned long long* acc;   // split K: exact integer sums (m x n x {re, im}), finished by k_oz_finalize
-                             // (zero on entry; the finaliser zeroes what it read)
+  int kexact;                // K blocks per exact accumulation (chunk)
+  int kchunk;                // split K: K blocks per CTA layer (blockIdx.z); 0 = all
+  unsigned long long* acc;   // split K: exact integer sums (m x n x {re, im}, wide: {re hi, re lo, im hi, im lo}),
+                             // finished by k_oz_finalize (zero on entry; the finaliser zeroes what it read)
 };
 
 // alpha v + beta c_old for one output value (the scaled product v):
 // alpha = +-1, beta in {0, 1} take one multiply and at most one add.
-__device__ __forceinline__ cplx oz_combine(const OzArgs& a, cplx v, cplx c_old, bool plain) {
+__device__ __forceinline__ cplx oz_combine(const OzArgs& a, cplx beta, cplx v, cplx c_old, bool plain) {
   if (plain) {
     if (a.alpha.x < 0.0) v = cmake(-v.x, -v.y);
-    if (a.beta.x != 0.0) v = cadd(c_old, v);
+    if (beta.x != 0.0) v = cadd(c_old, v);
     return v;
   }
   v = cmul(a.alpha, v);
-  if (a.beta.x != 0.0 || a.beta.y != 0.0) v = cfma(a.beta, c_old, v);
+  if (beta.x != 0.0 || beta.y != 0.0) v = cfma(beta, c_old, v);
   return v;
-}
-
-// Final scaling and accumulation of one output value (shared by the GEMM and
-// the split-K finaliser).
-__device__ __forceinline__ void oz_store(const OzArgs& a, int row, int col, double vr, double vi, double wint,
-                                         bool plain) {
-  double f = a.sA[row] * a.sB[col] * wint;
-  if (a.rs) f *= a.rs[row];
-  if (a.cs) f *= a.cs[col];
-  cplx v = cmake(vr * f, vi * f);
-  cplx* cp = &a.C[(size_t)col * a.ldc + row];
-  if (plain) {
-    // alpha = +-1, beta in {0, 1}: one multiply and at most one add per value
-    if (a.alpha.x < 0.0) v = cmake(-v.x, -v.y);
-    if (a.beta.x != 0.0) v = cadd(*cp, v);
-  } else {
-    v = cmul(a.alpha, v);
-    if (a.beta.x != 0.0 || a.beta.y != 0.0) v = cfma(a.beta, *cp, v);
-  }
-  *cp = v;
 }
 
 __device__ __forceinline__ bool oz_plain(const OzArgs& a) {
@@ -229,16 +144,97 @@ __device__ __forceinline__ bool oz_plain(const OzArgs& a) {
          (a.beta.x == 0.0 || a.beta.x == 1.0);
 }
 
+// The exact value of a wide sum is hi 2^WIDE_SHIFT(bits) + lo.
+__host__ __device__ constexpr int oz_wide_groups() { return 4; }   // groups of the low word
+__device__ __forceinline__ int oz_wide_shift(int bits) { return oz_wide_groups() * bits; }
+
+// (double)v 2^e, rounded to nearest even exactly as __ll2double_rn(v) * 2^e,
+// on the integer units and without branches, for -1022 <= e <= 960 (every
+// |v| < 2^63 then gives a normal double): |v| is shifted so that its leading
+// one sits at bit 63, the 53 high bits are rounded to nearest even at bit 11,
+// and a carry out of the significand steps the biased exponent by addition.
+__device__ __forceinline__ double ll_ldexp(long long v, int e) {
+  const unsigned long long sgn = (unsigned long long)v & 0x8000000000000000ull;
+  const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  const int lz = __clzll((long long)m) & 63;   // 64 for m = 0, masked; the select below covers it
+  const unsigned long long mn = m << lz;
+  unsigned long long q = mn >> 11;
+  const unsigned rem = (unsigned)mn & 0x7FFu;
+  q += (rem + (unsigned)(q & 1ull)) > 0x400u ? 1ull : 0ull;
+  const long long be = 63 - lz + e + 1023;
+  const unsigned long long bits = sgn | ((unsigned long long)(be - 1) << 52) + q;
+  return m ? __longlong_as_double((long long)bits) : 0.0;
+}
+
+// The same for the exact sum hi 2^sh + lo (|sum| < 2^100, sh < 64), rounded
+// once: the 128-bit magnitude is normalised to bit 127 and the words below
+// the rounding position enter as a sticky bit.  Normal results for
+// -1022 <= e <= 900.
+__device__ __forceinline__ double wide_ldexp(long long hi, long long lo, int sh, int e) {
+  const unsigned long long h0 = (unsigned long long)hi;
+  unsigned long long l = h0 << sh;
+  unsigned long long h = (unsigned long long)(hi >> (64 - sh));
+  l += (unsigned long long)lo;
+  h += (unsigned long long)(lo >> 63) + (l < (unsigned long long)lo ? 1ull : 0ull);
+  const bool neg = (long long)h < 0;
+  if (neg) {
+    l = 0ull - l;
+    h = ~h + (l == 0ull ? 1ull : 0ull);
+  }
+  int ex = e + 64;
+  if (h == 0ull) { h = l; l = 0ull; ex = e; }
+  const int lz = __clzll((long long)h) & 63;
+  const unsigned long long m = lz ? (h << lz) | (l >> (64 - lz)) : h;
+  const bool sticky = (l << lz) != 0ull;
+  unsigned long long q = m >> 11;
+  const unsigned rem = (unsigned)m & 0x7FFu;
+  q += (rem + ((unsigned)(q & 1ull) | (sticky ? 1u : 0u))) > 0x400u ? 1ull : 0ull;
+  const long long be = 63 - lz + ex + 1023;
+  const unsigned long long bits = (neg ? 0x8000000000000000ull : 0ull) | ((unsigned long long)(be - 1) << 52) + q;
+  return h ? __longlong_as_double((long long)bits) : 0.0;
+}
+
+// An exact sum times 2^e.  window: e lies where every sum gives a normal
+// double (integer route); otherwise the FP64 route with its range handling.
+template <bool WIDE>
+__device__ __forceinline__ double oz_value(long long hi, long long lo, int sh, int e, bool window) {
+  if constexpr (WIDE) {
+    if (window) return wide_ldexp(hi, lo, sh, e);
+    return ldexp(wide_ldexp(hi, lo, sh, 0), e);
+  } else {
+    if (window) return ll_ldexp(hi, e);
+    return ldexp(__ll2double_rn(hi), e);
+  }
+}
+__device__ __forceinline__ bool oz_window(int e) { return e >= -1022 && e <= 900; }
+constexpr int OZ_EXPO_NAN = 1 << 20;   // exponent of a NaN scale: no window, NaN results
+__device__ __forceinline__ int oz_expo(double scale) {   // E of the stored scale 2^(E-1)
+  const int f = expo_field(scale);
+  return f == 0x7FF ? OZ_EXPO_NAN : f - 1022;
+}
+
+template <bool WIDE>
 __global__ void k_oz_finalize(OzArgs a) {
-  const double wint = ldexp(1.0, -a.bits * (a.S + 1));
+  const int e0 = -a.bits * (a.S + 1), sh = oz_wide_shift(a.bits);
   const bool plain = oz_plain(a);
   const size_t total = (size_t)a.m * a.n;
+  constexpr int W = WIDE ? 2 : 1;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
     const int col = (int)(e / a.m), row = (int)(e - (size_t)col * a.m);
-    const long long vr = (long long)a.acc[2 * e], vi = (long long)a.acc[2 * e + 1];
-    a.acc[2 * e] = 0ull;
-    a.acc[2 * e + 1] = 0ull;
-    oz_store(a, row, col, __ll2double_rn(vr), __ll2double_rn(vi), wint, plain);
+    long long v[2 * W];
+#pragma unroll
+    for (int q = 0; q < 2 * W; ++q) {
+      v[q] = (long long)a.acc[2 * W * e + q];
+      a.acc[2 * W * e + q] = 0ull;
+    }
+    const int ex = oz_expo(a.sA[row]) + oz_expo(a.sB[col]);
+    cplx r = cmake(oz_value<WIDE>(v[0], v[W - 1], sh, e0 + ex, oz_window(e0 + ex)),
+                   oz_value<WIDE>(v[W], v[2 * W - 1], sh, e0 + ex, oz_window(e0 + ex)));
+    if (ex > OZ_EXPO_NAN / 2) r = cmake(nan(""), nan(""));
+    if (a.rs || a.cs) r = cscale(r, (a.rs ? a.rs[row] : 1.0) * (a.cs ? a.cs[col] : 1.0));
+    cplx* cp = &a.C[(size_t)col * a.ldc + row];
+    const bool rd = a.beta.x != 0.0 || a.beta.y != 0.0;
+    *cp = oz_combine(a, a.beta, r, rd ? *cp : cmake(0.0, 0.0), plain);
   }
 }
 
@@ -259,13 +255,13 @@ __global__ void k_oz_finalize(OzArgs a) {
 //     cp.async.bulk.tensor (128-byte swizzle) onto mbarriers;
 //   * warp 1 allocates TMEM, and one lane issues tcgen05.mma for every pair
 //     (p, q) with p + q <= S + 1 into group p + q, releasing each A slot and
-//     B buffer with tcgen05.commit and marking a tile's accumulators final
-//     with a commit; before the first MMA of the next tile it waits until
-//     the epilogue has read the accumulators out of TMEM;
-//   * warps 2-9 (two per TMEM lane quarter, one half of the columns each)
-//     read the S exact FP32 group sums of a tile with tcgen05.ld, release
-//     TMEM, combine the sums exactly in 64-bit integers (Horner in 2^bits),
-//     then scale and store as before.
+//     B buffer with tcgen05.commit and marking a chunk's accumulators final
+//     with a commit; before the first MMA of the next chunk (of this tile or
+//     the next) it waits until the epilogue has read them out of TMEM;
+//   * warps 2-17 (four per TMEM lane quarter, 8 columns each) read the S
+//     exact FP32 group sums of a chunk with tcgen05.ld, release TMEM, combine
+//     the sums exactly in 64-bit integers (Horner in 2^bits; two words above
+//     61 bits), then round, scale and store.
 // Every wait is bounded; on a timeout the kernel sets an error bit, drains
 // what it issued (bounded) and frees its TMEM.
 constexpr int TC_BM = 128;                      // rows of C per CTA (TMEM lanes)
@@ -273,7 +269,7 @@ constexpr int TC_BN = 32;                       // complex columns of C per CTA 
 constexpr int TC_BK = 64;                       // BF16 per K block: one 128-byte swizzle row
 constexpr int TC_MAXS = 8;                      // S groups x 64 TMEM columns <= 512
 constexpr int TC_ARING = 6;                     // A-slice stages (S <= 6: one K block of A in flight)
-constexpr int TC_EPI_WARPS = 8;                 // epilogue warps 2-9: two per TMEM lane quarter
+constexpr int TC_EPI_WARPS = 16;                // epilogue warps 2-17: four per TMEM lane quarter, 8 columns each
 constexpr int TC_THREADS = 32 * (2 + TC_EPI_WARPS);   // warp 0 TMA, warp 1 MMA (and TMEM allocation)
 constexpr int TC_A_TILE = TC_BM * TC_BK * 2;    // 16 KB
 constexpr int TC_B_HALF = TC_BN * TC_BK * 2;    // 4 KB: 32 rows of B'_re or of B'_im
@@ -366,42 +362,21 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-// 32 TMEM lanes (this warp's quarter) x 16 consecutive 32-bit columns; the
+// 32 TMEM lanes (this warp's quarter) x 8 consecutive 32-bit columns; the
 // registers are valid after tc_wait_ld
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
       : "r"(taddr));
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// (double)v 2^e, rounded to nearest even exactly as __ll2double_rn(v) * 2^e,
-// on the integer units and without branches, for -1022 <= e <= 960 (every
-// |v| < 2^63 then gives a normal double): |v| is shifted so that its leading
-// one sits at bit 63, the 53 high bits are rounded to nearest even at bit 11,
-// and a carry out of the significand steps the biased exponent by addition.
-__device__ __forceinline__ double ll_ldexp(long long v, int e) {
-  const unsigned long long sgn = (unsigned long long)v & 0x8000000000000000ull;
-  const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
-  const int lz = __clzll((long long)m) & 63;   // 64 for m = 0, masked; the select below covers it
-  const unsigned long long mn = m << lz;
-  unsigned long long q = mn >> 11;
-  const unsigned rem = (unsigned)mn & 0x7FFu;
-  q += (rem + (unsigned)(q & 1ull)) > 0x400u ? 1ull : 0ull;
-  const long long be = 63 - lz + e + 1023;
-  const unsigned long long bits = sgn | ((unsigned long long)(be - 1) << 52) + q;
-  return m ? __longlong_as_double((long long)bits) : 0.0;
-}
-// the exponent window in which ll_ldexp is exact for every 64-bit value
-__device__ __forceinline__ bool ll_ldexp_safe(int e) { return e >= -1022 && e <= 960; }
 
 struct TcMaps {
   CUtensorMap a, bre, bim;   // (Kp, rows, S) BF16 slices, box (64, 128 | 32, 1), 128-byte swizzle
 };
 
-template <bool INT>
+template <bool WIDE, int BITS>   // BITS: slice width, 0 = a.bits
 __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_constant__ TcMaps maps, OzArgs a,
                                                              int* err) {
   if (a.active && *a.active == 0) return;   // flush with nothing pending (uniform over the grid)
@@ -414,7 +389,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
   const uint32_t sA = base + 2u * S * TC_B_TILE;                // [TC_ARING] A tiles of 16 KB
   const uint32_t sBar = sA + TC_ARING * TC_A_TILE;              // barriers
   uint64_t* bars = reinterpret_cast<uint64_t*>(basep + (sBar - base));
-  // barrier slots: full_b 0-1, empty_b 2-3, full_a FA.., empty_a EA.., a tile's
+  // barrier slots: full_b 0-1, empty_b 2-3, full_a FA.., empty_a EA.., a chunk's
   // accumulators final ACC, TMEM drained by the epilogue TE, MMA thread done DONE
   constexpr int FA = 4, EA = FA + TC_ARING, ACC = EA + TC_ARING, TE = ACC + 1, DONE = TE + 1, NBAR = DONE + 1;
   auto bar = [&](int k) { return sBar + 8u * k; };
@@ -505,11 +480,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
     // ---- MMA issuer ----
     if (lane == 0) {
       int a_use = 0;
+      int vt = 0;   // chunks finished so far (over all tiles)
       for (int u = 0; u < U && !*s_abort; ++u) {
-        const int tt = u / nkb, kbi = u % nkb, bb = u & 1;
-        if (kbi == 0 && tt > 0) {
-          // the epilogue has read tile tt - 1's accumulators out of TMEM
-          if (!mbar_wait(bar(TE), (tt - 1) & 1, err, s_abort)) break;
+        const int kbi = u % nkb, bb = u & 1;
+        const bool chunk0 = kbi % a.kexact == 0;   // first K block of an exact accumulation
+        if (chunk0 && u > 0) {
+          // the epilogue has read the previous chunk's accumulators out of TMEM
+          if (!mbar_wait(bar(TE), (vt - 1) & 1, err, s_abort)) break;
           tc_fence_after();
         }
         if (!mbar_wait(bar(bb), (u >> 1) & 1, err, s_abort)) break;
@@ -526,164 +503,138 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
             const uint32_t d = tmem + (uint32_t)(p + q) * (2 * TC_BN);
 #pragma unroll
             for (int kk = 0; kk < TC_BK / 16; ++kk)
-              tc_mma(d, ad + 2u * kk, bd + 2u * kk, (kbi == 0 && p == 0 && kk == 0) ? 0u : 1u);
+              tc_mma(d, ad + 2u * kk, bd + 2u * kk, (chunk0 && p == 0 && kk == 0) ? 0u : 1u);
           }
           tc_commit(bar(EA + slot));  // A slot free once these MMAs have read it
         }
         tc_commit(bar(2 + bb));       // B buffer free
         if (!ok) break;
-        if (kbi == nkb - 1) tc_commit(bar(ACC));   // tile tt's accumulators final
+        if ((kbi + 1) % a.kexact == 0 || kbi == nkb - 1) {
+          tc_commit(bar(ACC));        // this chunk's accumulators final
+          ++vt;
+        }
       }
       tc_commit(bar(DONE));           // every MMA issued has completed (the abort path waits on it)
     }
   } else if (U > 0) {
-    // ---- epilogue: warps 2-9, two per TMEM lane quarter (warp % 4); warp w
-    //      takes the 16 columns of half (w - 2) / 4 of each tile ----
+    // ---- epilogue: warps 2-17, four per TMEM lane quarter (warp % 4); warp w
+    //      takes the 8 columns of group (w - 2) / 4 of each tile, chunk by chunk
+    //      (chunks after the first are added to the C the same thread stored) ----
     const int quarter = warp & 3;
-    const int h = (warp - 2) >> 2;
-    const bool fast = INT && oz_plain(a) && !a.rs && !a.cs && !a.acc;
-    const bool add = a.beta.x != 0.0;
-    const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16);
-    const double wint = INT ? ldexp(1.0, -a.bits * (S + 1)) : 1.0;
-    const bool plain = oz_plain(a);
-    for (int tt = 0; tt < my_tiles; ++tt) {
+    const int cg = (warp - 2) >> 2;
+    const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(8 * cg);
+    const int bits = BITS ? BITS : a.bits;
+    const int sh = oz_wide_shift(bits), e0 = -bits * (S + 1);
+    const int ghi = WIDE ? S - oz_wide_groups() : S;   // groups of the (high) word
+    const bool plain = oz_plain(a), neg = a.alpha.x < 0.0;
+    const bool simple = plain && !a.rs && !a.cs;   // alpha = +-1, beta in {0, 1}, no extra scalings
+    const int nch = (nkb + a.kexact - 1) / a.kexact;
+    for (int vt = 0; vt < my_tiles * nch; ++vt) {
       int i0, j0;
-      tile_of(tt, i0, j0);
+      tile_of(vt / nch, i0, j0);
+      j0 += 8 * cg;
+      const bool first = vt % nch == 0;
       const int row = i0 + 32 * quarter + lane;
-      const bool waited = mbar_wait(bar(ACC), tt & 1, err, s_abort);
+      const bool waited = mbar_wait(bar(ACC), vt & 1, err, s_abort);
       // tcgen05.ld is warp-collective: the decision must be uniform over the warp
       const bool have = __all_sync(0xffffffffu, waited && !*s_abort);
       if (!have) break;
+      __syncwarp();
       tc_fence_after();
-      {
-        typedef typename std::conditional<INT, long long, double>::type acc_t;
-        acc_t ar[16], ai[16];
+      long long ar[8], ai[8], lr[WIDE ? 8 : 1], li[WIDE ? 8 : 1];
 #pragma unroll
-        for (int c = 0; c < 16; ++c) { ar[c] = 0; ai[c] = 0; }
+      for (int c = 0; c < 8; ++c) { ar[c] = 0; ai[c] = 0; }
+#pragma unroll
+      for (int c = 0; c < (WIDE ? 8 : 1); ++c) { lr[c] = 0; li[c] = 0; }
 #pragma unroll 1
-        for (int g = 0; g < S; ++g) {
-          uint32_t ur[16], ui[16];
-          tc_ld16(tq + (uint32_t)(g * 2 * TC_BN + 16 * h), ur);
-          tc_ld16(tq + (uint32_t)(g * 2 * TC_BN + TC_BN + 16 * h), ui);
+      for (int g = 0; g < ghi; ++g) {
+        uint32_t ur[8], ui[8];
+        tc_ld8(tq + (uint32_t)(g * 2 * TC_BN), ur);
+        tc_ld8(tq + (uint32_t)(g * 2 * TC_BN + TC_BN), ui);
+        tc_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          ar[c] = (ar[c] << bits) + (long long)__float2int_rn(__uint_as_float(ur[c]));
+          ai[c] = (ai[c] << bits) + (long long)__float2int_rn(__uint_as_float(ui[c]));
+        }
+      }
+      if constexpr (WIDE) {
+#pragma unroll 1
+        for (int g = ghi; g < S; ++g) {
+          uint32_t ur[8], ui[8];
+          tc_ld8(tq + (uint32_t)(g * 2 * TC_BN), ur);
+          tc_ld8(tq + (uint32_t)(g * 2 * TC_BN + TC_BN), ui);
           tc_wait_ld();
-          float vr[16], vi[16];
 #pragma unroll
-          for (int c = 0; c < 16; ++c) { vr[c] = __uint_as_float(ur[c]); vi[c] = __uint_as_float(ui[c]); }
-          if constexpr (INT) {
-            const long long step = 1ll << a.bits;
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              ar[c] = ar[c] * step + (long long)__float2int_rn(vr[c]);
-              ai[c] = ai[c] * step + (long long)__float2int_rn(vi[c]);
-            }
-          } else {
-            const double wgt = ldexp(1.0, -a.bits * (g + 2));
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              ar[c] = fma(wgt, (double)vr[c], ar[c]);
-              ai[c] = fma(wgt, (double)vi[c], ai[c]);
-            }
+          for (int c = 0; c < 8; ++c) {
+            lr[c] = (lr[c] << bits) + (long long)__float2int_rn(__uint_as_float(ur[c]));
+            li[c] = (li[c] << bits) + (long long)__float2int_rn(__uint_as_float(ui[c]));
           }
         }
-        // this tile's accumulators are all in registers: TMEM may take the next tile
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(TE));
-        if (row < a.m) {
-          if (INT && a.acc) {
+      }
+      // this chunk's accumulators are all in registers: TMEM may take the next chunk
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(TE));
+      if (row >= a.m) continue;
+      if (a.acc) {
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
-              const int col = j0 + 16 * h + c;
-              if (col < a.n) {
-                unsigned long long* qa = a.acc + 2 * ((size_t)col * a.m + row);
-                atomicAdd(qa, (unsigned long long)ar[c]);
-                atomicAdd(qa + 1, (unsigned long long)ai[c]);
-              }
-            }
-          } else if (fast) {
-            // the scale sA sB 2^-bits(S+1) is a power of two: the value is the
-            // exact integer converted with that exponent on the integer units
-            // (GB300 issues FP64 at a small fraction of its integer rate); the
-            // only FP64 operation left is the addition of the old C (beta = 1)
-            const int e_row = expo_field(a.sA[row]) - 1023 - a.bits * (S + 1);
-            const bool neg = a.alpha.x < 0.0;
-            // two passes of 8 columns: the old C values of a pass are loaded
-            // together while the next tile's MMAs run (the arrays are indexed
-            // only by unrolled constants, so they stay in registers)
-#pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              cplx pre[8];
-              int e_col[8];
-#pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                const int col = j0 + 16 * h + 8 * hh + c;
-                pre[c] = (add && col < a.n) ? a.C[(size_t)col * a.ldc + row] : cmake(0.0, 0.0);
-                e_col[c] = col < a.n ? expo_field(a.sB[col]) - 1023 : 0;
-              }
-              bool safe = true;
-#pragma unroll
-              for (int c = 0; c < 8; ++c) safe = safe && ll_ldexp_safe(e_row + e_col[c]);
-              if (safe) {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                  const int col = j0 + 16 * h + 8 * hh + c;
-                  if (col < a.n) {
-                    const long long vr = neg ? -(long long)ar[8 * hh + c] : (long long)ar[8 * hh + c];
-                    const long long vi = neg ? -(long long)ai[8 * hh + c] : (long long)ai[8 * hh + c];
-                    cplx v = cmake(ll_ldexp(vr, e_row + e_col[c]), ll_ldexp(vi, e_row + e_col[c]));
-                    if (add) v = cadd(pre[c], v);
-                    a.C[(size_t)col * a.ldc + row] = v;
-                  }
-                }
-              } else {
-                // results that may leave the normal range: the FP64 route
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                  const int col = j0 + 16 * h + 8 * hh + c;
-                  if (col < a.n) {
-                    const long long vr = neg ? -(long long)ar[8 * hh + c] : (long long)ar[8 * hh + c];
-                    const long long vi = neg ? -(long long)ai[8 * hh + c] : (long long)ai[8 * hh + c];
-                    cplx v = cmake(ldexp(__ll2double_rn(vr), e_row + e_col[c]),
-                                   ldexp(__ll2double_rn(vi), e_row + e_col[c]));
-                    if (add) v = cadd(pre[c], v);
-                    a.C[(size_t)col * a.ldc + row] = v;
-                  }
-                }
-              }
-            }
+        for (int c = 0; c < 8; ++c) {
+          if (j0 + c >= a.n) continue;
+          unsigned long long* qa = a.acc + (WIDE ? 4 : 2) * ((size_t)(j0 + c) * a.m + row);
+          atomicAdd(qa, (unsigned long long)ar[c]);
+          if constexpr (WIDE) {
+            atomicAdd(qa + 1, (unsigned long long)lr[c]);
+            atomicAdd(qa + 2, (unsigned long long)ai[c]);
+            atomicAdd(qa + 3, (unsigned long long)li[c]);
           } else {
-            // per pass of 8 columns every load (scales, old C) is issued before
-            // the first store, so they are in flight together
-            double fr = a.sA[row] * wint;
-            if (a.rs) fr *= a.rs[row];
-            const bool rd = a.beta.x != 0.0 || a.beta.y != 0.0;
+            atomicAdd(qa + 1, (unsigned long long)ai[c]);
+          }
+        }
+        continue;
+      }
+      const cplx beta = first ? a.beta : cmake(1.0, 0.0);
+      const bool rd = beta.x != 0.0 || beta.y != 0.0;
+      // the scale sA sB 2^-bits(S+1) is a power of two: the value is the exact
+      // integer rounded once with that exponent on the integer units (GB300
+      // issues FP64 at a small fraction of its integer rate); the FP64
+      // operations left are the extra scalings and the addition of the old C.
+      // Two passes of 4 columns, the loads (scales, old C) of a pass issued
+      // before its first store.
+      const int e_row = oz_expo(a.sA[row]) + e0;
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              double fc[8];
-              cplx cold[8];
+      for (int hh = 0; hh < 8; hh += 4) {
+        cplx cold[4];
+        int e_col[4];
+        bool window = true;
 #pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                const int col = j0 + 16 * h + 8 * hh + c;
-                fc[c] = 0.0;
-                cold[c] = cmake(0.0, 0.0);
-                if (col < a.n) {
-                  fc[c] = a.sB[col];
-                  if (a.cs) fc[c] *= a.cs[col];
-                  if (rd) cold[c] = a.C[(size_t)col * a.ldc + row];
-                }
-              }
+        for (int c = 0; c < 4; ++c) {
+          const int col = j0 + hh + c;
+          const bool in = col < a.n;
+          cold[c] = rd && in ? a.C[(size_t)col * a.ldc + row] : cmake(0.0, 0.0);
+          e_col[c] = in ? oz_expo(a.sB[col]) + e_row : 0;
+          window = window && oz_window(e_col[c]);
+        }
+        if (window && simple) {
 #pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                const int col = j0 + 16 * h + 8 * hh + c;
-                if (col < a.n) {
-                  const double f = fr * fc[c];
-                  double vr, vi;
-                  if constexpr (INT) { vr = __ll2double_rn(ar[8 * hh + c]); vi = __ll2double_rn(ai[8 * hh + c]); }
-                  else { vr = ar[8 * hh + c]; vi = ai[8 * hh + c]; }
-                  a.C[(size_t)col * a.ldc + row] = oz_combine(a, cmake(vr * f, vi * f), cold[c], plain);
-                }
-              }
-            }
+          for (int c = 0; c < 4; ++c) {
+            if (j0 + hh + c >= a.n) continue;
+            cplx v = cmake(oz_value<WIDE>(ar[hh + c], lr[WIDE ? hh + c : 0], sh, e_col[c], true),
+                           oz_value<WIDE>(ai[hh + c], li[WIDE ? hh + c : 0], sh, e_col[c], true));
+            if (neg) v = cmake(-v.x, -v.y);
+            if (rd) v = cadd(cold[c], v);
+            a.C[(size_t)(j0 + hh + c) * a.ldc + row] = v;
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int col = j0 + hh + c;
+            if (col >= a.n) continue;
+            cplx v = cmake(oz_value<WIDE>(ar[hh + c], lr[WIDE ? hh + c : 0], sh, e_col[c], window),
+                           oz_value<WIDE>(ai[hh + c], li[WIDE ? hh + c : 0], sh, e_col[c], window));
+            if (e_col[c] > OZ_EXPO_NAN / 2) v = cmake(nan(""), nan(""));
+            if (a.rs || a.cs) v = cscale(v, (a.rs ? a.rs[row] : 1.0) * (a.cs ? a.cs[col] : 1.0));
+            a.C[(size_t)col * a.ldc + row] = oz_combine(a, beta, v, cold[c], plain);
           }
         }
       }
@@ -711,11 +662,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
 
 }  // namespace
 
-// Slice count S and width `bits` for a product with inner dimension K and a
-// target of `target_bits` mantissa bits: the smallest S whose widest exact
-// width bits = floor((24 - log2(K' S)) / 2) (at most 8, the BF16 integer range)
-// reaches the target.  Returns false when no S <= 8 does (the product keeps one
-// TMEM accumulator of 64 columns per group: 8 groups fill the 512 columns).
+// Slice count S and width `bits` of the mixed form's products with inner
+// dimension K and a target of target_bits mantissa bits: the smallest S whose
+// widest exact width in one accumulation over all of K, bits = floor((24 -
+// log2(K' S)) / 2) (at most 8, the BF16 integer range), reaches the target.
+// Returns false when no S <= 8 does (the product keeps one TMEM accumulator
+// of 64 columns per group: 8 groups fill the 512 columns).
 bool ozaki_plan(int K, int target_bits, int* S_out, int* bits_out) {
   const double kp = 2.0 * ((K + 15) / 16 * 16);
   for (int S = 2; S <= TC_MAXS; ++S) {
@@ -729,6 +681,11 @@ bool ozaki_plan(int K, int target_bits, int* S_out, int* bits_out) {
     }
   }
   return false;
+}
+
+// K blocks of 64 per exact accumulation: 64 blocks (S + 2) 2^(2 bits - 2) <= 2^24
+static int oz_chunk_blocks(int S, int bits) {
+  return (int)((1ll << (24 - 2 * bits + 2)) / (S + 2) / TC_BK);
 }
 
 OzSlices ozaki_slices(void* scratch, int m, int n, int K, int S, int bits) {
@@ -798,35 +755,31 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
                                const double* colscale, int S, int bits, void* scratch, size_t scratch_bytes,
                                unsigned long long* acc, size_t acc_bytes, cudaStream_t st, const int* active,
                                int splitk, int* kernels, int* err, bool persistent, bool presliced) {
-  if (S < 1 || S > TC_MAXS || bits < 1 || bits > 8) return cudaErrorInvalidValue;
+  if (S < 1 || S > TC_MAXS || bits < 1 || bits > 8 || !err) return cudaErrorInvalidValue;
   const int Kpad = (k + 15) / 16 * 16;
   const size_t Kp = 2 * (size_t)Kpad;
-  // exactness of the FP32 group sums: Kp * S * 2^(2 bits) <= 2^24
-  if ((double)Kp * S * ldexp(1.0, 2 * bits) > 16777216.0) return cudaErrorInvalidValue;
   if (ozaki_scratch_bytes(m, nn, k, S) > scratch_bytes) return cudaErrorInvalidValue;
   const OzSlices sl = ozaki_slices(scratch, m, nn, k, S, bits);
-  __nv_bfloat16 *As = sl.As, *Bre = sl.Bre, *Bim = sl.Bim;
-  double *sA = sl.sA, *sB = sl.sB;
-  const bool tiled = opA == 'N' && opB == 'T' && Kpad <= OZ_TILED_KMAX;
-  if (presliced) {
-    // the slices are already in scratch (cut by the delayed local-update kernel)
-  } else if (tiled) {
+  if (!presliced) {   // otherwise the slices are already in scratch (cut by the delayed local-update kernel)
+    const size_t smem = (size_t)SPLIT_V * (k + 1) * sizeof(cplx);
+    static SmemLimit limit_split;
+    if (cudaError_t e = limit_split.raise((const void*)k_oz_split, SPLIT_V * (1024 + 1) * (int)sizeof(cplx));
+        e != cudaSuccess)
+      return e;
     const int vecs = m > nn ? m : nn;
-    k_oz_split_tiled<<<dim3((vecs + OZ_TILED_V - 1) / OZ_TILED_V, 2), 32 * OZ_TILED_V, 0, st>>>(A, lda, m, B, ldb, nn, k, Kpad, S, bits, As, Bre, Bim,
-                                                               sA, sB, active);
-  } else {
-    k_oz_split_rows<<<m, 128, 0, st>>>(A, lda, opA, m, k, Kpad, S, bits, As, sA, active);
-    k_oz_split_cols<<<nn, 128, 0, st>>>(B, ldb, opB, k, nn, Kpad, S, bits, Bre, Bim, sB, active);
+    k_oz_split<<<dim3((vecs + SPLIT_V - 1) / SPLIT_V, 2), 64 * SPLIT_V, smem, st>>>(A, lda, opA, B, ldb, opB, k, sl,
+                                                                                   active);
   }
   OzArgs a;
-  a.As = As; a.Bre = Bre; a.Bim = Bim; a.sA = sA; a.sB = sB;
+  a.sA = sl.sA; a.sB = sl.sB;
   a.m = m; a.n = nn; a.Kp = (int)Kp; a.S = S; a.bits = bits;
   a.alpha = alpha; a.beta = beta; a.C = C; a.ldc = ldc; a.rs = rowscale; a.cs = colscale; a.active = active;
-  // |sum_t g_t 2^{bits (S+1-t)}| < 2^{24 + bits (S-1) + 1}: exact in int64 below 2^63
-  a.int_combine = 24 + bits * (S - 1) <= 61 ? 1 : 0;
+  // |sum_t g_t 2^{bits (S+1-t)}| < 2^{24 + bits (S-1) + 1}: one 64-bit word below 2^62, else two words
+  const bool wide = 24 + bits * (S - 1) > 61;
+  a.kexact = oz_chunk_blocks(S, bits);
   a.kchunk = 0;
   a.acc = nullptr;
-  if (S > TC_MAXS || !err) return cudaErrorInvalidValue;
+  if (a.kexact < 1) return cudaErrorInvalidValue;
   // persistent CTAs: one per SM (each holds the whole TMEM), every CTA takes
   // tiles x, x + grid, ... and overlaps a tile's epilogue with the next tile's
   // MMAs; otherwise one CTA per tile (chains sharing the GPU: short CTAs let
@@ -835,8 +788,8 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
   const int sms = sm_count_of_current_device();
   dim3 grid(persistent && ntiles > sms ? sms : ntiles);
   const int ksteps = (int)((Kp + TC_BK - 1) / TC_BK);
-  if (splitk > 1 && a.int_combine && !active && ksteps > 1 && acc &&
-      (size_t)m * nn * 2 * sizeof(unsigned long long) <= acc_bytes) {
+  if (splitk > 1 && !active && ksteps > 1 && acc &&
+      (size_t)m * nn * (wide ? 4 : 2) * sizeof(unsigned long long) <= acc_bytes) {
     // split K over blockIdx.z: exact 64-bit integer partial sums in acc, which
     // is zero between products (zeroed at allocation, re-zeroed by the finaliser)
     if (splitk > ksteps) splitk = ksteps;
@@ -844,30 +797,28 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
     grid.z = (ksteps + a.kchunk - 1) / a.kchunk;
     a.acc = acc;
   }
-  if (kernels) *kernels = (a.acc ? 4 : 3) - (presliced ? 2 : tiled ? 1 : 0);
+  if (kernels) *kernels = (a.acc ? 3 : 2) - (presliced ? 1 : 0);
   {
     TcMaps maps;
-    if (!encode_slices(&maps.a, As, Kp, m, S, TC_BM) || !encode_slices(&maps.bre, Bre, Kp, nn, S, TC_BN) ||
-        !encode_slices(&maps.bim, Bim, Kp, nn, S, TC_BN))
+    if (!encode_slices(&maps.a, sl.As, Kp, m, S, TC_BM) || !encode_slices(&maps.bre, sl.Bre, Kp, nn, S, TC_BN) ||
+        !encode_slices(&maps.bim, sl.Bim, Kp, nn, S, TC_BN))
       return cudaErrorInvalidValue;
-    static SmemLimit limit_int, limit_fp;
-    const size_t smem = tc_smem_bytes(S);
-    if (a.int_combine) {
-      if (cudaError_t e = limit_int.raise((const void*)k_oz_gemm_tc<true>, (int)tc_smem_bytes(TC_MAXS));
-          e != cudaSuccess)
-        return e;
-      k_oz_gemm_tc<true><<<grid, TC_THREADS, smem, st>>>(maps, a, err);
-    } else {
-      if (cudaError_t e = limit_fp.raise((const void*)k_oz_gemm_tc<false>, (int)tc_smem_bytes(TC_MAXS));
-          e != cudaSuccess)
-        return e;
-      k_oz_gemm_tc<false><<<grid, TC_THREADS, smem, st>>>(maps, a, err);
-    }
+    // the widths of the default targets are compiled in: 5, 6, 7 (40 bits, by K), 7 in two words (56 bits)
+    static SmemLimit limits[6];
+    const int which = wide ? (bits == 7 ? 4 : 5) : bits == 5 ? 0 : bits == 6 ? 1 : bits == 7 ? 2 : 3;
+    void (*const kernels_tc[6])(TcMaps, OzArgs, int*) = {k_oz_gemm_tc<false, 5>, k_oz_gemm_tc<false, 6>,
+                                                         k_oz_gemm_tc<false, 7>, k_oz_gemm_tc<false, 0>,
+                                                         k_oz_gemm_tc<true, 7>,  k_oz_gemm_tc<true, 0>};
+    if (cudaError_t e = limits[which].raise((const void*)kernels_tc[which], (int)tc_smem_bytes(TC_MAXS));
+        e != cudaSuccess)
+      return e;
+    kernels_tc[which]<<<grid, TC_THREADS, tc_smem_bytes(S), st>>>(maps, a, err);
   }
   if (a.acc) {
     const size_t total = (size_t)m * nn;
     const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-    k_oz_finalize<<<blocks, 256, 0, st>>>(a);
+    if (wide) k_oz_finalize<true><<<blocks, 256, 0, st>>>(a);
+    else k_oz_finalize<false><<<blocks, 256, 0, st>>>(a);
   }
   return cudaGetLastError();
 }

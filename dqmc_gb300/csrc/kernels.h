@@ -132,8 +132,6 @@ cudaError_t launch_trsm_left_upper(const cplx* T, const int* order, const cplx* 
 // lower: unit lower triangular; else upper with reciprocal diagonal rdiag
 cudaError_t launch_trsm_diag_block(const cplx* T, int ldT, const cplx* rdiag, cplx* Y, int ldY, int j0, int b, int m,
                                    bool lower, cudaStream_t st);
-// Y <- L^-1 Y, L unit lower triangular (strictly lower part of Lc)
-cudaError_t launch_trsm_left_lower_unit(const cplx* Lc, cplx* Y, int n, int m, cudaStream_t st);
 // Results of the LU with partial pivoting P A = L U (zgetrf semantics).
 struct LUWork {
   int* perm;         // (n) row perm[i] of A is row i of P A
@@ -204,6 +202,7 @@ cudaError_t measure_peak_fp64(int device, double* tflops);
 
 // ---- split-precision complex GEMM (k_ozaki.cu) ----
 bool ozaki_plan(int K, int target_bits, int* S, int* bits);
+constexpr int OZ_FP64_S = 8, OZ_FP64_BITS = 7;   // slices of the FP64 form's products: 56 mantissa bits at any K
 size_t ozaki_scratch_bytes(int m, int n, int K, int S);
 // where launch_ozaki_zgemm keeps the slices of an m x n x K product in scratch
 OzSlices ozaki_slices(void* scratch, int m, int n, int K, int S, int bits);
