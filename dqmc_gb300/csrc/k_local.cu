@@ -23,6 +23,7 @@
 // Proposal streams use fixed slots: delta[:, i] and unif[i] belong to site
 // i of this call; unif[i] decides only when p_acc <= 1, exactly as
 // `p_acc > 1.0 || rand() < p_acc`.
+#include <cooperative_groups.h>
 #include "common.cuh"
 #include "kernels.h"
 #include "oz_slice.cuh"
@@ -323,15 +324,13 @@ __global__ void __launch_bounds__(LU_THREADS, 2) k_local_updates(LocalUpdateArgs
 }
 
 // ---------------------------------------------------------------------------
-// delayed rank-k updates: G_cur = G + X Y with X (n x 4k), Y (4k x n)
+// delayed updates: windows of sites decided on one thread-block cluster
 // ---------------------------------------------------------------------------
-// On GB300 every FP64 warp instruction occupies a sub-partition's FP64 unit
-// for tens of cycles, so the per-site chain is kept short and split over
-// warps: the per-site constants come from a prepare kernel run once per
-// slice, the 4x4 block G_cur[i + rN, i + cN] is read from a cache that the
-// owner CTA of site i keeps current, and the decision runs on three warps
-// at once (det and 1/det; the adjugate; the action difference).
-
+// A round takes the next W sites of the slice (a window).  The Metropolis
+// decisions of its sites need G only on the window's own 4W rows and columns,
+// so one cluster keeps that block in shared memory and decides the window
+// there (k_local_window); the whole chip then forms the rank-4p factors of the
+// p accepted sites (k_local_factors) and applies them as one product (flush).
 // Per-site constants of slice l: one warp per site.  Lanes of even parity
 // evaluate the old-field block (power -1), odd lanes the proposed one.
 __global__ void __launch_bounds__(128) k_local_prepare(LocalUpdateArgs a, SitePrep* __restrict__ prep, int* state) {
@@ -385,273 +384,297 @@ __global__ void __launch_bounds__(128) k_local_prepare(LocalUpdateArgs a, SitePr
   }
 }
 
-// det M by the Laplace expansion along rows {0, 1}: the 2x2 minors T_ab of
-// rows {0, 1} (lanes 0-5) and B_ab of rows {2, 3} (lanes 6-11), pairs (a, b)
-// in the order (0,1) (0,2) (0,3) (1,2) (1,3) (2,3), and
-// det = sum_ab (-1)^(a+b+1) T_ab B_(complement of ab); m[r][c] in lane 4r+c.
-// The sum is complete in lane 0 (lanes 0-7 take part in it).
-__device__ __forceinline__ cplx det_laplace(cplx m, int lane) {
-  const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
-  const int mi = lane < 12 ? lane : 0;
-  const int pr = mi < 6 ? 0 : 2, pp = mi < 6 ? mi : mi - 6;
-  const cplx e00 = shfl_c(m, 4 * pr + pa[pp]), e01 = shfl_c(m, 4 * pr + pb[pp]);
-  const cplx e10 = shfl_c(m, 4 * (pr + 1) + pa[pp]), e11 = shfl_c(m, 4 * (pr + 1) + pb[pp]);
-  const cplx minor = csub(cmul(e00, e11), cmul(e01, e10));
-  // lane pp < 6: T_pp times B of the complementary pair (index 5 - pp, in lane 11 - pp)
-  const cplx bc = shfl_c(minor, lane < 6 ? 11 - lane : 0);
-  cplx term = cmake(0.0, 0.0);
-  if (lane < 6) {
-    term = cmul(minor, bc);
-    if (lane == 1 || lane == 4) term = cmake(-term.x, -term.y);   // (a + b) even: (0,2), (1,3)
-  }
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) term = cadd(term, shfl_c(term, lane ^ o));
-  return term;
-}
 
-// adj(M)[r][c] = cofactor C[c][r] for lane 4r+c (lanes < 16), from the 2x2
-// minors of rows {0,1} and {2,3} (Laplace expansion of each 3x3 minor along
-// its single row from the other pair); m[r][c] in lane 4r+c.
-__device__ __forceinline__ cplx adjugate_entry(cplx m, int lane) {
-  // pair index of columns (a, b), a < b: 0:(0,1) 1:(0,2) 2:(0,3) 3:(1,2) 4:(1,3) 5:(2,3)
-  const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
-  // lanes 0-5: top minors T_ab (rows 0, 1); lanes 6-11: bottom minors B_ab (rows 2, 3)
-  const int mi = lane < 12 ? lane : 0;
-  const int pr = mi < 6 ? 0 : 2, pp = mi < 6 ? mi : mi - 6;
-  const cplx e00 = shfl_c(m, 4 * pr + pa[pp]), e01 = shfl_c(m, 4 * pr + pb[pp]);
-  const cplx e10 = shfl_c(m, 4 * (pr + 1) + pa[pp]), e11 = shfl_c(m, 4 * (pr + 1) + pb[pp]);
-  const cplx minor = csub(cmul(e00, e11), cmul(e01, e10));
-  // lane 4r+c: cofactor with row c and column r removed
-  const int r = (lane >> 2) & 3, c = lane & 3;
-  const int rr = c, cc = r;                        // removed row / column
-  const int other = rr < 2 ? 1 - rr : 5 - rr;      // remaining row of the removed row's pair
-  const int base = rr < 2 ? 6 : 0;                 // minors of the complementary pair
-  int cols[3];
-  for (int t = 0, q = 0; t < 4; ++t) if (t != cc) cols[q++] = t;
-  cplx d3 = cmake(0.0, 0.0);
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const int u = a == 0 ? cols[1] : cols[0];
-    const int v = a == 2 ? cols[1] : cols[2];
-    const int pidx = u == 0 ? (v - 1) : (u == 1 ? v + 1 : 5);   // (0,1)0 (0,2)1 (0,3)2 (1,2)3 (1,3)4 (2,3)5
-    const cplx mn = shfl_c(minor, base + pidx);
-    const cplx ent = shfl_c(m, 4 * other + cols[a]);
-    const cplx t = cmul(ent, mn);
-    d3 = (a == 1) ? csub(d3, t) : cadd(d3, t);
-  }
-  if ((rr + cc) & 1) d3 = cmake(-d3.x, -d3.y);
-  return d3;
-}
-
-// The words of site i that the delayed kernel keeps in shared memory: the
-// SitePrep (Delta_i, the proposed eV entries, the field difference and the
-// prepared action parts), then the Metropolis uniform and the proposal delta.
-constexpr int kSiteEv = 32, kSiteDiff = 36, kSiteUnif = 44, kSiteProp = 45, kSiteWords = 48;
+// Words of a site kept in shared memory: its SitePrep (Delta_i, the proposed
+// eV entries, the field difference, the prepared action parts) and the
+// Metropolis uniform.
+constexpr int kSiteEv = 32, kSiteDiff = 36, kSiteUnif = 44, kSiteWords = 46;
 static_assert(sizeof(SitePrep) == 44 * sizeof(double), "SitePrep is read as 44 words");
 static_assert(offsetof(SitePrep, ev) == kSiteEv * sizeof(double), "SitePrep.ev");
 static_assert(offsetof(SitePrep, diff) == kSiteDiff * sizeof(double), "SitePrep.diff");
 static_assert(offsetof(SitePrep, dsA) == (kSiteDiff + 3) * sizeof(double), "SitePrep.dsA");
-__device__ __forceinline__ double site_word(const LocalUpdateArgs& a, const DelayedArgs& d, int i, int k) {
-  if (k < 44) return __ldcg(reinterpret_cast<const double*>(d.prep + i) + k);
-  if (k == kSiteUnif) return __ldg(&a.unif[i]);
-  return __ldg(&a.delta[3 * i + (k - kSiteProp)]);
+
+constexpr int WIN_THREADS = 256;
+constexpr int WIN_MAXC = 16;               // CTAs per cluster
+
+// Work split of the 4x4 algebra below: lane = 2 entry + part, so a lane owns
+// the real or the imaginary part of one of 16 entries.  An FP64 warp
+// instruction costs 64 cycles whatever its active lanes, so this halves the
+// instructions of a complex product per entry.
+//
+// x with its sign flipped where `flip`, on the integer units (a negation that
+// is not an operand of an FP64 instruction costs one itself).
+__device__ __forceinline__ double flip_sign(double x, bool flip) {
+  return __hiloint2double(__double2hiint(x) ^ (flip ? 0x80000000 : 0), __double2loint(x));
+}
+// Component `part` of a b, as two terms: a.x u + a.y w.
+__device__ __forceinline__ void win_uw(cplx b, int part, double& u, double& w) {
+  u = part ? b.y : b.x;
+  w = flip_sign(part ? b.x : b.y, !part);
+}
+// Component of sum_k A[r][k] B[k][c] (4x4 blocks, rows of A lda apart, of B 4 apart).
+__device__ __forceinline__ double win_mul4(const cplx* A, int lda, const cplx* B, int r, int c, int part) {
+  double v0 = 0.0, v1 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const cplx x = A[r * lda + k];
+    double u, w;
+    win_uw(B[4 * k + c], part, u, w);
+    double& v = k < 2 ? v0 : v1;
+    v = fma(x.x, u, v);
+    v = fma(x.y, w, v);
+  }
+  return v0 + v1;
+}
+// The 12 two-row minors of M = I + Delta (I - g) = (I + Delta) - Delta g
+// (src/local_updates.jl:49-55), g a 4x4 block with rows ld apart: minors of
+// rows {0, 1} in mn[0..5], of rows {2, 3} in mn[6..11], column pairs (0,1)
+// (0,2) (0,3) (1,2) (1,3) (2,3).  One warp; m (16) and mn (12) are its scratch.
+__device__ __forceinline__ void win_minors(const cplx* delta, const cplx* g, int ld, cplx* m, cplx* mn, int lane) {
+  const int idx = lane >> 1, part = lane & 1, r = idx >> 2, c = idx & 3;
+  double v0 = part ? delta[idx].y : delta[idx].x + (r == c ? 1.0 : 0.0), v1 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const cplx x = delta[4 * r + k];
+    double u, w;
+    win_uw(g[k * ld + c], part, u, w);
+    double& v = k < 2 ? v0 : v1;
+    v = fma(-x.x, u, v);
+    v = fma(-x.y, w, v);
+  }
+  reinterpret_cast<double*>(m)[lane] = v0 + v1;
+  __syncwarp();
+  if (lane < 24) {
+    const int mi = lane >> 1, pr = mi < 6 ? 0 : 2, pp = mi < 6 ? mi : mi - 6;
+    const int pa = pp < 3 ? 0 : (pp < 5 ? 1 : 2), pb = pp < 3 ? pp + 1 : (pp < 5 ? pp - 1 : 3);
+    const cplx e00 = m[4 * pr + pa], e01 = m[4 * pr + pb], e10 = m[4 * pr + 4 + pa], e11 = m[4 * pr + 4 + pb];
+    double u, w, u2, w2;
+    win_uw(e11, part, u, w);
+    win_uw(e10, part, u2, w2);
+    const double t1 = fma(e00.y, w, e00.x * u), t2 = fma(e01.y, w2, e01.x * u2);
+    reinterpret_cast<double*>(mn)[lane] = t1 - t2;
+  }
+  __syncwarp();
+}
+// det M = sum over the column pairs of +-(top minor)(complementary bottom
+// minor); real part in lane 0, imaginary part in lane 1.
+__device__ __forceinline__ double win_det(const cplx* mn, int lane) {
+  const int pp = lane >> 1, part = lane & 1;
+  double t = 0.0;
+  if (pp < 6) {
+    const cplx top = mn[pp];
+    double u, w;
+    win_uw(mn[11 - pp], part, u, w);
+    t = fma(top.y, w, top.x * u);
+    t = flip_sign(t, pp == 1 || pp == 4);
+  }
+#pragma unroll
+  for (int o = 8; o > 1; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+// Component of adj(M)[r][c] (cofactor C[c][r]) of this lane: the 3x3 minor
+// expanded along the remaining row of the removed row's pair, over the
+// two-row minors of the other pair.
+__device__ __forceinline__ double win_adj(const cplx* m, const cplx* mn, int lane) {
+  const int idx = lane >> 1, part = lane & 1, rr = idx & 3, cc = idx >> 2;   // removed row, column
+  const int other = rr < 2 ? 1 - rr : 5 - rr, base = rr < 2 ? 6 : 0;
+  int cols[3];
+#pragma unroll
+  for (int t = 0; t < 3; ++t) cols[t] = t + (t >= cc ? 1 : 0);
+  double d[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const int u0 = q == 0 ? cols[1] : cols[0], v0 = q == 2 ? cols[1] : cols[2];
+    const int pidx = u0 == 0 ? v0 - 1 : (u0 == 1 ? v0 + 1 : 5);
+    const cplx x = m[4 * other + cols[q]];
+    double u, w;
+    win_uw(mn[base + pidx], part, u, w);
+    d[q] = fma(x.y, w, x.x * u);
+  }
+  return flip_sign((d[0] - d[1]) + d[2], (rr + cc) & 1);
 }
 
-// Processes sites state[0] .. N-1 until k accepted updates are pending or the
-// slice ends; state[0] is left at the next site and state[1] at the number of
-// pending factors.  The flush G += X Y (a separate GEMM launch over the first
-// 4 state[1] columns) follows every round.
+// Words that travel between the CTAs of the cluster validate themselves, so
+// that no fence stands between writing and reading them: a decision carries
+// its step, and a slot of K = M^-1 Delta holds this NaN (which no arithmetic
+// produces) until its 8-byte words arrive.
+constexpr unsigned long long kWinEmpty = 0x7FF8DEADBEEF0001ull;
+__device__ __forceinline__ void st_cluster(void* p, unsigned long long v) {   // p: generic address of cluster shared memory
+  asm volatile("st.relaxed.cluster.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster(int* p, int v) {
+  asm volatile("st.relaxed.cluster.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// polls of words in this CTA's own shared memory
+__device__ __forceinline__ int ld_poll(const int* p) {
+  int v;
+  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+  return v;
+}
+// Release and acquire at cluster scope for shared memory only (a full
+// fence.acq_rel.cluster took 950 cycles).
+__device__ __forceinline__ void fence_release_shared() {
+  asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void fence_acquire_shared() {
+  asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
+}
+// 1 / x by Newton's iteration from a single-precision seed (2^-23, 2^-46,
+// then FP64 round-off): four dependent FMAs where the division takes twice
+// that; outside the single-precision range the division.
+__device__ __forceinline__ double recip_newton(double x) {
+  const int e = (__double2hiint(x) >> 20) & 0x7FF;
+  if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / x;
+  double y = (double)__frcp_rn((float)x);
+  y = fma(fma(-x, y, 1.0), y, y);
+  return fma(fma(-x, y, 1.0), y, y);
+}
+// a < b on the integer units (FP64 compares cost FP64 instructions) where the
+// bit patterns order like the values: non-negative a and b, b finite
+__device__ __forceinline__ bool less_fast(double a, double b) {
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  if ((x | y) >= 0 && (int)(y >> 52) != 0x7FF) return x < y;
+  return a < b;
+}
+__device__ __forceinline__ bool finite_bits(double x) { return ((__double2hiint(x) >> 20) & 0x7FF) != 0x7FF; }
+__device__ __forceinline__ bool zero_bits(double x) { return (__double_as_longlong(x) << 1) == 0; }
+constexpr int kWinPolls = 1 << 22;   // bound of every wait on another CTA (about 0.1 s)
+
+__device__ __forceinline__ void named_bar(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void named_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Decides the window of sites state[0] .. state[0] + W - 1 (fewer at the
+// slice's end; it also ends once d.k sites are accepted) on one cluster of C
+// CTAs.  Site s of the window (0-based) belongs to CTA s mod C, which holds its
+// 4 rows of the window's block of G (4 x 4W, column 4 s' + flavour).
 //
-// One CTA per SM; CTA b owns sites j = b, b + grid, ...  On each acceptance
-// it forms the 4 rows j + rN of the new X columns (one warp, 8 lanes per row)
-// and the 4 columns j + cN of the new Y rows (another warp), refreshes the
-// cached diagonal block of j, and publishes the number of acceptances it has
-// folded into site j.  Deciding site i waits only for that counter of site
-// i's owner (no grid-wide barrier per acceptance).  With CACHE the owner
-// also keeps its X rows / Y columns in shared memory, so the new factor
-// entries need no global loads.
-template <bool CACHE>
-__global__ void __launch_bounds__(LU_THREADS, 1) k_local_delayed(LocalUpdateArgs a, DelayedArgs d) {
-  unsigned bar_epoch = 0;
-  GridBarrierExit bar_exit(a.bar);
+// The next C undecided sites are evaluated at once, one per CTA, each as if
+// the ones before it were rejected; the first accepted one, in order, is the
+// chain's next acceptance, and the ones before it are rejected for good.  The
+// chain therefore costs one step per accepted site (and none per rejected
+// one).  Roles of the warps in a step:
+//   0  det M and the decision;          1  K = M^-1 Delta, pushed to all CTAs;
+//   2  exp(-dS), then 1 / det;          3  publishes the decision, polls all CTAs';
+//   4-7  read the accepted site's rows b = G[a, .] from its owner;
+//   0, 1  A = G[r, a] K of the own undecided rows, then the diagonal block of
+//         the next candidate, with which they start its evaluation at once;
+//   3-7  the rest of G[r, .] += A b, beside that evaluation.
+// Rows of decided sites stay as they were when decided.
+//
+// For the factors of the accepted sites a_1 .. a_p (in order), with
+// K_j = M_j^-1 Delta_j, the kernel leaves, per pair, the 4x4 blocks
+// b_i[a_j] = G_{i-1}[a_i, a_j] (i < j) and A_i[a_j] = ((G_{i-1} - I)[a_j, a_i] K_i
+// (i < j; kept in the columns of a_i, which are no longer needed).
+//
+// Bound: the chain of dependent FP64 operations of a step, about 100 cycles
+// each (64 to issue one).  The kernel this replaces formed all n rows and
+// columns of each acceptance before the next decision and took 7.6 us per
+// accepted and 3.6 us per rejected site at n = 1024.
+__global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a, DelayedArgs d, int W) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const ModelConst& mc = a.mc;
-  const int N = mc.N, n = mc.n, L = mc.L, K4 = 4 * d.k;
-  __shared__ int s_first, s_ok;
-  if (threadIdx.x == 0) s_first = __ldcg(&d.state[0]);
-  __syncthreads();
-  const int first = s_first;
-  // every round follows a flush of the previous round's factors, so nothing
-  // is pending at its start; clearing the count here also keeps the flush
-  // after a round with no sites left from applying the factors again
-  int p = 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) d.state[1] = 0;
-  if (first >= N) return;   // slice done: nothing to do in this round (uniform over the grid)
-  const int owned = (N - blockIdx.x + gridDim.x - 1) / gridDim.x;   // sites j = blockIdx.x + t grid
-  extern __shared__ double4_16a smem_local[];
-  cplx* s_blk = reinterpret_cast<cplx*>(smem_local);                   // (owned, 16) G_cur blocks
-  cplx* s_xn = s_blk + (size_t)16 * owned;                              // (4 sites, 4 x 4) new X rows
-  cplx* s_yn = s_xn + 64;                                              // (4 sites, 4 x 4) new Y columns
-  cplx* Ysm = s_yn + 64;                                               // (4k x 4): Y[j, i + cN]
-  cplx* Xsm = Ysm + (size_t)K4 * 4;                                    // (4 x 4k): X[i + rN, j]
-  cplx* s_xrow = Xsm + (size_t)K4 * 4;                                 // CACHE: (owned, 4, 4k) X[j', j + rN]
-  cplx* s_ycol = s_xrow + (CACHE ? (size_t)owned * 4 * K4 : 0);        // CACHE: (owned, 4, 4k) Y[j', j + cN]
-  double* phis = reinterpret_cast<double*>(s_ycol + (CACHE ? (size_t)owned * 4 * K4 : 0));   // (3, N)
-  __shared__ cplx s_adj[2][16];     // adj(M)[r][c] (double-buffered by site parity)
-  __shared__ cplx s_det[2];
-  __shared__ double s_expds[2];
-  // the decision, taken by whichever of the det lane and the exp(-dS) lane
-  // finishes second (s_dcnt counts their arrivals), read by all after the
-  // barrier: bit 0 accepted, bit 1 non-finite determinant
-  __shared__ int s_dcnt[2], s_dec[2];
-  __shared__ double s_pacc[2];
-  // per site (slot i & 1), read during the previous site's decision: the
-  // SitePrep words, the Metropolis uniform and the proposal (site_word), and
-  // the site's G_cur block, current if no acceptance came in between
-  // (s_gp = the pending count it was read at, -1 if not read).  Three buffers
-  // by site (i mod 3): while site i is decided, site i + 1's are written, and
-  // a thread still finishing site i - 1 (after its decision barrier, before
-  // site i's) reads that site's words, so the three must be distinct.
-  __shared__ double s_site[3][kSiteWords];
-  __shared__ cplx s_gblk[3][16];
-  __shared__ int s_gp[3];
-  // CTA 0: exp(-dS) of the round's accepted sites in order; the tracked action
-  // gets the same additions -log(exp(-dS)) in the same order once the round
-  // ends, off the per-site chain (no read-modify-write of global memory per site)
-  __shared__ double s_expq[64];
-  // mixed form: every CTA cuts the BF16 slices of its own rows of X and
-  // columns of Y (K = 4 pend entries each, zeros up to Kpad) for the flush
-  // that follows, so the flush needs no slicing launch
-  auto slice_round = [&](int pend) {
-    if (d.sl.As == nullptr || pend == 0) return;
-    __syncthreads();   // every thread's X / Y entries of the round are stored
-    const int K = 4 * pend, ln = threadIdx.x & 31;
-    for (int t = threadIdx.x >> 5; t < 8 * owned; t += blockDim.x >> 5) {
-      const int ts = t >> 3, sub = (t >> 1) & 3, side = t & 1;
-      const int rc = blockIdx.x + ts * gridDim.x + sub * N;
-      const cplx* src = side ? d.Y : d.X;
-      // with CACHE the entries come from this CTA's shared-memory copies (no L2 round trip)
-      const cplx* own = CACHE ? (side ? s_ycol : s_xrow) + (size_t)(4 * ts + sub) * K4 : nullptr;
-      oz_slice_vec(d.sl, side, rc, K, [&](int jj) { return CACHE ? own[jj] : ldcg_c(&src[(size_t)jj * n + rc]); },
-                   ln);
-    }
-  };
-  auto finish_round = [&](int pend) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && pend > 0) {
-      double act = *a.action;
-      for (int t = 0; t < pend; ++t) act += -log(s_expq[t]);
-      *a.action = act;
-      *a.n_acc += pend;
-    }
-  };
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int l = a.slice0;
-  for (int k = threadIdx.x; k < 3 * N; k += blockDim.x) phis[k] = a.phi[(size_t)3 * N * l + k];
-  for (int e = threadIdx.x; e < 16 * owned; e += blockDim.x) {
-    const int j = blockIdx.x + (e >> 4) * gridDim.x, r = (e >> 2) & 3, c = e & 3;
-    s_blk[e] = ldcg_c(&a.G[(size_t)(j + c * N) * n + j + r * N]);
+  const int N = mc.N, n = mc.n, L = mc.L;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int first = __ldcg(&d.state[0]);
+  if (first >= N) {   // slice done (uniform over the cluster): nothing for the flush either
+    if (rank == 0 && tid == 0) d.state[1] = 0;
+    return;
   }
-  // publication counters of the owned sites start the round at 0
-  for (int t = threadIdx.x; t < owned; t += blockDim.x) d.pub[blockIdx.x + t * gridDim.x] = 0;
-  // the first site's words and G block (nothing is pending at the round's start)
-  if (threadIdx.x < kSiteWords) s_site[first % 3][threadIdx.x] = site_word(a, d, first, threadIdx.x);
-  if (threadIdx.x >= 64 && threadIdx.x < 80) {
-    const int e = threadIdx.x - 64, r = e >> 2, c = e & 3;
-    s_gblk[first % 3][e] = ldcg_c(&a.G[(size_t)(first + c * N) * n + first + r * N]);
+  const int we = min(W, N - first);                       // sites of this window
+  const int owned = rank < we ? (we - rank + C - 1) / C : 0;   // sites rank + t C
+  const int own_max = (W + C - 1) / C;
+  const int LD = 4 * W + 1;
+  extern __shared__ double4_16a smem_win[];
+  cplx* Gs = reinterpret_cast<cplx*>(smem_win);           // (4 own_max, LD)
+  cplx* brow = Gs + (size_t)4 * own_max * LD;             // (4, 4W) rows of the accepted site
+  cplx* As = brow + 16 * W;                               // (4 own_max, 4): G[r, a] M^-1 Delta
+  double* site = reinterpret_cast<double*>(As + 16 * own_max);   // (own_max, kSiteWords)
+  double* prop = site + (size_t)own_max * kSiteWords;     // (W, 3) proposals
+  double* phis = prop + 3 * W + (W & 1);                  // (3, N) field of the slice
+  __shared__ cplx s_m[2][16], s_mn[2][12], s_adj[16], s_g[2][16];
+  __shared__ cplx s_k[3][WIN_MAXC][16];                   // K of the accepting candidates, by step mod 3 and owner
+  __shared__ int s_pub[2][WIN_MAXC];                      // (step + 1) << 1 | accepted, by parity (both written by the owners)
+  __shared__ double s_exp[2], s_det[2];
+  __shared__ cplx s_inv;
+  __shared__ int s_acc[WIN_MAX], s_fin[2], s_dec[2], s_flag[2];
+  if (tid < 2 * WIN_MAXC) s_pub[0][tid] = 0;
+  for (int e = tid; e < 3 * 2 * WIN_MAXC * 16; e += WIN_THREADS)
+    reinterpret_cast<unsigned long long*>(s_k)[e] = kWinEmpty;
+  for (int e = tid; e < owned * 16 * we; e += WIN_THREADS) {
+    const int rr = e / (4 * we), c = e - rr * 4 * we, t = rr >> 2, r = rr & 3;
+    Gs[(size_t)rr * LD + c] =
+        ldcg_c(&a.G[(size_t)(first + (c >> 2) + (c & 3) * N) * n + first + rank + t * C + r * N]);
   }
-  if (threadIdx.x == 0) { s_gp[first % 3] = 0; s_dcnt[0] = 0; s_dcnt[1] = 0; }
-  if (!grid_barrier(a.bar, a.err, bar_epoch)) return;
+  for (int e = tid; e < owned * kSiteWords; e += WIN_THREADS) {
+    const int t = e / kSiteWords, k = e - t * kSiteWords, gi = first + rank + t * C;
+    site[e] = k < 44 ? __ldcg(reinterpret_cast<const double*>(d.prep + gi) + k) : (k == kSiteUnif ? a.unif[gi] : 0.0);
+  }
+  for (int e = tid; e < 3 * we; e += WIN_THREADS) prop[e] = a.delta[3 * first + e];
+  for (int e = tid; e < 3 * N; e += WIN_THREADS) phis[e] = __ldcg(&a.phi[(size_t)3 * N * a.slice0 + e]);
+  cl.sync();   // also: every CTA of the cluster runs before its shared memory is written remotely
 
-  // phase-1 role of this warp in the first pass of owned sites
-  const int sub = lane >> 3, qg = (lane >> 1) & 3, h = lane & 1;
-  const bool isX = (wid & 1) == 0;
-
-  for (int i = first; i < N; ++i) {
-    const int J = 4 * p;   // pending columns of X / rows of Y
-    const int slot = i & 1;                                       // decision values
-    const int rs = i % 3, nrs = rs == 2 ? 0 : rs + 1;             // read-ahead buffers of sites i, i + 1
-    const double* sw = s_site[rs];                                // this site's words
-    const cplx* sdelta = reinterpret_cast<const cplx*>(sw);      // Delta_i, row-major
-    // the block read ahead is current unless an acceptance came in between
-    const bool have_g = s_gp[rs] == p;
-    // the Metropolis decision from det M and exp(-dS) (src/local_updates.jl:20-30),
-    // by the second of the two lanes that produce them
-    auto arrive_decide = [&]() {
-      __threadfence_block();
-      if (atomicAdd(&s_dcnt[slot], 1) == 1) {
-        __threadfence_block();
-        const cplx dt = s_det[slot];
-        const double pa = s_expds[slot] * dt.x;
-        const bool bad = !isfinite(dt.x) || !isfinite(dt.y) || (dt.x == 0.0 && dt.y == 0.0);
-        const bool ac = !bad && (pa > 1.0 || sw[kSiteUnif] < pa);
-        s_pacc[slot] = pa;
-        s_dec[slot] = (ac ? 1 : 0) | (bad ? 2 : 0);
-        s_dcnt[slot] = 0;
-      }
-    };
-    // ---- otherwise wait until the owner of site i has folded in all p acceptances ----
-    if (p > 0 && !have_g) {
-      if (threadIdx.x == 0) {
-        volatile int* f = d.pub + i;
-        int ok = 1;
-        long long spins = 0;
-        while (*f < p) {
-          if ((++spins & 1023) == 0) {
-            if (spins > (1ll << 24)) { atomicOr(a.err, 2); ok = 0; break; }
-            if (*(volatile int*)a.err & 2) { ok = 0; break; }
-          }
-        }
-        __threadfence();
-        s_ok = ok;
-      }
-      __syncthreads();
-      if (!s_ok) return;
+  const int part = lane & 1, r = lane >> 3, c = (lane >> 1) & 3;   // this lane's component of a 4x4 block
+  int cur = 0, p = 0;
+  bool ok = true, fresh = true;   // fresh: the candidate's diagonal block is to be read from Gs
+  // a CTA leaves the loop once all its sites are decided; every CTA in it has a
+  // candidate, publishes at every step and waits for all of them, so none can
+  // be two steps ahead of another and two buffers by step parity suffice.  A
+  // slot of K is emptied two steps after its use: every candidate's decision
+  // of the next step has then been seen, and with it the K it pushed (only
+  // accepting candidates push, and those either are waited for or stay in the
+  // loop).
+  for (int step = 0; owned > 0 && cur < we && p < d.k; ++step) {
+    const int par = step & 1, kslot = step % 3;
+    const int sc = cur + (rank - cur % C + C) % C;   // this CTA's candidate: its first undecided site
+    const int t = sc / C;
+    const double* sw = site + (size_t)t * kSiteWords;
+    const cplx* delta = reinterpret_cast<const cplx*>(sw);
+    const int ncand = min(C, we - cur);
+    double kv = 0.0;   // warp 1: this lane's component of K
+    if (wid < 2 && fresh) {
+      reinterpret_cast<double*>(s_g[wid])[lane] =
+          reinterpret_cast<const double*>(Gs + (size_t)(4 * t + r) * LD + 4 * sc + c)[part];
+      __syncwarp();
     }
-    // ---- G entries of the first pass's phase 1 (independent of the decision) ----
-    cplx gq_pref = cmake(0.0, 0.0);
-    if ((wid >> 1) < owned) {
-      const int rc = blockIdx.x + (wid >> 1) * gridDim.x + sub * N;
-      if (isX) {
-        gq_pref = ldcg_c(&a.G[(size_t)(i + qg * N) * n + rc]);
-        if (rc == i + qg * N) gq_pref.x -= 1.0;
-      } else {
-        gq_pref = ldcg_c(&a.G[(size_t)rc * n + i + qg * N]);
-      }
-    }
-    if (wid == 4 || wid == 6) {
-      // ---- M = I + Delta (I - G_cur_ii), lane 4r+c holds M[r][c] (src/local_updates.jl:49-55) ----
-      const int r = (lane >> 2) & 3, c = lane & 3;
-      cplx g = cmake(0.0, 0.0), drow[4];
-      if (lane < 16) {
-        g = have_g ? s_gblk[rs][lane] : ldcg_c(&d.blk[(size_t)16 * i + lane]);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) drow[k] = sdelta[4 * r + k];
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) drow[k] = cmake(0.0, 0.0);
-      }
-      const cplx mt = cmake((r == c ? 1.0 : 0.0) - g.x, -g.y);   // (I - G_ii)[r][c]
-      // M[r][c] = I + sum_k Delta[r][k] (I - G_ii)[k][c], as two independent pairs
-      const cplx m01 = cfma(drow[1], shfl_c(mt, 4 + c), cmul(drow[0], shfl_c(mt, c)));
-      const cplx m23 = cfma(drow[3], shfl_c(mt, 12 + c), cmul(drow[2], shfl_c(mt, 8 + c)));
-      cplx m = cadd(m01, m23);
-      if (r == c) m.x += 1.0;
-      if (wid == 4) {
-        // det M (Laplace expansion by 2x2 minors); lane 0's sum is the one
-        // used everywhere, so every CTA decides bit for bit alike
-        const cplx det = det_laplace(m, lane);
-        if (lane == 0) {
-          s_det[slot] = det;
-          arrive_decide();
-        }
-      } else {
-        const cplx adj = adjugate_entry(m, lane);
-        if (lane < 16) s_adj[slot][lane] = adj;
-      }
-    } else if (wid == 5) {
-      // ---- boson action difference: prepared part + space-neighbour coupling;
-      //      lanes 0-2 sum the neighbours' component c = lane (the same four
-      //      additions in the same order), lane 0 takes the rest ----
-      const int y = i % L, x = i / L;
+    if (wid == 0) {
+      win_minors(delta, s_g[0], 4, s_m[0], s_mn[0], lane);
+      const double det = win_det(s_mn[0], lane);
+      if (lane < 2) s_det[lane] = det;
+      __syncwarp();
+      named_arrive(4, 64);   // det for warp 2
+      named_bar(1, 64);      // exp(-dS) from warp 2
+      const double dx = __shfl_sync(0xffffffffu, det, 0), dy = __shfl_sync(0xffffffffu, det, 1);
+      const double ex = s_exp[par];
+      const double pa = ex * dx;
+      const bool bad = !finite_bits(dx) || !finite_bits(dy) || (zero_bits(dx) && zero_bits(dy));
+      const bool ac = !bad && (less_fast(1.0, pa) || less_fast(sw[kSiteUnif], pa));   // src/local_updates.jl:20-30
+      if (lane == 0) s_flag[par] = (ac ? 1 : 0) | (bad ? 2 : 0);
+      __syncwarp();
+      named_arrive(3, 96);   // decision for warps 1 and 3
+    } else if (wid == 1) {
+      win_minors(delta, s_g[1], 4, s_m[1], s_mn[1], lane);
+      reinterpret_cast<double*>(s_adj)[lane] = win_adj(s_m[1], s_mn[1], lane);
+      __syncwarp();
+      const double kp = win_mul4(s_adj, 4, delta, r, c, part);
+      const double o = __shfl_xor_sync(0xffffffffu, kp, 1);
+      named_bar(5, 64);      // 1 / det from warp 2
+      const cplx inv = s_inv;
+      kv = fma(o, flip_sign(inv.y, !part), kp * inv.x);
+      named_bar(3, 96);
+      if (s_flag[par] & 1)
+        for (int q = 0; q < C; ++q)
+          st_cluster(cl.map_shared_rank(reinterpret_cast<double*>(s_k[kslot][rank]) + lane, q),
+                     (unsigned long long)__double_as_longlong(kv));
+    } else if (wid == 2) {
+      // boson action difference: prepared part + space-neighbour coupling;
+      // lanes 0-2 sum the neighbours' component c = lane, lane 0 takes the rest
+      const int gi = first + sc, y = gi % L, x = gi / L;
       const int nbs[4] = {(y + 1) % L + L * x, y + L * ((x + 1) % L), (y - 1 + L) % L + L * x,
                           y + L * ((x - 1 + L) % L)};
       double os = 0.0;
@@ -661,193 +684,303 @@ __global__ void __launch_bounds__(LU_THREADS, 1) k_local_delayed(LocalUpdateArgs
       if (lane == 0) {
         const double osc[3] = {os, os1, os2};
         double sdot = 0.0;
-        for (int c = 0; c < 3; ++c) sdot += osc[c] * sw[kSiteDiff + c];
+        for (int q = 0; q < 3; ++q) sdot += osc[q] * sw[kSiteDiff + q];
         double dS = sw[kSiteDiff + 3];
         dS += 0.5 * mc.dtau * (sw[kSiteDiff + 4] - 2.0 * sdot);
         dS += sw[kSiteDiff + 5];
-        s_expds[slot] = exp(-dS);
-        arrive_decide();
+        s_exp[par] = exp(-dS);
       }
-    } else if (wid == 7 && i + 1 < N) {
-      // ---- site i + 1's G_cur block, ahead of time: current if site i is
-      //      rejected and its owner has folded in all p acceptances by now ----
-      int v = p;   // nothing pending: G itself is current
-      if (p > 0) {
-        if (lane == 0) v = (int)ld_acquire_u32(reinterpret_cast<const unsigned*>(d.pub + i + 1));
-        v = __shfl_sync(0xffffffffu, v, 0);
+      __syncwarp();
+      named_arrive(1, 64);
+      named_bar(4, 64);
+      if (lane == 0) {
+        const double dx = s_det[0], dy = s_det[1];
+        const double rd = recip_newton(fma(dx, dx, dy * dy));
+        s_inv = cmake(dx * rd, flip_sign(dy * rd, true));
       }
-      if (v >= p && lane < 16) {
-        const int r = lane >> 2, c = lane & 3, j = i + 1;
-        s_gblk[nrs][lane] = p == 0 ? ldcg_c(&a.G[(size_t)(j + c * N) * n + j + r * N])
-                                     : ldcg_c(&d.blk[(size_t)16 * j + lane]);
-      }
-      if (lane == 0) s_gp[nrs] = v >= p ? p : -1;
-    }
-    if (wid < 4) {
-      // ---- site i + 1's words (warp 3), then the pending factor entries
-      //      touching site i (128 threads, loads issued together) ----
-      // (the words are loaded first and stored last, so that their latency
-      // overlaps the staging loads)
-      const bool words = wid == 3 && i + 1 < N;
-      double w0 = 0.0, w1 = 0.0;
-      if (words) {
-        w0 = site_word(a, d, i + 1, lane);
-        if (lane + 32 < kSiteWords) w1 = site_word(a, d, i + 1, lane + 32);
-      }
-      constexpr int kStage = 128;
-      for (int t = threadIdx.x; t < 4 * J; t += 2 * kStage) {
-        const int t2 = t + kStage;
-        const int j1 = t >> 2, c1 = t & 3, j2 = t2 >> 2, c2 = t2 & 3;
-        const cplx y1 = ldcg_c(&d.Y[(size_t)j1 * n + i + c1 * N]);
-        const cplx x1 = ldcg_c(&d.X[(size_t)j1 * n + i + c1 * N]);
-        cplx y2 = cmake(0.0, 0.0), x2 = cmake(0.0, 0.0);
-        if (t2 < 4 * J) {
-          y2 = ldcg_c(&d.Y[(size_t)j2 * n + i + c2 * N]);
-          x2 = ldcg_c(&d.X[(size_t)j2 * n + i + c2 * N]);
-        }
-        Ysm[4 * j1 + c1] = y1;
-        Xsm[(size_t)c1 * K4 + j1] = x1;
-        if (t2 < 4 * J) {
-          Ysm[4 * j2 + c2] = y2;
-          Xsm[(size_t)c2 * K4 + j2] = x2;
+      __syncwarp();
+      named_arrive(5, 64);
+    } else if (wid == 3) {
+      // empty the K slots of two steps ago; the own rows are complete (barrier 6
+      // below): order both before the decision
+      for (int e = lane; e < 2 * WIN_MAXC * 16; e += 32)
+        reinterpret_cast<unsigned long long*>(s_k[(step + 1) % 3])[e] = kWinEmpty;
+      __syncwarp();
+      fence_release_shared();
+      named_bar(3, 96);
+      const int flag = s_flag[par];
+      if (lane < C) st_cluster(cl.map_shared_rank(&s_pub[par][rank], lane), (step + 1) << 1 | (flag & 1));
+      // the first accepted candidate in site order (the same in every CTA) once
+      // all candidates are published; -2: gave up waiting
+      int acc3 = -2;
+      for (int it = 0; it < kWinPolls; ++it) {
+        int v = (step + 1) << 1;
+        if (lane < ncand) v = ld_poll(&s_pub[par][(cur + lane) % C]);
+        if (__all_sync(0xffffffffu, v >> 1 == step + 1)) {
+          const unsigned hit = __ballot_sync(0xffffffffu, v & 1);
+          acc3 = hit ? cur + __ffs(hit) - 1 : -1;
+          break;
         }
       }
-      if (words) {
-        s_site[nrs][lane] = w0;
-        if (lane + 32 < kSiteWords) s_site[nrs][lane + 32] = w1;
-      }
+      fence_acquire_shared();
+      if (lane == 0) s_dec[par] = acc3;
     }
     __syncthreads();
-    // ---- Metropolis decision (the same in every CTA); thread 0 writes its effects ----
-    const int dec = s_dec[slot];
-    const bool acc = (dec & 1) != 0, bad = (dec & 2) != 0;
-    const cplx det = s_det[slot];
-    const double exp_dS = s_expds[slot];
-    const double pacc = s_pacc[slot];
-    if (threadIdx.x == 0) {
-      if (acc)
-        for (int q = 0; q < 3; ++q) phis[3 * i + q] += sw[kSiteProp + q];
-      if (blockIdx.x == 0) {
-        if (bad) atomicOr(a.err, DQMC_KERR_NONFINITE);
-        if (a.acc_out) a.acc_out[i] = (uint8_t)acc;
-        if (a.det_out) a.det_out[i] = det;
-        if (a.pacc_out) a.pacc_out[i] = pacc;
-        if (acc) {
-          double* pg = &a.phi[((size_t)N * l + i) * 3];
-          pg[0] = phis[3 * i]; pg[1] = phis[3 * i + 1]; pg[2] = phis[3 * i + 2];
-          if (a.evtab) {
-            EvEntry ev;
-            ev.C = sw[kSiteEv]; ev.Sr = sw[kSiteEv + 1]; ev.Si = sw[kSiteEv + 2]; ev.R = sw[kSiteEv + 3];
-            reinterpret_cast<EvEntry*>(a.evtab)[(size_t)N * l + i] = ev;
-          }
-          s_expq[p] = exp_dS;   // the action and the count are updated at the round's end
-        }
-      }
+    const int acc = s_dec[par];
+    if (acc == -2) {
+      ok = false;
+      break;
     }
-    // the decision values are double-buffered by site parity: a rejected site
-    // needs no barrier here; an accepted one synchronises in the passes below
-    if (!acc) continue;
-    // ---- new factor columns: X[:, J+k] = (G_cur[:, i + qN] - I[:, i + qN]) adj(M),
-    //      Y[J+k, :] = Delta G_cur[i + qN, :] / det  (X Y = (G_cur - I) M^-1 Delta G_cur) ----
-    // owned sites in passes of 4: site t of a pass -> warps 2t (X rows) and 2t+1 (Y columns)
-    for (int t0 = 0; t0 < owned; t0 += 4) {
-      const int ts = t0 + (wid >> 1);
-      if (ts < owned) {
-        const int j = blockIdx.x + ts * gridDim.x;
-        const int rc = j + sub * N;   // X: row rc; Y: column rc
-        cplx gq = gq_pref;
-        if (t0 > 0) {
-          if (isX) {
-            gq = ldcg_c(&a.G[(size_t)(i + qg * N) * n + rc]);
-            if (rc == i + qg * N) gq.x -= 1.0;
-          } else {
-            gq = ldcg_c(&a.G[(size_t)rc * n + i + qg * N]);
-          }
-        }
-        cplx inv = cmake(0.0, 0.0);
-        if (!isX) {
-          const cplx det = s_det[slot];
-          const double rd = 1.0 / (det.x * det.x + det.y * det.y);
-          inv = cmake(det.x * rd, -det.y * rd);
-        }
-        cplx part = cmake(0.0, 0.0);
-        const cplx* own = CACHE ? (isX ? s_xrow : s_ycol) + (size_t)(4 * ts + sub) * K4 : nullptr;
-        if (isX) {
-          if (CACHE) {
-            for (int jj = h; jj < J; jj += 2) part = cfma(own[jj], Ysm[4 * jj + qg], part);
-          } else {
-            for (int jj = h; jj < J; jj += 2) part = cfma(ldcg_c(&d.X[(size_t)jj * n + rc]), Ysm[4 * jj + qg], part);
-          }
-        } else {
-          if (CACHE) {
-            for (int jj = h; jj < J; jj += 2) part = cfma(Xsm[(size_t)qg * K4 + jj], own[jj], part);
-          } else {
-            for (int jj = h; jj < J; jj += 2) part = cfma(Xsm[(size_t)qg * K4 + jj], ldcg_c(&d.Y[(size_t)jj * n + rc]), part);
-          }
-        }
-        part = cadd(part, shfl_c(part, lane ^ 1));
-        const cplx gcur = cadd(gq, part);   // G_cur[rc, i + qN] (- delta) or G_cur[i + qN, rc]
-        // output k = qg of this lane over q' = 2h, 2h + 1, then the pair sum
-        const int ko = qg;
-        const cplx g0 = shfl_c(gcur, 8 * sub + 4 * h), g1 = shfl_c(gcur, 8 * sub + 4 * h + 2);
-        cplx prod;
-        if (isX) prod = cfma(g1, s_adj[slot][4 * (2 * h + 1) + ko], cmul(g0, s_adj[slot][4 * (2 * h) + ko]));
-        else prod = cfma(sdelta[4 * ko + 2 * h + 1], g1, cmul(sdelta[4 * ko + 2 * h], g0));
-        prod = cadd(prod, shfl_c(prod, lane ^ 1));
-        if (!isX) prod = cmul(prod, inv);
-        if (h == 0) {
-          const int ls = ts - t0;
-          if (isX) {
-            d.X[(size_t)(J + ko) * n + rc] = prod;
-            s_xn[16 * ls + 4 * sub + ko] = prod;        // X_new[j + sub N, k]
-          } else {
-            d.Y[(size_t)(J + ko) * n + rc] = prod;
-            s_yn[16 * ls + 4 * ko + sub] = prod;        // Y_new[k, j + sub N]
-          }
-          if (CACHE) const_cast<cplx*>(own)[J + ko] = prod;
-        }
+    const int last = acc >= 0 ? acc : cur + ncand - 1;   // sites cur .. last are decided
+    if (sc <= last && wid == 3 && lane == 0) {
+      const int gi = first + sc, flag = s_flag[par];
+      if (flag & 2) atomicOr(a.err, DQMC_KERR_NONFINITE);
+      if (a.acc_out) a.acc_out[gi] = (uint8_t)(flag & 1);
+      if (a.det_out) a.det_out[gi] = cmake(s_det[0], s_det[1]);
+      if (a.pacc_out) a.pacc_out[gi] = s_exp[par] * s_det[0];
+    }
+    cur = last + 1;
+    const int t0 = rank > last ? 0 : (last - rank) / C + 1;   // own undecided sites t0 .. owned - 1
+    fresh = true;
+    if (acc < 0) {
+      if (t0 >= owned) break;
+      __syncthreads();   // s_det, s_flag read
+      continue;
+    }
+    const int owner = acc % C, ta = acc / C;
+    if (rank == owner && wid == 1) reinterpret_cast<double*>(d.wk + 16 * p)[lane] = kv;   // for the factors
+    if (wid == 2) {
+      // field, interaction table, order of acceptances
+      const int gi = first + acc;
+      if (lane < 3) {
+        const double v = phis[3 * gi + lane] + prop[3 * acc + lane];
+        phis[3 * gi + lane] = v;
+        if (rank == owner) a.phi[((size_t)N * a.slice0 + gi) * 3 + lane] = v;
+      } else if (lane == 3) {
+        s_acc[p] = acc;
+        if (rank == owner) d.wexp[p] = s_exp[par];
+      } else if (lane == 4 && rank == owner && a.evtab) {
+        const double* se = site + (size_t)ta * kSiteWords + kSiteEv;
+        EvEntry ev;
+        ev.C = se[0]; ev.Sr = se[1]; ev.Si = se[2]; ev.R = se[3];
+        reinterpret_cast<EvEntry*>(a.evtab)[(size_t)N * a.slice0 + gi] = ev;
       }
-      __syncthreads();
-      // ---- refresh the cached blocks of the pass's sites (needed by later sites only) ----
-      if (!(wid & 1)) {
-        const int ls = wid >> 1, tsr = t0 + ls;
-        const int j = blockIdx.x + tsr * gridDim.x;
-        if (tsr < owned && j > i) {
-          // entry e = 4r + c of the block: lanes e and e + 16 take k = 0, 1 and
-          // k = 2, 3 of X_new[r, k] Y_new[k, c], then add the halves
-          const int e = lane & 15, r = e >> 2, c = e & 3, k0 = (lane >> 4) * 2;
-          cplx b = lane < 16 ? s_blk[16 * tsr + e] : cmake(0.0, 0.0);
-          b = cfma(s_xn[16 * ls + 4 * r + k0], s_yn[16 * ls + 4 * k0 + c], b);
-          b = cfma(s_xn[16 * ls + 4 * r + k0 + 1], s_yn[16 * ls + 4 * (k0 + 1) + c], b);
-          b = cadd(b, shfl_c(b, lane ^ 16));
-          if (lane < 16) {
-            s_blk[16 * tsr + e] = b;
-            d.blk[(size_t)16 * j + e] = b;
-          }
-        }
-      }
-      __syncthreads();   // s_xn / s_yn reused by the next pass; all stores precede the publication
+      __syncwarp();
     }
     ++p;
-    if (p == d.k || i == N - 1) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) { d.state[0] = i + 1; d.state[1] = p; }
-      finish_round(p);
-      slice_round(p);
-      return;   // the flush follows as its own launch
+    if (t0 >= owned) break;
+    if (wid != 2) {
+      // ---- apply the acceptance to the own undecided rows (7 warps) ----
+      const int left = owned - t0, cols = 4 * (we - acc - 1), c0 = 4 * (acc + 1);
+      const int s0 = rank + t0 * C;   // the next candidate
+      double gv = 0.0;                // warps 0, 1: this lane's component of its diagonal block
+      if (wid < 2) {
+        gv = reinterpret_cast<const double*>(Gs + (size_t)(4 * t0 + r) * LD + 4 * s0 + c)[part];
+        const cplx* k = s_k[kslot][owner];
+        bool here = false;
+        for (int it = 0; it < kWinPolls && !here; ++it) {
+          const int w0 = ld_poll(reinterpret_cast<const int*>(k) + 2 * lane);
+          const int w1 = ld_poll(reinterpret_cast<const int*>(k) + 2 * lane + 1);
+          here = __all_sync(0xffffffffu, w0 != (int)(kWinEmpty & 0xffffffffu) || w1 != (int)(kWinEmpty >> 32));
+        }
+        fence_acquire_shared();
+        __syncwarp();
+        ok = ok && here;
+        for (int ts = t0 + wid; ts < owned; ts += 2) {
+          const double v = win_mul4(Gs + (size_t)4 * ts * LD + 4 * acc, LD, k, r, c, part);
+          reinterpret_cast<double*>(As + 16 * ts)[lane] = v;
+          __syncwarp();
+          reinterpret_cast<double*>(Gs + (size_t)(4 * ts + r) * LD + 4 * acc + c)[part] = v;
+        }
+      } else if (wid >= 4) {
+        const int q = wid - 4;
+        const cplx* src = cl.map_shared_rank(Gs + (size_t)(4 * ta + q) * LD + c0, owner);
+        cplx* dst = brow + q * 4 * W + c0;
+        for (int cc = lane; cc < cols; cc += 64) {
+          const bool two = cc + 32 < cols;
+          const cplx x0 = src[cc], x1 = two ? src[cc + 32] : cmake(0.0, 0.0);
+          dst[cc] = x0;
+          if (two) dst[cc + 32] = x1;
+        }
+      }
+      named_bar(2, WIN_THREADS - 32);
+      if (wid < 2) {
+        // G[row, cc] += sum_q A[row][q] b[q][cc]
+        const cplx* ar = As + 4 * (4 * t0 + r);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          double u, w;
+          win_uw(brow[q * 4 * W + 4 * s0 + c], part, u, w);
+          gv = fma(ar[q].x, u, gv);
+          gv = fma(ar[q].y, w, gv);
+        }
+        reinterpret_cast<double*>(s_g[wid])[lane] = gv;
+        __syncwarp();
+      } else {
+        // one entry per lane: two independent chains (real, imaginary) hide the
+        // FP64 latency that one leaves exposed
+        const float icols = 1.0f / (float)cols;
+        for (int e = tid - 96; e < 4 * left * cols; e += 160) {
+          const int rr = (int)(((float)e + 0.5f) * icols), cc = c0 + e - rr * cols, row = 4 * t0 + rr;
+          const cplx* ar = As + 4 * row;
+          cplx v = Gs[(size_t)row * LD + cc];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const cplx x = ar[q], y = brow[q * 4 * W + cc];
+            v.x = fma(x.x, y.x, v.x);
+            v.y = fma(x.x, y.y, v.y);
+            v.x = fma(-x.y, y.y, v.x);
+            v.y = fma(x.y, y.x, v.y);
+          }
+          Gs[(size_t)row * LD + cc] = v;
+        }
+        named_bar(6, 160);   // warps 3-7: the own rows are complete
+      }
     }
-    // ---- publish: the owned later sites now include p acceptances (the CTA
-    //      barrier above orders every thread's stores before this fence) ----
-    if (threadIdx.x == 0) {
-      __threadfence();
-      for (int t = 0; t < owned; ++t) {
-        const int j = blockIdx.x + t * gridDim.x;
-        if (j > i) *(volatile int*)(d.pub + j) = p;
+    fresh = false;
+  }
+  if (!ok) atomicOr(a.err, DQMC_KERR_BARRIER_TIMEOUT);
+  if (wid == 2 && lane == 0) {
+    s_fin[0] = p;
+    s_fin[1] = cur;
+  }
+  cl.sync();   // every CTA is done; the owner of the last site has seen all decisions
+  const int lastr = (we - 1) % C;
+  p = *cl.map_shared_rank(&s_fin[0], lastr);
+  cur = *cl.map_shared_rank(&s_fin[1], lastr);
+  __syncthreads();
+  if (rank != lastr) {
+    for (int e = tid; e < p; e += WIN_THREADS) s_acc[e] = cl.map_shared_rank(&s_acc[0], lastr)[e];
+  }
+  cl.sync();   // no shared memory is read remotely any more
+  // ---- the accepted sites' blocks for k_local_factors, the round's state ----
+  for (int e = tid; e < p * p * 16; e += WIN_THREADS) {
+    const int j = e / (16 * p), i = (e >> 4) - j * p, q = e & 15;
+    const int sj = s_acc[j];
+    if (sj % C != rank || i == j) continue;
+    d.wblk[((size_t)j * WIN_MAX + i) * 16 + q] = Gs[(size_t)(4 * (sj / C) + (q >> 2)) * LD + 4 * s_acc[i] + (q & 3)];
+  }
+  if (rank == 0 && wid == 0) {
+    if (lane < p) d.wsite[lane] = first + s_acc[lane];
+    // the tracked action: -log(exp(-dS)) of the accepted sites, added in order
+    const double lg = lane < p ? -log(__ldcg(&d.wexp[lane])) : 0.0;
+    double act = lane == 0 ? *a.action : 0.0;
+    for (int q = 0; q < p; ++q) {
+      const double v = __shfl_sync(0xffffffffu, lg, q);
+      if (lane == 0) act += v;
+    }
+    if (lane == 0) {
+      d.state[0] = first + cur;
+      d.state[1] = p;
+      if (p > 0) {
+        *a.action = act;
+        *a.n_acc += p;
       }
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) { d.state[0] = N; d.state[1] = p; }
-  finish_round(p);
-  slice_round(p);
+}
+
+// The rank-4p factors of a window: G += X Y with
+//   X[:, j] = ((G - I)[:, a_j] + sum_{i<j} X[:, i] b_i[a_j]) K_j,
+//   Y[j, :] = G[a_j, :] + sum_{i<j} A_i[a_j] Y[i, :]
+// (blocks from k_local_window): every row of X and every column of Y is an
+// independent recurrence of p steps.  8 SPLIT lanes per vector: 4 components x
+// {real, imaginary} x SPLIT shares of the sum over i; the vector and the blocks
+// are in shared memory.  At the end each vector is cut into the BF16 slices of
+// the flush (or stored in FP64 when the product slices it itself).
+// Bound: FP64 issue, 8 (4p)^2 / 2 multiply-adds per vector; SPLIT grows as n
+// falls, so that small lattices still fill the sub-partitions.
+constexpr int FAC_THREADS = 128;
+template <int SPLIT>
+__global__ void __launch_bounds__(FAC_THREADS) k_local_factors(LocalUpdateArgs a, DelayedArgs d) {
+  const int p = __ldcg(&d.state[1]);
+  if (p == 0) return;   // uniform over the grid
+  constexpr int VPW = 4 / SPLIT, VPC = VPW * (FAC_THREADS / 32);
+  const int n = a.mc.n, N = a.mc.N;
+  const int side = blockIdx.y, v0 = blockIdx.x * VPC;   // side 0: rows of X, 1: columns of Y
+  extern __shared__ double4_16a smem_fac[];
+  cplx* coef = reinterpret_cast<cplx*>(smem_fac);       // (p (p - 1) / 2, 4, 4): [c][q] of step j, term i < j
+  cplx* kk = coef + (size_t)8 * p * (p - 1);            // (p, 4, 4) K_j (X)
+  const int ldx = 4 * d.k + 1;
+  cplx* xs = kk + 16 * p;                               // (VPC, ldx) the vectors
+  __shared__ cplx s_t[VPC][4];
+  __shared__ int s_site[WIN_MAX];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid < p) s_site[tid] = __ldcg(&d.wsite[tid]);
+#pragma unroll 4
+  for (int e = tid; e < 8 * p * (p - 1); e += FAC_THREADS) {
+    // pair index (j, i): j (j - 1) / 2 + i
+    const int pr = e >> 4, q = e & 15;
+    int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)pr)) * 0.5f);
+    while (j * (j - 1) / 2 > pr) --j;
+    while ((j + 1) * j / 2 <= pr) ++j;
+    const int i = pr - j * (j - 1) / 2;
+    coef[e] = side == 0 ? ldcg_c(&d.wblk[((size_t)i * WIN_MAX + j) * 16 + q])
+                        : ldcg_c(&d.wblk[((size_t)j * WIN_MAX + i) * 16 + 4 * (q & 3) + (q >> 2)]);
+  }
+  if (side == 0)
+    for (int e = tid; e < 16 * p; e += FAC_THREADS) kk[e] = ldcg_c(&d.wk[e]);
+  __syncthreads();
+#pragma unroll 4
+  for (int e = tid; e < 4 * p * VPC; e += FAC_THREADS) {
+    const int v = side == 0 ? e % VPC : e / (4 * p), jq = side == 0 ? e / VPC : e - v * 4 * p;
+    const int ai = s_site[jq >> 2] + (jq & 3) * N;
+    cplx g = side == 0 ? ldcg_c(&a.G[(size_t)ai * n + v0 + v]) : ldcg_c(&a.G[(size_t)(v0 + v) * n + ai]);
+    if (side == 0 && ai == v0 + v) g.x -= 1.0;
+    xs[v * ldx + jq] = g;
+  }
+  __syncthreads();
+  const int part = lane & 1, q = (lane >> 1) & 3, sp = (lane >> 3) % SPLIT, v = wid * VPW + lane / (8 * SPLIT);
+  cplx* x = xs + v * ldx;
+  for (int j = 0; j < p; ++j) {
+    const cplx* cj = coef + (size_t)8 * j * (j - 1);
+    double t0 = 0.0, t1 = 0.0;
+    if (sp == 0) t0 = part ? x[4 * j + q].y : x[4 * j + q].x;
+    for (int i = sp; i < j; i += SPLIT) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const cplx xv = x[4 * i + c];
+        double u, w;
+        win_uw(cj[16 * i + 4 * c + q], part, u, w);
+        t0 = fma(xv.x, u, t0);
+        t1 = fma(xv.y, w, t1);
+      }
+    }
+    double t = t0 + t1;
+#pragma unroll
+    for (int o = 8; o < 8 * SPLIT; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (side == 0) {
+      if (sp == 0) reinterpret_cast<double*>(&s_t[v][q])[part] = t;
+      __syncwarp();
+      double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const cplx tv = s_t[v][c];
+        double u, w;
+        win_uw(kk[16 * j + 4 * c + q], part, u, w);
+        r0 = fma(tv.x, u, r0);
+        r1 = fma(tv.y, w, r1);
+      }
+      t = r0 + r1;
+    }
+    __syncwarp();
+    if (sp == 0) reinterpret_cast<double*>(x + 4 * j + q)[part] = t;
+    __syncwarp();
+  }
+  if (d.sl.As) {
+#pragma unroll 1
+    for (int u = 0; u < VPW; ++u) {
+      const cplx* xv = xs + (wid * VPW + u) * ldx;
+      oz_slice_vec(d.sl, side, v0 + wid * VPW + u, 4 * p, [&](int k) { return xv[k]; }, lane);
+    }
+  } else {
+    __syncthreads();
+    cplx* out = side == 0 ? d.X : d.Y;
+    for (int e = tid; e < 4 * p * VPC; e += FAC_THREADS) {
+      const int vv = e % VPC, jq = e / VPC;
+      out[(size_t)jq * n + v0 + vv] = xs[vv * ldx + jq];
+    }
+  }
 }
 
 // Condition of the graph's WHILE node that repeats [delayed round, flush]:
@@ -882,37 +1015,89 @@ cudaError_t launch_local_prepare(const LocalUpdateArgs& a, SitePrep* prep, int* 
   return cudaGetLastError();
 }
 
-static size_t local_delayed_smem(int N, int k, int grid, bool cache) {
-  const size_t owned = (size_t)(N + grid - 1) / grid;
-  size_t c = 16 * owned + 128 + (size_t)2 * 16 * k;
-  if (cache) c += 2 * owned * 4 * 4 * (size_t)k;
-  return c * sizeof(cplx) + (size_t)3 * N * sizeof(double);
+// Cluster size of the window kernel on the current device: 16 CTAs where the
+// device can schedule one (a non-portable size), else 8; 0 if neither.
+static size_t window_smem(int N, int W, int C) {
+  const size_t own = (size_t)(W + C - 1) / C;
+  return (4 * own * (4 * W + 1) + 16 * W + 16 * own) * sizeof(cplx) +
+         (own * kSiteWords + 3 * W + (W & 1) + 3 * N) * sizeof(double);
 }
 
-cudaError_t launch_local_delayed(const LocalUpdateArgs& a, const DelayedArgs& d, int sm_count, cudaStream_t st,
-                                 int max_grid) {
-  constexpr size_t kMaxSmem = 200 * 1024;
-  const int N = a.mc.N;
-  int grid = sm_count;    // one CTA per SM
-  if (grid > N) grid = N;
-  if (max_grid > 0 && grid > max_grid) grid = max_grid;
-  const bool cache = local_delayed_smem(N, d.k, grid, true) <= kMaxSmem;
-  const size_t smem = local_delayed_smem(N, d.k, grid, cache);
-  if (smem > kMaxSmem) return cudaErrorInvalidValue;
-  static SmemLimit limit_cache, limit_plain;
-  if (cudaError_t ea = limit_cache.raise((const void*)k_local_delayed<true>, (int)kMaxSmem); ea != cudaSuccess)
-    return ea;
-  if (cudaError_t ea = limit_plain.raise((const void*)k_local_delayed<false>, (int)kMaxSmem); ea != cudaSuccess)
-    return ea;
-  const void* fn = cache ? (const void*)k_local_delayed<true> : (const void*)k_local_delayed<false>;
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, LU_THREADS, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  LocalUpdateArgs ca = a;
-  DelayedArgs cd = d;
-  void* args[] = {&ca, &cd};
-  return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(LU_THREADS), args, smem, st);
+static cudaLaunchConfig_t window_config(cudaLaunchAttribute* attr, int C, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(WIN_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+static cudaError_t window_cluster(int* C) {
+  static std::mutex mu;
+  static int cached[64] = {};
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (cached[dev] == 0) {
+    const void* fn = (const void*)k_local_window;
+    if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); e != cudaSuccess)
+      return e;
+    for (int c = WIN_MAXC; c >= 8 && cached[dev] == 0; c /= 2) {
+      const size_t smem = window_smem(256, WIN_MAX, c);   // the largest lattice and window
+      if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          e != cudaSuccess)
+        return e;
+      cudaLaunchAttribute attr[1];
+      const cudaLaunchConfig_t cfg = window_config(attr, c, smem, nullptr);
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        clusters = 0;
+      }
+      if (clusters >= 1) cached[dev] = c;
+    }
+    if (cached[dev] == 0) return cudaErrorNotSupported;
+    // 8-CTA clusters (batched chains) hold up to four sites per CTA
+    if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)window_smem(256, WIN_MAX, 8));
+        e != cudaSuccess)
+      return e;
+  }
+  *C = cached[dev];
+  return cudaSuccess;
+}
+
+int local_window_sites(int k) { return k < WIN_MAX ? k : WIN_MAX; }
+
+cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster) {
+  int C = 0;
+  if (cudaError_t e = window_cluster(&C); e != cudaSuccess) return e;
+  if (max_cluster > 0 && C > 8 && max_cluster < C) C = 8;
+  const int W = local_window_sites(d.k);
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = window_config(attr, C, window_smem(a.mc.N, W, C), st);
+  return cudaLaunchKernelEx(&cfg, k_local_window, a, d, W);
+}
+
+cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st) {
+  const int n = a.mc.n, W = local_window_sites(d.k);
+  // lanes per vector: 2 n vectors on about 600 sub-partitions, one warp each
+  const int split = n <= 304 ? 4 : n <= 608 ? 2 : 1;
+  const int vpc = 16 / split;   // n = 4 L^2 with L even: a multiple of 16
+  const size_t smem = ((size_t)8 * W * (W - 1) + 16 * W + (size_t)vpc * (4 * d.k + 1)) * sizeof(cplx);
+  static SmemLimit limits[3];
+  void (*const fns[3])(LocalUpdateArgs, DelayedArgs) = {k_local_factors<1>, k_local_factors<2>, k_local_factors<4>};
+  const int which = split == 4 ? 2 : split - 1;
+  if (cudaError_t e = limits[which].raise((const void*)fns[which], (int)smem); e != cudaSuccess) return e;
+  fns[which]<<<dim3(n / vpc, 2), FAC_THREADS, smem, st>>>(a, d);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_local_updates(const LocalUpdateArgs& a, int sm_count, cudaStream_t st, int max_grid) {

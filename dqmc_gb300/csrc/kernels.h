@@ -46,8 +46,9 @@ struct LocalUpdateArgs {
   ModelConst mc;
 };
 cudaError_t launch_local_updates(const LocalUpdateArgs& a, int sm_count, cudaStream_t st, int max_grid = 0);
-// delayed rank-k form: pending factors X (n x 4k, column-major) and Y (4k x n,
-// row j at Y + j*n); state[0] = next site of the slice, state[1] = pending accepts
+// delayed form, in rounds (windows of sites): state[0] = next site of the
+// slice, state[1] = acceptances of the round, whose factors X Y the flush
+// (a GEMM launch over the first 4 state[1] columns) adds to G
 // Per-site data of one slice, prepared once before its first delayed round
 // (the old field of a site cannot change before its own visit).
 struct SitePrep {
@@ -67,19 +68,25 @@ struct OzSlices {
   double *sA, *sB;
   int m, n, Kpad, S, bits;
 };
+constexpr int WIN_MAX = 32;   // most sites of a window (a window takes min(k, 32))
 struct DelayedArgs {
   cplx* X;
   cplx* Y;
   int* state;
-  int k;
+  int k;                   // most acceptances of a round
   const SitePrep* prep;    // (N) from launch_local_prepare for this slice
-  cplx* blk;               // (N, 16) cache of the diagonal blocks G_cur[j + rN, j + cN]
-  int* pub;                // (N) acceptances of the current round folded into site j's data
-  OzSlices sl;             // mixed form: the flush's slices, cut by the owners at the round's end
-                           // (sl.As null: the flush slices X and Y itself)
+  int* wsite;              // (WIN_MAX) sites accepted in the window, in order
+  cplx* wk;                // (WIN_MAX, 16) their M^-1 Delta
+  double* wexp;            // (WIN_MAX) their exp(-dS)
+  cplx* wblk;              // (WIN_MAX, WIN_MAX, 16) their 4x4 blocks (k_local_window)
+  OzSlices sl;             // the flush's slices, cut by launch_local_factors
+                           // (sl.As null: X and Y are stored and the flush slices them itself)
 };
-cudaError_t launch_local_delayed(const LocalUpdateArgs& a, const DelayedArgs& d, int sm_count, cudaStream_t st,
-                                 int max_grid = 0);
+// Decides the next window of the slice on one cluster (max_cluster > 0: at most that many CTAs, >= 8).
+cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster);
+// The factors X (n x 4p, column-major) and Y (4p x n, row j at Y + j n) of the window's p acceptances.
+cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st);
+int local_window_sites(int k);
 // Sets the WHILE condition of a captured round loop (see local_updates_dev):
 // another round while state[0] < N, state[2] < max_rounds and *err == 0.
 cudaError_t launch_round_cond(cudaGraphConditionalHandle hc, int* state, int N, int max_rounds, const int* err,
