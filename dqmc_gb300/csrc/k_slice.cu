@@ -242,34 +242,37 @@ __global__ void k_build_evtab(const double* __restrict__ phi, EvEntry* __restric
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-static int pick_cols_per_cta(int n) {
-  // ~32 KB of slab per CTA keeps 4-6 CTAs per SM and >= 2 waves of work.
-  int c = 32768 / (16 * n);
-  if (c < 1) c = 1;
-  if (c > 64) c = 64;
-  return c;
+// One column (two rows: a 32-byte sector of a column-major row) per CTA, with a
+// thread per site block.  The layers are bound by FP64 issue, so what counts is
+// that the work spreads evenly over the sub-partitions: slabs of 32 KB left
+// n = 64 on 2 CTAs and n = 256 on 32 (28 us per slice at either size), n = 400 on
+// 80, and at n = 1024 some SMs with 4 slabs and others with 3.
+static int slice_threads(int units) {
+  const int t = (units + 31) / 32 * 32;
+  return t < 32 ? 32 : (t > 256 ? 256 : t);
 }
 
 cudaError_t launch_apply_cols(cplx* A, int n, const ModelConst& mc, const void* evtab, int first_slice0,
                               int count, int step, int mode, const double* colscale, cudaStream_t st) {
-  int cpc = pick_cols_per_cta(n);
+  const int cpc = 1;
   int grid = (n + cpc - 1) / cpc;
   size_t smem = (size_t)cpc * n * sizeof(cplx) + (size_t)mc.N * sizeof(EvEntry);
   static SmemLimit smem_limit;
-  if (cudaError_t ea = smem_limit.raise((const void*)k_apply_cols, 200 * 1024); ea != cudaSuccess) return ea;
-  k_apply_cols<<<grid, 256, smem, st>>>(A, n, cpc, mc, (const EvEntry*)evtab, first_slice0, count, step, mode,
-                                         colscale);
+  if (cudaError_t ea = smem_limit.raise((const void*)k_apply_cols, 64 * 1024); ea != cudaSuccess) return ea;
+  k_apply_cols<<<grid, slice_threads(mc.N * cpc), smem, st>>>(A, n, cpc, mc, (const EvEntry*)evtab, first_slice0, count,
+                                                               step, mode, colscale);
   return cudaGetLastError();
 }
 
 cudaError_t launch_apply_rows(cplx* A, int n, const ModelConst& mc, const void* evtab, int first_slice0,
                               int count, int step, int mode, cudaStream_t st) {
-  int rpc = pick_cols_per_cta(n);
+  const int rpc = 2;
   int grid = (n + rpc - 1) / rpc;
   size_t smem = (size_t)rpc * n * sizeof(cplx) + (size_t)mc.N * sizeof(EvEntry);
   static SmemLimit smem_limit;
-  if (cudaError_t ea = smem_limit.raise((const void*)k_apply_rows, 200 * 1024); ea != cudaSuccess) return ea;
-  k_apply_rows<<<grid, 256, smem, st>>>(A, n, rpc, mc, (const EvEntry*)evtab, first_slice0, count, step, mode);
+  if (cudaError_t ea = smem_limit.raise((const void*)k_apply_rows, 64 * 1024); ea != cudaSuccess) return ea;
+  k_apply_rows<<<grid, slice_threads(mc.N * rpc), smem, st>>>(A, n, rpc, mc, (const EvEntry*)evtab, first_slice0, count,
+                                                               step, mode);
   return cudaGetLastError();
 }
 
