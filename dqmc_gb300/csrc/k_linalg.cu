@@ -1090,14 +1090,14 @@ __global__ void __launch_bounds__(128) k_trsm_left_upper(const cplx* __restrict_
 // columns, in shared memory once (no L2 round trip inside the dependent
 // column steps); each warp solves one column with its b values in registers
 // (row lane + 32 i in slot i) and broadcasts y_q by shuffle.
-constexpr int TRSM_DB_WARPS = 8;
+constexpr int TRSM_DB_WARPS = 8;   // all stage the triangle; the first `warps` of them solve a column each
 __device__ __forceinline__ int trsm_pack_lower(int q, int b) { return q * (b - 1) - q * (q - 1) / 2; }
 __device__ __forceinline__ int trsm_pack_upper(int q) { return q * (q - 1) / 2; }
 
 __global__ void __launch_bounds__(32 * TRSM_DB_WARPS) k_trsm_diag_block(const cplx* __restrict__ T, int ldT,
                                                                        const cplx* __restrict__ rdiag,
                                                                        cplx* __restrict__ Y, int ldY, int j0, int b,
-                                                                       int m, int lower) {
+                                                                       int m, int lower, int warps) {
   extern __shared__ double4_16a smem_tdb[];
   cplx* tp = reinterpret_cast<cplx*>(smem_tdb);   // (b (b - 1) / 2) packed strict triangle
   cplx* rd = tp + (size_t)b * (b - 1) / 2;        // (b) reciprocal diagonal (upper)
@@ -1122,8 +1122,8 @@ __global__ void __launch_bounds__(32 * TRSM_DB_WARPS) k_trsm_diag_block(const cp
   if (!lower)
     for (int q = threadIdx.x; q < b; q += blockDim.x) rd[q] = __ldg(&rdiag[j0 + q]);
   __syncthreads();
-  const int col = blockIdx.x * TRSM_DB_WARPS + wid;
-  if (col >= m) return;
+  const int col = blockIdx.x * warps + wid;
+  if (wid >= warps || col >= m) return;
   cplx* yg = Y + (size_t)col * ldY + j0;
   cplx y[4];
 #pragma unroll
@@ -1356,8 +1356,18 @@ cudaError_t launch_trsm_diag_block(const cplx* T, int ldT, const cplx* rdiag, cp
   static SmemLimit smem_limit;
   constexpr int kMaxTdb = (int)((128 * 127 / 2 + 128) * sizeof(cplx));   // b = 128
   if (cudaError_t ea = smem_limit.raise((const void*)k_trsm_diag_block, kMaxTdb); ea != cudaSuccess) return ea;
-  k_trsm_diag_block<<<(m + TRSM_DB_WARPS - 1) / TRSM_DB_WARPS, 32 * TRSM_DB_WARPS, smem, st>>>(
-      T, ldT, rdiag, Y, ldY, j0, b, m, lower ? 1 : 0);
+  // one column per warp and as few warps per SM as the m columns allow: a
+  // solve is a chain of b FP64 steps, and warps that share a sub-partition
+  // double it (m = 256, b = 64: 32 CTAs of 8 warps 48 and 79 us, lower and upper)
+  int sms = 152;
+  if (int dev = 0; cudaGetDevice(&dev) == cudaSuccess) {
+    int v = 0;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0) sms = v;
+  }
+  int warps = (m + sms - 1) / sms;
+  if (warps > TRSM_DB_WARPS) warps = TRSM_DB_WARPS;
+  k_trsm_diag_block<<<(m + warps - 1) / warps, 32 * TRSM_DB_WARPS, smem, st>>>(T, ldT, rdiag, Y, ldY, j0, b, m,
+                                                                              lower ? 1 : 0, warps);
   return cudaGetLastError();
 }
 
