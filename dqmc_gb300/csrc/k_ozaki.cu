@@ -244,9 +244,9 @@ __global__ void k_oz_finalize(OzArgs a) {
 // A CTA computes 128 x 32 complex tiles of C, persistently: one CTA per SM
 // takes tiles x, x + grid, ... and the MMAs of a tile run while the epilogue
 // of the previous one converts and stores.  Each MMA is
-// M = 128, N = 64, K = 16 (kind::f16, BF16 in, FP32 out): its B operand
-// stacks the 32 columns of B'_re over the 32 of B'_im, so one accumulator
-// holds [Re | Im] of the tile.  Every group t = p + q (2 <= t <= S + 1) has
+// M = 128, K = 16 (kind::f16, BF16 in, FP32 out), N = 64 per B slice: the
+// slice's tile stacks the 32 columns of B'_re over the 32 of B'_im, so one
+// accumulator holds [Re | Im] of the tile.  Every group t = p + q (2 <= t <= S + 1) has
 // its own accumulator of 64 TMEM columns, all S live at once (S <= 8: 512
 // columns), so one pass over K serves every slice pair and each K block of
 // every slice is staged once:
@@ -277,8 +277,16 @@ constexpr int TC_B_TILE = 2 * TC_B_HALF;        // 8 KB
 // MMA instruction descriptor (kind::f16): D F32 (bits 4-5 = 1), A BF16 (bits
 // 7-9 = 1), B BF16 (bits 10-12 = 1), both K-major (bits 15, 16 = 0),
 // N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-constexpr uint32_t TC_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * TC_BN) >> 3 << 17) |
-                              ((uint32_t)TC_BM >> 4 << 24);
+__host__ __device__ constexpr uint32_t tc_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)n >> 3 << 17) | ((uint32_t)TC_BM >> 4 << 24);
+}
+// B slices of one MMA.  For a fixed A slice p the pairs (p, q), q = 0, 1, ...
+// write adjacent groups of 64 TMEM columns, and the B slices' tiles of 64 rows
+// are adjacent in shared memory, so up to 4 of them are one MMA of N = 256: the
+// tensor core then reads A (4 KB per K step) once for them.  At N = 64 the 6 KB
+// of operands per MMA took 48 cycles of shared-memory bandwidth for 32 of
+// arithmetic.
+constexpr int TC_NSTACK = 4;
 
 __host__ __device__ constexpr size_t tc_smem_bytes(int S) {
   return 1024 + (size_t)2 * S * TC_B_TILE + (size_t)TC_ARING * TC_A_TILE + 256;
@@ -349,11 +357,12 @@ __device__ __forceinline__ void tma_load3(uint32_t dst, const CUtensorMap* map, 
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                       uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(TC_IDESC), "r"(accumulate)
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 // arrives on the barrier once every tcgen05.mma issued so far by this thread has completed
@@ -497,13 +506,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
           if (!mbar_wait(bar(FA + slot), (a_use / TC_ARING) & 1, err, s_abort)) { ok = false; break; }
           tc_fence_after();
           const uint64_t ad = tc_desc(sA + (uint32_t)slot * TC_A_TILE);
-          for (int q = 0; q + p < S; ++q) {
-            // pair (p + 1, q + 1) belongs to group t = p + q + 2: accumulator columns (p + q) * 64
+          for (int q = 0; q + p < S; q += TC_NSTACK) {
+            // pairs (p + 1, q + 1 ..) belong to groups t = p + q + 2 ..: accumulator columns from (p + q) * 64
+            const int cnt = min(TC_NSTACK, S - p - q);
             const uint64_t bd = tc_desc(sB + (uint32_t)(bb * S + q) * TC_B_TILE);
             const uint32_t d = tmem + (uint32_t)(p + q) * (2 * TC_BN);
+            const uint32_t idesc = tc_idesc(2 * TC_BN * cnt);
 #pragma unroll
             for (int kk = 0; kk < TC_BK / 16; ++kk)
-              tc_mma(d, ad + 2u * kk, bd + 2u * kk, (chunk0 && p == 0 && kk == 0) ? 0u : 1u);
+              tc_mma(d, ad + 2u * kk, bd + 2u * kk, idesc, (chunk0 && p == 0 && kk == 0) ? 0u : 1u);
           }
           tc_commit(bar(EA + slot));  // A slot free once these MMAs have read it
         }
