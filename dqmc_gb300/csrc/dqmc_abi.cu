@@ -83,20 +83,13 @@ struct dqmc_handle {
   LUWork lu{};                // LU of the D-scale separated calculate_greens
   LUPanel lup{};              // blocked LU: pivots and per-step candidate copies
   cplx* lu_L = nullptr;       // (n x n) unit lower factor of the unblocked LU (strict lower part)
-  int* lu_pivrow = nullptr;   // (2) unblocked LU: next pivot row by step parity
   double* lu_scales = nullptr;   // (4n) 1/max(Dl,1), min(Dl,1), 1/max(Dr,1), min(Dr,1)
-  // block sizes of the mixed-form factorisations and the LU panel grid
-  // (DQMC_TUNE="wy=128,trsm=64,lu_grid=64,lu_small=576" overrides; lu_grid 0
-  // = one CTA per SM; n <= lu_small takes the unblocked LU).  Defaults
-  // measured at L=16 on GB300: WY 32/64/128 -> 213/128/102 ms per sweep,
-  // triangular solves 32/64/128 -> 119/97/107 ms, LU panel grid 32/64/152 ->
-  // 186/184/194 ms; LU per sweep blocked/unblocked: n = 144 9.0/5.8 ms,
-  // n = 576 39.8/33.9 ms, n = 1024 184/232 ms.
-  int wy_block = 128, trsm_block = 64, lu_grid = 64, lu_small = 576;
-  // LU panels on one thread-block cluster of this many CTAs (16 or 8; 0: the
-  // cooperative grid of lu_grid CTAs; DQMC_TUNE "lu_cluster=").  The grid is
-  // the default: at n = 1024 both took about 0.3 ms per panel (the cluster's
-  // FP64 work on 16 SMs offsets its cheaper barriers) and 141 ms of LU per sweep
+  // block sizes of the factorisations (DQMC_TUNE="wy=128,trsm=64,lu_small=576"
+  // overrides; n <= lu_small takes the unblocked LU).  Defaults measured at
+  // L=16 on GB300: WY 32/64/128 -> 213/128/102 ms per sweep, triangular solves
+  // 32/64/128 -> 119/97/107 ms
+  int wy_block = 128, trsm_block = 64, lu_small = 576;
+  // CTAs of an LU panel's cluster (DQMC_TUNE "lu_cluster=" 16 or 8; 0: 16 where the device schedules it)
   int lu_cluster = 0;
   cplx* wy_v = nullptr;       // (n x kWyMax) reflector block
   cplx* wy_s = nullptr;       // (kWyMax^2) Vb^H Vb
@@ -504,15 +497,24 @@ int trsm_blocked(dqmc_handle* h, const cplx* T, const cplx* rdiag, cplx* Y, bool
 
 // zgetrf of A (n x n, in place: L strict lower, U upper) in panels of LU_PB
 // columns: panel factorisation with partial pivoting, the panel's row
-// exchanges on the other columns, U12 = L11^-1 A12, A22 -= L21 U12 (a GEMM,
-// split-BF16 in the mixed form).  lu.perm, lu.udiag, lu.rdiag on return.
-// For n <= lu_small the unblocked cooperative LU runs instead (one launch;
-// L then in lu_L).  *Lm receives the matrix whose strict lower part is L.
+// exchanges on the other columns, U12 = L11^-1 A12, A22 -= L21 U12 (a split
+// GEMM).  lu.perm, lu.udiag, lu.rdiag on return.  For n <= lu_small every entry
+// stays in FP64 multiply-adds, column after column (the panels of the same
+// kernel and k_lu_trail; L then in lu_L): at these sizes that costs less than
+// the blocked form's launches.  *Lm receives the matrix whose strict lower
+// part is L.
 int lu_blocked(dqmc_handle* h, cplx* A, const cplx** Lm) {
   const int n = h->n;
+  const int cap = h->lu_cluster > 0 ? h->lu_cluster : h->coop_cap;
   if (n <= h->lu_small) {
-    LUKernel w{h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lu_pivrow, h->qr.bar, h->err_d};
-    LAUNCH(DQMC_K_LU, 8.0 * n3(h) / 3.0, 32.0 * n2(h), launch_lup(A, h->lu_L, n, w, h->sm_count, h->st, h->coop_cap));
+    for (int p0 = 0; p0 < n; p0 += LU_PB) {
+      const int b = n - p0 < LU_PB ? n - p0 : LU_PB;
+      LAUNCH(DQMC_K_LU, 8.0 * (n - p0) * b * b / 2.0, 32.0 * (n - p0) * b,
+             launch_lu_unblocked_panel(A, h->lu_L, n, p0, b, h->lup, cap, h->st));
+      if (n > LU_PB)
+        LAUNCH(DQMC_K_LU, 8.0 * (n - p0 - b) * (n - p0) * b, 32.0 * (n - p0) * n,
+               launch_lu_trail(A, h->lu_L, n, p0, b, h->lup, h->st));
+    }
     *Lm = h->lu_L;
     return DQMC_OK;
   }
@@ -521,10 +523,8 @@ int lu_blocked(dqmc_handle* h, cplx* A, const cplx** Lm) {
   for (int p0 = 0; p0 < n; p0 += LU_PB) {
     const int b = n - p0 < LU_PB ? n - p0 : LU_PB;
     const int m = n - p0 - b;
-    int lu_cap = h->coop_cap;
-    if (h->lu_grid > 0 && (lu_cap == 0 || h->lu_grid < lu_cap)) lu_cap = h->lu_grid;
     LAUNCH(DQMC_K_LU, 8.0 * (n - p0) * b * b / 2.0, 32.0 * (n - p0) * b,
-           launch_lu_panel(A, n, p0, b, h->lup, h->sm_count, h->st, lu_cap, h->lu_cluster));
+           launch_lu_panel(A, n, p0, b, h->lup, cap, h->st));
     LAUNCH(DQMC_K_LU, 0.0, 64.0 * b * n, launch_lu_apply_swaps(A, n, p0, b, h->lup.piv, h->lu.perm, h->st));
     if (m > 0) {
       LAUNCH(DQMC_K_LU, 4.0 * b * b * m, 32.0 * b * m,
@@ -924,7 +924,7 @@ void free_all(dqmc_handle* h) {
                   h->Tr, h->Dl, h->Dr, h->W1, h->W2, h->W3, h->W4, h->D1, h->d2, h->ord1, h->qr.vn1,
                   h->qr.vn2, h->qr.order, h->qr.tau, h->qr.beta, h->qr.V, h->qr.bar, h->qr.cand_v, h->qr.cand_q, h->delta_d, h->unif_d,
                   h->acc_d, h->det_d, h->pacc_d, h->action_d, h->nacc_d, h->Acol, h->Brow, h->bar, h->err_d,
-                  h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wblk, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.cand_rows, h->lup.rowk, h->lu_L, h->lu_pivrow, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
+                  h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wblk, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   clear_graphs(h);
@@ -1250,7 +1250,6 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
     int v = 0;
     if (const char* q = std::strstr(tune, "wy=")) if (std::sscanf(q + 3, "%d", &v) == 1 && v >= 16 && v <= kWyMax) h->wy_block = v;
     if (const char* q = std::strstr(tune, "trsm=")) if (std::sscanf(q + 5, "%d", &v) == 1 && v >= 16 && v <= 128) h->trsm_block = v;
-    if (const char* q = std::strstr(tune, "lu_grid=")) if (std::sscanf(q + 8, "%d", &v) == 1 && v >= 0) h->lu_grid = v;
     if (const char* q = std::strstr(tune, "lu_small=")) if (std::sscanf(q + 9, "%d", &v) == 1 && v >= 0) h->lu_small = v;
     if (const char* q = std::strstr(tune, "lu_cluster=")) if (std::sscanf(q + 11, "%d", &v) == 1 && (v == 0 || v == 8 || v == 16)) h->lu_cluster = v;
   }
@@ -1297,13 +1296,12 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
   A((void**)&h->lu.perm, n * sizeof(int)); A((void**)&h->lu.udiag, n * sizeof(cplx));
   A((void**)&h->lu.rdiag, n * sizeof(cplx));
   A((void**)&h->lu_scales, 4 * n * sizeof(double));
-  A((void**)&h->lu_L, n * n * sizeof(cplx)); A((void**)&h->lu_pivrow, 2 * sizeof(int));
+  A((void**)&h->lu_L, n * n * sizeof(cplx));
   A((void**)&h->lup.piv, n * sizeof(int));
-  A((void**)&h->lup.cand_rows, (size_t)1024 * LU_PB * sizeof(cplx));
-  A((void**)&h->lup.rowk, (size_t)2 * LU_PB * sizeof(cplx));
-  h->lup.cand_v = h->qr.cand_v;
-  h->lup.cand_r = h->qr.cand_q;
-  h->lup.bar = h->qr.bar;
+  A((void**)&h->lup.src, n * sizeof(int));
+  h->lup.perm = h->lu.perm;
+  h->lup.udiag = h->lu.udiag;
+  h->lup.rdiag = h->lu.rdiag;
   h->lup.err = h->err_d;
   h->delay = p->delay > 1 ? p->delay : 16;
   {

@@ -10,7 +10,6 @@
 // factor comes out directly in the un-permuted ("T = R[:, invperm(p)]")
 // layout that the UDT decomposition needs.
 #include <cfloat>
-#include <cooperative_groups.h>
 #include "common.cuh"
 #include "kernels.h"
 
@@ -421,24 +420,6 @@ __global__ void __launch_bounds__(QR_THREADS) k_qrp(cplx* __restrict__ A, int n,
     for (int q = threadIdx.x; q < n; q += blockDim.x) w.order[q] = order[q];
 }
 
-// ---------------------------------------------------------------------------
-// LU pivot search helpers: candidates compared on the bit patterns of the
-// non-negative |Re| + |Im| (first row of maximal value, as izamax)
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ bool piv_better(double v, int r, double bv, int br) {
-  const long long a = __double_as_longlong(v), b = __double_as_longlong(bv);   // v >= 0
-  return a > b || (a == b && r < br);
-}
-
-__device__ __forceinline__ void warp_argmax(double& best, int& row) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int orow = __shfl_xor_sync(0xffffffffu, row, o);
-    if (piv_better(ob, orow, best, row)) { best = ob; row = orow; }
-  }
-}
-
 // Block j of the compact-WY form of Q = H_0 ... H_{n-1}: Vb (m x b, m = n - jb,
 // leading dimension m) = rows jb.. of reflector columns jb..jb+b; a reflector
 // with tau = 0 is the identity and is stored as v = 0 with tau' = 1, so that
@@ -453,490 +434,6 @@ __global__ void k_wy_prep(const cplx* __restrict__ V, const cplx* __restrict__ t
     const bool ident = t.x == 0.0 && t.y == 0.0;
     Vb[e] = ident ? cmake(0.0, 0.0) : V[(size_t)(jb + c) * n + jb + r];
     if (r == 0) trd[c] = ident ? cmake(1.0, 0.0) : t;
-  }
-}
-
-// Unblocked LU with partial pivoting (cooperative, one grid barrier per
-// column step), for small n where the blocked form's launches dominate:
-// P A = L U as LAPACK zgetf2 (pivot: first row of maximal |Re| + |Im|, as
-// izamax), rows exchanged physically in the trailing columns.  Column k of
-// A is read, never written, in step k: the multipliers go to Lb (strictly
-// lower part; earlier columns receive the same row exchanges) and the
-// diagonal of U to udiag, so the CTAs need no ordering among themselves
-// inside a step.  The owner of column k+1 publishes the next pivot row.
-__global__ void __launch_bounds__(QR_THREADS) k_lup(cplx* __restrict__ A, cplx* __restrict__ Lb, int n, LUKernel w) {
-  unsigned bar_epoch = 0;
-  GridBarrierExit bar_exit(w.bar);
-  extern __shared__ double smem_lu[];
-  cplx* v = reinterpret_cast<cplx*>(smem_lu);   // (n) column k after the row exchange (rows > k)
-  int* perm = reinterpret_cast<int*>(v + n);    // (n) position -> original row
-  __shared__ cplx s_rinv;
-  __shared__ int s_piv;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int warps = QR_THREADS / 32;
-  const int scal_warp = warps - 1;
-  for (int q = threadIdx.x; q < n; q += blockDim.x) perm[q] = q;
-  if (blockIdx.x == 0 && wid == 0) {
-    double best = 0.0;
-    int row = n;
-    for (int r = lane; r < n; r += 32) {
-      const cplx x = A[r];
-      const double a = fabs(x.x) + fabs(x.y);
-      if (piv_better(a, r, best, row)) { best = a; row = r; }
-    }
-    warp_argmax(best, row);
-    if (lane == 0) w.pivrow[0] = row < n ? row : 0;
-  }
-  if (!grid_barrier(w.bar, w.err, bar_epoch)) return;
-
-  const int chunk = (n + gridDim.x - 1) / gridDim.x;   // rows of Lb written by this CTA
-  for (int k = 0; k < n; ++k) {
-    if (threadIdx.x == 0) s_piv = __ldcg(&w.pivrow[k & 1]);
-    __syncthreads();
-    const int p = s_piv;
-    const cplx* colk = A + (size_t)k * n;
-    const cplx piv = ldcg_c(&colk[p]);
-    for (int r = k + 1 + threadIdx.x; r < n; r += blockDim.x) v[r] = ldcg_c(&colk[r == p ? k : r]);
-    if (threadIdx.x == 0 && p != k) { const int t = perm[k]; perm[k] = perm[p]; perm[p] = t; }
-    if (wid == scal_warp) {
-      const bool zero = piv.x == 0.0 && piv.y == 0.0;
-      const cplx rinv = zero ? cmake(0.0, 0.0) : cdiv(cmake(1.0, 0.0), piv);
-      if (lane == 0) {
-        s_rinv = rinv;
-        if (blockIdx.x == 0) {
-          w.udiag[k] = piv;
-          w.rdiag[k] = rinv;
-          if (zero) atomicOr(w.err, DQMC_KERR_SINGULAR);
-        }
-      }
-    }
-    // the same row exchange in the multiplier columns formed so far
-    if (p != k)
-      for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < k; j += gridDim.x * blockDim.x) {
-        cplx* lj = Lb + (size_t)j * n;
-        const cplx a = ldcg_c(&lj[k]), b = ldcg_c(&lj[p]);
-        lj[k] = b;
-        lj[p] = a;
-      }
-    __syncthreads();   // v, s_rinv
-    const cplx rinv = s_rinv;
-    {
-      const int r0 = blockIdx.x * chunk, r1 = r0 + chunk < n ? r0 + chunk : n;
-      for (int r = (r0 > k + 1 ? r0 : k + 1) + threadIdx.x; r < r1; r += blockDim.x)
-        Lb[(size_t)k * n + r] = cmul(v[r], rinv);
-    }
-    // ---- trailing columns j > k, dealt round-robin over the CTAs ----
-    const int rem = n - k - 1;
-    const int nq = (rem + 31) >> 5;   // warp-uniform slot count of rows k+1..n-1
-    for (int t = blockIdx.x + gridDim.x * wid; t < rem; t += gridDim.x * warps) {
-      const int j = k + 1 + t;
-      cplx* col = A + (size_t)j * n;
-      const cplx u = ldcg_c(&col[p]), wk = ldcg_c(&col[k]);
-      cplx x[QR_MAXT];
-#pragma unroll
-      for (int q = 0; q < QR_MAXT; ++q) {
-        if (q >= nq) break;
-        const int r = k + 1 + lane + 32 * q;
-        x[q] = r < n ? (r == p ? wk : ldcg_c(&col[r])) : cmake(0.0, 0.0);
-      }
-      const cplx c = cmul(u, rinv);   // a_rj -= (a_rk / piv) u_kj
-      double best = 0.0;
-      int brow = n;
-#pragma unroll
-      for (int q = 0; q < QR_MAXT; ++q) {
-        if (q >= nq) break;
-        const int r = k + 1 + lane + 32 * q;
-        if (r < n) {
-          const cplx vr = v[r];
-          x[q] = cmake(fma(-vr.x, c.x, fma(vr.y, c.y, x[q].x)), fma(-vr.x, c.y, fma(-vr.y, c.x, x[q].y)));
-          col[r] = x[q];
-          if (t == 0) {
-            const double a = fabs(x[q].x) + fabs(x[q].y);
-            if (piv_better(a, r, best, brow)) { best = a; brow = r; }
-          }
-        }
-      }
-      if (lane == 0) col[k] = u;
-      if (t == 0) {   // column k+1: pivot row of the next step
-        warp_argmax(best, brow);
-        if (lane == 0) w.pivrow[(k + 1) & 1] = brow < n ? brow : k + 1;
-      }
-    }
-    if (!grid_barrier(w.bar, w.err, bar_epoch)) return;
-  }
-  if (blockIdx.x == 0)
-    for (int q = threadIdx.x; q < n; q += blockDim.x) w.perm[q] = perm[q];
-}
-
-// ---------------------------------------------------------------------------
-// blocked LU with partial pivoting (zgetrf semantics, in place)
-// ---------------------------------------------------------------------------
-// Panel of LU_PB columns [p0, p0 + b) over rows [p0, n), rows dealt to the CTAs
-// in contiguous chunks.  Per column step the CTAs publish their pivot
-// candidate (|Re| + |Im|, row, and that row's panel values) and the owner of
-// row k publishes row k; after the grid barrier every CTA reads the pivot
-// row (the U row) and row k (which moves to the pivot's place) from those
-// copies, so no CTA reads a row another one is rewriting.
-__global__ void __launch_bounds__(256) k_lu_panel(cplx* __restrict__ A, int n, int p0, int b, LUPanel w) {
-  unsigned bar_epoch = 0;
-  GridBarrierExit bar_exit(w.bar);
-  extern __shared__ double4_16a smem_panel[];
-  cplx* prow = reinterpret_cast<cplx*>(smem_panel);   // (own rows, LU_PB): this CTA's rows of the panel
-  const int rows = n - p0;
-  const int chunk = (rows + gridDim.x - 1) / gridDim.x;
-  const int r0 = p0 + blockIdx.x * chunk;
-  const int r1 = r0 + chunk < n ? r0 + chunk : n;
-  const int nrw = r1 > r0 ? r1 - r0 : 0;
-  __shared__ cplx urow[LU_PB], krow[LU_PB];
-  __shared__ double s_v[8];
-  __shared__ int s_r[8];
-  __shared__ int s_p, s_wc;
-  __shared__ cplx s_rinv;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < nrw * b; e += blockDim.x) {
-    const int rr = e / b, j = e - rr * b;
-    prow[rr * LU_PB + j] = ldcg_c(&A[(size_t)(p0 + j) * n + r0 + rr]);
-  }
-  __syncthreads();
-
-  // candidate of this CTA for panel column jc over its rows >= rlo, published with the row's panel values
-  auto publish_candidate = [&](int jc, int rlo) {
-    double best = 0.0;
-    int brow = n;
-    for (int r = (r0 > rlo ? r0 : rlo) + threadIdx.x; r < r1; r += blockDim.x) {
-      const cplx x = prow[(r - r0) * LU_PB + jc];
-      const double a = fabs(x.x) + fabs(x.y);
-      if (piv_better(a, r, best, brow)) { best = a; brow = r; }
-    }
-    warp_argmax(best, brow);
-    if (lane == 0) { s_v[wid] = best; s_r[wid] = brow; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double bv = s_v[0]; int br = s_r[0];
-      for (int q = 1; q < (int)(blockDim.x >> 5); ++q)
-        if (piv_better(s_v[q], s_r[q], bv, br)) { bv = s_v[q]; br = s_r[q]; }
-      w.cand_v[blockIdx.x] = bv;
-      w.cand_r[blockIdx.x] = br;
-      s_r[0] = br;
-    }
-    __syncthreads();
-    const int br = s_r[0];
-    if (br < n)
-      for (int j = threadIdx.x; j < b; j += blockDim.x)
-        w.cand_rows[(size_t)blockIdx.x * LU_PB + j] = prow[(br - r0) * LU_PB + j];
-  };
-  auto publish_rowk = [&](int k, int slot) {
-    if (r0 <= k && k < r1)
-      for (int j = threadIdx.x; j < b; j += blockDim.x) w.rowk[slot * LU_PB + j] = prow[(k - r0) * LU_PB + j];
-  };
-
-  publish_candidate(0, p0);
-  publish_rowk(p0, 0);
-  if (!grid_barrier(w.bar, w.err, bar_epoch)) return;
-
-  for (int kk = 0; kk < b; ++kk) {
-    const int k = p0 + kk;
-    // ---- pivot: best candidate (first row of maximal |Re| + |Im|) ----
-    if (wid == 0) {
-      // all candidate loads in flight at once (grid <= 32 * CAND_PER_LANE), then the compares
-      double cvv[CAND_PER_LANE];
-      int crr[CAND_PER_LANE];
-#pragma unroll
-      for (int u = 0; u < CAND_PER_LANE; ++u) {
-        const int c = lane + 32 * u;
-        cvv[u] = 0.0;
-        crr[u] = n;
-        if (c < (int)gridDim.x) { cvv[u] = __ldcg(&w.cand_v[c]); crr[u] = __ldcg(&w.cand_r[c]); }
-      }
-      double best = 0.0;
-      int brow = n, bc = 0;
-#pragma unroll
-      for (int u = 0; u < CAND_PER_LANE; ++u)
-        if (piv_better(cvv[u], crr[u], best, brow)) { best = cvv[u]; brow = crr[u]; bc = lane + 32 * u; }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int orow = __shfl_xor_sync(0xffffffffu, brow, o), oc = __shfl_xor_sync(0xffffffffu, bc, o);
-        if (piv_better(ob, orow, best, brow)) { best = ob; brow = orow; bc = oc; }
-      }
-      if (lane == 0) { s_p = brow; s_wc = bc; }
-    }
-    __syncthreads();
-    const bool none = s_p >= n;   // all candidates zero: no exchange, singular pivot
-    const int p = none ? k : s_p;
-    for (int j = threadIdx.x; j < b; j += blockDim.x) {
-      const cplx kv = ldcg_c(&w.rowk[(kk & 1) * LU_PB + j]);
-      krow[j] = kv;
-      urow[j] = none ? kv : ldcg_c(&w.cand_rows[(size_t)s_wc * LU_PB + j]);
-    }
-    __syncthreads();
-    if (wid == 0) {
-      // 1 / pivot = conj(pv) / |pv|^2 (the D-scale separated matrix has no large scales)
-      const cplx pv = urow[kk];
-      const double d2 = pv.x * pv.x + pv.y * pv.y;
-      const bool zero = d2 == 0.0;
-      const double rd = zero ? 0.0 : 1.0 / d2;
-      if (lane == 0) {
-        s_rinv = cmake(pv.x * rd, -pv.y * rd);
-        if (zero) atomicOr(w.err, DQMC_KERR_SINGULAR);
-        if (blockIdx.x == 0) w.piv[k] = p;
-      }
-    }
-    // the exchanged rows: row k <- pivot row (U), row p <- old row k
-    if (r0 <= k && k < r1)
-      for (int j = threadIdx.x; j < b; j += blockDim.x) prow[(k - r0) * LU_PB + j] = urow[j];
-    if (p != k && r0 <= p && p < r1)
-      for (int j = threadIdx.x; j < b; j += blockDim.x) prow[(p - r0) * LU_PB + j] = krow[j];
-    __syncthreads();
-    const cplx rinv = s_rinv;
-    // ---- multipliers of the own rows below k, then the rank-1 update of the panel ----
-    const int ra = r0 > k + 1 ? r0 : k + 1;
-    const int nr = r1 > ra ? r1 - ra : 0;
-    for (int t = threadIdx.x; t < nr; t += blockDim.x) {
-      cplx* e = &prow[(ra + t - r0) * LU_PB + kk];
-      *e = cmul(*e, rinv);
-    }
-    __syncthreads();
-    const int nc = b - kk - 1;
-    for (int t = threadIdx.x; t < nr * nc; t += blockDim.x) {
-      const int rr = t % nr, jj = kk + 1 + t / nr;
-      cplx* rowp = &prow[(ra + rr - r0) * LU_PB];
-      const cplx l = rowp[kk], u = urow[jj], x = rowp[jj];
-      rowp[jj] = cmake(fma(-l.x, u.x, fma(l.y, u.y, x.x)), fma(-l.x, u.y, fma(-l.y, u.x, x.y)));
-    }
-    __syncthreads();
-    if (kk + 1 < b) {
-      publish_candidate(kk + 1, k + 1);
-      publish_rowk(k + 1, (kk + 1) & 1);
-    }
-    if (!grid_barrier(w.bar, w.err, bar_epoch)) return;
-  }
-  for (int e = threadIdx.x; e < nrw * b; e += blockDim.x) {
-    const int rr = e / b, j = e - rr * b;
-    A[(size_t)(p0 + j) * n + r0 + rr] = prow[rr * LU_PB + j];
-  }
-}
-
-// The same panel factorisation on one thread-block cluster of cs CTAs (8 or
-// 16, the rows dealt in contiguous chunks): each CTA keeps its candidate (value,
-// row and the row's panel values) and, when it holds it, the step's row k in
-// its own shared memory, double-buffered by step parity; the others read them
-// through distributed shared memory after one cluster barrier per column, in
-// place of the grid barrier and the round trips through L2.  Every CTA runs
-// the same loop, so every cluster barrier is met by all of them; the last
-// barrier of the loop also keeps each CTA's shared memory alive until the
-// others have read it.
-__global__ void __launch_bounds__(256) k_lu_panel_cluster(cplx* __restrict__ A, int n, int p0, int b, LUPanel w) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  const int cs = (int)cl.num_blocks(), q = (int)cl.block_rank();
-  extern __shared__ double4_16a smem_panel[];
-  cplx* prow = reinterpret_cast<cplx*>(smem_panel);   // (own rows, LU_PB): this CTA's rows of the panel
-  const int rows = n - p0;
-  const int chunk = (rows + cs - 1) / cs;
-  const int r0 = p0 + q * chunk;
-  const int r1 = r0 + chunk < n ? r0 + chunk : n;
-  const int nrw = r1 > r0 ? r1 - r0 : 0;
-  __shared__ cplx urow[LU_PB], krow[LU_PB];
-  __shared__ cplx c_row[2][LU_PB], k_row[2][LU_PB];
-  __shared__ double c_val[2];
-  __shared__ int c_r[2];
-  __shared__ double s_v[8];
-  __shared__ int s_r[8];
-  __shared__ int s_p, s_wc;
-  __shared__ cplx s_rinv;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < nrw * b; e += blockDim.x) {
-    const int rr = e / b, j = e - rr * b;
-    prow[rr * LU_PB + j] = ldcg_c(&A[(size_t)(p0 + j) * n + r0 + rr]);
-  }
-  __syncthreads();
-
-  // candidate of this CTA for panel column jc over its rows >= k (value, row,
-  // row values), and row k itself if this CTA holds it, into buffers par
-  auto publish = [&](int jc, int k, int par) {
-    double best = 0.0;
-    int brow = n;
-    for (int r = (r0 > k ? r0 : k) + threadIdx.x; r < r1; r += blockDim.x) {
-      const cplx x = prow[(r - r0) * LU_PB + jc];
-      const double a = fabs(x.x) + fabs(x.y);
-      if (piv_better(a, r, best, brow)) { best = a; brow = r; }
-    }
-    warp_argmax(best, brow);
-    if (lane == 0) { s_v[wid] = best; s_r[wid] = brow; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double bv = s_v[0]; int br = s_r[0];
-      for (int u = 1; u < (int)(blockDim.x >> 5); ++u)
-        if (piv_better(s_v[u], s_r[u], bv, br)) { bv = s_v[u]; br = s_r[u]; }
-      c_val[par] = bv;
-      c_r[par] = br;
-      s_r[0] = br;
-    }
-    __syncthreads();
-    const int br = s_r[0];
-    if (br < n)
-      for (int j = threadIdx.x; j < b; j += blockDim.x) c_row[par][j] = prow[(br - r0) * LU_PB + j];
-    if (r0 <= k && k < r1)
-      for (int j = threadIdx.x; j < b; j += blockDim.x) k_row[par][j] = prow[(k - r0) * LU_PB + j];
-  };
-
-  publish(0, p0, 0);
-  cl.sync();
-
-  for (int kk = 0; kk < b; ++kk) {
-    const int k = p0 + kk, par = kk & 1;
-    // ---- pivot: best of the cs candidates (first row of maximal |Re| + |Im|) ----
-    if (wid == 0) {
-      double best = 0.0;
-      int brow = n, bc = 0;
-      if (lane < cs) {
-        best = *cl.map_shared_rank(&c_val[par], lane);
-        brow = *cl.map_shared_rank(&c_r[par], lane);
-        bc = lane;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        const int orow = __shfl_xor_sync(0xffffffffu, brow, o), oc = __shfl_xor_sync(0xffffffffu, bc, o);
-        if (piv_better(ob, orow, best, brow)) { best = ob; brow = orow; bc = oc; }
-      }
-      if (lane == 0) { s_p = brow; s_wc = bc; }
-    }
-    __syncthreads();
-    const bool none = s_p >= n;   // all candidates zero: no exchange, singular pivot
-    const int p = none ? k : s_p;
-    {
-      const cplx* kr = cl.map_shared_rank(&k_row[par][0], (unsigned)((k - p0) / chunk));
-      const cplx* ur = cl.map_shared_rank(&c_row[par][0], (unsigned)s_wc);
-      for (int j = threadIdx.x; j < b; j += blockDim.x) {
-        const cplx kv = kr[j];
-        krow[j] = kv;
-        urow[j] = none ? kv : ur[j];
-      }
-    }
-    __syncthreads();
-    if (wid == 0) {
-      // 1 / pivot = conj(pv) / |pv|^2 (the D-scale separated matrix has no large scales)
-      const cplx pv = urow[kk];
-      const double d2 = pv.x * pv.x + pv.y * pv.y;
-      const bool zero = d2 == 0.0;
-      const double rd = zero ? 0.0 : 1.0 / d2;
-      if (lane == 0) {
-        s_rinv = cmake(pv.x * rd, -pv.y * rd);
-        if (zero) atomicOr(w.err, DQMC_KERR_SINGULAR);
-        if (q == 0) w.piv[k] = p;
-      }
-    }
-    // the exchanged rows: row k <- pivot row (U), row p <- old row k
-    if (r0 <= k && k < r1)
-      for (int j = threadIdx.x; j < b; j += blockDim.x) prow[(k - r0) * LU_PB + j] = urow[j];
-    if (p != k && r0 <= p && p < r1)
-      for (int j = threadIdx.x; j < b; j += blockDim.x) prow[(p - r0) * LU_PB + j] = krow[j];
-    __syncthreads();
-    const cplx rinv = s_rinv;
-    // ---- multipliers of the own rows below k, then the rank-1 update of the panel ----
-    const int ra = r0 > k + 1 ? r0 : k + 1;
-    const int nr = r1 > ra ? r1 - ra : 0;
-    for (int t = threadIdx.x; t < nr; t += blockDim.x) {
-      cplx* e = &prow[(ra + t - r0) * LU_PB + kk];
-      *e = cmul(*e, rinv);
-    }
-    __syncthreads();
-    const int nc = b - kk - 1;
-    for (int t = threadIdx.x; t < nr * nc; t += blockDim.x) {
-      const int rr = t % nr, jj = kk + 1 + t / nr;
-      cplx* rowp = &prow[(ra + rr - r0) * LU_PB];
-      const cplx l = rowp[kk], u = urow[jj], x = rowp[jj];
-      rowp[jj] = cmake(fma(-l.x, u.x, fma(l.y, u.y, x.x)), fma(-l.x, u.y, fma(-l.y, u.x, x.y)));
-    }
-    __syncthreads();
-    if (kk + 1 < b) publish(kk + 1, k + 1, (kk + 1) & 1);
-    cl.sync();
-  }
-  for (int e = threadIdx.x; e < nrw * b; e += blockDim.x) {
-    const int rr = e / b, j = e - rr * b;
-    A[(size_t)(p0 + j) * n + r0 + rr] = prow[rr * LU_PB + j];
-  }
-}
-
-// Row exchanges of one panel applied to the columns outside it, and to the
-// running permutation: the b exchanges (k, piv[k]) touch at most 2b rows,
-// whose net permutation warp 0 works out (panel rows indexed directly, rows
-// below the panel found by a ballot over the ones met so far); every column
-// is then gathered over those rows.
-__global__ void k_lu_apply_swaps(cplx* __restrict__ A, int n, int p0, int b, const int* __restrict__ piv,
-                                 int* __restrict__ perm) {
-  __shared__ int rowof[2 * LU_PB], src[2 * LU_PB], spiv[LU_PB];
-  __shared__ int s_cnt;
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    for (int s2 = lane; s2 < b; s2 += 32) {
-      rowof[s2] = p0 + s2;
-      src[s2] = p0 + s2;
-      spiv[s2] = piv[p0 + s2];
-    }
-    __syncwarp();
-    int cnt = b;
-    for (int kk = 0; kk < b; ++kk) {
-      const int k = p0 + kk, pr = spiv[kk];
-      if (pr == k) continue;   // warp-uniform
-      int sp = -1;
-      if (pr < p0 + b) {
-        sp = pr - p0;
-      } else {
-        for (int base = b; base < cnt && sp < 0; base += 32) {
-          const int s2 = base + lane;
-          const unsigned hit = __ballot_sync(0xffffffffu, s2 < cnt && rowof[s2] == pr);
-          if (hit) sp = base + __ffs(hit) - 1;
-        }
-        if (sp < 0) {
-          sp = cnt++;
-          if (lane == 0) { rowof[sp] = pr; src[sp] = pr; }
-        }
-      }
-      __syncwarp();
-      if (lane == 0) { const int t = src[kk]; src[kk] = src[sp]; src[sp] = t; }
-      __syncwarp();
-    }
-    if (lane == 0) s_cnt = cnt;
-  }
-  __syncthreads();
-  const int cnt = s_cnt;
-  // permutation (block 0): perm[rowof[s]] <- old perm[src[s]]
-  if (blockIdx.x == 0) {
-    __shared__ int pv[2 * LU_PB];
-    for (int s2 = threadIdx.x; s2 < cnt; s2 += blockDim.x) pv[s2] = perm[src[s2]];
-    __syncthreads();
-    for (int s2 = threadIdx.x; s2 < cnt; s2 += blockDim.x) perm[rowof[s2]] = pv[s2];
-  }
-  // columns outside the panel, one warp per column
-  const int lane = threadIdx.x & 31;
-  const int nw = blockDim.x >> 5;
-  for (int c = blockIdx.x * nw + (threadIdx.x >> 5); c < n; c += gridDim.x * nw) {
-    if (c >= p0 && c < p0 + b) continue;
-    cplx* col = A + (size_t)c * n;
-    cplx v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int s2 = lane + 32 * q;
-      if (s2 < cnt) v[q] = ldcg_c(&col[src[s2]]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int s2 = lane + 32 * q;
-      if (s2 < cnt) col[rowof[s2]] = v[q];
-    }
-  }
-}
-
-// udiag = diag(U) of the in-place LU, rdiag = 1 / udiag
-__global__ void k_lu_diag(const cplx* __restrict__ A, int n, cplx* __restrict__ udiag, cplx* __restrict__ rdiag) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const cplx d = A[(size_t)i * n + i];
-    udiag[i] = d;
-    rdiag[i] = (d.x == 0.0 && d.y == 0.0) ? cmake(0.0, 0.0) : cdiv(cmake(1.0, 0.0), d);
   }
 }
 
@@ -1374,101 +871,6 @@ cudaError_t launch_trsm_diag_block(const cplx* T, int ldT, const cplx* rdiag, cp
 cudaError_t launch_wy_prep(const cplx* V, const cplx* tau, int n, int jb, int b, cplx* Vb, cplx* trd,
                            cudaStream_t st) {
   k_wy_prep<<<grid_for((size_t)(n - jb) * b), 256, 0, st>>>(V, tau, n, jb, b, Vb, trd);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_lup(cplx* A, cplx* Lb, int n, LUKernel& w, int sm_count, cudaStream_t st, int max_grid) {
-  if (n > 32 * QR_MAXT) return cudaErrorInvalidValue;
-  size_t smem = (size_t)n * (sizeof(cplx) + sizeof(int));
-  static SmemLimit smem_limit;
-  if (cudaError_t ea = smem_limit.raise((const void*)k_lup, 64 * 1024); ea != cudaSuccess) return ea;
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lup, QR_THREADS, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  int grid = sm_count;
-  if (max_grid > 0 && grid > max_grid) grid = max_grid;
-  LUKernel copy = w;
-  void* args[] = {&A, &Lb, &n, &copy};
-  return cudaLaunchCooperativeKernel((void*)k_lup, dim3(grid), dim3(QR_THREADS), args, smem, st);
-}
-
-// One cluster of cs CTAs (16, else 8 when 16 cannot be scheduled); returns
-// cudaErrorNotSupported, with nothing launched, when neither fits.
-static cudaError_t launch_lu_panel_cluster(cplx* A, int n, int p0, int b, LUPanel& w, int cs, cudaStream_t st) {
-  constexpr size_t kMax = 160 * 1024;
-  static SmemLimit smem_limit;
-  static bool nonportable_set[64] = {};
-  int dev = 0;
-  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
-  if (cudaError_t ea = smem_limit.raise((const void*)k_lu_panel_cluster, (int)kMax); ea != cudaSuccess) return ea;
-  if (dev >= 0 && dev < 64 && !nonportable_set[dev]) {
-    if (cudaError_t e = cudaFuncSetAttribute((const void*)k_lu_panel_cluster,
-                                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        e != cudaSuccess)
-      return e;
-    nonportable_set[dev] = true;
-  }
-  for (int c = cs; c >= 8; c /= 2) {
-    const int chunk = (n - p0 + c - 1) / c;
-    const size_t smem = (size_t)chunk * LU_PB * sizeof(cplx);
-    if (smem > kMax) return cudaErrorNotSupported;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(c);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = c;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, (const void*)k_lu_panel_cluster, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      clusters = 0;
-    }
-    if (clusters < 1) continue;
-    return cudaLaunchKernelEx(&cfg, k_lu_panel_cluster, A, n, p0, b, w);
-  }
-  return cudaErrorNotSupported;
-}
-
-cudaError_t launch_lu_panel(cplx* A, int n, int p0, int b, LUPanel& w, int sm_count, cudaStream_t st, int max_grid,
-                            int cluster) {
-  if (b < 1 || b > LU_PB) return cudaErrorInvalidValue;
-  if (cluster >= 8) {
-    const cudaError_t e = launch_lu_panel_cluster(A, n, p0, b, w, cluster, st);
-    if (e != cudaErrorNotSupported) return e;
-  }
-  int grid = sm_count;
-  if (max_grid > 0 && grid > max_grid) grid = max_grid;
-  if (grid > n - p0) grid = n - p0;
-  if (grid > 32 * CAND_PER_LANE) grid = 32 * CAND_PER_LANE;
-  const int chunk = (n - p0 + grid - 1) / grid;
-  const size_t smem = (size_t)chunk * LU_PB * sizeof(cplx);
-  constexpr size_t kMax = 160 * 1024;
-  if (smem > kMax) return cudaErrorInvalidValue;   // grid too small for the panel rows
-  static SmemLimit smem_limit;
-  if (cudaError_t ea = smem_limit.raise((const void*)k_lu_panel, (int)kMax); ea != cudaSuccess) return ea;
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lu_panel, 256, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  LUPanel copy = w;
-  void* args[] = {&A, &n, &p0, &b, &copy};
-  return cudaLaunchCooperativeKernel((void*)k_lu_panel, dim3(grid), dim3(256), args, smem, st);
-}
-
-cudaError_t launch_lu_apply_swaps(cplx* A, int n, int p0, int b, const int* piv, int* perm, cudaStream_t st) {
-  k_lu_apply_swaps<<<(n + 7) / 8, 256, 0, st>>>(A, n, p0, b, piv, perm);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_lu_diag(const cplx* A, int n, cplx* udiag, cplx* rdiag, cudaStream_t st) {
-  k_lu_diag<<<(n + 255) / 256, 256, 0, st>>>(A, n, udiag, rdiag);
   return cudaGetLastError();
 }
 

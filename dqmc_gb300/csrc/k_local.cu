@@ -24,6 +24,7 @@
 // i of this call; unif[i] decides only when p_acc <= 1, exactly as
 // `p_acc > 1.0 || rand() < p_acc`.
 #include <cooperative_groups.h>
+#include "cluster.cuh"
 #include "common.cuh"
 #include "kernels.h"
 #include "oz_slice.cuh"
@@ -499,26 +500,6 @@ __device__ __forceinline__ double win_adj(const cplx* m, const cplx* mn, int lan
 // its step, and a slot of K = M^-1 Delta holds this NaN (which no arithmetic
 // produces) until its 8-byte words arrive.
 constexpr unsigned long long kWinEmpty = 0x7FF8DEADBEEF0001ull;
-__device__ __forceinline__ void st_cluster(void* p, unsigned long long v) {   // p: generic address of cluster shared memory
-  asm volatile("st.relaxed.cluster.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ void st_cluster(int* p, int v) {
-  asm volatile("st.relaxed.cluster.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-// polls of words in this CTA's own shared memory
-__device__ __forceinline__ int ld_poll(const int* p) {
-  int v;
-  asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
-  return v;
-}
-// Release and acquire at cluster scope for shared memory only (a full
-// fence.acq_rel.cluster took 950 cycles).
-__device__ __forceinline__ void fence_release_shared() {
-  asm volatile("fence.release.sync_restrict::shared::cta.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void fence_acquire_shared() {
-  asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory");
-}
 // 1 / x by Newton's iteration from a single-precision seed (2^-23, 2^-46,
 // then FP64 round-off): four dependent FMAs where the division takes twice
 // that; outside the single-precision range the division.
@@ -538,7 +519,6 @@ __device__ __forceinline__ bool less_fast(double a, double b) {
 }
 __device__ __forceinline__ bool finite_bits(double x) { return ((__double2hiint(x) >> 20) & 0x7FF) != 0x7FF; }
 __device__ __forceinline__ bool zero_bits(double x) { return (__double_as_longlong(x) << 1) == 0; }
-constexpr int kWinPolls = 1 << 22;   // bound of every wait on another CTA (about 0.1 s)
 
 __device__ __forceinline__ void named_bar(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -713,7 +693,7 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
       // the first accepted candidate in site order (the same in every CTA) once
       // all candidates are published; -2: gave up waiting
       int acc3 = -2;
-      for (int it = 0; it < kWinPolls; ++it) {
+      for (int it = 0; it < kClusterPolls; ++it) {
         int v = (step + 1) << 1;
         if (lane < ncand) v = ld_poll(&s_pub[par][(cur + lane) % C]);
         if (__all_sync(0xffffffffu, v >> 1 == step + 1)) {
@@ -731,6 +711,9 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
       ok = false;
       break;
     }
+    // orders warp 1's K words before this CTA's next decision (about 950 cycles,
+    // beside the reads of the accepted site's rows)
+    if (wid == 3) fence_cluster();
     const int last = acc >= 0 ? acc : cur + ncand - 1;   // sites cur .. last are decided
     if (sc <= last && wid == 3 && lane == 0) {
       const int gi = first + sc, flag = s_flag[par];
@@ -778,7 +761,7 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
         gv = reinterpret_cast<const double*>(Gs + (size_t)(4 * t0 + r) * LD + 4 * s0 + c)[part];
         const cplx* k = s_k[kslot][owner];
         bool here = false;
-        for (int it = 0; it < kWinPolls && !here; ++it) {
+        for (int it = 0; it < kClusterPolls && !here; ++it) {
           const int w0 = ld_poll(reinterpret_cast<const int*>(k) + 2 * lane);
           const int w1 = ld_poll(reinterpret_cast<const int*>(k) + 2 * lane + 1);
           here = __all_sync(0xffffffffu, w0 != (int)(kWinEmpty & 0xffffffffu) || w1 != (int)(kWinEmpty >> 32));

@@ -145,34 +145,26 @@ struct LUWork {
   cplx* udiag;       // (n) diagonal of U
   cplx* rdiag;       // (n) 1 / diagonal of U
 };
-// Unblocked cooperative LU (small n): U in A's strict upper part, L in Lb's strict lower part.
-struct LUKernel {
-  int* perm;
-  cplx* udiag;
-  cplx* rdiag;
-  int* pivrow;       // (2) pivot row of the next step, by step parity
-  GridBarrier* bar;
-  int* err;
-};
-cudaError_t launch_lup(cplx* A, cplx* Lb, int n, LUKernel& w, int sm_count, cudaStream_t st, int max_grid = 0);
 // compact-WY block jb..jb+b of the reflectors in V/tau: Vb ((n-jb) x b), trd (b) (tau, 1 for identity reflectors)
 cudaError_t launch_wy_prep(const cplx* V, const cplx* tau, int n, int jb, int b, cplx* Vb, cplx* trd,
                            cudaStream_t st);
-// Blocked LU (in place): panel factorisation of columns [p0, p0+b) (b <= LU_PB) over rows [p0, n)
+// LU panels of LU_PB columns on one cluster (k_lu.cu)
 constexpr int LU_PB = 64;
 struct LUPanel {
-  int* piv;            // (n) pivot row of each step
-  double* cand_v;      // (grid) per-CTA pivot candidates: |Re| + |Im|
-  int* cand_r;         // (grid) and row
-  cplx* cand_rows;     // (grid, LU_PB) the candidate rows' panel values
-  cplx* rowk;          // (2, LU_PB) row k of the step, by step parity
-  GridBarrier* bar;
+  int* piv;            // (n) blocked form: pivot position of each step
+  int* src;            // (n) unblocked form: row order of the panel, position -> row (both from p0)
+  int* perm;           // (n) unblocked form: running permutation, row perm[i] of A is row i of P A
+  cplx* udiag;         // (n) unblocked form: diagonal of U and its reciprocals
+  cplx* rdiag;
   int* err;
 };
-// cluster >= 8: the panel on one thread-block cluster of that many CTAs (16 or
-// 8; the cooperative grid when no cluster can be scheduled); 0: the grid
-cudaError_t launch_lu_panel(cplx* A, int n, int p0, int b, LUPanel& w, int sm_count, cudaStream_t st,
-                            int max_grid = 0, int cluster = 0);
+// blocked form, in place: panel [p0, p0+b) over rows [p0, n); max_cluster > 0: at most that many CTAs (>= 8)
+cudaError_t launch_lu_panel(cplx* A, int n, int p0, int b, const LUPanel& w, int max_cluster, cudaStream_t st);
+// unblocked form: U in A's strict upper part, L in Lb's strict lower part after
+// every panel and its trailing update (zgetf2 arithmetic, column by column)
+cudaError_t launch_lu_unblocked_panel(cplx* A, cplx* Lb, int n, int p0, int b, const LUPanel& w, int max_cluster,
+                                      cudaStream_t st);
+cudaError_t launch_lu_trail(cplx* A, cplx* Lb, int n, int p0, int b, const LUPanel& w, cudaStream_t st);
 // the panel's row exchanges applied to the columns outside [p0, p0+b) and to perm
 cudaError_t launch_lu_apply_swaps(cplx* A, int n, int p0, int b, const int* piv, int* perm, cudaStream_t st);
 cudaError_t launch_lu_diag(const cplx* A, int n, cplx* udiag, cplx* rdiag, cudaStream_t st);
