@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
         const int ps = pos[r0 + rr];
         if (ps < kk) continue;
         const cplx x = prow[rr * LU_LDP + kk];
-        const double a = fabs(x.x) + fabs(x.y);
+        double a = fabs(x.x) + fabs(x.y);
+        if (ps == kk && __double2hiint(a) < 0) a = 0.0;   // NaN: no candidate, but some row always is
         const int c = ps << 16 | (r0 + rr);
         if (piv_better(a, c, best, pk)) { best = a; pk = c; }
       }

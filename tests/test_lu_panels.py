@@ -37,3 +37,36 @@ def test_greens_of_udts(L, cluster, monkeypatch):
     assert np.max(np.abs(G - want)) < tol * max(1.0, np.max(np.abs(want)))
     assert abs(ld - ldw) < tol * n
     chain.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [4, 6, 14])
+def test_nan_leaves_the_chain_usable(L):
+    # a NaN is no pivot: it travels to the result, and the next call is as ever
+    from dqmc_gb300 import api
+    chain = api.DQMC(api.ModelParams(L=L, slices=10, safe_mult=10))
+    n = 4 * L * L
+    rng = np.random.default_rng(L)
+    udts = _udt(n, rng, 3.0) + _udt(n, rng, 2.0)
+    good, _ = chain.calculate_greens_udt(*udts)
+    for fill in (np.nan, -np.nan):
+        bad = [x.copy() for x in udts]
+        bad[0][:, n // 2] = fill
+        try:
+            G, _ = chain.calculate_greens_udt(*bad)
+            assert np.isnan(G).any()
+        except api.DQMCError:
+            pass
+        again, _ = chain.calculate_greens_udt(*udts)
+        assert np.array_equal(again, good)
+        A = np.array(udts[0])
+        u, d, t = chain.decompose_udt(A)
+        A[:, n // 3] = fill
+        try:
+            u1, d1, t1 = chain.decompose_udt(A)
+            assert np.isnan(u1).any() or np.isnan(d1).any() or np.isnan(t1).any()
+        except api.DQMCError:
+            pass
+        for x, y in zip(chain.decompose_udt(np.array(udts[0])), (u, d, t)):
+            assert np.array_equal(x, y)
+    chain.close()
