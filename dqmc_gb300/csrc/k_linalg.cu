@@ -116,6 +116,8 @@ __device__ double block_sum(double v, double* scratch) {
 // column-pivoted QR (cooperative, one grid barrier per column step)
 // ---------------------------------------------------------------------------
 constexpr int QR_THREADS = 256;
+constexpr int QR_WARPS = QR_THREADS / 32;              // the last one is the reflector warp
+constexpr int QR_REFL_WORDS = 10;                      // beta, tau, scal in 32-bit halves under the step's tag
 constexpr int QR_MAXT = 32;   // elements per lane of one column (n <= 1024)
 constexpr int CAND_PER_LANE = 8;   // per-CTA pivot candidates read per lane: grids of at most 256 CTAs
 
@@ -246,175 +248,258 @@ __device__ __forceinline__ double qr_finish_column(cplx (&x)[QR_MAXT], cplx* __r
   return vn1_new;
 }
 
-__global__ void __launch_bounds__(QR_THREADS) k_qrp(cplx* __restrict__ A, int n, QRWork w) {
-  unsigned bar_epoch = 0;
+// Column step k: the pivot column p (the first of maximal partial norm) gives the
+// reflector; every other column is updated and its norm downdated, one warp per
+// column, the remaining columns dealt round-robin over the CTAs.  One grid
+// barrier per step.  The reflector's scalars are a chain of a square root and two
+// divisions (about 5000 cycles with the norm), which every CTA runs ahead of time
+// for its own candidate while the grid barrier is under way, on its last warp
+// (which takes columns only once the others all have one).  The chosen one's
+// owner has published them by the time the others have read the column and
+// formed their first dot products.  Bound: FP64 issue while more than a few
+// hundred columns remain, then the latency of barrier, pivot column and norm
+// downdate.  Per sequence of calls, ms, formed after the barrier -> ahead:
+// n = 64 1.70 -> 1.53, 144 8.0 -> 7.4, 256 14.9 -> 14.4, 1024 52.6 -> 51.8.
+__global__ void __launch_bounds__(QR_THREADS, 1) k_qrp(cplx* __restrict__ A, int n, QRWork w) {
+  unsigned epoch = 0;
   GridBarrierExit bar_exit(w.bar);
   extern __shared__ double smem_qr[];
   cplx* v = reinterpret_cast<cplx*>(smem_qr);         // (n) pivot column: a_k at k, unscaled x below
   int* order = reinterpret_cast<int*>(v + n);         // (n) logical -> physical
-  __shared__ double red[32];
-  __shared__ int redi[32];
-  __shared__ double nsum[32];
+  __shared__ double red[QR_WARPS], nsum[QR_WARPS];
+  __shared__ int redi[QR_WARPS], redj[QR_WARPS];
   __shared__ cplx s_tau, s_scal;
+  __shared__ int s_ok, s_wc, s_rok;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int warps = QR_THREADS / 32;
-  const int scal_warp = warps - 1;   // holds no column while rem < (warps - 1) * grid
+  constexpr int warps = QR_WARPS, CT = 32 * (QR_WARPS - 1);   // CT: threads of the other warps
+  const bool refl_warp = wid == warps - 1;
   const int gwarp = blockIdx.x * warps + wid, nwarps = gridDim.x * warps;
   const double tol3z = sqrt(DBL_EPSILON);
 
   for (int q = threadIdx.x; q < n; q += blockDim.x) order[q] = q;
   // initial column norms (zgeqp3: vn1 = vn2 = ||A(:, j)||) and the first candidates
-  double cb = 0.0;
-  int cq = n;
+  double cbest = 0.0;
+  int cbq = n, cbj = 0;
   for (int j = gwarp; j < n; j += nwarps) {
     double s = 0.0;
     for (int r = lane; r < n; r += 32) s += cabs2(A[(size_t)j * n + r]);
     s = warp_sum(s);
     const double nv = sqrt(s), iv = nv > 0.0 ? 1.0 / nv : 0.0;
     if (lane == 0) { w.vn1[j] = nv; w.vn2[j] = nv; w.vn1[n + j] = iv; w.vn2[n + j] = iv; }
-    if (cand_better(nv, j, cb, cq)) { cb = nv; cq = j; }
+    if (cand_better(nv, j, cbest, cbq)) { cbest = nv; cbq = j; cbj = j; }
   }
-  if (lane == 0) { red[wid] = cb; redi[wid] = cq; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = red[0]; int bq = redi[0];
-    for (int q = 1; q < warps; ++q)
-      if (cand_better(red[q], redi[q], b, bq)) { b = red[q]; bq = redi[q]; }
-    w.cand_v[blockIdx.x] = b;
-    w.cand_q[blockIdx.x] = bq;
-  }
-  if (!grid_barrier(w.bar, w.err, bar_epoch)) return;
+  for (int e = threadIdx.x; e < 2 * QR_REFL_WORDS; e += blockDim.x)   // this CTA's reflector slots are empty
+    w.refl[((size_t)(e / QR_REFL_WORDS) * gridDim.x + blockIdx.x) * QR_REFL_WORDS + e % QR_REFL_WORDS] = 0ull;
 
   const int chunk = (n + gridDim.x - 1) / gridDim.x;   // rows of V written by this CTA
   for (int k = 0; k < n; ++k) {
     const int rem = n - k - 1;
     const int nq = (n - k + 31) >> 5;   // warp-uniform: no FP64 work on fully masked slots
     const int t_first = blockIdx.x + gridDim.x * wid;
-    // the first column of this warp, read while the pivot is chosen; if the
-    // pivot exchange moves another column to its position, it is read again
+    const int par = k & 1;
+    // ---- this CTA's candidate of step k (lane 0 of each warp holds its best) ----
+    if (lane == 0) { red[wid] = cbest; redi[wid] = cbq; redj[wid] = cbj; }
+    __syncthreads();   // the columns of step k - 1 are stored
+    double cb = red[0];
+    int cq = redi[0], cj = redj[0];
+#pragma unroll
+    for (int q = 1; q < warps; ++q)
+      if (cand_better(red[q], redi[q], cb, cq)) { cb = red[q]; cq = redi[q]; cj = redj[q]; }
+    ++epoch;
+    if (wid == 0) {
+      // ---- arrive at the grid barrier with the candidate, wait, choose the pivot ----
+      int ok = 1;
+      if (lane == 0) {
+        w.cand_v[par * gridDim.x + blockIdx.x] = cb;
+        w.cand_q[par * gridDim.x + blockIdx.x] = cq;
+        __threadfence();
+        atomicAdd(&w.bar->count, 1u);
+        long long spins = 0;
+        while (ld_acquire_u32(&w.bar->count) < epoch * gridDim.x) {
+          if ((++spins & 1023) == 0) {
+            if (spins > (1ll << 26)) { atomicOr(w.err, 2); ok = 0; break; }
+            if (*(volatile int*)w.err & 2) { ok = 0; break; }
+          }
+        }
+        __threadfence();
+        s_ok = ok;
+      }
+      __syncwarp();
+    } else if (cq < n) {
+      // ---- the reflector of this CTA's candidate (zlarfg): partial squared norms
+      //      of its column below row k, summed as 8 warps with rows 256 apart per
+      //      thread; the reflector warp takes the first warp's share as well ----
+      cplx x0 = cmake(0.0, 0.0);
+      for (int wp = refl_warp ? 0 : wid; wp < warps; wp += refl_warp ? warps - 1 : warps) {
+        double xn2 = 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int r = k + 32 * wp + lane + u * QR_THREADS;
+          if (r < n) {
+            const cplx x = ldcg_c(&A[(size_t)cj * n + r]);
+            if (u == 0 && wp == 0) x0 = x;
+            if (r > k) xn2 = fma(x.x, x.x, fma(x.y, x.y, xn2));
+          }
+        }
+        xn2 = warp_sum(xn2);
+        if (lane == 0) nsum[wp] = xn2;
+      }
+      __syncwarp();
+      if (!refl_warp) {
+        asm volatile("bar.arrive 1, 224;" ::: "memory");
+      } else {
+        asm volatile("bar.sync 1, 224;" ::: "memory");
+        double t = lane < warps ? nsum[lane] : 0.0;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);   // warps <= 8
+        const cplx alpha = cmake(__shfl_sync(0xffffffffu, x0.x, 0), __shfl_sync(0xffffffffu, x0.y, 0));
+        t = __shfl_sync(0xffffffffu, t, 0);
+        double beta;
+        cplx tau, scal;
+        if (t == 0.0 && alpha.y == 0.0) {
+          tau = cmake(0.0, 0.0);
+          beta = alpha.x;
+          scal = cmake(0.0, 0.0);
+        } else {
+          const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + t);
+          beta = alpha.x >= 0.0 ? -nrm : nrm;
+          const double rb = 1.0 / beta;
+          tau = cmake((beta - alpha.x) * rb, -alpha.y * rb);
+          // scal = 1 / (alpha - beta), formed on (alpha - beta) / nrm (modulus in [1, 2])
+          const double an = fabs(rb);
+          const cplx dd = cmake((alpha.x - beta) * an, alpha.y * an);
+          const double rd = an / (dd.x * dd.x + dd.y * dd.y);
+          scal = cmake(dd.x * rd, -dd.y * rd);
+        }
+        // words of 32 bits under the step's tag validate themselves
+        if (lane < QR_REFL_WORDS) {
+          const int c = lane >> 1;
+          const double val = c == 0 ? beta : c == 1 ? tau.x : c == 2 ? tau.y : c == 3 ? scal.x : scal.y;
+          const unsigned half = lane & 1 ? (unsigned)__double2loint(val) : (unsigned)__double2hiint(val);
+          unsigned long long* o = w.refl + ((size_t)par * gridDim.x + blockIdx.x) * QR_REFL_WORDS + lane;
+          asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(o), "l"((unsigned long long)(k + 1) << 32 | half)
+                       : "memory");
+        }
+      }
+    }
+    // ---- column warps: the barrier is passed; first columns read while the pivot
+    //      is chosen (read again if the exchange moves another column there) ----
     cplx x[QR_MAXT];
     int j_pre = -1;
-    if (t_first < rem && wid != scal_warp) {
-      j_pre = order[k + 1 + t_first];
-      qr_load(x, A + (size_t)j_pre * n, k, n, nq, lane);
-    }
-    // ---- pivot: best of the per-CTA candidates (first position of maximal norm), warp 0 ----
-    if (wid == 0) {
-      // all candidate loads in flight at once (grid <= 32 * CAND_PER_LANE), then the compares
-      double cvv[CAND_PER_LANE];
-      int cqq[CAND_PER_LANE];
+    if (!refl_warp) {
+      asm volatile("bar.sync 2, 224;" ::: "memory");
+      if (s_ok) {
+        if (t_first < rem) {
+          j_pre = order[k + 1 + t_first];
+          qr_load(x, A + (size_t)j_pre * n, k, n, nq, lane);
+        }
+        // best of the per-CTA candidates (first position of maximal norm), warp 0
+        if (wid == 0) {
+          // all candidate loads in flight at once (grid <= 32 * CAND_PER_LANE), then the compares
+          double cvv[CAND_PER_LANE];
+          int cqq[CAND_PER_LANE];
 #pragma unroll
-      for (int u = 0; u < CAND_PER_LANE; ++u) {
-        const int c = lane + 32 * u;
-        cvv[u] = 0.0;
-        cqq[u] = n;
-        if (c < (int)gridDim.x) { cvv[u] = __ldcg(&w.cand_v[c]); cqq[u] = __ldcg(&w.cand_q[c]); }
-      }
-      double best = 0.0;
-      int bestq = n;
+          for (int u = 0; u < CAND_PER_LANE; ++u) {
+            const int c = lane + 32 * u;
+            cvv[u] = 0.0;
+            cqq[u] = n;
+            if (c < (int)gridDim.x) {
+              cvv[u] = __ldcg(&w.cand_v[par * gridDim.x + c]);
+              cqq[u] = __ldcg(&w.cand_q[par * gridDim.x + c]);
+            }
+          }
+          double best = 0.0;
+          int bestq = n, bc = 0;
 #pragma unroll
-      for (int u = 0; u < CAND_PER_LANE; ++u)
-        if (cand_better(cvv[u], cqq[u], best, bestq)) { best = cvv[u]; bestq = cqq[u]; }
+          for (int u = 0; u < CAND_PER_LANE; ++u)
+            if (cand_better(cvv[u], cqq[u], best, bestq)) { best = cvv[u]; bestq = cqq[u]; bc = lane + 32 * u; }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        double ob = __shfl_xor_sync(0xffffffffu, best, o);
-        int oq = __shfl_xor_sync(0xffffffffu, bestq, o);
-        if (cand_better(ob, oq, best, bestq)) { best = ob; bestq = oq; }
-      }
-      if (lane == 0) {
-        if (bestq < k || bestq >= n) bestq = k;   // no candidate: keep the order
-        int t = order[k]; order[k] = order[bestq]; order[bestq] = t;
+          for (int o = 16; o > 0; o >>= 1) {
+            double ob = __shfl_xor_sync(0xffffffffu, best, o);
+            int oq = __shfl_xor_sync(0xffffffffu, bestq, o), oc = __shfl_xor_sync(0xffffffffu, bc, o);
+            if (cand_better(ob, oq, best, bestq)) { best = ob; bestq = oq; bc = oc; }
+          }
+          if (lane == 0) {
+            const bool none = bestq < k || bestq >= n;   // NaN in every remaining column: keep the order
+            s_wc = none ? -1 : bc;
+            if (none) bestq = k;
+            int t = order[k]; order[k] = order[bestq]; order[bestq] = t;
+          }
+          __syncwarp();
+        }
       }
     }
     __syncthreads();
-    const int p = order[k];
-    // ---- reflector from A[k:n, p] (zlarfg): partial squared norms, 4 loads per thread at n <= 1024 ----
-    double xn2 = 0.0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int r = k + threadIdx.x + u * QR_THREADS;
-      if (r < n) {
-        cplx x = ldcg_c(&A[(size_t)p * n + r]);
-        v[r] = x;
-        if (r > k) xn2 = fma(x.x, x.x, fma(x.y, x.y, xn2));
-      }
-    }
-    xn2 = warp_sum(xn2);
-    if (lane == 0) nsum[wid] = xn2;
-    __syncthreads();
-    // ---- one warp forms beta, tau and the reflector scale while the others
-    //      start the dot products of their first column (which need neither) ----
-    if (wid == scal_warp) {
-      double t = lane < warps ? nsum[lane] : 0.0;
-#pragma unroll
-      for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);   // warps <= 8
-      const cplx alpha = v[k];
-      double beta;
-      cplx tau, scal;
-      if (t == 0.0 && alpha.y == 0.0) {
-        tau = cmake(0.0, 0.0);
-        beta = alpha.x;
-        scal = cmake(0.0, 0.0);
-      } else {
-        const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + t);
-        beta = alpha.x >= 0.0 ? -nrm : nrm;
-        const double rb = 1.0 / beta;
-        tau = cmake((beta - alpha.x) * rb, -alpha.y * rb);
-        // scal = 1 / (alpha - beta), formed on (alpha - beta) / nrm (modulus in [1, 2])
-        const double an = fabs(rb);
-        const cplx dd = cmake((alpha.x - beta) * an, alpha.y * an);
-        const double rd = an / (dd.x * dd.x + dd.y * dd.y);
-        scal = cmake(dd.x * rd, -dd.y * rd);
-      }
-      if (lane == 0) {
-        s_tau = tau;
-        s_scal = scal;
-        if (blockIdx.x == 0) { w.tau[k] = tau; w.beta[k] = beta; }
-      }
-    }
-    // ---- apply H_k^H to the remaining columns, downdate their norms ----
-    // remaining logical positions k+1..n-1 are dealt round-robin over the CTAs
-    // first, so every SM keeps an equal share of the columns as k grows
-    double cbest = 0.0;
-    int cbq = n;
+    if (!s_ok) return;
+    // ---- the reflector warp fetches the chosen reflector; the column warps read
+    //      the pivot column and form their first dot products (which need neither) ----
     cplx s_first = cmake(0.0, 0.0);
     int j_first = -1;
-    if (t_first < rem && wid != scal_warp) {
-      j_first = order[k + 1 + t_first];
-      if (j_first != j_pre) qr_load(x, A + (size_t)j_first * n, k, n, nq, lane);
-      s_first = qr_dot(x, v, k, n, nq, lane);
+    if (refl_warp) {
+      const int wc = s_wc;
+      const unsigned long long* src = w.refl + ((size_t)par * gridDim.x + max(wc, 0)) * QR_REFL_WORDS + lane;
+      unsigned long long word = 0x7FF8000000000000ull >> (lane & 1 ? 0 : 32);   // halves of a NaN: the reflector of NaN columns
+      bool here = wc < 0;
+      for (long long spins = 0; !here && spins < (1ll << 22); ++spins) {
+        if (lane < QR_REFL_WORDS)
+          asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(word) : "l"(src) : "memory");
+        here = __all_sync(0xffffffffu, lane >= QR_REFL_WORDS || (unsigned)(word >> 32) == (unsigned)(k + 1));
+      }
+      if (!here && lane == 0) atomicOr(w.err, 2);
+      double f[5];
+#pragma unroll
+      for (int c = 0; c < 5; ++c)
+        f[c] = __hiloint2double((int)__shfl_sync(0xffffffffu, (unsigned)word, 2 * c),
+                                (int)__shfl_sync(0xffffffffu, (unsigned)word, 2 * c + 1));
+      if (lane == 0) {
+        s_tau = cmake(f[1], f[2]);
+        s_scal = cmake(f[3], f[4]);
+        s_rok = here ? 1 : 0;
+        if (blockIdx.x == 0) { w.tau[k] = cmake(f[1], f[2]); w.beta[k] = f[0]; }
+      }
+    } else {
+      const int p = order[k];
+#pragma unroll
+      for (int u = 0; u < 5; ++u) {   // n <= 1024 < 5 CT
+        const int r = k + threadIdx.x + u * CT;
+        if (r < n) v[r] = ldcg_c(&A[(size_t)p * n + r]);
+      }
+      asm volatile("bar.sync 2, 224;" ::: "memory");
+      if (t_first < rem) {
+        j_first = order[k + 1 + t_first];
+        if (j_first != j_pre) qr_load(x, A + (size_t)j_first * n, k, n, nq, lane);
+        s_first = qr_dot(x, v, k, n, nq, lane);
+      }
     }
     __syncthreads();   // tau, scal visible
+    if (!s_rok) return;
     const cplx ctau = cconj(s_tau), scal = s_scal;
+    cbest = 0.0;
+    cbq = n;
+    cbj = 0;
     // rows of V written by this CTA: v = (1, scal x_{k+1..n}), zero above k
     for (int r = blockIdx.x * chunk + threadIdx.x; r < n && r < (blockIdx.x + 1) * chunk; r += blockDim.x)
       w.V[(size_t)k * n + r] = r < k ? cmake(0.0, 0.0) : (r == k ? cmake(1.0, 0.0) : cmul(v[r], scal));
+    // ---- apply H_k^H to the remaining columns, downdate their norms ----
+    // remaining logical positions k+1..n-1 are dealt round-robin over the CTAs
+    // first, so every SM keeps an equal share of the columns as k grows
     if (j_first >= 0) {
       const double nv = qr_finish_column(x, A + (size_t)j_first * n, v, k, n, nq, lane, j_first, s_first, ctau, scal,
                                          w, tol3z);
-      if (lane == 0 && cand_better(nv, k + 1 + t_first, cbest, cbq)) { cbest = nv; cbq = k + 1 + t_first; }
+      if (lane == 0 && cand_better(nv, k + 1 + t_first, cbest, cbq)) {
+        cbest = nv; cbq = k + 1 + t_first; cbj = j_first;
+      }
     }
-    // further columns of this warp (more columns than warps), and the scal
+    // further columns of this warp (more columns than warps), and the reflector
     // warp's share when it has one
-    for (int t = (wid == scal_warp ? t_first : t_first + gridDim.x * warps); t < rem; t += gridDim.x * warps) {
+    for (int t = refl_warp ? t_first : t_first + gridDim.x * warps; t < rem; t += gridDim.x * warps) {
       const int qpos = k + 1 + t;
       const int j = order[qpos];
       cplx* col = A + (size_t)j * n;
       const cplx s0 = qr_load_dot(x, col, v, k, n, nq, lane);
       const double nv = qr_finish_column(x, col, v, k, n, nq, lane, j, s0, ctau, scal, w, tol3z);
-      if (lane == 0 && cand_better(nv, qpos, cbest, cbq)) { cbest = nv; cbq = qpos; }
+      if (lane == 0 && cand_better(nv, qpos, cbest, cbq)) { cbest = nv; cbq = qpos; cbj = j; }
     }
-    // this CTA's candidate for the next pivot (lane 0 of each warp holds its best)
-    if (lane == 0) { red[wid] = cbest; redi[wid] = cbq; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double b = red[0]; int bq = redi[0];
-      for (int q = 1; q < warps; ++q)
-        if (cand_better(red[q], redi[q], b, bq)) { b = red[q]; bq = redi[q]; }
-      w.cand_v[blockIdx.x] = b;
-      w.cand_q[blockIdx.x] = bq;
-    }
-    if (!grid_barrier(w.bar, w.err, bar_epoch)) return;
   }
   if (blockIdx.x == 0)
     for (int q = threadIdx.x; q < n; q += blockDim.x) w.order[q] = order[q];

@@ -110,8 +110,9 @@ struct QRWork {
   cplx* tau;         // (n)
   double* beta;      // (n) real diagonal of R in logical order
   cplx* V;           // (n, n) Householder vectors, column k = v_k (v_k[k] = 1, zero above)
-  double* cand_v;    // (grid) per-CTA pivot candidates: norm
-  int* cand_q;       // (grid) and logical position
+  double* cand_v;    // (2 grid) per-CTA pivot candidates, by step parity: norm
+  int* cand_q;       // (2 grid) and logical position
+  unsigned long long* refl;   // (2 grid, 10) and their reflectors
   GridBarrier* bar;
   int* err;
 };
