@@ -241,7 +241,8 @@ __global__ void k_oz_finalize(OzArgs a) {
 // ---------------------------------------------------------------------------
 // tcgen05 engine: TMA-staged slices, tensor-core MMAs into TMEM accumulators
 // ---------------------------------------------------------------------------
-// A CTA computes 128 x 32 complex tiles of C, persistently: one CTA per SM
+// A CTA computes 128 x BN complex tiles of C (BN = 32, 16 or 8; the figures below
+// are for 32), persistently: one CTA per SM
 // takes tiles x, x + grid, ... and the MMAs of a tile run while the epilogue
 // of the previous one converts and stores.  Each MMA is
 // M = 128, K = 16 (kind::f16, BF16 in, FP32 out), N = 64 per B slice: the
@@ -265,15 +266,14 @@ __global__ void k_oz_finalize(OzArgs a) {
 // Every wait is bounded; on a timeout the kernel sets an error bit, drains
 // what it issued (bounded) and frees its TMEM.
 constexpr int TC_BM = 128;                      // rows of C per CTA (TMEM lanes)
-constexpr int TC_BN = 32;                       // complex columns of C per CTA (MMA N = 64)
+constexpr int TC_BN = 32;                       // complex columns of C per tile, at most (BN of the kernel: 32, 16 or 8)
 constexpr int TC_BK = 64;                       // BF16 per K block: one 128-byte swizzle row
 constexpr int TC_MAXS = 8;                      // S groups x 64 TMEM columns <= 512
 constexpr int TC_ARING = 6;                     // A-slice stages (S <= 6: one K block of A in flight)
-constexpr int TC_EPI_WARPS = 16;                // epilogue warps 2-17: four per TMEM lane quarter, 8 columns each
+constexpr int TC_EPI_WARPS = 16;                // epilogue warps 2-17: four per TMEM lane quarter, BN / 4 columns each
 constexpr int TC_THREADS = 32 * (2 + TC_EPI_WARPS);   // warp 0 TMA, warp 1 MMA (and TMEM allocation)
 constexpr int TC_A_TILE = TC_BM * TC_BK * 2;    // 16 KB
-constexpr int TC_B_HALF = TC_BN * TC_BK * 2;    // 4 KB: 32 rows of B'_re or of B'_im
-constexpr int TC_B_TILE = 2 * TC_B_HALF;        // 8 KB
+__host__ __device__ constexpr int tc_b_half(int bn) { return bn * TC_BK * 2; }   // 4 KB at BN = 32: BN rows of B'_re or of B'_im
 // MMA instruction descriptor (kind::f16): D F32 (bits 4-5 = 1), A BF16 (bits
 // 7-9 = 1), B BF16 (bits 10-12 = 1), both K-major (bits 15, 16 = 0),
 // N >> 3 at bits 17-22, M >> 4 at bits 24-28.
@@ -282,17 +282,17 @@ __host__ __device__ constexpr uint32_t tc_idesc(int n) {
 }
 // B slices of one MMA.  For a fixed A slice p the pairs (p, q), q = 0, 1, ...
 // write adjacent groups of 64 TMEM columns, and the B slices' tiles of 64 rows
-// are adjacent in shared memory, so up to 4 of them are one MMA of N = 256: the
+// are adjacent in shared memory, so up to 4 of them (at BN = 32) are one MMA of N = 256: the
 // tensor core then reads A (4 KB per K step) once for them.  At N = 64 the 6 KB
 // of operands per MMA took 48 cycles of shared-memory bandwidth for 32 of
 // arithmetic.
-constexpr int TC_NSTACK = 4;
+__host__ __device__ constexpr int tc_nstack(int bn) { return 128 / bn; }
 
-__host__ __device__ constexpr size_t tc_smem_bytes(int S) {
-  return 1024 + (size_t)2 * S * TC_B_TILE + (size_t)TC_ARING * TC_A_TILE + 256;
+__host__ __device__ constexpr size_t tc_smem_bytes(int S, int bn) {
+  return 1024 + (size_t)4 * S * tc_b_half(bn) + (size_t)TC_ARING * TC_A_TILE + 256;
 }
-__host__ __device__ constexpr uint32_t tc_tmem_cols(int S) {
-  return S <= 2 ? 128u : (S <= 4 ? 256u : 512u);
+__host__ __device__ constexpr uint32_t tc_tmem_cols(int S, int bn) {   // S groups of 2 bn columns, a power of two
+  return S * bn <= 16 ? 32u : (S * bn <= 32 ? 64u : (S * bn <= 64 ? 128u : (S * bn <= 128 ? 256u : 512u)));
 }
 
 // Shared-memory matrix descriptor of a K-major operand tile written by TMA
@@ -371,13 +371,23 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-// 32 TMEM lanes (this warp's quarter) x 8 consecutive 32-bit columns; the
+// 32 TMEM lanes (this warp's quarter) x W consecutive 32-bit columns; the
 // registers are valid after tc_wait_ld
-__device__ __forceinline__ void tc_ld8(uint32_t taddr, uint32_t* r) {
+template <int W>
+__device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&r)[W]) {
+  static_assert(W == 2 || W == 4 || W == 8, "widths used by the epilogue");
+  if constexpr (W == 2) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr));
+  } else if constexpr (W == 4) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+  } else {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
       : "r"(taddr));
+  }
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -385,16 +395,17 @@ struct TcMaps {
   CUtensorMap a, bre, bim;   // (Kp, rows, S) BF16 slices, box (64, 128 | 32, 1), 128-byte swizzle
 };
 
-template <bool WIDE, int BITS>   // BITS: slice width, 0 = a.bits
+template <bool WIDE, int BITS, int BN>   // BITS: slice width, 0 = a.bits
 __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_constant__ TcMaps maps, OzArgs a,
                                                              int* err) {
+  constexpr int TC_B_HALF = tc_b_half(BN), TC_B_TILE = 2 * TC_B_HALF, NSTACK = tc_nstack(BN), CPW = BN / 4, PC = CPW < 4 ? CPW : 4;
   if (a.active && *a.active == 0) return;   // flush with nothing pending (uniform over the grid)
   extern __shared__ uint8_t tc_smem_raw[];
   const uint32_t raw = smem_u32(tc_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* basep = tc_smem_raw + (base - raw);
   const int S = a.S;
-  const uint32_t sB = base;                                     // [2][S] B tiles of 8 KB
+  const uint32_t sB = base;                                     // [2][S] B tiles
   const uint32_t sA = base + 2u * S * TC_B_TILE;                // [TC_ARING] A tiles of 16 KB
   const uint32_t sBar = sA + TC_ARING * TC_A_TILE;              // barriers
   uint64_t* bars = reinterpret_cast<uint64_t*>(basep + (sBar - base));
@@ -407,7 +418,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // output tiles, taken persistently: CTA x handles tiles x, x + gridDim.x, ...
   // (tile t: row block t / tiles_x, column block t % tiles_x)
-  const int tiles_x = (a.n + TC_BN - 1) / TC_BN;
+  const int tiles_x = (a.n + BN - 1) / BN;
   const int ntiles = tiles_x * ((a.m + TC_BM - 1) / TC_BM);
   const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   const int nkb_all = (a.Kp + TC_BK - 1) / TC_BK;
@@ -418,9 +429,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
   auto tile_of = [&](int tt, int& i0, int& j0) {
     const int t = (int)blockIdx.x + tt * (int)gridDim.x;
     i0 = (t / tiles_x) * TC_BM;
-    j0 = (t % tiles_x) * TC_BN;
+    j0 = (t % tiles_x) * BN;
   };
-  const uint32_t ncols = tc_tmem_cols(S);
+  const uint32_t ncols = tc_tmem_cols(S, BN);
 
   if (threadIdx.x == 0) {
     for (int k = 0; k < 2; ++k) { mbar_init(bar(k), 1); mbar_init(bar(2 + k), 1); }
@@ -506,12 +517,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
           if (!mbar_wait(bar(FA + slot), (a_use / TC_ARING) & 1, err, s_abort)) { ok = false; break; }
           tc_fence_after();
           const uint64_t ad = tc_desc(sA + (uint32_t)slot * TC_A_TILE);
-          for (int q = 0; q + p < S; q += TC_NSTACK) {
+          for (int q = 0; q + p < S; q += NSTACK) {
             // pairs (p + 1, q + 1 ..) belong to groups t = p + q + 2 ..: accumulator columns from (p + q) * 64
-            const int cnt = min(TC_NSTACK, S - p - q);
+            const int cnt = min(NSTACK, S - p - q);
             const uint64_t bd = tc_desc(sB + (uint32_t)(bb * S + q) * TC_B_TILE);
-            const uint32_t d = tmem + (uint32_t)(p + q) * (2 * TC_BN);
-            const uint32_t idesc = tc_idesc(2 * TC_BN * cnt);
+            const uint32_t d = tmem + (uint32_t)(p + q) * (2 * BN);
+            const uint32_t idesc = tc_idesc(2 * BN * cnt);
 #pragma unroll
             for (int kk = 0; kk < TC_BK / 16; ++kk)
               tc_mma(d, ad + 2u * kk, bd + 2u * kk, idesc, (chunk0 && p == 0 && kk == 0) ? 0u : 1u);
@@ -529,11 +540,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
     }
   } else if (U > 0) {
     // ---- epilogue: warps 2-17, four per TMEM lane quarter (warp % 4); warp w
-    //      takes the 8 columns of group (w - 2) / 4 of each tile, chunk by chunk
+    //      takes the CPW columns of group (w - 2) / 4 of each tile, chunk by chunk
     //      (chunks after the first are added to the C the same thread stored) ----
     const int quarter = warp & 3;
     const int cg = (warp - 2) >> 2;
-    const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(8 * cg);
+    const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(CPW * cg);
     const int bits = BITS ? BITS : a.bits;
     const int sh = oz_wide_shift(bits), e0 = -bits * (S + 1);
     const int ghi = WIDE ? S - oz_wide_groups() : S;   // groups of the (high) word
@@ -543,7 +554,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
     for (int vt = 0; vt < my_tiles * nch; ++vt) {
       int i0, j0;
       tile_of(vt / nch, i0, j0);
-      j0 += 8 * cg;
+      j0 += CPW * cg;
       const bool first = vt % nch == 0;
       const int row = i0 + 32 * quarter + lane;
       const bool waited = mbar_wait(bar(ACC), vt & 1, err, s_abort);
@@ -552,19 +563,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
       if (!have) break;
       __syncwarp();
       tc_fence_after();
-      long long ar[8], ai[8], lr[WIDE ? 8 : 1], li[WIDE ? 8 : 1];
+      long long ar[CPW], ai[CPW], lr[WIDE ? CPW : 1], li[WIDE ? CPW : 1];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) { ar[c] = 0; ai[c] = 0; }
+      for (int c = 0; c < CPW; ++c) { ar[c] = 0; ai[c] = 0; }
 #pragma unroll
-      for (int c = 0; c < (WIDE ? 8 : 1); ++c) { lr[c] = 0; li[c] = 0; }
+      for (int c = 0; c < (WIDE ? CPW : 1); ++c) { lr[c] = 0; li[c] = 0; }
 #pragma unroll 1
       for (int g = 0; g < ghi; ++g) {
-        uint32_t ur[8], ui[8];
-        tc_ld8(tq + (uint32_t)(g * 2 * TC_BN), ur);
-        tc_ld8(tq + (uint32_t)(g * 2 * TC_BN + TC_BN), ui);
+        uint32_t ur[CPW], ui[CPW];
+        tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN), ur);
+        tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN + BN), ui);
         tc_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < CPW; ++c) {
           ar[c] = (ar[c] << bits) + (long long)__float2int_rn(__uint_as_float(ur[c]));
           ai[c] = (ai[c] << bits) + (long long)__float2int_rn(__uint_as_float(ui[c]));
         }
@@ -572,12 +583,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
       if constexpr (WIDE) {
 #pragma unroll 1
         for (int g = ghi; g < S; ++g) {
-          uint32_t ur[8], ui[8];
-          tc_ld8(tq + (uint32_t)(g * 2 * TC_BN), ur);
-          tc_ld8(tq + (uint32_t)(g * 2 * TC_BN + TC_BN), ui);
+          uint32_t ur[CPW], ui[CPW];
+          tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN), ur);
+          tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN + BN), ui);
           tc_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
+          for (int c = 0; c < CPW; ++c) {
             lr[c] = (lr[c] << bits) + (long long)__float2int_rn(__uint_as_float(ur[c]));
             li[c] = (li[c] << bits) + (long long)__float2int_rn(__uint_as_float(ui[c]));
           }
@@ -590,7 +601,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
       if (row >= a.m) continue;
       if (a.acc) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < CPW; ++c) {
           if (j0 + c >= a.n) continue;
           unsigned long long* qa = a.acc + (WIDE ? 4 : 2) * ((size_t)(j0 + c) * a.m + row);
           atomicAdd(qa, (unsigned long long)ar[c]);
@@ -610,16 +621,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
       // integer rounded once with that exponent on the integer units (GB300
       // issues FP64 at a small fraction of its integer rate); the FP64
       // operations left are the extra scalings and the addition of the old C.
-      // Two passes of 4 columns, the loads (scales, old C) of a pass issued
-      // before its first store.
+      // Passes of 4 columns (2 at BN = 8), the loads (scales, old C) of a pass
+      // issued before its first store.
       const int e_row = oz_expo(a.sA[row]) + e0;
 #pragma unroll
-      for (int hh = 0; hh < 8; hh += 4) {
-        cplx cold[4];
-        int e_col[4];
+      for (int hh = 0; hh < CPW; hh += PC) {
+        cplx cold[PC];
+        int e_col[PC];
         bool window = true;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < PC; ++c) {
           const int col = j0 + hh + c;
           const bool in = col < a.n;
           cold[c] = rd && in ? a.C[(size_t)col * a.ldc + row] : cmake(0.0, 0.0);
@@ -628,7 +639,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
         }
         if (window && simple) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < PC; ++c) {
             if (j0 + hh + c >= a.n) continue;
             cplx v = cmake(oz_value<WIDE>(ar[hh + c], lr[WIDE ? hh + c : 0], sh, e_col[c], true),
                            oz_value<WIDE>(ai[hh + c], li[WIDE ? hh + c : 0], sh, e_col[c], true));
@@ -638,7 +649,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
           }
         } else {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < PC; ++c) {
             const int col = j0 + hh + c;
             if (col >= a.n) continue;
             cplx v = cmake(oz_value<WIDE>(ar[hh + c], lr[WIDE ? hh + c : 0], sh, e_col[c], window),
@@ -761,6 +772,34 @@ static bool encode_slices(CUtensorMap* map, const __nv_bfloat16* base, size_t Kp
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int BN>
+static cudaError_t launch_tc(int which, dim3 grid, int S, cudaStream_t st, const TcMaps& maps, const OzArgs& a,
+                             int* err) {
+  static SmemLimit limits[6];
+  void (*const kernels_tc[6])(TcMaps, OzArgs, int*) = {k_oz_gemm_tc<false, 5, BN>, k_oz_gemm_tc<false, 6, BN>,
+                                                       k_oz_gemm_tc<false, 7, BN>, k_oz_gemm_tc<false, 0, BN>,
+                                                       k_oz_gemm_tc<true, 7, BN>,  k_oz_gemm_tc<true, 0, BN>};
+  if (cudaError_t e = limits[which].raise((const void*)kernels_tc[which], (int)tc_smem_bytes(TC_MAXS, BN));
+      e != cudaSuccess)
+    return e;
+  kernels_tc[which]<<<grid, TC_THREADS, tc_smem_bytes(S, BN), st>>>(maps, a, err);
+  return cudaSuccess;
+}
+
+// Complex columns BN of a tile: as narrow as keeps all tiles (times the layers of
+// split K) in one wave.  A tile's time is 3 us until its first MMA, the MMAs and
+// 8 us of epilogue at BN = 32, and the last two shrink with BN; A, in
+// exchange, is read by more CTAs, which a long K does not repay beyond one wave.
+// Flush of 16 sites, us, BN = 32 / 16 / 8: n = 256 23 / 19 / 17, n = 400 (56 bits)
+// 27 / 22 / 24, n = 576 20 / 19 / 21, n = 1024 31 / 34 / 44; product of n = 256
+// 35 / 31 / 39, of n = 576 105 / 131 / 178.
+static int tc_width(int m, int nn, int layers, int ksteps, int sms) {
+  const int rows = (m + TC_BM - 1) / TC_BM, most = ksteps <= 4 ? sms + sms / 4 : sms;
+  for (int bn = 8; bn < TC_BN; bn *= 2)
+    if (rows * ((nn + bn - 1) / bn) * layers <= most) return bn;
+  return TC_BN;
+}
+
 cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                                const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rowscale,
                                const double* colscale, int S, int bits, void* scratch, size_t scratch_bytes,
@@ -795,35 +834,33 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
   // tiles x, x + grid, ... and overlaps a tile's epilogue with the next tile's
   // MMAs; otherwise one CTA per tile (chains sharing the GPU: short CTAs let
   // the other chains' kernels in between)
-  const int ntiles = ((nn + TC_BN - 1) / TC_BN) * ((m + TC_BM - 1) / TC_BM);
   const int sms = sm_count_of_current_device();
-  dim3 grid(persistent && ntiles > sms ? sms : ntiles);
   const int ksteps = (int)((Kp + TC_BK - 1) / TC_BK);
+  int layers = 1;
   if (splitk > 1 && !active && ksteps > 1 && acc &&
       (size_t)m * nn * (wide ? 4 : 2) * sizeof(unsigned long long) <= acc_bytes) {
     // split K over blockIdx.z: exact 64-bit integer partial sums in acc, which
     // is zero between products (zeroed at allocation, re-zeroed by the finaliser)
     if (splitk > ksteps) splitk = ksteps;
     a.kchunk = (ksteps + splitk - 1) / splitk;
-    grid.z = (ksteps + a.kchunk - 1) / a.kchunk;
+    layers = (ksteps + a.kchunk - 1) / a.kchunk;
     a.acc = acc;
   }
+  const int bn = persistent ? tc_width(m, nn, layers, ksteps, sms) : TC_BN;
+  const int ntiles = ((nn + bn - 1) / bn) * ((m + TC_BM - 1) / TC_BM);
+  const dim3 grid(persistent && ntiles > sms ? sms : ntiles, 1, layers);
   if (kernels) *kernels = (a.acc ? 3 : 2) - (presliced ? 1 : 0);
   {
     TcMaps maps;
-    if (!encode_slices(&maps.a, sl.As, Kp, m, S, TC_BM) || !encode_slices(&maps.bre, sl.Bre, Kp, nn, S, TC_BN) ||
-        !encode_slices(&maps.bim, sl.Bim, Kp, nn, S, TC_BN))
+    if (!encode_slices(&maps.a, sl.As, Kp, m, S, TC_BM) || !encode_slices(&maps.bre, sl.Bre, Kp, nn, S, bn) ||
+        !encode_slices(&maps.bim, sl.Bim, Kp, nn, S, bn))
       return cudaErrorInvalidValue;
     // the widths of the default targets are compiled in: 5, 6, 7 (40 bits, by K), 7 in two words (56 bits)
-    static SmemLimit limits[6];
     const int which = wide ? (bits == 7 ? 4 : 5) : bits == 5 ? 0 : bits == 6 ? 1 : bits == 7 ? 2 : 3;
-    void (*const kernels_tc[6])(TcMaps, OzArgs, int*) = {k_oz_gemm_tc<false, 5>, k_oz_gemm_tc<false, 6>,
-                                                         k_oz_gemm_tc<false, 7>, k_oz_gemm_tc<false, 0>,
-                                                         k_oz_gemm_tc<true, 7>,  k_oz_gemm_tc<true, 0>};
-    if (cudaError_t e = limits[which].raise((const void*)kernels_tc[which], (int)tc_smem_bytes(TC_MAXS));
-        e != cudaSuccess)
-      return e;
-    kernels_tc[which]<<<grid, TC_THREADS, tc_smem_bytes(S), st>>>(maps, a, err);
+    const cudaError_t e = bn == 32 ? launch_tc<32>(which, grid, S, st, maps, a, err)
+                        : bn == 16 ? launch_tc<16>(which, grid, S, st, maps, a, err)
+                                   : launch_tc<8>(which, grid, S, st, maps, a, err);
+    if (e != cudaSuccess) return e;
   }
   if (a.acc) {
     const size_t total = (size_t)m * nn;

@@ -152,3 +152,21 @@ def test_nan_and_inf_reach_the_product():
         want[:, 140] = False
         assert np.array_equal(ok, want)
     chain.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,bits", [(2, 0), (2, 56), (4, 0), (4, 56), (6, 0), (6, 48), (8, 0), (10, 0), (12, 0)])
+def test_tile_width_keeps_the_bits(L, bits):
+    # tiles of 8 (n <= 144), 16 (n = 256, with split K) and 32 columns: sums are
+    # exact, so the product is that of the 32 columns which chains in flight take
+    from dqmc_gb300 import api
+    n = 4 * L * L
+    rng = np.random.default_rng(L)
+    A, B = _matrix("rows", n, rng), _matrix("plain", n, rng)
+    got = []
+    for inflight in (0, 8):
+        chain = api.DQMC(api.ModelParams(L=L, slices=10, safe_mult=10, precision="mixed", ozaki_bits=bits,
+                                         inflight=inflight))
+        got.append(chain.gemm_check(A, B, 1))
+        chain.close()
+    assert np.array_equal(got[0], got[1])
