@@ -76,8 +76,10 @@ struct dqmc_handle {
   int* dstate = nullptr;
   SitePrep* prep = nullptr;   // (N) per-site constants of the slice being updated
   int* wsite = nullptr;       // (WIN_MAX) accepted sites of the window
-  cplx* wk = nullptr;         // (WIN_MAX, 16) and (WIN_MAX, WIN_MAX, 16): their blocks (DelayedArgs)
-  cplx* wblk = nullptr;
+  cplx* wk = nullptr;         // (WIN_MAX, 16) and (WIN_MAX, 4, 4 WIN_MAX): their blocks and rows (DelayedArgs)
+  cplx* wrow = nullptr;
+  int* wflag = nullptr;       // (WIN_MAX + 1) published acceptances, (1) followers' arrivals
+  bool follow = false;        // the windows' factors are formed by follower clusters of the same launch
   double* wexp = nullptr;     // (WIN_MAX) and their exp(-dS)
   int greens_method = DQMC_GREENS_SCALES;
   LUWork lu{};                // LU of the D-scale separated calculate_greens
@@ -882,18 +884,20 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
   a.err = h->err_d;
   a.mc = h->mc;
   const int n = h->n, k = h->delay;
-  DelayedArgs d{h->Xd, h->Yd, h->dstate, k, h->prep, h->wsite, h->wk, h->wexp, h->wblk, {}};
+  DelayedArgs d{h->Xd, h->Yd, h->dstate, k, h->prep, h->wsite, h->wk, h->wexp, h->wrow, h->wflag, h->wflag + WIN_MAX + 1, {}};
   // the factor kernel cuts the flush's slices
   int S = 0, bits = 0;
   const bool presliced = oz_plan(h, 4 * k, &S, &bits) && ozaki_scratch_bytes(n, n, 4 * k, S) <= h->oz_bytes;
   if (presliced) d.sl = ozaki_slices(h->oz_scratch, n, n, 4 * k, S, bits);
-  LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_prepare(a, h->prep, h->dstate, h->st));
+  LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_prepare(a, h->prep, h->dstate, h->wflag, h->st));
   // a round consumes a whole window of sites or k acceptances
   const int w = local_window_sites(k);
   const int rounds = (h->N + w - 1) / w + 1;
   auto round = [&]() -> int {
-    LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_window(a, d, h->st, h->coop_cap));
-    LAUNCH(DQMC_K_FLUSH, 0.0, 0.0, launch_local_factors(a, d, h->st));
+    // followers only where the chain has the GPU to itself
+    const bool follow = h->follow && h->coop_cap == 0;
+    LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_window(a, d, h->st, h->coop_cap, follow));
+    if (!follow) LAUNCH(DQMC_K_FLUSH, 0.0, 0.0, launch_local_factors(a, d, h->st));
     // flush G += X Y over the 4p new columns (p read on the device; no work when p = 0)
     return zgemm_general(h, n, n, 4 * k, 'N', 'T', cmake(1, 0), h->Xd, n, h->Yd, n, cmake(1, 0), h->G, n, nullptr,
                          nullptr, true, DQMC_K_FLUSH, h->dstate + 1, presliced);
@@ -924,7 +928,7 @@ void free_all(dqmc_handle* h) {
                   h->Tr, h->Dl, h->Dr, h->W1, h->W2, h->W3, h->W4, h->D1, h->d2, h->ord1, h->qr.vn1,
                   h->qr.vn2, h->qr.order, h->qr.tau, h->qr.beta, h->qr.V, h->qr.bar, h->qr.cand_v, h->qr.cand_q, h->qr.refl, h->delta_d, h->unif_d,
                   h->acc_d, h->det_d, h->pacc_d, h->action_d, h->nacc_d, h->Acol, h->Brow, h->bar, h->err_d,
-                  h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wblk, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
+                  h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wrow, h->wflag, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   clear_graphs(h);
@@ -1313,7 +1317,9 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
     A((void**)&h->wsite, WIN_MAX * sizeof(int));
     A((void**)&h->wk, (size_t)WIN_MAX * 16 * sizeof(cplx));
     A((void**)&h->wexp, WIN_MAX * sizeof(double));
-    A((void**)&h->wblk, (size_t)WIN_MAX * WIN_MAX * 16 * sizeof(cplx));
+    A((void**)&h->wrow, (size_t)WIN_MAX * 16 * WIN_MAX * sizeof(cplx));
+    A((void**)&h->wflag, (WIN_MAX + 2) * sizeof(int));
+    if (ok) h->follow = local_window_follows((int)n, h->delay);
   }
   A((void**)&h->wy_v, (size_t)n * kWyMax * sizeof(cplx));
   A((void**)&h->wy_s, (size_t)kWyMax * kWyMax * sizeof(cplx));

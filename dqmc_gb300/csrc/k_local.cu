@@ -23,6 +23,7 @@
 // Proposal streams use fixed slots: delta[:, i] and unif[i] belong to site
 // i of this call; unif[i] decides only when p_acc <= 1, exactly as
 // `p_acc > 1.0 || rand() < p_acc`.
+#include <algorithm>
 #include <cooperative_groups.h>
 #include "cluster.cuh"
 #include "common.cuh"
@@ -334,13 +335,15 @@ __global__ void __launch_bounds__(LU_THREADS, 2) k_local_updates(LocalUpdateArgs
 // p accepted sites (k_local_factors) and applies them as one product (flush).
 // Per-site constants of slice l: one warp per site.  Lanes of even parity
 // evaluate the old-field block (power -1), odd lanes the proposed one.
-__global__ void __launch_bounds__(128) k_local_prepare(LocalUpdateArgs a, SitePrep* __restrict__ prep, int* state) {
+__global__ void __launch_bounds__(128) k_local_prepare(LocalUpdateArgs a, SitePrep* __restrict__ prep, int* state,
+                                                       int* wflag) {
   const ModelConst& mc = a.mc;
   const int N = mc.N, M = mc.M, l = a.slice0;
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 4 + (threadIdx.x >> 5);
   // delayed rounds of this slice start from site 0 with nothing pending
-  if (state && blockIdx.x == 0 && threadIdx.x == 0) { state[0] = 0; state[1] = 0; state[2] = 0; }
+  if (blockIdx.x == 0 && threadIdx.x == 0) { state[0] = 0; state[1] = 0; state[2] = 0; }
+  if (blockIdx.x == 0 && threadIdx.x <= WIN_MAX) wflag[threadIdx.x] = 0;   // flags carry the window's first site
   if (i >= N) return;
   const double* po = &a.phi[((size_t)N * l + i) * 3];
   const double old[3] = {po[0], po[1], po[2]};
@@ -527,6 +530,200 @@ __device__ __forceinline__ void named_arrive(int id, int threads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The rank-4p factors of a window: G += X Y with
+//   X[:, j] = ((G - I)[:, a_j] + sum_{i<j} X[:, i] b_i[a_j]) K_j,
+//   Y[j, :] = G[a_j, :] + sum_{i<j} A_i[a_j] Y[i, :]
+// (rows of the accepted sites from k_local_window): every row of X and every
+// column of Y is an independent recurrence of p steps, taken by 8 SPLIT lanes of a
+// warp: 4 components x {real, imaginary} x SPLIT shares of the sum over i.  At
+// the end each vector is cut into the BF16 slices of the flush (or stored in
+// FP64 when the product slices it itself).
+// Bound: FP64 issue, 8 (4p)^2 / 2 multiply-adds per vector.
+struct FacLane {
+  int part, q, sp, v;   // this lane's component, share of the sum and vector of its warp
+};
+template <int SPLIT>
+__device__ __forceinline__ FacLane fac_lane() {
+  const int lane = threadIdx.x & 31;
+  return {lane & 1, (lane >> 1) & 3, (lane >> 3) % SPLIT, lane / (8 * SPLIT)};
+}
+// Step j of one vector x (4 p entries; entry 4 j + q holds g on entry): cj the
+// blocks of the terms i < j, [i][c][q]; kj the block K_j (X only); t scratch of 4.
+template <int SPLIT>
+__device__ __forceinline__ void fac_step(const FacLane& f, cplx* x, int j, const cplx* cj, const cplx* kj, cplx* ts) {
+  double t0 = 0.0, t1 = 0.0;
+  if (f.sp == 0) t0 = f.part ? x[4 * j + f.q].y : x[4 * j + f.q].x;
+#pragma unroll 1
+  for (int i = f.sp; i < j; i += SPLIT) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const cplx xv = x[4 * i + c];
+      double u, w;
+      win_uw(cj[16 * i + 4 * c + f.q], f.part, u, w);
+      t0 = fma(xv.x, u, t0);
+      t1 = fma(xv.y, w, t1);
+    }
+  }
+  double t = t0 + t1;
+#pragma unroll
+  for (int o = 8; o < 8 * SPLIT; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (kj) {
+    if (f.sp == 0) reinterpret_cast<double*>(&ts[f.q])[f.part] = t;
+    __syncwarp();
+    double r0 = 0.0, r1 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const cplx tv = ts[c];
+      double u, w;
+      win_uw(kj[4 * c + f.q], f.part, u, w);
+      r0 = fma(tv.x, u, r0);
+      r1 = fma(tv.y, w, r1);
+    }
+    t = r0 + r1;
+  }
+  __syncwarp();
+  if (f.sp == 0) reinterpret_cast<double*>(x + 4 * j + f.q)[f.part] = t;
+  __syncwarp();
+}
+// block element e (4 c + q of the step) of term i in step j: X takes b_i[a_j],
+// Y the transpose of A_i[a_j]; si, sj: the sites' places in the window
+__device__ __forceinline__ cplx fac_coef(const DelayedArgs& d, int side, int j, int i, int sj, int si, int e) {
+  const int c = e >> 2, q = e & 3;
+  return side == 0 ? ldcg_c(&d.wrow[((size_t)i * 4 + c) * (4 * WIN_MAX) + 4 * sj + q])
+                   : ldcg_c(&d.wrow[((size_t)j * 4 + q) * (4 * WIN_MAX) + 4 * si + c]);
+}
+// entry q of step j before the recurrence, of vector v
+__device__ __forceinline__ cplx fac_entry(const LocalUpdateArgs& a, int side, int site, int q, int v) {
+  const int n = a.mc.n, ai = site + q * a.mc.N;
+  cplx g = side == 0 ? ldcg_c(&a.G[(size_t)ai * n + v]) : ldcg_c(&a.G[(size_t)v * n + ai]);
+  if (side == 0 && ai == v) g.x -= 1.0;
+  return g;
+}
+// a warp's VPW finished vectors from v0 on
+template <int VPW>
+__device__ __forceinline__ void fac_finish(const LocalUpdateArgs& a, const DelayedArgs& d, int side, int v0, int p,
+                                           const cplx* xs, int ldx) {
+  const int lane = threadIdx.x & 31, n = a.mc.n;
+#pragma unroll 1
+  for (int u = 0; u < VPW; ++u) {
+    const cplx* xv = xs + u * ldx;
+    if (d.sl.As) {
+      oz_slice_vec(d.sl, side, v0 + u, 4 * p, [&](int k) { return xv[k]; }, lane);
+    } else {
+      cplx* out = side == 0 ? d.X : d.Y;
+      for (int jq = lane; jq < 4 * p; jq += 32) out[(size_t)jq * n + v0 + u] = xv[jq];
+    }
+  }
+}
+
+// The factors as a launch of their own, after the window (chains that share the
+// GPU).  SPLIT grows as n falls, so that small lattices still fill the
+// sub-partitions.
+constexpr int FAC_THREADS = 128;
+template <int SPLIT>
+__global__ void __launch_bounds__(FAC_THREADS) k_local_factors(LocalUpdateArgs a, DelayedArgs d) {
+  const int p = __ldcg(&d.state[1]);
+  if (p == 0) return;   // uniform over the grid
+  constexpr int VPW = 4 / SPLIT, VPC = VPW * (FAC_THREADS / 32);
+  const int side = blockIdx.y, v0 = blockIdx.x * VPC;   // side 0: rows of X, 1: columns of Y
+  extern __shared__ double4_16a smem_fac[];
+  cplx* coef = reinterpret_cast<cplx*>(smem_fac);       // (p (p - 1) / 2, 4, 4): [c][q] of step j, term i < j
+  cplx* kk = coef + (size_t)8 * p * (p - 1);            // (p, 4, 4) K_j (X)
+  const int ldx = 4 * d.k + 1;
+  cplx* xs = kk + 16 * p;                               // (VPC, ldx) the vectors
+  __shared__ cplx s_t[VPC][4];
+  __shared__ int s_site[WIN_MAX];
+  const int tid = threadIdx.x, wid = tid >> 5;
+  const int base = __ldcg(&d.state[3]);
+  if (tid < p) s_site[tid] = __ldcg(&d.wsite[tid]);
+  __syncthreads();
+#pragma unroll 4
+  for (int e = tid; e < 8 * p * (p - 1); e += FAC_THREADS) {
+    // pair index (j, i): j (j - 1) / 2 + i
+    const int pr = e >> 4;
+    int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)pr)) * 0.5f);
+    while (j * (j - 1) / 2 > pr) --j;
+    while ((j + 1) * j / 2 <= pr) ++j;
+    const int i = pr - j * (j - 1) / 2;
+    coef[e] = fac_coef(d, side, j, i, s_site[j], s_site[i], e & 15);
+  }
+  if (side == 0)
+    for (int e = tid; e < 16 * p; e += FAC_THREADS) kk[e] = ldcg_c(&d.wk[e]);
+#pragma unroll 4
+  for (int e = tid; e < 4 * p * VPC; e += FAC_THREADS) {
+    const int v = side == 0 ? e % VPC : e / (4 * p), jq = side == 0 ? e / VPC : e - v * 4 * p;
+    xs[v * ldx + jq] = fac_entry(a, side, base + s_site[jq >> 2], jq & 3, v0 + v);
+  }
+  __syncthreads();
+  const FacLane f = fac_lane<SPLIT>();
+  const int v = wid * VPW + f.v;
+  for (int j = 0; j < p; ++j)
+    fac_step<SPLIT>(f, xs + v * ldx, j, coef + (size_t)8 * j * (j - 1), side == 0 ? kk + 16 * j : nullptr, s_t[v]);
+  fac_finish<VPW>(a, d, side, v0 + wid * VPW, p, xs + wid * VPW * ldx, ldx);
+}
+
+// The factors beside the window (a chain that has the GPU to itself): a CTA of
+// a follower cluster takes step j of its VPC = 4 WARPS / SPLIT vectors as soon as
+// the window's cluster has published the j-th acceptance, so that only the last
+// step and the slicing are left when the window is decided.  One warp per CTA
+// polls: a poll of every warp keeps the word's L2 slice busy.
+template <int SPLIT, int WARPS>
+__device__ void fac_follow(const LocalUpdateArgs& a, const DelayedArgs& d, int first, int blk, cplx* smem) {
+  constexpr int VPW = 4 / SPLIT, VPC = VPW * WARPS, T = 32 * WARPS;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, n = a.mc.n;
+  const int ctas = (n + VPC - 1) / VPC, side = blk < ctas ? 0 : 1;
+  if (blk >= 2 * ctas) return;
+  const int v0 = (blk - side * ctas) * VPC, nv = min(VPC, n - v0);   // nv: a multiple of 4
+  const int ldx = 4 * d.k + 1;
+  cplx* xs = smem;                          // (VPC, ldx)
+  cplx* cj = xs + VPC * ldx;                // (WIN_MAX, 4, 4)
+  cplx* kj = cj + 16 * WIN_MAX;             // (4, 4)
+  cplx* ts = kj + 16;                       // (VPC, 4)
+  int* sites = reinterpret_cast<int*>(ts + 4 * VPC);   // (WIN_MAX) and the word of the step
+  const FacLane f = fac_lane<SPLIT>();
+  const int v = wid * VPW + f.v;
+  int j = 0;
+  for (;; ++j) {
+    if (wid == 0) {
+      int w = 0;
+      bool here = false;
+      for (int it = 0; it < kClusterPolls && !here; ++it) {
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(w) : "l"(d.wflag + j) : "memory");
+        here = __all_sync(0xffffffffu, (w >> 9) == first + 1);
+      }
+      __threadfence();
+      if (lane == 0) sites[WIN_MAX] = here ? w : -1;
+    }
+    named_bar(1, T);   // also: the coefficients of the step before are read
+    const int w = sites[WIN_MAX];
+    if (w < 0) {
+      if (tid == 0) atomicOr(a.err, DQMC_KERR_BARRIER_TIMEOUT);
+      return;
+    }
+    if (!(w & 256)) break;   // no further acceptance
+    const int sj = w & 255;
+    if (tid == 0) sites[j] = sj;
+    for (int e = tid; e < 16 * j; e += T) cj[e] = fac_coef(d, side, j, e >> 4, sj, sites[e >> 4], e & 15);
+    if (tid < 4 * nv) {
+      const int u = side == 0 ? tid % nv : tid >> 2, q = side == 0 ? tid / nv : tid & 3;
+      xs[u * ldx + 4 * j + q] = fac_entry(a, side, first + sj, q, v0 + u);
+    }
+    if (side == 0 && tid >= T - 16) kj[tid - (T - 16)] = ldcg_c(&d.wk[16 * j + tid - (T - 16)]);
+    named_bar(1, T);
+    if (wid * VPW < nv) fac_step<SPLIT>(f, xs + v * ldx, j, cj, side == 0 ? kj : nullptr, ts + 4 * v);
+  }
+  if (j > 0 && wid * VPW < nv) fac_finish<VPW>(a, d, side, v0 + wid * VPW, j, xs + wid * VPW * ldx, ldx);
+}
+
+// Vectors of a follower CTA: the fewest that keep the followers within 7
+// clusters of 16 CTAs.  With the window's own these have a GPC each; an eighth
+// shares its SMs with another (n > 896), which doubles the time of its steps.
+__host__ __device__ constexpr int fac_vpc(int n) { return n <= 224 ? 4 : (n <= 448 ? 8 : 16); }
+// and their words of shared memory
+__host__ __device__ constexpr int fac_follow_smem(int n, int k) {
+  return fac_vpc(n) * (4 * k + 1) + 16 * WIN_MAX + 16 + 4 * fac_vpc(n) + WIN_MAX / 4 + 1;
+}
+
 // Decides the window of sites state[0] .. state[0] + W - 1 (fewer at the
 // slice's end; it also ends once d.k sites are accepted) on one cluster of C
 // CTAs.  Site s of the window (0-based) belongs to CTA s mod C, which holds its
@@ -545,10 +742,12 @@ __device__ __forceinline__ void named_arrive(int id, int threads) {
 //   3-7  the rest of G[r, .] += A b, beside that evaluation.
 // Rows of decided sites stay as they were when decided.
 //
-// For the factors of the accepted sites a_1 .. a_p (in order), with
-// K_j = M_j^-1 Delta_j, the kernel leaves, per pair, the 4x4 blocks
-// b_i[a_j] = G_{i-1}[a_i, a_j] (i < j) and A_i[a_j] = ((G_{i-1} - I)[a_j, a_i] K_i
-// (i < j; kept in the columns of a_i, which are no longer needed).
+// For the factors of the accepted sites a_1 .. a_p (in order) the kernel leaves
+// K_j = M_j^-1 Delta_j and the rows of a_j as they were when it was accepted: in
+// the columns of a later site a_l they are b_j[a_l] = G_{j-1}[a_j, a_l], in those of
+// an earlier one A_i[a_j] = (G_{i-1} - I)[a_j, a_i] K_i (which takes the place of the
+// column once it is no longer needed).  With follower clusters (gridDim.x > C)
+// those form the factors at the same time, acceptance by acceptance.
 //
 // Bound: the chain of dependent FP64 operations of a step, about 100 cycles
 // each (64 to issue one).  The kernel this replaces formed all n rows and
@@ -562,15 +761,33 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
   const int N = mc.N, n = mc.n, L = mc.L;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int first = __ldcg(&d.state[0]);
-  if (first >= N) {   // slice done (uniform over the cluster): nothing for the flush either
-    if (rank == 0 && tid == 0) d.state[1] = 0;
+  extern __shared__ double4_16a smem_win[];
+  const int followers = (int)gridDim.x - C;   // their CTAs, in clusters after the window's
+  if (first >= N) {   // slice done (uniform over the grid): nothing for the flush either
+    if (blockIdx.x == 0 && tid == 0) d.state[1] = 0;
+    return;
+  }
+  if ((int)blockIdx.x >= C) {
+    __syncthreads();
+    if (tid == 0) {   // the state has been read: the window may advance it
+      __threadfence();
+      atomicAdd(d.arrive, 1);
+    }
+    const int blk = (int)blockIdx.x - C, vpc = fac_vpc(n);
+    cplx* sm = reinterpret_cast<cplx*>(smem_win);
+    if (vpc == 4) {
+      if (wid < 4) fac_follow<4, 4>(a, d, first, blk, sm);
+    } else if (vpc == 8) {
+      fac_follow<4, 8>(a, d, first, blk, sm);
+    } else {
+      fac_follow<2, 8>(a, d, first, blk, sm);
+    }
     return;
   }
   const int we = min(W, N - first);                       // sites of this window
   const int owned = rank < we ? (we - rank + C - 1) / C : 0;   // sites rank + t C
   const int own_max = (W + C - 1) / C;
   const int LD = 4 * W + 1;
-  extern __shared__ double4_16a smem_win[];
   cplx* Gs = reinterpret_cast<cplx*>(smem_win);           // (4 own_max, LD)
   cplx* brow = Gs + (size_t)4 * own_max * LD;             // (4, 4W) rows of the accepted site
   cplx* As = brow + 16 * W;                               // (4 own_max, 4): G[r, a] M^-1 Delta
@@ -731,7 +948,30 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
       continue;
     }
     const int owner = acc % C, ta = acc / C;
-    if (rank == owner && wid == 1) reinterpret_cast<double*>(d.wk + 16 * p)[lane] = kv;   // for the factors
+    if (rank == owner) {
+      // K and the rows of the accepted site for the factors, published by warp 4
+      if (wid == 1) {
+        reinterpret_cast<double*>(d.wk + 16 * p)[lane] = kv;
+        __syncwarp();
+        named_arrive(7, 160);
+      } else if (wid >= 4) {
+        const cplx* src = Gs + (size_t)(4 * ta + wid - 4) * LD;
+        cplx* dst = d.wrow + ((size_t)p * 4 + wid - 4) * (4 * WIN_MAX);
+        for (int cc = lane; cc < 4 * we; cc += 32) dst[cc] = src[cc];
+        __syncwarp();
+        if (wid > 4) {
+          named_arrive(7, 160);
+        } else {
+          named_bar(7, 160);
+          if (lane == 0) {
+            __threadfence();
+            asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(d.wflag + p), "r"((first + 1) << 9 | 256 | acc)
+                         : "memory");
+          }
+          __syncwarp();
+        }
+      }
+    }
     if (wid == 2) {
       // field, interaction table, order of acceptances
       const int gi = first + acc;
@@ -823,12 +1063,14 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
     fresh = false;
   }
   if (!ok) atomicOr(a.err, DQMC_KERR_BARRIER_TIMEOUT);
+  const int lastr = (we - 1) % C;   // has seen all decisions
+  if (followers > 0 && rank == lastr && tid == 0)   // no further acceptance
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(d.wflag + p), "r"((first + 1) << 9) : "memory");
   if (wid == 2 && lane == 0) {
     s_fin[0] = p;
     s_fin[1] = cur;
   }
   cl.sync();   // every CTA is done; the owner of the last site has seen all decisions
-  const int lastr = (we - 1) % C;
   p = *cl.map_shared_rank(&s_fin[0], lastr);
   cur = *cl.map_shared_rank(&s_fin[1], lastr);
   __syncthreads();
@@ -836,15 +1078,17 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
     for (int e = tid; e < p; e += WIN_THREADS) s_acc[e] = cl.map_shared_rank(&s_acc[0], lastr)[e];
   }
   cl.sync();   // no shared memory is read remotely any more
-  // ---- the accepted sites' blocks for k_local_factors, the round's state ----
-  for (int e = tid; e < p * p * 16; e += WIN_THREADS) {
-    const int j = e / (16 * p), i = (e >> 4) - j * p, q = e & 15;
-    const int sj = s_acc[j];
-    if (sj % C != rank || i == j) continue;
-    d.wblk[((size_t)j * WIN_MAX + i) * 16 + q] = Gs[(size_t)(4 * (sj / C) + (q >> 2)) * LD + 4 * s_acc[i] + (q & 3)];
-  }
+  // ---- the round's state ----
   if (rank == 0 && wid == 0) {
-    if (lane < p) d.wsite[lane] = first + s_acc[lane];
+    if (lane < p) d.wsite[lane] = s_acc[lane];
+    if (lane == 0 && followers > 0) {
+      // the followers have read the state (bounded wait)
+      bool here = false;
+      for (int it = 0; it < kClusterPolls && !here; ++it) here = *(volatile int*)d.arrive == followers;
+      if (!here) atomicOr(a.err, DQMC_KERR_BARRIER_TIMEOUT);
+      *(volatile int*)d.arrive = 0;
+    }
+    __syncwarp();
     // the tracked action: -log(exp(-dS)) of the accepted sites, added in order
     const double lg = lane < p ? -log(__ldcg(&d.wexp[lane])) : 0.0;
     double act = lane == 0 ? *a.action : 0.0;
@@ -855,113 +1099,11 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
     if (lane == 0) {
       d.state[0] = first + cur;
       d.state[1] = p;
+      d.state[3] = first;
       if (p > 0) {
         *a.action = act;
         *a.n_acc += p;
       }
-    }
-  }
-}
-
-// The rank-4p factors of a window: G += X Y with
-//   X[:, j] = ((G - I)[:, a_j] + sum_{i<j} X[:, i] b_i[a_j]) K_j,
-//   Y[j, :] = G[a_j, :] + sum_{i<j} A_i[a_j] Y[i, :]
-// (blocks from k_local_window): every row of X and every column of Y is an
-// independent recurrence of p steps.  8 SPLIT lanes per vector: 4 components x
-// {real, imaginary} x SPLIT shares of the sum over i; the vector and the blocks
-// are in shared memory.  At the end each vector is cut into the BF16 slices of
-// the flush (or stored in FP64 when the product slices it itself).
-// Bound: FP64 issue, 8 (4p)^2 / 2 multiply-adds per vector; SPLIT grows as n
-// falls, so that small lattices still fill the sub-partitions.
-constexpr int FAC_THREADS = 128;
-template <int SPLIT>
-__global__ void __launch_bounds__(FAC_THREADS) k_local_factors(LocalUpdateArgs a, DelayedArgs d) {
-  const int p = __ldcg(&d.state[1]);
-  if (p == 0) return;   // uniform over the grid
-  constexpr int VPW = 4 / SPLIT, VPC = VPW * (FAC_THREADS / 32);
-  const int n = a.mc.n, N = a.mc.N;
-  const int side = blockIdx.y, v0 = blockIdx.x * VPC;   // side 0: rows of X, 1: columns of Y
-  extern __shared__ double4_16a smem_fac[];
-  cplx* coef = reinterpret_cast<cplx*>(smem_fac);       // (p (p - 1) / 2, 4, 4): [c][q] of step j, term i < j
-  cplx* kk = coef + (size_t)8 * p * (p - 1);            // (p, 4, 4) K_j (X)
-  const int ldx = 4 * d.k + 1;
-  cplx* xs = kk + 16 * p;                               // (VPC, ldx) the vectors
-  __shared__ cplx s_t[VPC][4];
-  __shared__ int s_site[WIN_MAX];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  if (tid < p) s_site[tid] = __ldcg(&d.wsite[tid]);
-#pragma unroll 4
-  for (int e = tid; e < 8 * p * (p - 1); e += FAC_THREADS) {
-    // pair index (j, i): j (j - 1) / 2 + i
-    const int pr = e >> 4, q = e & 15;
-    int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)pr)) * 0.5f);
-    while (j * (j - 1) / 2 > pr) --j;
-    while ((j + 1) * j / 2 <= pr) ++j;
-    const int i = pr - j * (j - 1) / 2;
-    coef[e] = side == 0 ? ldcg_c(&d.wblk[((size_t)i * WIN_MAX + j) * 16 + q])
-                        : ldcg_c(&d.wblk[((size_t)j * WIN_MAX + i) * 16 + 4 * (q & 3) + (q >> 2)]);
-  }
-  if (side == 0)
-    for (int e = tid; e < 16 * p; e += FAC_THREADS) kk[e] = ldcg_c(&d.wk[e]);
-  __syncthreads();
-#pragma unroll 4
-  for (int e = tid; e < 4 * p * VPC; e += FAC_THREADS) {
-    const int v = side == 0 ? e % VPC : e / (4 * p), jq = side == 0 ? e / VPC : e - v * 4 * p;
-    const int ai = s_site[jq >> 2] + (jq & 3) * N;
-    cplx g = side == 0 ? ldcg_c(&a.G[(size_t)ai * n + v0 + v]) : ldcg_c(&a.G[(size_t)(v0 + v) * n + ai]);
-    if (side == 0 && ai == v0 + v) g.x -= 1.0;
-    xs[v * ldx + jq] = g;
-  }
-  __syncthreads();
-  const int part = lane & 1, q = (lane >> 1) & 3, sp = (lane >> 3) % SPLIT, v = wid * VPW + lane / (8 * SPLIT);
-  cplx* x = xs + v * ldx;
-  for (int j = 0; j < p; ++j) {
-    const cplx* cj = coef + (size_t)8 * j * (j - 1);
-    double t0 = 0.0, t1 = 0.0;
-    if (sp == 0) t0 = part ? x[4 * j + q].y : x[4 * j + q].x;
-    for (int i = sp; i < j; i += SPLIT) {
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const cplx xv = x[4 * i + c];
-        double u, w;
-        win_uw(cj[16 * i + 4 * c + q], part, u, w);
-        t0 = fma(xv.x, u, t0);
-        t1 = fma(xv.y, w, t1);
-      }
-    }
-    double t = t0 + t1;
-#pragma unroll
-    for (int o = 8; o < 8 * SPLIT; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (side == 0) {
-      if (sp == 0) reinterpret_cast<double*>(&s_t[v][q])[part] = t;
-      __syncwarp();
-      double r0 = 0.0, r1 = 0.0;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const cplx tv = s_t[v][c];
-        double u, w;
-        win_uw(kk[16 * j + 4 * c + q], part, u, w);
-        r0 = fma(tv.x, u, r0);
-        r1 = fma(tv.y, w, r1);
-      }
-      t = r0 + r1;
-    }
-    __syncwarp();
-    if (sp == 0) reinterpret_cast<double*>(x + 4 * j + q)[part] = t;
-    __syncwarp();
-  }
-  if (d.sl.As) {
-#pragma unroll 1
-    for (int u = 0; u < VPW; ++u) {
-      const cplx* xv = xs + (wid * VPW + u) * ldx;
-      oz_slice_vec(d.sl, side, v0 + wid * VPW + u, 4 * p, [&](int k) { return xv[k]; }, lane);
-    }
-  } else {
-    __syncthreads();
-    cplx* out = side == 0 ? d.X : d.Y;
-    for (int e = tid; e < 4 * p * VPC; e += FAC_THREADS) {
-      const int vv = e % VPC, jq = e / VPC;
-      out[(size_t)jq * n + v0 + vv] = xs[vv * ldx + jq];
     }
   }
 }
@@ -993,8 +1135,8 @@ static size_t local_smem_bytes(int N) {
   return (size_t)N * (16 * sizeof(cplx) + sizeof(EvEntry)) + (size_t)3 * N * sizeof(double);
 }
 
-cudaError_t launch_local_prepare(const LocalUpdateArgs& a, SitePrep* prep, int* state, cudaStream_t st) {
-  k_local_prepare<<<(a.mc.N + 3) / 4, 128, 0, st>>>(a, prep, state);
+cudaError_t launch_local_prepare(const LocalUpdateArgs& a, SitePrep* prep, int* state, int* wflag, cudaStream_t st) {
+  k_local_prepare<<<(a.mc.N + 3) / 4, 128, 0, st>>>(a, prep, state, wflag);
   return cudaGetLastError();
 }
 
@@ -1047,9 +1189,9 @@ static cudaError_t window_cluster(int* C) {
       if (clusters >= 1) cached[dev] = c;
     }
     if (cached[dev] == 0) return cudaErrorNotSupported;
-    // 8-CTA clusters (batched chains) hold up to four sites per CTA
-    if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)window_smem(256, WIN_MAX, 8));
+    // 8-CTA clusters (batched chains) hold up to four sites per CTA; the followers of the deepest windows
+    const size_t most = std::max(window_smem(256, WIN_MAX, 8), (size_t)fac_follow_smem(1024, 64) * sizeof(cplx));
+    if (cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         e != cudaSuccess)
       return e;
   }
@@ -1059,14 +1201,47 @@ static cudaError_t window_cluster(int* C) {
 
 int local_window_sites(int k) { return k < WIN_MAX ? k : WIN_MAX; }
 
-cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster) {
+// Follower clusters of a window launch.
+static int follower_clusters(int n, int C) { return (2 * ((n + fac_vpc(n) - 1) / fac_vpc(n)) + C - 1) / C; }
+
+cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster,
+                                bool follow) {
   int C = 0;
   if (cudaError_t e = window_cluster(&C); e != cudaSuccess) return e;
   if (max_cluster > 0 && C > 8 && max_cluster < C) C = 8;
   const int W = local_window_sites(d.k);
-  cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t cfg = window_config(attr, C, window_smem(a.mc.N, W, C), st);
+  size_t smem = window_smem(a.mc.N, W, C);
+  cudaLaunchAttribute attr[2];
+  if (follow) {
+    const size_t fs = (size_t)fac_follow_smem(a.mc.n, d.k) * sizeof(cplx);
+    if (fs > smem) smem = fs;
+  }
+  cudaLaunchConfig_t cfg = window_config(attr, C, smem, st);
+  if (follow) {
+    // cooperative: the followers wait on the window's cluster, so all are resident together
+    cfg.gridDim = dim3(C * (1 + follower_clusters(a.mc.n, C)));
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+    cfg.numAttrs = 2;
+  }
   return cudaLaunchKernelEx(&cfg, k_local_window, a, d, W);
+}
+
+bool local_window_follows(int n, int k) {
+  int C = 0;
+  if (window_cluster(&C) != cudaSuccess) return false;
+  const int W = local_window_sites(k);
+  size_t smem = window_smem(n / 4, W, C);
+  const size_t fs = (size_t)fac_follow_smem(n, k) * sizeof(cplx);
+  if (fs > smem) smem = fs;
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = window_config(attr, C, smem, nullptr);
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, (const void*)k_local_window, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return clusters >= 1 + follower_clusters(n, C);
 }
 
 cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st) {

@@ -58,8 +58,8 @@ struct SitePrep {
   double dsA, dsQ, dsB;    // boson action difference, space-neighbour coupling excluded
   double pad[2];
 };
-// state (2 ints, nullable): delayed-round state of the slice, zeroed here
-cudaError_t launch_local_prepare(const LocalUpdateArgs& a, SitePrep* prep, int* state, cudaStream_t st);
+// state (delayed-round state of the slice) and wflag are zeroed here
+cudaError_t launch_local_prepare(const LocalUpdateArgs& a, SitePrep* prep, int* state, int* wflag, cudaStream_t st);
 // BF16 slices of the operands of an m x n x K split-BF16 product in its
 // scratch block: As S x (m x Kp), Bre / Bim S x (n x Kp) (K contiguous, Kp =
 // 2 Kpad), row scales sA (m), column scales sB (n)
@@ -75,15 +75,20 @@ struct DelayedArgs {
   int* state;
   int k;                   // most acceptances of a round
   const SitePrep* prep;    // (N) from launch_local_prepare for this slice
-  int* wsite;              // (WIN_MAX) sites accepted in the window, in order
+  int* wsite;              // (WIN_MAX) sites accepted in the window, in order, from its first site state[3]
   cplx* wk;                // (WIN_MAX, 16) their M^-1 Delta
   double* wexp;            // (WIN_MAX) their exp(-dS)
-  cplx* wblk;              // (WIN_MAX, WIN_MAX, 16) their 4x4 blocks (k_local_window)
+  cplx* wrow;              // (WIN_MAX, 4, 4 WIN_MAX) their rows of the window's block (k_local_window)
+  int* wflag;              // (WIN_MAX + 1) acceptances published to the follower clusters
+  int* arrive;             // followers that have read the state (zero between launches)
   OzSlices sl;             // the flush's slices, cut by launch_local_factors
                            // (sl.As null: X and Y are stored and the flush slices them itself)
 };
 // Decides the next window of the slice on one cluster (max_cluster > 0: at most that many CTAs, >= 8).
-cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster);
+cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster,
+                                bool follow);
+// whether the window can have follower clusters that form its factors (else launch_local_factors)
+bool local_window_follows(int n, int k);
 // The factors X (n x 4p, column-major) and Y (4p x n, row j at Y + j n) of the window's p acceptances.
 cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st);
 int local_window_sites(int k);

@@ -59,3 +59,28 @@ def test_full_and_nearly_empty_windows(unif, rate):
     accepts only those with p > 1."""
     got = _run(P, 16, 0, unif=unif)
     assert rate is None or got == rate
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L,delay", [(8, 16), (10, 3), (12, 16), (14, 40), (16, 16)])
+def test_factors_beside_the_window(L, delay):
+    """Follower clusters of 8 and 16 vectors per CTA, ragged last CTAs among
+    them, against the factors as a launch of their own (chains in flight): the
+    sums are the same up to the split over lanes, 4 p terms of FP64 rounding per
+    window and at most 2 N / 16 windows."""
+    from dqmc_gb300 import api
+    calls = 2
+    phi = R.synthetic_field(L * L, 10, 70 + L)
+    delta, u = R.synthetic_streams(L * L, calls, 0.2, 80 + L)
+    got = []
+    for inflight in (0, 8):
+        c = api.DQMC(api.ModelParams(L=L, slices=10, safe_mult=10, delay=delay, inflight=inflight), phi)
+        c.init()
+        res = c.sweep(calls, delta, u, return_accepted=True)
+        got.append((res["accepted_mask"], np.array(c.greens), c.get_field()))
+        c.close()
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][2], got[1][2])
+    windows = 2 * calls * (L * L // 16 + 1)
+    tol = windows * 4 * 32 * 2.3e-16
+    assert np.max(np.abs(got[0][1] - got[1][1])) < tol * max(1.0, np.max(np.abs(got[1][1])))
