@@ -353,7 +353,10 @@ int gemm(dqmc_handle* h, char opA, char opB, const cplx* A, const cplx* B, cplx*
 }
 // pivoted QR of A (destroyed) -> T (physical layout), D; reflectors in h->qr
 int qrp(dqmc_handle* h, cplx* A, cplx* T, double* D) {
-  LAUNCH(DQMC_K_QRP, 16.0 / 3.0 * n3(h), 32.0 * n2(h), launch_qrp(A, h->n, h->qr, h->sm_count, h->st, h->coop_cap));
+  int kernels = 1;
+  LAUNCH(DQMC_K_QRP, 16.0 / 3.0 * n3(h), 32.0 * n2(h),
+         launch_qrp(A, h->n, h->qr, h->sm_count, h->st, h->coop_cap, &kernels));
+  h->launches += kernels - 1;
   LAUNCH(DQMC_K_MISC, 0.0, 32.0 * n2(h), launch_qrp_finalize(A, T, D, h->n, h->qr, h->st));
   return DQMC_OK;
 }
@@ -926,7 +929,7 @@ void host_model_constants(dqmc_handle* h) { fill_model_const(h->p, h->mc); }
 void free_all(dqmc_handle* h) {
   void* ptrs[] = {h->phi, h->evtab, h->G, h->Gtmp, h->u_stack, h->d_stack, h->t_stack, h->Ul, h->Ur, h->Tl,
                   h->Tr, h->Dl, h->Dr, h->W1, h->W2, h->W3, h->W4, h->D1, h->d2, h->ord1, h->qr.vn1,
-                  h->qr.vn2, h->qr.order, h->qr.tau, h->qr.beta, h->qr.V, h->qr.bar, h->qr.cand_v, h->qr.cand_q, h->qr.refl, h->delta_d, h->unif_d,
+                  h->qr.vn2, h->qr.order, h->qr.tau, h->qr.beta, h->qr.V, h->qr.bar, h->qr.cand_v, h->qr.cand_q, h->qr.refl, h->qr.slots, h->qr.cols, h->qr.run, h->delta_d, h->unif_d,
                   h->acc_d, h->det_d, h->pacc_d, h->action_d, h->nacc_d, h->Acol, h->Brow, h->bar, h->err_d,
                   h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wrow, h->wflag, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
   for (void* q : ptrs)
@@ -1293,6 +1296,9 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
   A((void**)&h->qr.bar, sizeof(GridBarrier));
   A((void**)&h->qr.cand_v, 1024 * sizeof(double)); A((void**)&h->qr.cand_q, 1024 * sizeof(int));
   A((void**)&h->qr.refl, (size_t)2 * 256 * 10 * sizeof(unsigned long long));
+  A((void**)&h->qr.slots, (size_t)2 * 160 * 160 * 2 * sizeof(unsigned long long));
+  A((void**)&h->qr.cols, qr_column_words((int)n, h->sm_count) * sizeof(unsigned long long));
+  A((void**)&h->qr.run, sizeof(unsigned));
   A((void**)&h->action_d, sizeof(double)); A((void**)&h->nacc_d, 2 * sizeof(int));
   A((void**)&h->Acol, 4 * n * sizeof(cplx)); A((void**)&h->Brow, 4 * n * sizeof(cplx));
   A((void**)&h->bar, sizeof(GridBarrier)); A((void**)&h->err_d, sizeof(int));

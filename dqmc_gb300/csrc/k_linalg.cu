@@ -10,6 +10,7 @@
 // factor comes out directly in the un-permuted ("T = R[:, invperm(p)]")
 // layout that the UDT decomposition needs.
 #include <cfloat>
+#include <type_traits>
 #include "common.cuh"
 #include "kernels.h"
 
@@ -260,7 +261,7 @@ __device__ __forceinline__ double qr_finish_column(cplx (&x)[QR_MAXT], cplx* __r
 // hundred columns remain, then the latency of barrier, pivot column and norm
 // downdate.  Per sequence of calls, ms, formed after the barrier -> ahead:
 // n = 64 1.70 -> 1.53, 144 8.0 -> 7.4, 256 14.9 -> 14.4, 1024 52.6 -> 51.8.
-__global__ void __launch_bounds__(QR_THREADS, 1) k_qrp(cplx* __restrict__ A, int n, QRWork w) {
+__global__ void __launch_bounds__(QR_THREADS, 1) k_qrp(cplx* __restrict__ A, int n, int kend, QRWork w) {
   unsigned epoch = 0;
   GridBarrierExit bar_exit(w.bar);
   extern __shared__ double smem_qr[];
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(QR_THREADS, 1) k_qrp(cplx* __restrict__ A, int
     w.refl[((size_t)(e / QR_REFL_WORDS) * gridDim.x + blockIdx.x) * QR_REFL_WORDS + e % QR_REFL_WORDS] = 0ull;
 
   const int chunk = (n + gridDim.x - 1) / gridDim.x;   // rows of V written by this CTA
-  for (int k = 0; k < n; ++k) {
+  for (int k = 0; k < kend; ++k) {
     const int rem = n - k - 1;
     const int nq = (n - k + 31) >> 5;   // warp-uniform: no FP64 work on fully masked slots
     const int t_first = blockIdx.x + gridDim.x * wid;
@@ -556,6 +557,468 @@ __global__ void k_lu_logdet(const cplx* __restrict__ udiag, const double* __rest
   }
   s = block_sum(s, red);
   if (threadIdx.x == 0) out[0] = s;
+}
+
+// ---------------------------------------------------------------------------
+// column-pivoted QR with the columns in registers (cooperative)
+// ---------------------------------------------------------------------------
+// Steps k0 .. n - 1 of k_qrp when at most four columns per SM remain: one column
+// per warp and sub-partition, from the launch's start to its pivot step, so no
+// step loads or stores columns, and a CTA's chain from one pivot to the next
+// passes no grid barrier.  Per step:
+//   warps 0-3   a column each: its norm as the CTA's bid for the next pivot; the
+//               update of the step before (beside the exchange), which the bidding
+//               column publishes; then the dot product and the norm;
+//   warp 4      publishes the CTA's bid, polls all CTAs', picks the pivot;
+//   warps 4-11  fetch the pivot column, sum its squares, write rows of V;
+//   warp 5      the reflector's scalars (in every CTA: a second way through L2
+//               costs more than the sum and the chain of a root and two divisions).
+// A norm that has to be recomputed (the guard of zlaqp2) needs the update and a
+// further pass.  It is below 2^-12 of its last exact value, so the CTA bids with
+// its best exact norm if that is larger, else with the bound, and the pivot is
+// waited for only where a bound turns out to be the best bid.
+// What CTAs publish validates itself: a bid is one 16-byte word with the step's
+// tag, columns are 32-bit halves under the tag.  Buffers alternate by step:
+// nobody publishes step k + 2 before all have published step k + 1, which they
+// do after reading everything of step k.
+// Rows stay with their lanes (row base + 32 q + lane), and the sums over a
+// column rotate to the lanes that k_qrp has them in: same terms in the same
+// order, so both kernels give the same bits.
+// Bound: latency; a step of n = 144 is update, the way through L2, squares and
+// scalars (6000 cycles) and the norm downdate (2000).  From n = 400 on the passes
+// over a column at one FP64 instruction per 64 cycles and sub-partition take over.
+// Per sequence of calls, ms, k_qrp -> this: n = 64 1.53 -> 1.24, 144 7.4 -> 5.9,
+// 256 14.4 -> 10.8, 400 31.7 -> 24.4, 576 41.4 -> 36.0, 1024 (the last 608 columns)
+// 51.8 -> 49.6.
+constexpr int QC_COLS = 4, QC_HELP = 8;
+constexpr int QC_THREADS = 32 * (QC_COLS + QC_HELP);
+// named barriers
+constexpr int QC_B_BIDS = 1, QC_B_NORMS = 2, QC_B_PIVOT = 3, QC_B_TAU = 4, QC_B_EXACT = 5, QC_B_COL = 8, QC_B_COLTAU = 12;
+constexpr int QC_SLOTS = 5;                     // candidates polled per lane: grids of at most 160 CTAs
+constexpr int QC_POLLS = 1 << 20;               // bound of every wait (about a second)
+constexpr long long QC_NONE = -0x7FFFFFFFFFFFFFFFll - 1;   // key of a CTA without columns
+
+__device__ __forceinline__ void qc_sync(int id, int warps) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(32 * warps) : "memory");
+}
+__device__ __forceinline__ void qc_arrive(int id, int warps) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(32 * warps) : "memory");
+}
+__device__ __forceinline__ void qc_store16(unsigned long long* p, unsigned long long a, unsigned long long b) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p), "l"(a),
+               "l"(b)
+               : "memory");
+}
+__device__ __forceinline__ void qc_load16(const unsigned long long* p, unsigned long long& a, unsigned long long& b) {
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
+               : "=l"(a), "=l"(b)
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ unsigned long long qc_word(unsigned tag, int half) {
+  return (unsigned long long)tag << 32 | (unsigned)half;
+}
+// a == b ? x : y, kept a select (as an indexed read the columns would live in local memory)
+__device__ __forceinline__ double qc_select(int a, int b, double x, double y) {
+  double r;
+  asm("{\n .reg .pred p;\n setp.eq.s32 p, %1, %2;\n selp.f64 %0, %3, %4, p;\n}\n" : "=d"(r) : "r"(a), "r"(b), "d"(x), "d"(y));
+  return r;
+}
+// norms order like their bit patterns; a NaN with its sign set comes last
+__device__ __forceinline__ long long qc_key(double norm) {
+  const long long b = __double_as_longlong(norm);
+  return b < 0 ? -1 : b;
+}
+
+template <int NQ>   // rows from k0's group of 32 on, in groups of 32
+__global__ void __launch_bounds__(QC_THREADS, 1) k_qr_cols(cplx* __restrict__ A, int n, int k0, QRWork w) {
+  extern __shared__ double smem_qc[];
+  const int base = k0 & ~31, rows = n - base;
+  cplx* vbuf = reinterpret_cast<cplx*>(smem_qc);   // (2, rows) pivot columns, by step parity
+  __shared__ long long s_key[2][QC_COLS], s_exact[2][QC_COLS];
+  __shared__ int s_pos[2][QC_COLS], s_phys[2][QC_COLS], s_def[2][QC_COLS];
+  __shared__ int s_win[2][3];                      // pivot: CTA, logical position, column
+  __shared__ double s_norm[QC_HELP];
+  __shared__ cplx s_tau[2], s_scal[2];
+  __shared__ int s_abort;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, G = gridDim.x;
+  const unsigned run = *(volatile unsigned*)w.run + 1u;   // tags differ from those of earlier launches and of k_qrp
+  if (threadIdx.x == 0) s_abort = 0;
+  __syncthreads();
+  volatile int* abort = &s_abort;
+  unsigned long long* slot = w.slots;                               // (2, to, from, 2)
+  unsigned long long* cols = w.cols;                                // (2, G, rows, 4)
+  auto give_up = [&] {   // nothing is waited for any more; the results are void
+    if (!*abort) { atomicOr(w.err, DQMC_KERR_BARRIER_TIMEOUT); *abort = 1; }
+  };
+  // The CTA's candidate among the columns with an exact norm, in key; open: a
+  // deferred column (s_def, key a bound) may be better, bound its bound.
+  auto cta_best = [&](int par, long long& key, bool& open, long long& bound) {
+    int c = 0;
+    key = QC_NONE;
+    bound = QC_NONE;
+#pragma unroll
+    for (int q = 0; q < QC_COLS; ++q) {
+      const long long kq = s_key[par][q];
+      if (s_def[par][q]) {
+        if (kq > bound) bound = kq;
+      } else if (kq > key || (kq == key && s_pos[par][q] < s_pos[par][c])) {
+        key = kq;
+        c = q;
+      }
+    }
+    open = bound != QC_NONE && bound >= key;
+    return c;
+  };
+  auto cta_best_exact = [&](int par, long long& key) {
+    int c = 0;
+    key = s_exact[par][0];
+#pragma unroll
+    for (int q = 1; q < QC_COLS; ++q)
+      if (s_exact[par][q] > key || (s_exact[par][q] == key && s_pos[par][q] < s_pos[par][c])) {
+        key = s_exact[par][q];
+        c = q;
+      }
+    return c;
+  };
+
+  // warp 4: this CTA's bid to all, theirs, the pivot of step k
+  auto pick_pivot = [&](int k) {
+    const int par = k & 1;
+    const unsigned tag = run * 2048u + (unsigned)k + 1u;
+    qc_sync(QC_B_BIDS, QC_COLS + 1);
+    long long key, bound;
+    bool open;
+    int c = cta_best(par, key, open, bound);
+    // a mailbox per receiver: polled by one CTA each, where common slots would
+    // serialise 150 pollers in a few L2 slices
+    auto publish = [&](long long kq, unsigned meta) {
+      for (int e = lane; e < G; e += 32)
+        qc_store16(slot + (((size_t)par * G + e) * G + blockIdx.x) * 2, (unsigned long long)kq,
+                   (unsigned long long)tag << 32 | meta);
+    };
+    if (open) {
+      publish(bound, 0x80000000u);
+      qc_sync(QC_B_EXACT, QC_COLS + 1);
+      c = cta_best_exact(par, key);
+    }
+    publish(key, (unsigned)(s_pos[par][c] << 16 | s_phys[par][c]));
+    const unsigned long long* sl = slot + ((size_t)par * G + blockIdx.x) * G * 2;
+    unsigned long long kk[QC_SLOTS], mm[QC_SLOTS];
+    unsigned have = 0;
+#pragma unroll
+    for (int u = 0; u < QC_SLOTS; ++u)
+      if (lane + 32 * u >= G) { have |= 1u << u; kk[u] = (unsigned long long)QC_NONE; mm[u] = 0xFFFFFFFFull; }
+    for (int it = 0;; ++it) {
+#pragma unroll
+      for (int u = 0; u < QC_SLOTS; ++u)
+        if (!(have >> u & 1)) qc_load16(sl + 2 * (lane + 32 * u), kk[u], mm[u]);
+#pragma unroll
+      for (int u = 0; u < QC_SLOTS; ++u)
+        if ((unsigned)(mm[u] >> 32) == tag) have |= 1u << u;
+      if (__all_sync(0xffffffffu, have == (1u << QC_SLOTS) - 1)) break;
+      if (it >= QC_POLLS || ((it & 1023) == 1023 && (*abort || (*(volatile int*)w.err & DQMC_KERR_BARRIER_TIMEOUT)))) {
+        give_up();
+        break;
+      }
+    }
+    __syncwarp();
+    // the best; a bound that is best (m < 0, before equal exact norms) is waited for
+    long long bk;
+    int bm, bc;
+    for (int it = 0;; ++it) {
+      bk = QC_NONE;
+      bm = 0x7FFFFFFF;
+      bc = 0;
+#pragma unroll
+      for (int u = 0; u < QC_SLOTS; ++u) {
+        const int m = (int)(unsigned)mm[u];
+        if (lane + 32 * u < G && ((long long)kk[u] > bk || ((long long)kk[u] == bk && m < bm))) {
+          bk = (long long)kk[u]; bm = m; bc = lane + 32 * u;
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const long long ok = __shfl_xor_sync(0xffffffffu, bk, o);
+        const int om = __shfl_xor_sync(0xffffffffu, bm, o), oc = __shfl_xor_sync(0xffffffffu, bc, o);
+        if (ok > bk || (ok == bk && om < bm)) { bk = ok; bm = om; bc = oc; }
+      }
+      if (bm >= 0) break;
+      if (it >= QC_POLLS || ((it & 1023) == 1023 && (*abort || (*(volatile int*)w.err & DQMC_KERR_BARRIER_TIMEOUT)))) {
+        give_up();
+        break;
+      }
+#pragma unroll
+      for (int u = 0; u < QC_SLOTS; ++u)
+        if (lane + 32 * u < G && (int)(unsigned)mm[u] < 0) qc_load16(sl + 2 * (lane + 32 * u), kk[u], mm[u]);
+    }
+    if (lane == 0) {
+      s_win[par][0] = bc;
+      s_win[par][1] = (bm >> 16) & 0x7FFF;
+      s_win[par][2] = min(bm & 0xFFFF, n - 1);
+    }
+    __syncwarp();
+  };
+
+  if (wid < QC_COLS) {
+    // ---- a column ----
+    const int i0 = blockIdx.x + G * wid;
+    bool active = i0 < n - k0;
+    int pos = k0 + i0, phys = 0;
+    cplx x[NQ];
+    double vn1 = 0.0, vn2 = 0.0, inv1 = 0.0, inv2 = 0.0;
+    if (active) {
+      phys = k0 ? __ldcg(&w.order[pos]) : pos;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        const int r = base + lane + 32 * q;
+        x[q] = r < n ? ldcg_c(&A[(size_t)phys * n + r]) : cmake(0.0, 0.0);
+      }
+      if (k0) {
+        vn1 = __ldcg(&w.vn1[phys]); vn2 = __ldcg(&w.vn2[phys]);
+        inv1 = __ldcg(&w.vn1[n + phys]); inv2 = __ldcg(&w.vn2[n + phys]);
+      } else {
+        double s = 0.0;
+        for (int r = lane; r < n; r += 32) s += cabs2(A[(size_t)phys * n + r]);
+        s = warp_sum(s);
+        vn1 = sqrt(s);
+        inv1 = vn1 > 0.0 ? 1.0 / vn1 : 0.0;
+        vn2 = vn1;
+        inv2 = inv1;
+      }
+    }
+    const double tol3z = sqrt(DBL_EPSILON);
+    bool pending = false, deferred = false;   // the update by the step before; its norm too
+    cplx f = cmake(0.0, 0.0), fs = cmake(0.0, 0.0);
+    // x -= c v of step k (c = f at r = k, fs below, v_k = 1); TAIL: squares below row k
+    // pub: the new rows below k go to this CTA's published column of step k + 1
+    auto publish = [&](int k, int q) {
+      const unsigned tag = run * 2048u + (unsigned)k + 1u;
+      unsigned long long* p = cols + (((size_t)(k & 1) * G + blockIdx.x) * rows + 32 * q + lane) * 4;
+      asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(qc_word(tag, __double2hiint(x[q].x))),
+                   "l"(qc_word(tag, __double2loint(x[q].x)))
+                   : "memory");
+      asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p + 2),
+                   "l"(qc_word(tag, __double2hiint(x[q].y))), "l"(qc_word(tag, __double2loint(x[q].y)))
+                   : "memory");
+    };
+    auto update = [&](int k, auto tail, bool pub) {
+      const cplx* v = vbuf + (size_t)(k & 1) * rows;
+      double tp = 0.0;
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        if (base + 32 * q + 31 < k || base + 32 * q >= n) continue;   // warp-uniform
+        const int r = base + lane + 32 * q;
+        if (r >= k && r < n) {
+          const cplx vr = r == k ? cmake(1.0, 0.0) : v[r - base];
+          const cplx c = r == k ? f : fs;
+          x[q] = cmake(fma(-c.x, vr.x, fma(c.y, vr.y, x[q].x)), fma(-c.x, vr.y, fma(-c.y, vr.x, x[q].y)));
+          if (decltype(tail)::value && r > k) tp = fma(x[q].x, x[q].x, fma(x[q].y, x[q].y, tp));
+          if (pub && r > k) publish(k + 1, q);
+        }
+      }
+      return tp;
+    };
+    for (int k = k0; k < n; ++k) {
+      const int par = k & 1, d = k - base;
+      const unsigned tag = run * 2048u + (unsigned)k + 1u;
+      if (lane == 0) {
+        // a deferred norm is below vn2 sqrt(tol3z): twice that as a power of two
+        s_key[par][wid] = !active ? QC_NONE : qc_key(deferred ? vn2 * 0x1p-12 : vn1);
+        s_def[par][wid] = deferred ? 1 : 0;
+        s_pos[par][wid] = pos;
+        s_phys[par][wid] = phys;
+      }
+      qc_sync(QC_B_BIDS, QC_COLS + 1);
+      long long best, bound;
+      bool open;
+      int cw = cta_best(par, best, open, bound);
+      const bool early = active && !open && cw == wid;   // this column is the CTA's bid
+      if (deferred) {
+        const double tp = update(k - 1, std::true_type{}, false);
+        const double tail = warp_sum(__shfl_sync(0xffffffffu, tp, (lane + d - 1) & 31));
+        vn1 = sqrt(tail);   // k - 1 < n - 1
+        inv1 = vn1 > 0.0 ? 1.0 / vn1 : 0.0;
+        vn2 = vn1;
+        inv2 = inv1;
+      } else if (pending) {
+        update(k - 1, std::false_type{}, early);
+      }
+      if (open) {   // uniform over the CTA
+        if (lane == 0) s_exact[par][wid] = active ? qc_key(vn1) : QC_NONE;
+        qc_sync(QC_B_EXACT, QC_COLS + 1);
+        cw = cta_best_exact(par, best);
+      }
+      if (active && cw == wid && !(early && pending)) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          const int r = base + lane + 32 * q;
+          if (r >= k && r < n) publish(k, q);
+        }
+      }
+      pending = deferred = false;
+      // this column's element of row k, for all lanes
+      cplx ak = cmake(0.0, 0.0);
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        ak.x = qc_select(q, d >> 5, x[q].x, ak.x);
+        ak.y = qc_select(q, d >> 5, x[q].y, ak.y);
+      }
+      ak = cmake(__shfl_sync(0xffffffffu, ak.x, d & 31), __shfl_sync(0xffffffffu, ak.y, d & 31));
+      const int rot = (lane + d) & 31;   // the lane with k_qrp's rows k + lane, k + lane + 32, ...
+      qc_sync(QC_B_COL + wid, 1 + QC_HELP);   // pivot known, its column in vbuf
+      const int wpos = s_win[par][1];
+      cplx s0 = cmake(0.0, 0.0);
+      if (active && pos == wpos) {
+        // the pivot: its rows above k are final
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          const int r = base + lane + 32 * q;
+          if (r < k) A[(size_t)phys * n + r] = x[q];
+        }
+        active = false;
+      } else if (active) {
+        if (pos == k) pos = wpos;
+        const cplx* v = vbuf + (size_t)par * rows;
+        cplx sp = cmake(0.0, 0.0);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+          if (base + 32 * q + 31 <= k || base + 32 * q >= n) continue;   // warp-uniform
+          const int r = base + lane + 32 * q;
+          if (r > k && r < n) sp = cfma_conj(v[r - base], x[q], sp);
+        }
+        s0 = warp_sum_c(cmake(__shfl_sync(0xffffffffu, sp.x, rot), __shfl_sync(0xffffffffu, sp.y, rot)));
+      }
+      qc_sync(QC_B_COLTAU + wid, 2);   // tau, scal
+      if (active) {
+        const cplx ctau = cconj(s_tau[par]), scal = s_scal[par];
+        // v^H a = a_k + conj(scal) s0
+        const cplx s = cfma_conj(scal, s0, ak);
+        f = cmul(ctau, s);     // a_k -= f
+        fs = cmul(f, scal);    // a_r -= f scal x_r, r > k
+        pending = true;
+        if (vn1 != 0.0) {      // the norm downdate of qr_finish_column
+          const cplx xk = csub(ak, f);
+          double temp = 1.0 - (cabs2(xk) * inv1) * inv1;
+          temp = temp > 0.0 ? temp : 0.0;
+          const double r2 = vn1 * inv2;
+          if (temp * r2 * r2 <= tol3z) {
+            deferred = true;   // recomputed beside the exchange of the next step
+          } else {
+            const double rs = rsqrt(temp);
+            vn1 = vn1 * temp * rs;
+            inv1 = inv1 * rs;
+          }
+        }
+      }
+    }
+  } else {
+    // ---- the other warps ----
+    const int hw = wid - QC_COLS, tid = 32 * hw + lane, chunk = (n + G - 1) / G;
+    constexpr int T = 32 * QC_HELP, U = (32 * NQ + T - 1) / T;
+    for (int k = k0; k < n; ++k) {
+      const int par = k & 1;
+      const unsigned tag = run * 2048u + (unsigned)k + 1u;
+      if (hw == 0) pick_pivot(k);
+      qc_sync(QC_B_PIVOT, QC_HELP);
+      // the pivot column; thread t holds rows k + t, k + t + 256, ... (as in k_qrp)
+      cplx* v = vbuf + (size_t)par * rows;
+      const unsigned long long* src = cols + ((size_t)par * G + s_win[par][0]) * rows * 4;
+      unsigned have = 0;
+      double xn2 = 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k + tid + T * u >= n) have |= 1u << u;
+      const unsigned mine = ~have;
+      cplx z[U];
+      for (int it = 0; have != (1u << U) - 1; ++it) {
+        unsigned long long q0[U], q1[U], q2[U], q3[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (!(have >> u & 1)) {
+            const unsigned long long* p = src + (size_t)(k + tid + T * u - base) * 4;
+            asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(q0[u]), "=l"(q1[u]) : "l"(p) : "memory");
+            asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(q2[u]), "=l"(q3[u]) : "l"(p + 2) : "memory");
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (!(have >> u & 1) && (unsigned)(q0[u] >> 32) == tag && (unsigned)(q1[u] >> 32) == tag &&
+              (unsigned)(q2[u] >> 32) == tag && (unsigned)(q3[u] >> 32) == tag) {
+            have |= 1u << u;
+            z[u] = cmake(__hiloint2double((int)(unsigned)q0[u], (int)(unsigned)q1[u]),
+                         __hiloint2double((int)(unsigned)q2[u], (int)(unsigned)q3[u]));
+            v[k + tid + T * u - base] = z[u];
+          }
+        if (it >= QC_POLLS || ((it & 1023) == 1023 && *abort)) {
+          if (have != (1u << U) - 1) give_up();
+          break;
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < QC_COLS; ++c) qc_arrive(QC_B_COL + c, 1 + QC_HELP);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if ((mine & have) >> u & 1)
+          if (u > 0 || tid > 0) xn2 = fma(z[u].x, z[u].x, fma(z[u].y, z[u].y, xn2));
+      xn2 = warp_sum(xn2);
+      if (lane == 0) s_norm[hw] = xn2;
+      __syncwarp();
+      if (hw != 1) {
+        qc_arrive(QC_B_NORMS, QC_HELP);
+      } else {
+        qc_sync(QC_B_NORMS, QC_HELP);
+        // zlarfg, as in k_qrp
+        double t = lane < QC_HELP ? s_norm[lane] : 0.0;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        const cplx alpha = v[k - base];
+        double beta;
+        cplx tau, scal;
+        if (t == 0.0 && alpha.y == 0.0) {
+          tau = cmake(0.0, 0.0);
+          beta = alpha.x;
+          scal = cmake(0.0, 0.0);
+        } else {
+          const double nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + t);
+          beta = alpha.x >= 0.0 ? -nrm : nrm;
+          const double rb = 1.0 / beta;
+          tau = cmake((beta - alpha.x) * rb, -alpha.y * rb);
+          const double an = fabs(rb);
+          const cplx dd = cmake((alpha.x - beta) * an, alpha.y * an);
+          const double rd = an / (dd.x * dd.x + dd.y * dd.y);
+          scal = cmake(dd.x * rd, -dd.y * rd);
+        }
+        if (lane == 0) {
+          s_tau[par] = tau;
+          s_scal[par] = scal;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < QC_COLS; ++c) qc_arrive(QC_B_COLTAU + c, 2);
+        if (lane == 0 && blockIdx.x == 0) {
+          w.tau[k] = tau;
+          w.beta[k] = beta;
+          w.order[k] = s_win[par][2];
+        }
+      }
+      qc_sync(QC_B_TAU, QC_HELP);
+      const cplx scal = s_scal[par];
+      const int r1 = min(n, ((int)blockIdx.x + 1) * chunk);
+      for (int r = blockIdx.x * chunk + tid; r < r1; r += T)
+        w.V[(size_t)k * n + r] = r < k ? cmake(0.0, 0.0) : (r == k ? cmake(1.0, 0.0) : cmul(v[r - base], scal));
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {   // the last CTA out counts the launch
+    __threadfence();
+    if (atomicAdd(&w.bar->exits, 1u) == (unsigned)G - 1) {
+      w.bar->exits = 0;
+      *w.run = run & 0xFFFFFu;
+      __threadfence();
+    }
+  }
 }
 
 // T (physical layout) = D^-1 R, zero below the logical diagonal; D = |beta|.
@@ -890,23 +1353,59 @@ cudaError_t launch_zgemm(int m, int nn, int k, char opA, char opB, cplx alpha, c
   return cudaGetLastError();
 }
 
-cudaError_t launch_qrp(cplx* A, int n, QRWork& w, int sm_count, cudaStream_t st, int max_grid) {
-  if (n > 32 * QR_MAXT) return cudaErrorInvalidValue;
-  size_t smem = (size_t)n * (sizeof(cplx) + sizeof(int));
-  static SmemLimit smem_limit;
-  if (cudaError_t ea = smem_limit.raise((const void*)k_qrp, 64 * 1024); ea != cudaSuccess) return ea;
-  int per_sm = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_qrp, QR_THREADS, smem);
-  if (e != cudaSuccess) return e;
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  int grid = sm_count;   // one CTA per SM; remaining columns are dealt round-robin over all CTAs
+// Columns that k_qr_cols can hold (0: none) and the words of its published columns.
+static int qr_resident_columns(int n, int sm_count, int max_grid) {
+  int grid = sm_count < 32 * QC_SLOTS ? sm_count : 32 * QC_SLOTS;
   if (max_grid > 0 && grid > max_grid) grid = max_grid;
-  if (grid > 32 * CAND_PER_LANE) grid = 32 * CAND_PER_LANE;
-  QRWork copy = w;
-  void* args[] = {&A, &n, &copy};
-  return cudaLaunchCooperativeKernel((void*)k_qrp, dim3(grid), dim3(QR_THREADS), args, smem, st);
+  const int held = QC_COLS * grid;
+  if (held >= n) return n;
+  return max_grid > 0 ? 0 : held;   // chains that share the GPU: all of the columns or none
+}
+size_t qr_column_words(int n, int sm_count) {
+  const int held = qr_resident_columns(n, sm_count, 0), base = (n - held) & ~31;
+  return (size_t)2 * ((held + QC_COLS - 1) / QC_COLS) * (n - base) * 4;
 }
 
+template <int NQ>
+static cudaError_t launch_qr_cols(cplx* A, int n, int k0, QRWork& w, cudaStream_t st) {
+  const int base = k0 & ~31, grid = (n - k0 + QC_COLS - 1) / QC_COLS;
+  QRWork copy = w;
+  void* args[] = {&A, &n, &k0, &copy};
+  return cudaLaunchCooperativeKernel((void*)k_qr_cols<NQ>, dim3(grid), dim3(QC_THREADS), args,
+                                     (size_t)2 * (n - base) * sizeof(cplx), st);
+}
+
+// The last columns, as many as the SMs hold, by k_qr_cols; k_qrp takes the steps
+// before (n > 608 on 152 SMs) or, where the held ones are too few, all.
+cudaError_t launch_qrp(cplx* A, int n, QRWork& w, int sm_count, cudaStream_t st, int max_grid, int* kernels) {
+  if (n > 32 * QR_MAXT) return cudaErrorInvalidValue;
+  int held = qr_resident_columns(n, sm_count, max_grid), kend = n - held;
+  *kernels = (kend > 0 ? 1 : 0) + (held > 0 ? 1 : 0);
+  if (kend > 0) {
+    size_t smem = (size_t)n * (sizeof(cplx) + sizeof(int));
+    static SmemLimit smem_limit;
+    if (cudaError_t ea = smem_limit.raise((const void*)k_qrp, 64 * 1024); ea != cudaSuccess) return ea;
+    int per_sm = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_qrp, QR_THREADS, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    int grid = sm_count;   // one CTA per SM; remaining columns are dealt round-robin over all CTAs
+    if (max_grid > 0 && grid > max_grid) grid = max_grid;
+    if (grid > 32 * CAND_PER_LANE) grid = 32 * CAND_PER_LANE;
+    QRWork copy = w;
+    void* args[] = {&A, &n, &kend, &copy};
+    e = cudaLaunchCooperativeKernel((void*)k_qrp, dim3(grid), dim3(QR_THREADS), args, smem, st);
+    if (e != cudaSuccess || held == 0) return e;
+  }
+  const int nq = (n - (kend & ~31) + 31) / 32;   // at most 21 (640 held columns)
+  if (nq <= 2) return launch_qr_cols<2>(A, n, kend, w, st);
+  if (nq <= 5) return launch_qr_cols<5>(A, n, kend, w, st);
+  if (nq <= 8) return launch_qr_cols<8>(A, n, kend, w, st);
+  if (nq <= 13) return launch_qr_cols<13>(A, n, kend, w, st);
+  if (nq <= 18) return launch_qr_cols<18>(A, n, kend, w, st);
+  if (nq <= 21) return launch_qr_cols<21>(A, n, kend, w, st);
+  return cudaErrorInvalidValue;
+}
 cudaError_t launch_qrp_finalize(cplx* A, cplx* T, double* D, int n, const QRWork& w, cudaStream_t st) {
   k_qrp_finalize<<<grid_for((size_t)n * n), 256, n * sizeof(int), st>>>(A, T, D, n, w.order, w.beta);
   return cudaGetLastError();

@@ -118,6 +118,9 @@ struct QRWork {
   double* cand_v;    // (2 grid) per-CTA pivot candidates, by step parity: norm
   int* cand_q;       // (2 grid) and logical position
   unsigned long long* refl;   // (2 grid, 10) and their reflectors
+  unsigned long long* slots;  // k_qr_cols: (2, grid, grid, 2) candidates and
+  unsigned long long* cols;   // (2 grid, rows, 4) their columns, under tags
+  unsigned* run;              // launches of k_qr_cols
   GridBarrier* bar;
   int* err;
 };
@@ -126,7 +129,8 @@ struct QRWork {
 // logical position of each physical column) holds R in physical column
 // order; V/tau hold the reflectors; order/beta the pivots and diag(R).
 // max_grid > 0 caps the cooperative grid (chains sharing the GPU)
-cudaError_t launch_qrp(cplx* A, int n, QRWork& w, int sm_count, cudaStream_t st, int max_grid = 0);
+cudaError_t launch_qrp(cplx* A, int n, QRWork& w, int sm_count, cudaStream_t st, int max_grid, int* kernels);
+size_t qr_column_words(int n, int sm_count);   // size of QRWork::cols
 // After launch_qrp: D[k] = |beta[k]|, T (physical layout) = D^-1 R with zeros below.
 cudaError_t launch_qrp_finalize(cplx* A, cplx* T, double* D, int n, const QRWork& w, cudaStream_t st);
 // X (m x n) <- X * Q  with Q = H_0 ... H_{n-1} (reflectors in w).  Also used
