@@ -78,7 +78,7 @@ struct dqmc_handle {
   int* wsite = nullptr;       // (WIN_MAX) accepted sites of the window
   cplx* wk = nullptr;         // (WIN_MAX, 16) and (WIN_MAX, 4, 4 WIN_MAX): their blocks and rows (DelayedArgs)
   cplx* wrow = nullptr;
-  int* wflag = nullptr;       // (WIN_MAX + 1) published acceptances, (1) followers' arrivals
+  int* wflag = nullptr;       // (WIN_MAX + 1) published acceptances, (2) followers' arrivals, clusters started
   bool follow = false;        // the windows' factors are formed by follower clusters of the same launch
   double* wexp = nullptr;     // (WIN_MAX) and their exp(-dS)
   int greens_method = DQMC_GREENS_SCALES;
@@ -1324,7 +1324,7 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
     A((void**)&h->wk, (size_t)WIN_MAX * 16 * sizeof(cplx));
     A((void**)&h->wexp, WIN_MAX * sizeof(double));
     A((void**)&h->wrow, (size_t)WIN_MAX * 16 * WIN_MAX * sizeof(cplx));
-    A((void**)&h->wflag, (WIN_MAX + 2) * sizeof(int));
+    A((void**)&h->wflag, (WIN_MAX + 3) * sizeof(int));
     if (ok) h->follow = local_window_follows((int)n, h->delay);
   }
   A((void**)&h->wy_v, (size_t)n * kWyMax * sizeof(cplx));

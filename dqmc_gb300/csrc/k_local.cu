@@ -753,36 +753,32 @@ __host__ __device__ constexpr int fac_follow_smem(int n, int k) {
 // each (64 to issue one).  The kernel this replaces formed all n rows and
 // columns of each acceptance before the next decision and took 7.6 us per
 // accepted and 3.6 us per rejected site at n = 1024.
-__global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a, DelayedArgs d, int W) {
+__global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a, DelayedArgs d, int W, int C) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
-  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int rank = (int)cl.block_rank();
   const ModelConst& mc = a.mc;
   const int N = mc.N, n = mc.n, L = mc.L;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if ((int)cl.num_blocks() != C) {   // not the clusters that shared memory was sized for
+    if (tid == 0) atomicOr(a.err, DQMC_KERR_BAD_SHAPE);
+    return;
+  }
   const int first = __ldcg(&d.state[0]);
   extern __shared__ double4_16a smem_win[];
   const int followers = (int)gridDim.x - C;   // their CTAs, in clusters after the window's
   if (first >= N) {   // slice done (uniform over the grid): nothing for the flush either
-    if (blockIdx.x == 0 && tid == 0) d.state[1] = 0;
+    if (blockIdx.x == 0 && tid == 0) d.state[1] = 0;   // read by nobody in this launch
     return;
   }
-  if ((int)blockIdx.x >= C) {
-    __syncthreads();
-    if (tid == 0) {   // the state has been read: the window may advance it
-      __threadfence();
-      atomicAdd(d.arrive, 1);
-    }
-    const int blk = (int)blockIdx.x - C, vpc = fac_vpc(n);
-    cplx* sm = reinterpret_cast<cplx*>(smem_win);
-    if (vpc == 4) {
-      if (wid < 4) fac_follow<4, 4>(a, d, first, blk, sm);
-    } else if (vpc == 8) {
-      fac_follow<4, 8>(a, d, first, blk, sm);
-    } else {
-      fac_follow<2, 8>(a, d, first, blk, sm);
-    }
-    return;
+  // With followers, the first cluster to start takes the window: whoever waits
+  // then waits for a cluster that runs, in whatever order clusters are placed.
+  // Every cluster loads the window meanwhile.
+  __shared__ int s_ticket;
+  int ticket = 0;
+  if (followers > 0) {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (rank == 0 && tid == 0) ticket = atomicAdd(d.arrive + 1, 1);
   }
   const int we = min(W, N - first);                       // sites of this window
   const int owned = rank < we ? (we - rank + C - 1) / C : 0;   // sites rank + t C
@@ -814,7 +810,27 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
   }
   for (int e = tid; e < 3 * we; e += WIN_THREADS) prop[e] = a.delta[3 * first + e];
   for (int e = tid; e < 3 * N; e += WIN_THREADS) phis[e] = __ldcg(&a.phi[(size_t)3 * N * a.slice0 + e]);
+  if (followers > 0) {
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every CTA of the cluster runs
+    if (rank == 0 && tid < C) *cl.map_shared_rank(&s_ticket, tid) = __shfl_sync((1u << C) - 1, ticket, 0);
+  }
   cl.sync();   // also: every CTA of the cluster runs before its shared memory is written remotely
+  if (followers > 0 && s_ticket > 0) {
+    if (tid == 0) {   // the state has been read: the window may advance it
+      __threadfence();
+      atomicAdd(d.arrive, 1);
+    }
+    const int blk = (s_ticket - 1) * C + rank, vpc = fac_vpc(n);
+    cplx* sm = reinterpret_cast<cplx*>(smem_win);
+    if (vpc == 4) {
+      if (wid < 4) fac_follow<4, 4>(a, d, first, blk, sm);
+    } else if (vpc == 8) {
+      fac_follow<4, 8>(a, d, first, blk, sm);
+    } else {
+      fac_follow<2, 8>(a, d, first, blk, sm);
+    }
+    return;
+  }
 
   const int part = lane & 1, r = lane >> 3, c = (lane >> 1) & 3;   // this lane's component of a 4x4 block
   int cur = 0, p = 0;
@@ -1086,7 +1102,8 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
       bool here = false;
       for (int it = 0; it < kClusterPolls && !here; ++it) here = *(volatile int*)d.arrive == followers;
       if (!here) atomicOr(a.err, DQMC_KERR_BARRIER_TIMEOUT);
-      *(volatile int*)d.arrive = 0;
+      d.arrive[0] = 0;
+      d.arrive[1] = 0;
     }
     __syncwarp();
     // the tracked action: -log(exp(-dS)) of the accepted sites, added in order
@@ -1211,20 +1228,14 @@ cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, 
   if (max_cluster > 0 && C > 8 && max_cluster < C) C = 8;
   const int W = local_window_sites(d.k);
   size_t smem = window_smem(a.mc.N, W, C);
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];
   if (follow) {
     const size_t fs = (size_t)fac_follow_smem(a.mc.n, d.k) * sizeof(cplx);
     if (fs > smem) smem = fs;
   }
   cudaLaunchConfig_t cfg = window_config(attr, C, smem, st);
-  if (follow) {
-    // cooperative: the followers wait on the window's cluster, so all are resident together
-    cfg.gridDim = dim3(C * (1 + follower_clusters(a.mc.n, C)));
-    attr[1].id = cudaLaunchAttributeCooperative;
-    attr[1].val.cooperative = 1;
-    cfg.numAttrs = 2;
-  }
-  return cudaLaunchKernelEx(&cfg, k_local_window, a, d, W);
+  if (follow) cfg.gridDim = dim3(C * (1 + follower_clusters(a.mc.n, C)));
+  return cudaLaunchKernelEx(&cfg, k_local_window, a, d, W, C);
 }
 
 bool local_window_follows(int n, int k) {

@@ -80,7 +80,7 @@ struct DelayedArgs {
   double* wexp;            // (WIN_MAX) their exp(-dS)
   cplx* wrow;              // (WIN_MAX, 4, 4 WIN_MAX) their rows of the window's block (k_local_window)
   int* wflag;              // (WIN_MAX + 1) acceptances published to the follower clusters
-  int* arrive;             // followers that have read the state (zero between launches)
+  int* arrive;             // (2) followers that have read the state, clusters started (zero between launches)
   OzSlices sl;             // the flush's slices, cut by launch_local_factors
                            // (sl.As null: X and Y are stored and the flush slices them itself)
 };
