@@ -1139,6 +1139,11 @@ constexpr int TRSM_DB_WARPS = 8;   // all stage the triangle; the first `warps` 
 __device__ __forceinline__ int trsm_pack_lower(int q, int b) { return q * (b - 1) - q * (q - 1) / 2; }
 __device__ __forceinline__ int trsm_pack_upper(int q) { return q * (q - 1) / 2; }
 
+// a b with the multiply-adds spelled out (which product a compiler contracts depends on the context)
+__device__ __forceinline__ cplx trsm_scale(cplx a, cplx b) {
+  return cmake(__fma_rn(a.x, b.x, -__dmul_rn(a.y, b.y)), __fma_rn(a.y, b.x, __dmul_rn(a.x, b.y)));
+}
+template <int NS>   // slots of 32 rows, b <= 32 NS
 __global__ void __launch_bounds__(32 * TRSM_DB_WARPS) k_trsm_diag_block(const cplx* __restrict__ T, int ldT,
                                                                        const cplx* __restrict__ rdiag,
                                                                        cplx* __restrict__ Y, int ldY, int j0, int b,
@@ -1170,49 +1175,85 @@ __global__ void __launch_bounds__(32 * TRSM_DB_WARPS) k_trsm_diag_block(const cp
   const int col = blockIdx.x * warps + wid;
   if (wid >= warps || col >= m) return;
   cplx* yg = Y + (size_t)col * ldY + j0;
-  cplx y[4];
+  cplx y[NS];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < NS; ++i) {
     const int r = lane + 32 * i;
     y[i] = r < b ? yg[r] : cmake(0.0, 0.0);
   }
-  auto bcast = [&](int q) {
-    const int slot = q >> 5, src = q & 31;
-    const cplx v = slot == 0 ? y[0] : slot == 1 ? y[1] : slot == 2 ? y[2] : y[3];
+  auto bcast = [&](cplx v, int src) {
     return cmake(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
   };
+  auto sub = [&](cplx& v, cplx yq, cplx t) {
+    v = cmake(fma(-yq.x, t.x, fma(yq.y, t.y, v.x)), fma(-yq.x, t.y, fma(-yq.y, t.x, v.y)));
+  };
+  // Column q of the triangle is read one step ahead, and the slot that holds
+  // the next step's row is updated first: the chain of a step is then a shuffle
+  // and two FMAs (upper: four), about 200 cycles, and the FP64 issue of the
+  // slots, 256 cycles each, is what is left.  Solves of b rows, us, before -> now:
+  // b = 64 lower 34 -> 21, upper 44 -> 31 (m <= 608), upper 69 -> 44 (m = 1024);
+  // b = 128 upper 89 -> 79.
+  cplx t[NS], tn[NS];
   if (lower) {
-    for (int q = 0; q < b - 1; ++q) {
-      const cplx yq = bcast(q);
+    auto load = [&](int q, cplx (&o)[NS]) {
       const cplx* tq = tp + trsm_pack_lower(q, b) - q - 1;   // tq[r], r > q
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (32 * i + 31 <= q || 32 * i >= b) continue;   // warp-uniform
+      for (int i = 0; i < NS; ++i) {
         const int r = lane + 32 * i;
-        if (r > q && r < b) {
-          const cplx t = tq[r];
-          y[i] = cmake(fma(-yq.x, t.x, fma(yq.y, t.y, y[i].x)), fma(-yq.x, t.y, fma(-yq.y, t.x, y[i].y)));
+        if (r > q && r < b) o[i] = tq[r];
+      }
+    };
+    load(0, tn);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      for (int j = 0; j < 32; ++j) {
+        const int q = 32 * s + j;
+        if (q >= b - 1) break;
+#pragma unroll
+        for (int i = s; i < NS; ++i) t[i] = tn[i];
+        const cplx yq = bcast(y[s], j);
+        load(q + 1, tn);
+#pragma unroll
+        for (int i = s; i < NS; ++i) {
+          const int r = lane + 32 * i;
+          if (r > q && r < b) sub(y[i], yq, t[i]);
         }
       }
     }
   } else {
-    for (int q = b - 1; q >= 0; --q) {
-      const cplx yq = cmul(bcast(q), rd[q]);
+    auto load = [&](int q, cplx (&o)[NS]) {
       const cplx* tq = tp + trsm_pack_upper(q);   // tq[r], r < q
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (32 * i > q) continue;   // warp-uniform
+      for (int i = 0; i < NS; ++i) {
         const int r = lane + 32 * i;
-        if (r == q) y[i] = yq;
-        else if (r < q) {
-          const cplx t = tq[r];
-          y[i] = cmake(fma(-yq.x, t.x, fma(yq.y, t.y, y[i].x)), fma(-yq.x, t.y, fma(-yq.y, t.x, y[i].y)));
+        if (r < q) o[i] = tq[r];
+      }
+    };
+    load(b - 1, tn);
+    cplx dn = rd[b - 1];
+#pragma unroll
+    for (int s = NS - 1; s >= 0; --s) {
+      for (int j = 31; j >= 0; --j) {
+        const int q = 32 * s + j;
+        if (q >= b) continue;
+#pragma unroll
+        for (int i = 0; i <= s; ++i) t[i] = tn[i];
+        const cplx yq = trsm_scale(bcast(y[s], j), dn);
+        if (q > 0) {
+          load(q - 1, tn);
+          dn = rd[q - 1];
+        }
+#pragma unroll
+        for (int i = s; i >= 0; --i) {
+          const int r = lane + 32 * i;
+          if (r == q) y[i] = yq;
+          else if (r < q) sub(y[i], yq, t[i]);
         }
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < NS; ++i) {
     const int r = lane + 32 * i;
     if (r < b) yg[r] = y[i];
   }
@@ -1434,9 +1475,12 @@ cudaError_t launch_trsm_diag_block(const cplx* T, int ldT, const cplx* rdiag, cp
   if (b < 1 || b > 128) return cudaErrorInvalidValue;
   if (!lower && !rdiag) return cudaErrorInvalidValue;
   const size_t smem = ((size_t)b * (b - 1) / 2 + b) * sizeof(cplx);
-  static SmemLimit smem_limit;
   constexpr int kMaxTdb = (int)((128 * 127 / 2 + 128) * sizeof(cplx));   // b = 128
-  if (cudaError_t ea = smem_limit.raise((const void*)k_trsm_diag_block, kMaxTdb); ea != cudaSuccess) return ea;
+  static SmemLimit smem_limits[3];
+  const int which = b <= 32 ? 0 : (b <= 64 ? 1 : 2);
+  void (*const kernels[3])(const cplx*, int, const cplx*, cplx*, int, int, int, int, int, int) = {
+      k_trsm_diag_block<1>, k_trsm_diag_block<2>, k_trsm_diag_block<4>};
+  if (cudaError_t ea = smem_limits[which].raise((const void*)kernels[which], kMaxTdb); ea != cudaSuccess) return ea;
   // one column per warp and as few warps per SM as the m columns allow: a
   // solve is a chain of b FP64 steps, and warps that share a sub-partition
   // double it (m = 256, b = 64: 32 CTAs of 8 warps 48 and 79 us, lower and upper)
@@ -1447,8 +1491,8 @@ cudaError_t launch_trsm_diag_block(const cplx* T, int ldT, const cplx* rdiag, cp
   }
   int warps = (m + sms - 1) / sms;
   if (warps > TRSM_DB_WARPS) warps = TRSM_DB_WARPS;
-  k_trsm_diag_block<<<(m + warps - 1) / warps, 32 * TRSM_DB_WARPS, smem, st>>>(T, ldT, rdiag, Y, ldY, j0, b, m,
-                                                                              lower ? 1 : 0, warps);
+  kernels[which]<<<(m + warps - 1) / warps, 32 * TRSM_DB_WARPS, smem, st>>>(T, ldT, rdiag, Y, ldY, j0, b, m,
+                                                                           lower ? 1 : 0, warps);
   return cudaGetLastError();
 }
 
