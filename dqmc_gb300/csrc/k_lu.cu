@@ -32,6 +32,7 @@ __device__ __forceinline__ cplx lu_mul(cplx a, cplx b) {
 }
 
 constexpr int LU_THREADS = 256;
+__device__ __forceinline__ void lu_bar() { asm volatile("bar.sync 1, 224;" ::: "memory"); }   // warps 1-7
 constexpr int LU_LDP = LU_PB + 4;   // row stride of the panel in shared memory: 8 lanes on 2 rows x 4 columns miss no bank
 constexpr int LU_MAXC = 16;
 
@@ -48,15 +49,17 @@ __device__ __forceinline__ double lu_join(unsigned hi, unsigned lo) { return __h
 // move: every CTA keeps the map between rows and their positions after the
 // exchanges, and the rows go to their positions when the panel is written.
 //
-// Per column: each CTA finds its candidate and pushes it to the others;
-// everyone polls for all of them and picks the same winner;
-// one warp forms 1 / pivot while two others read the rest of the pivot row
-// from its owner; then every CTA updates its own rows.
+// Per column: everyone polls for all candidates and picks the same winner; one
+// warp forms 1 / pivot while two others read the rest of the pivot row from its
+// owner; then warp 0 updates the next column, finds this CTA's candidate in it
+// and pushes it, beside the other warps' update of the remaining columns, whose
+// end is pushed as well (the pivot row is read only after it).
 //
-// Bound: about 4000-5000 cycles of latency per column (a remote store or load
-// takes 1000, the reciprocal 1000-2000), plus 4 multiply-adds per entry on 16
-// SMs.  The cooperative grids this replaces paid a grid barrier and three
-// round trips through L2 per column, 10000-15000 cycles.
+// Bound: about 4500 cycles of latency per column (a remote store or load takes
+// 1000, the reciprocal 1000-1500); the multiply-adds, 4 per entry on 16 SMs, fit
+// beside them.  Panel of 64 columns, us: in turn -> overlapped n = 144 198 -> @A,
+// n = 576 235 -> @B, n = 1024 229 -> @C.  The cooperative grids before paid a grid
+// barrier and three round trips through L2 per column, 10000-15000 cycles.
 //
 // UNBLOCKED false: A in place, L below the diagonal (scaled multipliers, a -= l
 // u), w.piv for the other columns.  true: the factors of zgetf2 as the trailing
@@ -76,8 +79,8 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
   int* pos = reinterpret_cast<int*>(prow + (size_t)chunk * LU_LDP);   // (R) row -> position
   int* rowat = pos + R;                                      // (R) position -> row
   __shared__ LuCand s_cand[2][LU_MAXC];
-  __shared__ cplx urow[LU_PB], s_rinv[LU_PB], s_piv[LU_PB];
-  __shared__ int s_win[2], s_pk[2];
+  __shared__ cplx urow[LU_PB], us[LU_PB], s_rinv[LU_PB], s_piv[LU_PB];   // us: urow / pivot
+  __shared__ int s_win[2], s_pk[2], s_ready[LU_MAXC], s_late;   // s_ready: steps that CTA has finished
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   for (int e = tid; e < nrw * b; e += LU_THREADS) {
     const int j = e / nrw, rr = e - j * nrw;
@@ -85,50 +88,56 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
   }
   for (int i = tid; i < R; i += LU_THREADS) { pos[i] = i; rowat[i] = i; }
   for (int e = tid; e < 2 * LU_MAXC * 8; e += LU_THREADS) s_cand[0][0].w[e] = 0ull;
+  if (tid < LU_MAXC) s_ready[tid] = 0;
+  if (tid == 0) s_late = 0;
   cl.sync();   // also: every CTA of the cluster runs before its shared memory is written remotely
 
-  // threads per row: rows padded to a power of two (chunk <= 128)
-  int tpr = LU_THREADS;
-  while (tpr * chunk > LU_THREADS) tpr >>= 1;
-  const int row = tid / tpr, sub = tid - row * tpr;
-  bool ok = true;
+  // warps 1-7: threads per row (chunk <= 128)
+  const int tpr = max(1, (LU_THREADS - 32) / chunk);
+  const int row = tid < 32 ? LU_THREADS : (tid - 32) / tpr, sub = (tid - 32) - row * tpr;
+  const bool works = row < nrw && row * tpr + sub < LU_THREADS - 32;
+  // warp 0: the candidate (or none) of this CTA for column kk, rows rr = lane, lane + 32, ...
+  double best = 0.0;
+  int pk = 0x7FFFFFFF;   // position << 16 | row; the positions of the candidates are distinct
+  auto consider = [&](int kk, int rr, int ps, cplx x) {
+    double a = fabs(x.x) + fabs(x.y);
+    if (ps == kk && __double2hiint(a) < 0) a = 0.0;   // NaN: no candidate, but some row always is
+    const int c = ps << 16 | (r0 + rr);
+    if (piv_better(a, c, best, pk)) { best = a; pk = c; }
+  };
+  auto push = [&](int kk) {
+    const int par = kk & 1;
+    warp_argmax(best, pk);
+    const bool any = pk != 0x7FFFFFFF;
+    __syncwarp();
+    const cplx x = any ? prow[((pk & 0xFFFF) - r0) * LU_LDP + kk] : cmake(0.0, 0.0);
+    // lane c < 16 stores the first three words at CTA c, lane c + 16 the other four
+    const int c = lane & 15;
+    const unsigned long long tag = (unsigned long long)(kk + 1) << 32;
+    if (c < C) {
+      unsigned long long* o = cl.map_shared_rank(&s_cand[par][q].w[0], c);
+      if (lane < 16) {
+        st_cluster(o, tag | (unsigned)__double2hiint(best));
+        st_cluster(o + 1, tag | (unsigned)__double2loint(best));
+        st_cluster(o + 2, tag | (unsigned)pk);
+      } else {
+        st_cluster(o + 3, tag | (unsigned)__double2hiint(x.x));
+        st_cluster(o + 4, tag | (unsigned)__double2loint(x.x));
+        st_cluster(o + 5, tag | (unsigned)__double2hiint(x.y));
+        st_cluster(o + 6, tag | (unsigned)__double2loint(x.y));
+      }
+    }
+  };
+  if (wid == 0) {
+    for (int rr = lane; rr < nrw; rr += 32) consider(0, rr, r0 + rr, prow[rr * LU_LDP]);
+    push(0);
+  }
+  bool ok = true, mine = false;
+  cplx l = cmake(0.0, 0.0);
   for (int kk = 0; kk < b; ++kk) {
     const int par = kk & 1;
     cplx pvw = cmake(0.0, 0.0);   // warp 0: the pivot
     if (wid == 0) {
-      double best = 0.0;
-      int pk = 0x7FFFFFFF;   // position << 16 | row; the positions of the candidates are distinct
-      for (int rr = lane; rr < nrw; rr += 32) {
-        const int ps = pos[r0 + rr];
-        if (ps < kk) continue;
-        const cplx x = prow[rr * LU_LDP + kk];
-        double a = fabs(x.x) + fabs(x.y);
-        if (ps == kk && __double2hiint(a) < 0) a = 0.0;   // NaN: no candidate, but some row always is
-        const int c = ps << 16 | (r0 + rr);
-        if (piv_better(a, c, best, pk)) { best = a; pk = c; }
-      }
-      warp_argmax(best, pk);
-      const bool any = pk != 0x7FFFFFFF;
-      const cplx x = any ? prow[((pk & 0xFFFF) - r0) * LU_LDP + kk] : cmake(0.0, 0.0);
-      fence_release_shared();   // this CTA's rows of the previous step
-      {
-        // lane c < 16 stores the first three words at CTA c, lane c + 16 the other four
-        const int c = lane & 15;
-        const unsigned long long tag = (unsigned long long)(kk + 1) << 32;
-        if (c < C) {
-          unsigned long long* o = cl.map_shared_rank(&s_cand[par][q].w[0], c);
-          if (lane < 16) {
-            st_cluster(o, tag | (unsigned)__double2hiint(best));
-            st_cluster(o + 1, tag | (unsigned)__double2loint(best));
-            st_cluster(o + 2, tag | (unsigned)pk);
-          } else {
-            st_cluster(o + 3, tag | (unsigned)__double2hiint(x.x));
-            st_cluster(o + 4, tag | (unsigned)__double2loint(x.x));
-            st_cluster(o + 5, tag | (unsigned)__double2hiint(x.y));
-            st_cluster(o + 6, tag | (unsigned)__double2loint(x.y));
-          }
-        }
-      }
       // lane c polls CTA c's first three words, lane c + 16 the other four
       unsigned got[4] = {0u, 0u, 0u, 0u};
       bool here = false;
@@ -153,7 +162,6 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
           }
         }
       }
-      fence_acquire_shared();
       __syncwarp();
       best = 0.0;
       pk = 0x7FFFFFFF;
@@ -178,9 +186,11 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
       }
     }
     __syncthreads();
-    const int win = s_win[par], pk = s_pk[par];
+    const int win = s_win[par], pkw = s_pk[par];
     if (win < 0) { ok = false; break; }
-    const int ps = pk >> 16, o = pk & 0xFFFF;
+    // column kk - 1 is read no more: its multipliers take their place
+    if (!UNBLOCKED && mine && sub == 0) prow[(size_t)row * LU_LDP + kk - 1] = l;
+    const int ps = pkw >> 16, o = pkw & 0xFFFF;
     if (wid == 0) {
       const cplx pv = pvw;
       const bool zero = pv.x == 0.0 && pv.y == 0.0;
@@ -200,8 +210,14 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
         if (!UNBLOCKED && q == 0) w.piv[p0 + kk] = p0 + ps;
       }
     } else if (wid <= 2) {
+      // the pivot row, once its CTA has finished the step before
+      bool here = false;
+      for (int it = 0; it < kClusterPolls && !here; ++it) here = ld_poll(&s_ready[win]) >= kk;
+      fence_acquire_shared();
+      __syncwarp();
+      if (!here && lane == 0) s_late = 1;
       const int j = tid - 32;
-      if (j >= kk && j < b) urow[j] = cl.map_shared_rank(prow + (size_t)(o - win * chunk) * LU_LDP, win)[j];
+      if (j > kk && j < b) urow[j] = cl.map_shared_rank(prow + (size_t)(o - win * chunk) * LU_LDP, win)[j];
     } else if (wid == 3 && lane == 0) {
       const int o2 = rowat[kk];
       pos[o] = kk;
@@ -210,24 +226,50 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
       rowat[kk] = o;
     }
     __syncthreads();
-    if (UNBLOCKED) {
-      if (tid > kk && tid < b) urow[tid] = lu_mul(urow[tid], s_rinv[kk]);
-      __syncthreads();
-    }
-    cplx l = cmake(0.0, 0.0);
-    const bool mine = row < nrw && pos[r0 + row] > kk;
-    if (mine) {
-      cplx* pr = prow + (size_t)row * LU_LDP;
-      l = UNBLOCKED ? pr[kk] : lu_mul(pr[kk], s_rinv[kk]);
-      for (int j = kk + 1 + sub; j < b; j += tpr) {
-        const cplx u = urow[j], x = pr[j];
-        pr[j] = cmake(fma(-l.x, u.x, fma(l.y, u.y, x.x)), fma(-l.x, u.y, fma(-l.y, u.x, x.y)));
+    if (wid == 0) {
+      // column kk + 1 ahead of the others: its candidate is on its way while they work
+      best = 0.0;
+      pk = 0x7FFFFFFF;
+      if (kk + 1 < b) {
+        const cplx ri = s_rinv[kk];
+        const cplx u = UNBLOCKED ? lu_mul(urow[kk + 1], ri) : urow[kk + 1];
+        for (int rr = lane; rr < nrw; rr += 32) {
+          const int pr_pos = pos[r0 + rr];
+          if (pr_pos <= kk) continue;
+          cplx* pr = prow + (size_t)rr * LU_LDP;
+          const cplx lw = UNBLOCKED ? pr[kk] : lu_mul(pr[kk], ri), x0 = pr[kk + 1];
+          const cplx x = cmake(fma(-lw.x, u.x, fma(lw.y, u.y, x0.x)), fma(-lw.x, u.y, fma(-lw.y, u.x, x0.y)));
+          pr[kk + 1] = x;
+          consider(kk + 1, rr, pr_pos, x);
+        }
+        push(kk + 1);
+      }
+    } else {
+      if (UNBLOCKED) {
+        const int j = tid - 32;
+        if (j > kk && j < b) us[j] = lu_mul(urow[j], s_rinv[kk]);
+        lu_bar();
+      }
+      const cplx* uu = UNBLOCKED ? us : urow;
+      mine = works && pos[r0 + row] > kk;
+      if (mine) {
+        cplx* pr = prow + (size_t)row * LU_LDP;
+        l = UNBLOCKED ? pr[kk] : lu_mul(pr[kk], s_rinv[kk]);
+        for (int j = kk + 2 + sub; j < b; j += tpr) {
+          const cplx u = uu[j], x = pr[j];
+          pr[j] = cmake(fma(-l.x, u.x, fma(l.y, u.y, x.x)), fma(-l.x, u.y, fma(-l.y, u.x, x.y)));
+        }
+      }
+      lu_bar();
+      if (wid == 1) {
+        fence_release_shared();   // this CTA's rows
+        if (lane < C) st_cluster(cl.map_shared_rank(&s_ready[q], lane), kk + 1);
       }
     }
-    __syncthreads();
-    // column kk is read no more: its multipliers take their place
-    if (!UNBLOCKED && mine && sub == 0) prow[(size_t)row * LU_LDP + kk] = l;
   }
+  __syncthreads();
+  if (ok && !UNBLOCKED && mine && sub == 0) prow[(size_t)row * LU_LDP + b - 1] = l;
+  ok = ok && s_late == 0;
   if (!ok && tid == 0) atomicOr(w.err, DQMC_KERR_BARRIER_TIMEOUT);
   __syncthreads();
   if (ok) {
