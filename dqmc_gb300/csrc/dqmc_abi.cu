@@ -110,8 +110,13 @@ struct dqmc_handle {
   double *gb_d = nullptr, *gb_phi = nullptr;
   void* gb_evtab = nullptr;
   GridBarrier* bar = nullptr;
-  int* err_d = nullptr;
-  double* scal_d = nullptr;    // scalars: [0] sum log d2, [1] absdiff, [2] saved sum log d2, [3] instability max
+  int* err_d = nullptr;        // in scal_d[4]
+  // scalars: [0] sum log d2, [1] absdiff, [2] saved sum log d2, [3] instability max,
+  // [4] error bits, [5] acceptance counters
+  double* scal_d = nullptr;
+  // pinned host memory: [0 .. 5] scal_d as of the last wait, [6] rounds run, [7] a
+  // counter snapshot, [8 ..] the per-site outputs of one call
+  double* pin = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;   // brackets of the last enqueued sweep
   int pending_calls = 0;
   // ---- host state ----
@@ -227,10 +232,16 @@ void resolve_spans(dqmc_handle* h) {
   h->event_next = 0;
 }
 
-int check_device_error(dqmc_handle* h) {
-  int e = 0;
-  CU(cudaMemcpyAsync(&e, h->err_d, sizeof(int), cudaMemcpyDeviceToHost, h->st));
+constexpr int kPinScal = 6, kPinRounds = 6, kPinCount = 7, kPinOut = 8;
+
+// Waits for the stream with the call's scalars in pin.  One copy to pinned
+// memory and one wait: the error bits, instability and counters each copied to
+// pageable memory cost a further wait of 8-10 us.
+int wait_scalars(dqmc_handle* h) {
+  CU(cudaMemcpyAsync(h->pin, h->scal_d, kPinScal * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CU(cudaStreamSynchronize(h->st));
+  int e = 0;
+  std::memcpy(&e, h->pin + 4, sizeof(int));
   if (e == 0) return DQMC_OK;
   CU(cudaMemsetAsync(h->err_d, 0, sizeof(int), h->st));
   if (e & DQMC_KERR_BARRIER_TIMEOUT) return set_err(h, DQMC_ERR_TIMEOUT, "device barrier timed out");
@@ -239,13 +250,15 @@ int check_device_error(dqmc_handle* h) {
   return set_err(h, DQMC_ERR_CUDA, "device error flag " + std::to_string(e));
 }
 
-int read_instability(dqmc_handle* h);
-
+// Waits for the stream; folds the instability of the call into the maximum.
 int sync(dqmc_handle* h) {
-  CU(cudaStreamSynchronize(h->st));
+  const int rc = wait_scalars(h);
   if (h->timing) resolve_spans(h);
-  CHK(check_device_error(h));
-  return read_instability(h);
+  CHK(rc);
+  const double d = h->pin[3];
+  if (!(d <= h->max_instability)) h->max_instability = d;
+  if (!std::isfinite(d)) return set_err(h, DQMC_ERR_NONFINITE, "non-finite Green's function");
+  return DQMC_OK;
 }
 
 size_t nn_bytes(const dqmc_handle* h) { return (size_t)h->n * h->n * sizeof(cplx); }
@@ -614,16 +627,6 @@ int instability_check(dqmc_handle* h) {
   return DQMC_OK;
 }
 
-// Reads the running instability maximum (stream must be idle).
-int read_instability(dqmc_handle* h) {
-  double d = 0.0;
-  CU(cudaMemcpyAsync(&d, h->scal_d + 3, sizeof(double), cudaMemcpyDeviceToHost, h->st));
-  CU(cudaStreamSynchronize(h->st));
-  if (!(d <= h->max_instability)) h->max_instability = d;
-  if (!std::isfinite(d)) return set_err(h, DQMC_ERR_NONFINITE, "non-finite Green's function");
-  return DQMC_OK;
-}
-
 // build_stack (src/stack.jl:251-272)
 int build_stack(dqmc_handle* h) {
   CHK(stack_identity(h, 0));
@@ -918,22 +921,17 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
   return DQMC_OK;
 }
 
-int read_nacc(dqmc_handle* h, int* out) {
-  CU(cudaMemcpyAsync(out, h->nacc_d, sizeof(int), cudaMemcpyDeviceToHost, h->st));
-  CU(cudaStreamSynchronize(h->st));
-  return DQMC_OK;
-}
-
 void host_model_constants(dqmc_handle* h) { fill_model_const(h->p, h->mc); }
 
 void free_all(dqmc_handle* h) {
   void* ptrs[] = {h->phi, h->evtab, h->G, h->Gtmp, h->u_stack, h->d_stack, h->t_stack, h->Ul, h->Ur, h->Tl,
                   h->Tr, h->Dl, h->Dr, h->W1, h->W2, h->W3, h->W4, h->D1, h->d2, h->ord1, h->qr.vn1,
                   h->qr.vn2, h->qr.order, h->qr.tau, h->qr.beta, h->qr.V, h->qr.bar, h->qr.cand_v, h->qr.cand_q, h->qr.refl, h->qr.slots, h->qr.cols, h->qr.run, h->delta_d, h->unif_d,
-                  h->acc_d, h->det_d, h->pacc_d, h->action_d, h->nacc_d, h->Acol, h->Brow, h->bar, h->err_d,
+                  h->acc_d, h->det_d, h->pacc_d, h->action_d, h->Acol, h->Brow, h->bar,
                   h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wrow, h->wflag, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
   for (void* q : ptrs)
     if (q) cudaFree(q);
+  if (h->pin) cudaFreeHost(h->pin);
   clear_graphs(h);
   if (h->done) cudaEventDestroy(h->done);
   for (auto e : h->event_pool) cudaEventDestroy(e);
@@ -1299,10 +1297,15 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
   A((void**)&h->qr.slots, (size_t)2 * 160 * 160 * 2 * sizeof(unsigned long long));
   A((void**)&h->qr.cols, qr_column_words((int)n, h->sm_count) * sizeof(unsigned long long));
   A((void**)&h->qr.run, sizeof(unsigned));
-  A((void**)&h->action_d, sizeof(double)); A((void**)&h->nacc_d, 2 * sizeof(int));
+  A((void**)&h->action_d, sizeof(double));
   A((void**)&h->Acol, 4 * n * sizeof(cplx)); A((void**)&h->Brow, 4 * n * sizeof(cplx));
-  A((void**)&h->bar, sizeof(GridBarrier)); A((void**)&h->err_d, sizeof(int));
+  A((void**)&h->bar, sizeof(GridBarrier)); 
   A((void**)&h->scal_d, 8 * sizeof(double));
+  if (ok) {
+    h->err_d = reinterpret_cast<int*>(h->scal_d + 4);
+    h->nacc_d = reinterpret_cast<int*>(h->scal_d + 5);
+    ok = cudaHostAlloc((void**)&h->pin, kPinOut * sizeof(double) + (size_t)h->N * 25 + 16, cudaHostAllocDefault) == cudaSuccess;
+  }
   h->greens_method = p->greens_method == DQMC_GREENS_TWO_QR ? DQMC_GREENS_TWO_QR : DQMC_GREENS_SCALES;
   A((void**)&h->lu.perm, n * sizeof(int)); A((void**)&h->lu.udiag, n * sizeof(cplx));
   A((void**)&h->lu.rdiag, n * sizeof(cplx));
@@ -1418,16 +1421,23 @@ static int local_updates_host(dqmc_handle* h, const double* delta, const double*
   CHK(ensure_out_capacity(h, 1));
   CU(cudaMemcpyAsync(h->delta_d, delta, (size_t)3 * h->N * sizeof(double), cudaMemcpyHostToDevice, h->st));
   CU(cudaMemcpyAsync(h->unif_d, unif, (size_t)h->N * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  int before = 0;
-  CHK(read_nacc(h, &before));
+  CU(cudaMemcpyAsync(h->pin + kPinCount, h->nacc_d, sizeof(int), cudaMemcpyDeviceToHost, h->st));
   CHK(local_updates_dev(h, h->delta_d, h->unif_d, h->acc_d, h->det_d, h->pacc_d));
-  if (accepted) CU(cudaMemcpyAsync(accepted, h->acc_d, h->N, cudaMemcpyDeviceToHost, h->st));
-  if (detratio) CU(cudaMemcpyAsync(detratio, h->det_d, h->N * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
-  if (p_acc) CU(cudaMemcpyAsync(p_acc, h->pacc_d, h->N * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  // the outputs wait in pinned memory, so that one wait serves them all
+  const size_t N = h->N;
+  char* det = reinterpret_cast<char*>(h->pin + kPinOut);
+  char *pac = det + N * sizeof(cplx), *acc = pac + N * sizeof(double);
+  if (detratio) CU(cudaMemcpyAsync(det, h->det_d, N * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
+  if (p_acc) CU(cudaMemcpyAsync(pac, h->pacc_d, N * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  if (accepted) CU(cudaMemcpyAsync(acc, h->acc_d, N, cudaMemcpyDeviceToHost, h->st));
   CHK(sync(h));
+  if (detratio) std::memcpy(detratio, det, N * sizeof(cplx));
+  if (p_acc) std::memcpy(p_acc, pac, N * sizeof(double));
+  if (accepted) std::memcpy(accepted, acc, N);
   if (acc_rate) {
-    int after = 0;
-    CHK(read_nacc(h, &after));
+    int before = 0, after = 0;
+    std::memcpy(&before, h->pin + kPinCount, sizeof(int));
+    std::memcpy(&after, h->pin + 5, sizeof(int));
     *acc_rate = (double)(after - before) / h->N;
   }
   return DQMC_OK;
@@ -1554,15 +1564,15 @@ static int sweep_enqueue(dqmc_handle* h, int n_calls, const double* delta_dev, c
 
 // Waits for an enqueued sweep and fills the statistics.
 static int sweep_finish(dqmc_handle* h, dqmc_stats* stats) {
+  if (h->pending_while > 0)
+    CU(cudaMemcpyAsync(h->pin + kPinRounds, h->dstate + 4, sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->st));
   CHK(sync(h));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, h->ev0, h->ev1);
   int cnt[2] = {0, 0};
   unsigned long long rounds = 0;
-  CU(cudaMemcpyAsync(cnt, h->nacc_d, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->st));
-  if (h->pending_while > 0)
-    CU(cudaMemcpyAsync(&rounds, h->dstate + 4, sizeof(rounds), cudaMemcpyDeviceToHost, h->st));
-  CU(cudaStreamSynchronize(h->st));
+  std::memcpy(cnt, h->pin + 5, sizeof(cnt));
+  std::memcpy(&rounds, h->pin + kPinRounds, sizeof(rounds));
   if (h->pending_while > 0) {
     // the graph's counts hold one round body per WHILE node (a WHILE node
     // runs its body at least once): add the rounds that ran beyond those
@@ -1924,10 +1934,8 @@ int dqmc_calculate_greens_udt(dqmc_handle* h, const double* Ul, const double* Dl
   CU(cudaMemcpyAsync(h->Dr, Dr, dn, cudaMemcpyHostToDevice, h->st));
   CHK(calculate_greens_into(h, h->Gtmp));
   CHK(download_nn(h, G, h->Gtmp));
-  double sl = 0.0;
-  CU(cudaMemcpyAsync(&sl, h->scal_d, sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CHK(sync(h));
-  if (logdet) *logdet = -sl;
+  if (logdet) *logdet = -h->pin[0];
   return DQMC_OK;
 }
 
@@ -1945,10 +1953,8 @@ int dqmc_decompose_udt(dqmc_handle* h, const double* A, double* U, double* D, do
 int dqmc_logdet(dqmc_handle* h, double* logdet) {
   if (h) cudaSetDevice(h->device);
   if (!h || !logdet) return DQMC_ERR_ARG;
-  double sl = 0.0;
-  CU(cudaMemcpyAsync(&sl, h->scal_d + 2, sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CHK(sync(h));
-  *logdet = -sl;
+  *logdet = -h->pin[2];
   return DQMC_OK;
 }
 
@@ -1997,10 +2003,8 @@ int dqmc_calc_greens(dqmc_handle* h, int32_t slice, double* out, double* logdet)
   }
   CHK(calculate_greens_into(h, h->Gtmp));
   CHK(download_nn(h, out, h->Gtmp));
-  double sl = 0.0;
-  CU(cudaMemcpyAsync(&sl, h->scal_d, sizeof(double), cudaMemcpyDeviceToHost, h->st));
   CHK(sync(h));
-  if (logdet) *logdet = -sl;
+  if (logdet) *logdet = -h->pin[0];
   // the stack copies Ul..Tr were overwritten: restore nothing (propagate re-reads them from the stack)
   return DQMC_OK;
 }
@@ -2238,14 +2242,23 @@ int dqmc_measure_equal_time(dqmc_handle* h, const double* greens, double* etpc_p
   }
   if (!h->etc_d) CU(cudaMalloc(&h->etc_d, (size_t)6 * N * sizeof(double)));
   LAUNCH(DQMC_K_MISC, 0.0, 0.0, launch_equal_time_corr(src, h->L, h->etc_d, h->st));
-  const cudaMemcpyKind kind = device_ptrs ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
   double* outs[4] = {etpc_plus, etpc_minus, etcdc_plus, etcdc_minus};
   const size_t off[4] = {0, (size_t)N, (size_t)2 * N, (size_t)4 * N};
   const size_t cnt[4] = {(size_t)N, (size_t)N, (size_t)2 * N, (size_t)2 * N};
+  if (device_ptrs) {
+    for (int q = 0; q < 4; ++q)
+      if (outs[q])
+        CU(cudaMemcpyAsync(outs[q], h->etc_d + off[q], cnt[q] * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
+    CHK(sync(h));
+    return wait_scalars(h);
+  }
+  // one copy for the four arrays: a copy to pageable memory costs 8 us whatever its size
+  std::vector<double> host((size_t)6 * N);
+  CU(cudaMemcpyAsync(host.data(), h->etc_d, host.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  CHK(wait_scalars(h));   // waits for the stream
   for (int q = 0; q < 4; ++q)
-    if (outs[q]) CU(cudaMemcpyAsync(outs[q], h->etc_d + off[q], cnt[q] * sizeof(double), kind, h->st));
-  CHK(sync(h));
-  return check_device_error(h);
+    if (outs[q]) std::memcpy(outs[q], host.data() + off[q], cnt[q] * sizeof(double));
+  return DQMC_OK;
 }
 
 int dqmc_measure(dqmc_handle* h, double* greens_out, double* occupation, double* e_kin) {
@@ -2259,10 +2272,12 @@ int dqmc_measure(dqmc_handle* h, double* greens_out, double* occupation, double*
   CHK(wrap_greens(h, h->Gtmp, h->current_slice, 1));
   CHK(apply_rows(h, h->Gtmp, 0, 1, 1, 5));   // G Hb_half Ha_half
   CHK(apply_cols(h, h->Gtmp, 0, 1, 1, 6, nullptr));   // Ha_half^-1 Hb_half^-1 G
-  std::vector<double> g((size_t)2 * n * n);
-  CHK(download_nn(h, g.data(), h->Gtmp));
+  // straight into the caller's array: a buffer between costs its page faults and
+  // a second pass over n^2 (the hook and its correlators at n = 256 315 us with it, 211 without)
+  std::vector<double> own(greens_out ? 0 : (size_t)2 * n * n);
+  double* g = greens_out ? greens_out : own.data();
+  CHK(download_nn(h, g, h->Gtmp));
   CHK(sync(h));
-  if (greens_out) std::memcpy(greens_out, g.data(), g.size() * sizeof(double));
   auto Gre = [&](int r, int c) { return g[2 * ((size_t)c * n + r)]; };
   if (occupation) {
     double s = 0.0;
@@ -2393,7 +2408,7 @@ int dqmc_measure_zfpc(dqmc_handle* h, const double* Gt0, double* zfpc_plus, doub
       cudaMemcpyAsync(zfpc_minus, h->etc_d + N, N * sizeof(double), kind, h->st) != cudaSuccess) rc = DQMC_ERR_CUDA;
   if (rc == DQMC_OK && cudaStreamSynchronize(h->st) != cudaSuccess) rc = DQMC_ERR_CUDA;
   if (rc != DQMC_OK) return set_err(h, rc, "zfpc");
-  return check_device_error(h);
+  return wait_scalars(h);
 }
 
 // Shared body of the zero-frequency charge-density (which = 0) and
@@ -2479,7 +2494,7 @@ static int zero_frequency_measure(dqmc_handle* h, int which, const double* green
       }
     *sfdensity = 0.25 * (qx - qy);
   }
-  return check_device_error(h);
+  return wait_scalars(h);
 }
 
 int dqmc_measure_zfcdc(dqmc_handle* h, const double* greens, const double* Gt0, const double* G0t,

@@ -57,8 +57,8 @@ __device__ __forceinline__ double lu_join(unsigned hi, unsigned lo) { return __h
 //
 // Bound: about 4500 cycles of latency per column (a remote store or load takes
 // 1000, the reciprocal 1000-1500); the multiply-adds, 4 per entry on 16 SMs, fit
-// beside them.  Panel of 64 columns, us: in turn -> overlapped n = 144 198 -> @A,
-// n = 576 235 -> @B, n = 1024 229 -> @C.  The cooperative grids before paid a grid
+// beside them.  Panel of 64 columns, us: in turn -> overlapped n = 144 198 -> 178,
+// n = 576 235 -> 190, n = 1024 229 -> 185.  The cooperative grids before paid a grid
 // barrier and three round trips through L2 per column, 10000-15000 cycles.
 //
 // UNBLOCKED false: A in place, L below the diagonal (scaled multipliers, a -= l
