@@ -219,6 +219,166 @@ __global__ void k_apply_rows(cplx* __restrict__ A, int n, int rows_per_cta, Mode
   }
 }
 
+// The same application for small lattices (n <= 144): one column (NV = 1) or two
+// rows (NV = 2) per CTA with a thread per output component, 4 FP64 operations
+// per layer in a chain where a thread per block has 32 (plaquettes) or 40 (sites),
+// which left n = 64 with one busy sub-partition per CTA.  Layers go from one
+// buffer to the other.  B M is the same bits as above.  Chains of the other modes
+// (and B^dag M) stay with the kernels above: they feed the stabilisation, whose
+// 40-bit products amplify another rounding to their own error.
+// Bound: latency, a layer is about 500 cycles.  Columns and rows per sequence of
+// wraps, ms: n = 64 0.77 and 0.58 -> 0.40 and 0.41, n = 144 1.53 and 1.13 -> 0.88 and
+// 1.07; at n = 256 the blocks fill the sub-partitions (1.64 and 1.15 against 1.63 and 1.43).
+constexpr int SF_MAX = 144, SF_THREADS = 2 * SF_MAX;
+
+struct SlicePlace {   // a thread's component: its partners' offsets in the buffer
+  int pl[2][4];       // plaquette group 0, 1: corners i, j, m, n
+  int h[2];           // the component's own corner: (y odd) | (x odd) << 1
+  int s_off, r_off;   // interaction block: partners through S and R
+  int f, site;
+};
+
+template <int NV>
+__global__ void __launch_bounds__(SF_THREADS) k_slice_fine(cplx* __restrict__ A, int n, ModelConst mc,
+                                                          const EvEntry* __restrict__ evtab, int first, int count,
+                                                          int step, int mode, const double* __restrict__ colscale) {
+  constexpr int UPT = NV;   // components per thread: 2 n threads
+  __shared__ double buf[2][2 * SF_MAX * NV];
+  __shared__ EvEntry s_ev[2][SF_MAX / 4];
+  __shared__ double coef[2][2][4];   // [half][band][dy | dx << 1]
+  const int N = mc.N, L = mc.L, units = 2 * n * NV, T = blockDim.x;
+  const int r0 = blockIdx.x * NV;
+  if (threadIdx.x < 16) {
+    const int half = threadIdx.x >> 3, b = (threadIdx.x >> 2) & 1, k = threadIdx.x & 3;
+    const double ch = half ? mc.ch_h[b] : mc.ch_f[b], sh = half ? mc.sh_h[b] : mc.sh_f[b];
+    const double cv = half ? mc.cv_h[b] : mc.cv_f[b], sv = half ? mc.sv_h[b] : mc.sv_f[b];
+    coef[half][b][k] = (k & 2 ? sh : ch) * (k & 1 ? sv : cv);
+  }
+  // component w: part w & 1 of vector (w >> 1) % NV, element w / (2 NV)
+  auto global = [&](int w) -> double* {
+    const int e = w / (2 * NV), q = w % (2 * NV);
+    return reinterpret_cast<double*>(NV == 1 ? A + (size_t)r0 * n + e : A + (size_t)e * n + r0) + q;
+  };
+  SlicePlace pc[UPT];
+#pragma unroll
+  for (int u = 0; u < UPT; ++u) {
+    const int w = threadIdx.x + u * T;
+    if (w >= units) continue;
+    const int e = w / (2 * NV);
+    SlicePlace& c = pc[u];
+    buf[0][w] = NV == 1 || r0 + ((w >> 1) & 1) < n ? *global(w) : 0.0;
+    c.f = e / N;
+    c.site = e - c.f * N;
+    const int x = c.site / L, y = c.site - x * L;
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      const int hy = (y ^ g) & 1, hx = (x ^ g) & 1;
+      const int yo = hy ? (y == 0 ? L - 1 : y - 1) : (y + 1 == L ? 0 : y + 1);
+      const int xo = hx ? (x == 0 ? L - 1 : x - 1) : (x + 1 == L ? 0 : x + 1);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int ye = (k & 1) == hy ? y : yo, xe = (k >> 1) == hx ? x : xo;
+        c.pl[g][k] = w + (ye + L * xe - c.site) * 2 * NV;
+      }
+      c.h[g] = hy | hx << 1;
+    }
+    c.s_off = w + ((c.f ^ 1) - c.f) * N * 2 * NV;
+    c.r_off = w + (3 - 2 * c.f) * N * 2 * NV;
+  }
+  int cur = 0;   // the buffer that holds the vectors
+  auto plaquettes = [&](int g, int half, bool inverse) {
+#pragma unroll
+    for (int u = 0; u < UPT; ++u) {
+      const int w = threadIdx.x + u * T;
+      if (w >= units) continue;
+      const SlicePlace& c = pc[u];
+      const double* x = buf[cur];
+      const double* k = coef[half][c.f & 1];
+      double t[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int d = q ^ c.h[g];
+        const double v = k[d];
+        t[q] = inverse && (d == 1 || d == 2) ? -v : v;
+      }
+      const double xi = x[c.pl[g][0]], xj = x[c.pl[g][1]], xm = x[c.pl[g][2]], xn = x[c.pl[g][3]];
+      const double a = __fma_rn(t[0], xi, __dmul_rn(t[1], xj));
+      buf[cur ^ 1][w] = __fma_rn(t[3], xn, __fma_rn(t[2], xm, a));
+    }
+    cur ^= 1;
+    __syncthreads();
+  };
+  auto interaction = [&](const EvEntry* ev) {
+    const bool inv = mode == SLICE_LEFT_BINV || mode == SLICE_RIGHT_BINV;
+    const bool transpose = mode == SLICE_RIGHT_B || mode == SLICE_RIGHT_BINV;
+    const bool pre = mode == SLICE_LEFT_BINV || mode == SLICE_RIGHT_B;
+#pragma unroll
+    for (int u = 0; u < UPT; ++u) {
+      const int w = threadIdx.x + u * T;
+      if (w >= units) continue;
+      const SlicePlace& c = pc[u];
+      const double* x = buf[cur];
+      const bool im = w & 1;
+      const int b = c.f & 1;
+      const double m0 = inv ? mc.emu_inv[b] : mc.emu[b], m1 = inv ? mc.emu_inv[b ^ 1] : mc.emu[b ^ 1];
+      const EvEntry e = ev[c.site];
+      double xs = x[w], xr = x[c.r_off], sx = x[c.s_off & ~1], sy = x[c.s_off | 1];
+      if (pre) { xs *= m0; xr *= m1; sx *= m1; sy *= m1; }
+      // S: entry (0, 1) and (3, 2); conjugated for rows 1, 2 and for the transpose
+      const bool conj = transpose != (c.f == 1 || c.f == 2);
+      const double Sx = inv ? -e.Sr : e.Sr, S0 = inv ? -e.Si : e.Si, Sy = conj ? -S0 : S0;
+      const double R = inv ? -e.R : e.R;
+      double acc;
+      if (c.f == 0 || c.f == 3) acc = __fma_rn(R, xr, __dmul_rn(e.C, xs));
+      else acc = __fma_rn(e.C, xs, -__dmul_rn(R, xr));
+      double y = im ? fma(Sx, sy, fma(Sy, sx, acc)) : fma(Sx, sx, fma(-Sy, sy, acc));
+      if (!pre) y *= m0;
+      buf[cur ^ 1][w] = y;
+    }
+    cur ^= 1;
+    __syncthreads();
+  };
+  for (int i = threadIdx.x; i < N; i += T) s_ev[0][i] = evtab[(size_t)first * N + i];
+  __syncthreads();
+  for (int k = 0; k < count; ++k) {
+    const EvEntry* ev = s_ev[k & 1];
+    if (k + 1 < count)
+      for (int i = threadIdx.x; i < N; i += T) s_ev[(k + 1) & 1][i] = evtab[(size_t)(first + (k + 1) * step) * N + i];
+    switch (mode) {
+      case SLICE_LEFT_B:
+        interaction(ev);
+        plaquettes(1, 1, false); plaquettes(0, 0, false); plaquettes(1, 1, false);
+        break;
+      case SLICE_RIGHT_B:
+        plaquettes(1, 1, false); plaquettes(0, 0, false); plaquettes(1, 1, false);
+        interaction(ev);
+        break;
+      case SLICE_LEFT_BINV:
+        plaquettes(1, 1, true); plaquettes(0, 0, true); plaquettes(1, 1, true);
+        interaction(ev);
+        break;
+      case SLICE_RIGHT_BINV:
+        interaction(ev);
+        plaquettes(1, 1, true); plaquettes(0, 0, true); plaquettes(1, 1, true);
+        break;
+      case SLICE_EFF_RIGHT:
+        plaquettes(1, 1, false); plaquettes(0, 1, false);
+        break;
+      case SLICE_EFF_LEFT_INV:
+        plaquettes(1, 1, true); plaquettes(0, 1, true);
+        break;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UPT; ++u) {
+    const int w = threadIdx.x + u * T;
+    if (w >= units || (NV == 2 && r0 + ((w >> 1) & 1) >= n)) continue;
+    double v = buf[cur][w];
+    if (NV == 1 && colscale) v *= colscale[r0];
+    *global(w) = v;
+  }
+}
+
 // Per-site interaction entries for every slice from the field
 // (src/interactions.jl:52-64, power +1).
 __global__ void k_build_evtab(const double* __restrict__ phi, EvEntry* __restrict__ evtab, int N, int M,
@@ -254,6 +414,10 @@ static int slice_threads(int units) {
 
 cudaError_t launch_apply_cols(cplx* A, int n, const ModelConst& mc, const void* evtab, int first_slice0,
                               int count, int step, int mode, const double* colscale, cudaStream_t st) {
+  if (n <= SF_MAX && (mode == SLICE_LEFT_B || (mode != SLICE_LEFT_BDAG && count == 1))) {
+    k_slice_fine<1><<<n, 2 * n, 0, st>>>(A, n, mc, (const EvEntry*)evtab, first_slice0, count, step, mode, colscale);
+    return cudaGetLastError();
+  }
   const int cpc = 1;
   int grid = (n + cpc - 1) / cpc;
   size_t smem = (size_t)cpc * n * sizeof(cplx) + (size_t)mc.N * sizeof(EvEntry);
@@ -266,6 +430,11 @@ cudaError_t launch_apply_cols(cplx* A, int n, const ModelConst& mc, const void* 
 
 cudaError_t launch_apply_rows(cplx* A, int n, const ModelConst& mc, const void* evtab, int first_slice0,
                               int count, int step, int mode, cudaStream_t st) {
+  if (n <= SF_MAX && count == 1) {
+    k_slice_fine<2><<<(n + 1) / 2, 2 * n, 0, st>>>(A, n, mc, (const EvEntry*)evtab, first_slice0, count, step, mode,
+                                                   nullptr);
+    return cudaGetLastError();
+  }
   const int rpc = 2;
   int grid = (n + rpc - 1) / rpc;
   size_t smem = (size_t)rpc * n * sizeof(cplx) + (size_t)mc.N * sizeof(EvEntry);
