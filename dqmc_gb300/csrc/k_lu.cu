@@ -280,6 +280,7 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
       if (UNBLOCKED && ps > j) Lb[(size_t)(p0 + j) * n + p0 + ps] = lu_mul(x, s_rinv[j]);
     }
     if (UNBLOCKED && q == 0) {
+      __syncthreads();   // pos has been read by all warps
       if (tid < b) {
         w.udiag[p0 + tid] = s_piv[tid];
         w.rdiag[p0 + tid] = s_rinv[tid];
