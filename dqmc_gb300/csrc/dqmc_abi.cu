@@ -67,8 +67,6 @@ struct dqmc_handle {
   int out_cap = 0;
   double* action_d = nullptr;
   int* nacc_d = nullptr;
-  cplx* Acol = nullptr;
-  cplx* Brow = nullptr;
   // delayed updates: pending factors and {next site, pending count}
   int delay = 1;
   cplx* Xd = nullptr;
@@ -109,7 +107,6 @@ struct dqmc_handle {
   cplx *gb_u = nullptr, *gb_t = nullptr, *gb_G = nullptr;
   double *gb_d = nullptr, *gb_phi = nullptr;
   void* gb_evtab = nullptr;
-  GridBarrier* bar = nullptr;
   int* err_d = nullptr;        // in scal_d[4]
   // scalars: [0] sum log d2, [1] absdiff, [2] saved sum log d2, [3] instability max,
   // [4] error bits, [5] acceptance counters
@@ -526,7 +523,7 @@ int trsm_blocked(dqmc_handle* h, const cplx* T, const cplx* rdiag, cplx* Y, bool
 // part is L.
 int lu_blocked(dqmc_handle* h, cplx* A, const cplx** Lm) {
   const int n = h->n;
-  const int cap = h->lu_cluster > 0 ? h->lu_cluster : h->coop_cap;
+  const int cap = h->lu_cluster > 0 ? h->lu_cluster : (h->coop_cap > 0 ? 8 : 0);   // shared GPU: as the windows
   if (n <= h->lu_small) {
     for (int p0 = 0; p0 < n; p0 += LU_PB) {
       const int b = n - p0 < LU_PB ? n - p0 : LU_PB;
@@ -888,9 +885,6 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
   a.pacc_out = pacc_dev;
   a.action = h->action_d;
   a.n_acc = h->nacc_d;
-  a.Acol = h->Acol;
-  a.Brow = h->Brow;
-  a.bar = h->bar;
   a.err = h->err_d;
   a.mc = h->mc;
   const int n = h->n, k = h->delay;
@@ -912,7 +906,7 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
   auto round = [&]() -> int {
     // followers only where the chain has the GPU to itself
     const bool follow = h->follow && h->coop_cap == 0;
-    LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_window(a, d, h->st, h->coop_cap, follow));
+    LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_window(a, d, h->st, h->coop_cap > 0, follow));
     if (!follow) LAUNCH(DQMC_K_FLUSH, 0.0, 0.0, launch_local_factors(a, d, h->st));
     // flush G += X Y over the 4p new columns (p read on the device; no work when p = 0)
     return zgemm_general(h, n, n, 4 * k, 'N', 'T', cmake(1, 0), h->Xd, n, h->Yd, n, cmake(1, 0), h->G, n, nullptr,
@@ -937,7 +931,7 @@ void free_all(dqmc_handle* h) {
   void* ptrs[] = {h->phi, h->evtab, h->G, h->Gtmp, h->u_stack, h->d_stack, h->t_stack, h->Ul, h->Ur, h->Tl,
                   h->Tr, h->Dl, h->Dr, h->W1, h->W2, h->W3, h->W4, h->D1, h->d2, h->ord1, h->qr.vn1,
                   h->qr.vn2, h->qr.order, h->qr.tau, h->qr.beta, h->qr.V, h->qr.bar, h->qr.cand_v, h->qr.cand_q, h->qr.refl, h->qr.slots, h->qr.cols, h->qr.run, h->delta_d, h->unif_d,
-                  h->acc_d, h->det_d, h->pacc_d, h->action_d, h->Acol, h->Brow, h->bar,
+                  h->acc_d, h->det_d, h->pacc_d, h->action_d,
                   h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wrow, h->wflag, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -1311,8 +1305,6 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
   A((void**)&h->qr.cols, qr_column_words((int)n, h->sm_count) * sizeof(unsigned long long));
   A((void**)&h->qr.run, sizeof(unsigned));
   A((void**)&h->action_d, sizeof(double));
-  A((void**)&h->Acol, 4 * n * sizeof(cplx)); A((void**)&h->Brow, 4 * n * sizeof(cplx));
-  A((void**)&h->bar, sizeof(GridBarrier)); 
   A((void**)&h->scal_d, 8 * sizeof(double));
   if (ok) {
     h->err_d = reinterpret_cast<int*>(h->scal_d + 4);

@@ -1221,11 +1221,14 @@ int local_window_sites(int k) { return k < WIN_MAX ? k : WIN_MAX; }
 // Follower clusters of a window launch.
 static int follower_clusters(int n, int C) { return (2 * ((n + fac_vpc(n) - 1) / fac_vpc(n)) + C - 1) / C; }
 
-cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster,
+cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, bool shared,
                                 bool follow) {
   int C = 0;
   if (cudaError_t e = window_cluster(&C); e != cudaSuccess) return e;
-  if (max_cluster > 0 && C > 8 && max_cluster < C) C = 8;
+  // 16 free SMs in one GPC are rare beside other chains' QRs, which fill their SMs:
+  // with the LU panels likewise, 16 chains of L = 6 .. 12 484 -> 458 ms, 8 of L = 16
+  // 899 -> 772 ms per 40 calls
+  if (shared && C > 8) C = 8;
   const int W = local_window_sites(d.k);
   size_t smem = window_smem(a.mc.N, W, C);
   cudaLaunchAttribute attr[1];

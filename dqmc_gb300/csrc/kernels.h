@@ -84,8 +84,9 @@ struct DelayedArgs {
   OzSlices sl;             // the flush's slices, cut by launch_local_factors
                            // (sl.As null: X and Y are stored and the flush slices them itself)
 };
-// Decides the next window of the slice on one cluster (max_cluster > 0: at most that many CTAs, >= 8).
-cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, int max_cluster,
+// Decides the next window of the slice on one cluster of 16 CTAs, 8 when other
+// chains share the GPU.
+cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st, bool shared,
                                 bool follow);
 // whether the window can have follower clusters that form its factors (else launch_local_factors)
 bool local_window_follows(int n, int k);
