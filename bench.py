@@ -160,18 +160,15 @@ def measured_peaks():
     return {"hbm_gbs": 6800.0, "bf16_tflops": 1900.0}, "fallback"
 
 
-def flops_model(kind, t, n, accepted, delay=1, real_flushes=0):
+def flops_model(kind, t, n, accepted, real_flushes):
     """Algorithmic (FP64-equivalent flops, bytes) of one kernel kind over the
     launches in `t`.  The rank-4 update of an accepted site is 32 n^2 flops
-    and one read + write of G (32 n^2 bytes).  Immediate form (delay 1): the
-    local-update kernel does it.  Delayed form: the decision kernel only
-    decides and forms the new factor rows/columns (its cost is reported per
-    site, not as a rate); the flush does the rank-4k work, 32 n^2 flops per
-    accepted site, and moves G once per flush that carries work."""
+    and one read + write of G (32 n^2 bytes).  The window kernel decides and
+    forms the factors (its cost is reported per site, not as a rate); the flush
+    does the rank-4p work, 32 n^2 flops per accepted site, and moves G once per
+    flush that carries work."""
     k = t["kinds"][kind]
     if kind == "local_updates":
-        if delay <= 1:
-            return 32.0 * n * n * accepted, 32.0 * n * n * accepted
         return 0.0, 0.0
     if kind == "flush":
         return 32.0 * n * n * accepted, 32.0 * n * n * real_flushes
@@ -179,11 +176,12 @@ def flops_model(kind, t, n, accepted, delay=1, real_flushes=0):
 
 
 def real_flush_count(acc_flags, M, N, delay):
-    """Flushes with work in one sweep of delayed rounds: a round ends after
-    `delay` acceptances or at the end of the slice, so a slice with a
-    acceptances flushes ceil(a / delay) times with work."""
-    a = np.asarray(acc_flags, dtype=np.int64).reshape(M, N).sum(axis=1)
-    return int(np.sum((a + delay - 1) // delay))
+    """Flushes with work in one sweep: a round decides a window of
+    min(delay, 32) sites (16 for depths 0 and 1) and flushes with work when it
+    accepted any of them."""
+    w = min(delay, 32) if delay > 1 else 16
+    a = np.asarray(acc_flags, dtype=np.int64).reshape(M, N)
+    return int(sum(a[:, i:i + w].any(axis=1).sum() for i in range(0, N, w)))
 
 
 def cpu_baseline(p, phi, n_calls, seed, threads):
@@ -574,29 +572,28 @@ def _measure_form(api, chain, args, M, N, d_dev, u_dev, acc_dev, flush, world, s
                 ev_accepted=acc_ev, ev_flags=ev_flags, flags=flags, timed_launches=timed_launches)
 
 
-def kernel_rooflines(tim, n, N, M, accepted_ev, ev_flags, delay, form, peaks, fp64_peak):
+def kernel_rooflines(tim, n, N, M, accepted_ev, ev_flags, delay, peaks, fp64_peak):
     """Per kernel kind, over the one evented sweep: device ms, launches, share,
-    and the algorithmic rate against the bound of the kind.  Local updates of
-    the delayed form: microseconds per site and per accepted site (latency
+    and the algorithmic rate against the bound of the kind.  Local updates:
+    microseconds per site and per accepted site (latency
     bound); flush: algorithmic GB/s against HBM (G read and written once per
     flush with work) and FP64-equivalent TFLOP/s; split-BF16 GEMMs: tensor
     TFLOP/s against the BF16 peak; FP64 kinds against the FP64 peak."""
     kinds = tim["kinds"]
     tot_ms = sum(x["ms"] for x in kinds.values())
-    flushes = real_flush_count(ev_flags, M, N, delay) if delay > 1 else 0
+    flushes = real_flush_count(ev_flags, M, N, delay)
     pipe_of = {"slice_cols": "fp64", "slice_rows": "fp64", "qrp": "fp64", "ozaki_gemm": "tensor",
-               "flush": "tensor" if form == "mixed" else "fp64", "local_updates": "latency",
-               "lu": "fp64" if form == "fp64" else "fp64+tensor", "trsm": "fp64" if form == "fp64" else "fp64+tensor",
-               "apply_q": "fp64" if form == "fp64" else "fp64+tensor", "misc": "hbm", "zgemm": "fp64"}
+               "flush": "tensor", "local_updates": "latency", "lu": "fp64+tensor", "trsm": "fp64+tensor",
+               "apply_q": "fp64+tensor", "misc": "hbm", "zgemm": "fp64"}
     out = {}
     for k, v in kinds.items():
         if not v["launches"]:
             continue
         secs = max(1e-12, v["ms"] / 1000.0)
-        kfl, kby = flops_model(k, tim, n, accepted_ev, delay, flushes)
+        kfl, kby = flops_model(k, tim, n, accepted_ev, flushes)
         e = {"ms": round(v["ms"], 2), "launches": v["launches"], "share": round(v["ms"] / max(1e-9, tot_ms), 4),
              "pipe": pipe_of.get(k)}
-        if k == "local_updates" and delay > 1:
+        if k == "local_updates":
             e["us_per_site"] = round(1e6 * secs / (M * N), 3)
             e["us_per_accepted_site"] = round(1e6 * secs / max(1, accepted_ev), 3)
         elif k == "flush":
@@ -605,7 +602,7 @@ def kernel_rooflines(tim, n, N, M, accepted_ev, ev_flags, delay, form, peaks, fp
             e["hbm_gbs"] = round(kby / secs / 1e9, 1)
             e["hbm_frac"] = round(kby / secs / 1e9 / peaks["hbm_gbs"], 4) if peaks.get("hbm_gbs") else None
             e["fp64_equiv_tflops"] = round(kfl / secs / 1e12, 3)
-            e["tensor_tflops"] = round(v["flops"] / secs / 1e12, 1) if form == "mixed" else None
+            e["tensor_tflops"] = round(v["flops"] / secs / 1e12, 1)
         else:
             e["tflops"] = round(kfl / secs / 1e12, 3)
             e["gbs"] = round(kby / secs / 1e9, 1)
@@ -683,9 +680,9 @@ def run_ours(args, world, rank, local):
     tim = R["timing"]
     kinds = tim["kinds"]
     tot_ms = sum(x["ms"] for x in kinds.values())
-    per_kind = kernel_rooflines(tim, n, N, M, R["ev_accepted"], R["ev_flags"], R["delay"], head, peaks, fp64_peak)
+    per_kind = kernel_rooflines(tim, n, N, M, R["ev_accepted"], R["ev_flags"], R["delay"], peaks, fp64_peak)
     # the `roofline` key: the largest kind with a throughput bound (the
-    # delayed local updates are bound by their per-site dependency chain and
+    # local updates are bound by their per-site dependency chain and
     # are reported per site in `kernels`)
     dominant = max(kinds, key=lambda k: kinds[k]["ms"])
     bounded = {k: v for k, v in kinds.items() if k not in ("local_updates", "misc") and v["launches"]}

@@ -1,11 +1,13 @@
-// Local Metropolis updates of one time slice (plain FP64, rank-4 updates).
+// Local Metropolis updates of one time slice: windows of sites with their
+// factors and flush (the handle's updates, see "windows of sites" below), and
+// immediate rank-4 updates (the allocation-free entry point).
 //
 // Reference: src/local_updates.jl:1-95 (local_updates, calc_detratio,
 // update_greens!), src/action.jl:57-100 (calc_boson_action_diff),
 // src/interactions.jl:102-141 (interaction_matrix_exp_op!).
 //
-// One cooperative (co-resident) launch visits all N sites of the slice in
-// order.  Structure:
+// Immediate form: one cooperative (co-resident) launch visits all N sites of the
+// slice in order.  Structure:
 //   * prologue: every CTA builds, for all sites in parallel, the 4x4 block
 //     Delta_i = e^{+dtau V(phi_i)} e^{-dtau V(phi_i + delta_i)} - I into shared
 //     memory (the old field of a site cannot change before its own visit);
@@ -1157,8 +1159,6 @@ cudaError_t launch_local_prepare(const LocalUpdateArgs& a, SitePrep* prep, int* 
   return cudaGetLastError();
 }
 
-// Cluster size of the window kernel on the current device: 16 CTAs where the
-// device can schedule one (a non-portable size), else 8; 0 if neither.
 static size_t window_smem(int N, int W, int C) {
   const size_t own = (size_t)(W + C - 1) / C;
   return (4 * own * (4 * W + 1) + 16 * W + 16 * own) * sizeof(cplx) +
@@ -1180,6 +1180,8 @@ static cudaLaunchConfig_t window_config(cudaLaunchAttribute* attr, int C, size_t
   return cfg;
 }
 
+// Cluster size of the window kernel on the current device: 16 CTAs where the
+// device can schedule one (a non-portable size), else 8.
 static cudaError_t window_cluster(int* C) {
   static std::mutex mu;
   static int cached[64] = {};
