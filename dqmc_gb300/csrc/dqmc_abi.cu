@@ -56,6 +56,7 @@ struct dqmc_handle {
   size_t oz_bytes = 0;
   unsigned long long* oz_acc = nullptr;   // split-K integer sums, zero between products
   size_t oz_acc_bytes = 0;
+  bool guard = false;   // all products of the running call are guarded (zgemm_general)
   int oz_target = 40;   // mantissa bits kept per operand of the mixed form's products
   // local updates
   double* delta_d = nullptr;
@@ -314,13 +315,21 @@ int wrap_greens(dqmc_handle* h, cplx* gf, int slice, int direction) {
 
 // ---- dense kernels with their work models ----------------------------------
 // Every product goes through the split-BF16 GEMM: oz_target bits per operand
-// in the mixed form, 56 in the FP64 form.  56 bits leave no more error against
-// the exact product than FP64 FMA chains do (the slices are truncated at 2^-57
-// of a row's or column's largest entry and summed exactly, where an FMA chain
-// rounds K times at 2^-53) and take GB300's FP64 pipe, 1/1500 of its BF16 rate,
-// out of the product: n = 1024 8.3 -> 0.50 ms, n = 400 1.64 -> 0.09 ms, n = 64
-// 0.27 -> 0.04 ms (a 64 x 64 FMA tile is one SM's work), flush at n = 400 116 ->
-// 18 us.  allow_split = false keeps the FMA kernel (dqmc_gemm_check).
+// in the mixed form, 63 in the FP64 form (k_ozaki.cu), which takes GB300's FP64
+// pipe, 1/1500 of its BF16 rate, out of the product.  At 63 bits an element's error
+// is at most 0.01 of an FMA chain's, unless the large entries of its row meet the
+// small ones of its column; guard makes such elements FP64 dot products.  Guarded
+// are the updates of the LU and of the triangular solves, which divide by what
+// they leave (few elements: solves 4.71 -> 4.93 ms, LU 8.00 -> 8.13 ms in two
+// stabilisations at L = 16), and every product of operands that the caller gave.
+// In the others (T and U of the stack, Q, the flush) up to half of the elements
+// are of that kind, and guarded they would cost what the FMA kernel does (sweep
+// at L = 16 193 instead of 89 ms); there the rounding of entries of order one in
+// the QR, the LU and the windows, 2^8 above the split's error, is what reaches the
+// results.  Error of whole passes against 64-bit results, FMA kernels -> this:
+// sweeps at L = 4 2.1e-15 -> 1.9e-15, L = 10 1.4e-14 -> 1.1e-14, true G at L = 8
+// 1.1e-14 -> 9.1e-15.  allow_split = false keeps the FMA kernel
+// (dqmc_gemm_check).
 // tensor flops of one split-BF16 complex GEMM: S(S+1)/2 slice pairs x 2 real GEMMs with K' = 2K
 double ozaki_tensor_flops(double m, double nn, double k, int S) {
   const double kp = 2.0 * std::ceil(k / 16.0) * 16.0;
@@ -335,7 +344,8 @@ bool oz_plan(const dqmc_handle* h, int k, int* S, int* bits) {
 }
 int zgemm_general(dqmc_handle* h, int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                   const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rs, const double* cs,
-                  bool allow_split, int kind = -1, const int* active = nullptr, bool presliced = false) {
+                  bool allow_split, int kind = -1, const int* active = nullptr, bool presliced = false,
+                  bool guard = false) {
   if (allow_split) {
     int S = 0, bits = 0;
     if (!oz_plan(h, k, &S, &bits)) return set_err(h, DQMC_ERR_ARG, "no exact slicing for this K");
@@ -350,7 +360,7 @@ int zgemm_general(dqmc_handle* h, int m, int nn, int k, char opA, char opB, cplx
     LAUNCH(kind >= 0 ? kind : DQMC_K_OZGEMM, ozaki_tensor_flops(m, nn, k, S), gemm_bytes(m, nn, k),
            launch_ozaki_zgemm(m, nn, k, opA, opB, alpha, A, lda, B, ldb, beta, C, ldc, rs, cs, S, bits,
                               h->oz_scratch, h->oz_bytes, h->oz_acc, h->oz_acc_bytes, h->st, active, splitk,
-                              &kernels, h->err_d, h->coop_cap == 0, presliced));
+                              &kernels, h->err_d, h->coop_cap == 0, presliced, guard || h->guard));
     h->launches += kernels - 1;   // the slicing kernel and the split-K finaliser
     return DQMC_OK;
   }
@@ -515,11 +525,11 @@ int trsm_blocked(dqmc_handle* h, const cplx* T, const cplx* rdiag, cplx* Y, bool
     if (lower && j0 + bs < n) {
       // Y[j0+bs:, :] -= T[j0+bs:, j0:j0+bs] Y[j0:j0+bs, :]
       CHK(zgemm_general(h, n - j0 - bs, n, bs, 'N', 'N', cmake(-1, 0), T + (size_t)j0 * n + j0 + bs, n, Y + j0, n,
-                        cmake(1, 0), Y + j0 + bs, n, nullptr, nullptr, true, DQMC_K_TRSM));
+                        cmake(1, 0), Y + j0 + bs, n, nullptr, nullptr, true, DQMC_K_TRSM, nullptr, false, true));
     } else if (!lower && j0 > 0) {
       // Y[:j0, :] -= T[:j0, j0:j0+bs] Y[j0:j0+bs, :]
       CHK(zgemm_general(h, j0, n, bs, 'N', 'N', cmake(-1, 0), T + (size_t)j0 * n, n, Y + j0, n, cmake(1, 0), Y, n,
-                        nullptr, nullptr, true, DQMC_K_TRSM));
+                        nullptr, nullptr, true, DQMC_K_TRSM, nullptr, false, true));
     }
   }
   return DQMC_OK;
@@ -561,7 +571,7 @@ int lu_blocked(dqmc_handle* h, cplx* A, const cplx** Lm) {
              launch_trsm_diag_block(A, n, nullptr, A + (size_t)(p0 + b) * n, n, p0, b, m, true, h->st));
       CHK(zgemm_general(h, m, m, b, 'N', 'N', cmake(-1, 0), A + (size_t)p0 * n + p0 + b, n,
                         A + (size_t)(p0 + b) * n + p0, n, cmake(1, 0), A + (size_t)(p0 + b) * n + p0 + b, n, nullptr,
-                        nullptr, true, DQMC_K_LU));
+                        nullptr, true, DQMC_K_LU, nullptr, false, true));
     }
   }
   LAUNCH(DQMC_K_LU, 0.0, 32.0 * n, launch_lu_diag(A, n, h->lu.udiag, h->lu.rdiag, h->st));
@@ -1360,9 +1370,10 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
     if (oz_plan(h, 4 * h->delay, &S, &bits))
       h->oz_bytes = std::max(h->oz_bytes, ozaki_scratch_bytes((int)n, (int)n, 4 * h->delay, S));
     A(&h->oz_scratch, h->oz_bytes);
-    // split K is taken for fewer than sm_count / 2 output tiles of 64 x 64; two words per real sum above 42 bits
+    // split K is taken for fewer than sm_count / 2 output tiles of 64 x 64; two words per real sum above 42
+    // bits, and one for the magnitudes
     const size_t tiles = (size_t)(h->sm_count / 2 + 1);
-    h->oz_acc_bytes = std::min((size_t)n * n, tiles * 64 * 64) * 4 * sizeof(unsigned long long);
+    h->oz_acc_bytes = std::min((size_t)n * n, tiles * 64 * 64) * 5 * sizeof(unsigned long long);
     A((void**)&h->oz_acc, h->oz_acc_bytes);
   }
   if (!ok) return fail(DQMC_ERR_CUDA);
@@ -1961,7 +1972,10 @@ int dqmc_calculate_greens_udt(dqmc_handle* h, const double* Ul, const double* Dl
   CHK(upload_nn(h, h->Tr, Tr));
   CU(cudaMemcpyAsync(h->Dl, Dl, dn, cudaMemcpyHostToDevice, h->st));
   CU(cudaMemcpyAsync(h->Dr, Dr, dn, cudaMemcpyHostToDevice, h->st));
-  CHK(calculate_greens_into(h, h->Gtmp));
+  h->guard = true;
+  const int rc = calculate_greens_into(h, h->Gtmp);
+  h->guard = false;
+  CHK(rc);
   CHK(download_nn(h, G, h->Gtmp));
   CHK(sync(h));
   if (logdet) *logdet = -h->pin[0];
@@ -2358,13 +2372,11 @@ int dqmc_get_timing(dqmc_handle* h, dqmc_timing* t) {
 int dqmc_gemm_check(dqmc_handle* h, int32_t mode, const double* A, const double* B, double* C) {
   if (h) cudaSetDevice(h->device);
   if (!h || !A || !B || !C || (mode != 0 && mode != 1)) return DQMC_ERR_ARG;
-  if (mode == 1 && h->p.precision != DQMC_PREC_MIXED)
-    return set_err(h, DQMC_ERR_STATE, "mode 1 needs a handle created with DQMC_PREC_MIXED");
   const int n = h->n;
   CHK(upload_nn(h, h->W1, A));
   CHK(upload_nn(h, h->W2, B));
   CHK(zgemm_general(h, n, n, n, 'N', 'N', cmake(1, 0), h->W1, n, h->W2, n, cmake(0, 0), h->W3, n, nullptr, nullptr,
-                    mode == 1));
+                    mode == 1, -1, nullptr, false, true));
   CHK(download_nn(h, C, h->W3));
   return sync(h);
 }

@@ -17,14 +17,30 @@
 //    accumulator per t, over chunks of K' short enough that
 //    chunk (S + 2) 2^{2B - 2} <= 2^24 (the digit bounds above, summed over the
 //    pairs of a group): every partial sum is an integer of at most 24 bits, so
-//    the FP32 accumulation is exact whatever K is (S = 8 slices of 7 bits, the
-//    FP64 form's products: chunks of 384);
-//  * the group sums of a chunk are combined exactly in 64-bit integers (one for
-//    up to 61 bits, else a high and a low one) and the result rounded once to
-//    double with its power-of-two weight and the scales.
-// The only errors are the truncation of the slice expansion (2^{-B S - 1}
-// relative to sigma_i and tau_j), the dropped pairs p + q > S + 1 of the same
-// size, and one FP64 rounding per chunk.
+//    the FP32 accumulation is exact whatever K is (S = 9 slices of 7 bits, the
+//    FP64 form's products: chunks of 320);
+//  * the group sums of all chunks are combined exactly in 64-bit integers (one
+//    for up to 61 bits, else a high and a low one) and the result is rounded once
+//    to double with its power-of-two weight and the scales.
+// The errors besides that rounding are the truncation of the slice expansion
+// (2^{-B S - 1}, at least 2^{-62}, relative to sigma_i and tau_j) and the dropped
+// pairs p + q > S + 1 of the same size.  They go by the largest entries of row i
+// and column j: an entry far below them has fewer bits than in FP64.
+//
+// FP64 form (S = 9, "full"): below 2^-65 sqrt(2 K) sigma_i tau_j, where an FMA
+// chain's error is about 2^-54.5 M, M = sum_k |a_ik| |b_kj|.  That is 0.003 of it for
+// random entries (M = sqrt(2 K) / 4 in units of the scales; K = 16 .. 1024, exact
+// integers) and more than all of it below M = sqrt(2 K) / 2000, where the large
+// entries of the row meet the small ones of the column.  Products whose elements
+// are to be as good as FMA chains one by one (operands from the caller, the LU's
+// and the triangular solves' updates) are guarded: one BF16 magnitude per entry (a
+// float with its own exponent, down to 2^-60) is kept beside the slices, the tensor
+// cores sum M from them to 1%, and where M < 2^-8 sqrt(2 K) sigma_i tau_j (and the
+// sum with an old C is below that, too) the element is an FP64 dot product of the
+// operands instead (oz_dot).  At that limit the slices' error is 0.2 of the FMA
+// chain's.  The magnitudes are one more A tile per K block, a twelfth more of B and
+// 1 / 45 of the arithmetic.  Rows and columns with an Inf or NaN are dot products in
+// every full product, as long as it has its operands.
 // The tensor-core products run on tcgen05.mma (kind::f16, BF16 in, FP32
 // accumulators in tensor memory), with every operand tile staged by TMA
 // (cp.async.bulk.tensor) onto mbarriers; see the engine section below.
@@ -111,6 +127,11 @@ __global__ void __launch_bounds__(64 * SPLIT_V) k_oz_split(const cplx* __restric
 }
 
 struct OzArgs {
+  const cplx *A, *B;         // full form: the operands, op(A) (m x k) and op(B) (k x n) (null: sliced elsewhere)
+  int lda, ldb, k;
+  char opA, opB;
+  float theta;               // guarded: the least magnitude sum (in units of the scales) that the slices carry
+  int theta_e;               // ceil(log2(theta))
   const double* sA;          // (m) row scales 2^(E-1)
   const double* sB;          // (n) column scales
   int m, n, Kp, S, bits;
@@ -122,7 +143,8 @@ struct OzArgs {
   const int* active;         // optional: nothing to do when *active == 0
   int kexact;                // K blocks per exact accumulation (chunk)
   int kchunk;                // split K: K blocks per CTA layer (blockIdx.z); 0 = all
-  unsigned long long* acc;   // split K: exact integer sums (m x n x {re, im}, wide: {re hi, re lo, im hi, im lo}),
+  unsigned long long* acc;   // split K: exact integer sums (m x n x {re, im}, wide: {re hi, re lo, im hi, im lo},
+                             // guarded: and the magnitudes in 2^-40, rounded up),
                              // finished by k_oz_finalize (zero on entry; the finaliser zeroes what it read)
 };
 
@@ -213,36 +235,101 @@ __device__ __forceinline__ int oz_expo(double scale) {   // E of the stored scal
   return f == 0x7FF ? OZ_EXPO_NAN : f - 1022;
 }
 
-template <bool WIDE>
+// ---- full form: elements that the slices do not carry ----
+// Whether the slices carry an element of value v (old C included) and magnitude
+// sum mag, scales 2^ex: mag or, where v is a sum with the old C (sum), v itself is
+// large enough.  mag = 0: no term differs from zero.  Not finite: as k_zgemm has it.
+template <bool GUARD>
+__device__ __forceinline__ bool oz_carried(const OzArgs& a, float mag, int ex, cplx v, bool sum) {
+  const int f = max(expo_field(v.x), expo_field(v.y));
+  if (f == 0x7FF || ex > OZ_EXPO_NAN / 2) return false;
+  return !GUARD || mag >= a.theta || mag == 0.0f || (sum && f > 1023 + ex + a.theta_e);
+}
+// extra scalings one after the other (their product could leave the range of double)
+__device__ __forceinline__ cplx oz_scale2(const OzArgs& a, cplx v, int row, int col) {
+  if (a.rs) v = cscale(v, a.rs[row]);
+  if (a.cs) v = cscale(v, a.cs[col]);
+  return v;
+}
+// the elements C[row of this lane, col] for which need is set, one warp each: dot
+// products in FP64 multiply-adds over the operands (called by whole warps; C
+// still holds its old value there).  Bound: FP64 issue, 4 multiply-adds per term,
+// as for k_zgemm; rows of A are read 16 bytes per sector.
+__device__ __forceinline__ void oz_dot(const OzArgs& a, int row, int col, bool need) {
+  const int lane = threadIdx.x & 31, K = a.active ? min(a.k, 4 * *a.active) : a.k;
+  unsigned todo = __ballot_sync(0xffffffffu, need);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int r = __shfl_sync(0xffffffffu, row, src), c = __shfl_sync(0xffffffffu, col, src);
+    const cplx* pa = a.opA == 'N' ? a.A + r : a.A + (size_t)r * a.lda;
+    const cplx* pb = a.opB == 'N' ? a.B + (size_t)c * a.ldb : a.B + c;
+    const size_t sa = a.opA == 'N' ? a.lda : 1, sb = a.opB == 'N' ? 1 : a.ldb;
+    cplx s = cmake(0.0, 0.0);
+#pragma unroll 4
+    for (int k = lane; k < K; k += 32) {
+      cplx x = pa[k * sa], y = pb[k * sb];
+      if (a.opA == 'C') x = cconj(x);
+      if (a.opB == 'C') y = cconj(y);
+      s = cfma(x, y, s);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (lane == 0) {
+      cplx* cp = &a.C[(size_t)c * a.ldc + r];
+      s = cmul(a.alpha, oz_scale2(a, s, r, c));   // as k_zgemm, also for what is not finite
+      if (a.beta.x != 0.0 || a.beta.y != 0.0) s = cfma(a.beta, *cp, s);
+      *cp = s;
+    }
+    __syncwarp();
+  }
+}
+
+template <bool WIDE, bool FULL = false, bool GUARD = false>
 __global__ void k_oz_finalize(OzArgs a) {
   const int e0 = -a.bits * (a.S + 1), sh = oz_wide_shift(a.bits);
   const bool plain = oz_plain(a);
   const size_t total = (size_t)a.m * a.n;
-  constexpr int W = WIDE ? 2 : 1;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const int col = (int)(e / a.m), row = (int)(e - (size_t)col * a.m);
-    long long v[2 * W];
+  constexpr int W = WIDE ? 2 : 1, WORDS = 2 * W + (GUARD ? 1 : 0);
+  // whole warps stay in the loop (oz_dot)
+  for (size_t b = (size_t)blockIdx.x * blockDim.x; b < total; b += (size_t)gridDim.x * blockDim.x) {
+    const size_t e = b + threadIdx.x;
+    const bool in = e < total;
+    const int col = in ? (int)(e / a.m) : 0, row = in ? (int)(e - (size_t)col * a.m) : 0;
+    bool need = false;
+    if (in) {
+      long long v[WORDS];
 #pragma unroll
-    for (int q = 0; q < 2 * W; ++q) {
-      v[q] = (long long)a.acc[2 * W * e + q];
-      a.acc[2 * W * e + q] = 0ull;
+      for (int q = 0; q < WORDS; ++q) {
+        v[q] = (long long)a.acc[WORDS * e + q];
+        a.acc[WORDS * e + q] = 0ull;
+      }
+      const int ex = oz_expo(a.sA[row]) + oz_expo(a.sB[col]);
+      cplx r = cmake(oz_value<WIDE>(v[0], v[W - 1], sh, e0 + ex, oz_window(e0 + ex)),
+                     oz_value<WIDE>(v[W], v[2 * W - 1], sh, e0 + ex, oz_window(e0 + ex)));
+      if (ex > OZ_EXPO_NAN / 2) r = cmake(nan(""), nan(""));
+      if constexpr (FULL) r = oz_scale2(a, r, row, col);
+      else if (a.rs || a.cs) r = cscale(r, (a.rs ? a.rs[row] : 1.0) * (a.cs ? a.cs[col] : 1.0));
+      cplx* cp = &a.C[(size_t)col * a.ldc + row];
+      const bool rd = a.beta.x != 0.0 || a.beta.y != 0.0;
+      r = oz_combine(a, a.beta, r, rd ? *cp : cmake(0.0, 0.0), plain);
+      if constexpr (FULL)
+        need = a.A && !oz_carried<GUARD>(a, GUARD ? (float)v[WORDS - 1] * 0x1p-40f : 0.0f, ex, r,
+                                         rd && plain && !a.rs && !a.cs);
+      if (!need) *cp = r;
     }
-    const int ex = oz_expo(a.sA[row]) + oz_expo(a.sB[col]);
-    cplx r = cmake(oz_value<WIDE>(v[0], v[W - 1], sh, e0 + ex, oz_window(e0 + ex)),
-                   oz_value<WIDE>(v[W], v[2 * W - 1], sh, e0 + ex, oz_window(e0 + ex)));
-    if (ex > OZ_EXPO_NAN / 2) r = cmake(nan(""), nan(""));
-    if (a.rs || a.cs) r = cscale(r, (a.rs ? a.rs[row] : 1.0) * (a.cs ? a.cs[col] : 1.0));
-    cplx* cp = &a.C[(size_t)col * a.ldc + row];
-    const bool rd = a.beta.x != 0.0 || a.beta.y != 0.0;
-    *cp = oz_combine(a, a.beta, r, rd ? *cp : cmake(0.0, 0.0), plain);
+    if constexpr (FULL) oz_dot(a, row, col, need);
   }
 }
 
 // ---------------------------------------------------------------------------
 // tcgen05 engine: TMA-staged slices, tensor-core MMAs into TMEM accumulators
 // ---------------------------------------------------------------------------
-// A CTA computes 128 x BN complex tiles of C (BN = 32, 16 or 8; the figures below
-// are for 32), persistently: one CTA per SM
+// A CTA computes 128 x BN complex tiles of C (BN = 32, 16 or 8, in the full form
+// 24, 16 or 8; the figures below are for 32), persistently: one CTA per SM
 // takes tiles x, x + grid, ... and the MMAs of a tile run while the epilogue
 // of the previous one converts and stores.  Each MMA is
 // M = 128, K = 16 (kind::f16, BF16 in, FP32 out), N = 64 per B slice: the
@@ -259,19 +346,27 @@ __global__ void k_oz_finalize(OzArgs a) {
 //     B buffer with tcgen05.commit and marking a chunk's accumulators final
 //     with a commit; before the first MMA of the next chunk (of this tile or
 //     the next) it waits until the epilogue has read them out of TMEM;
-//   * warps 2-17 (four per TMEM lane quarter, 8 columns each) read the S
-//     exact FP32 group sums of a chunk with tcgen05.ld, release TMEM, combine
-//     the sums exactly in 64-bit integers (Horner in 2^bits; two words above
-//     61 bits), then round, scale and store.
+//   * the other warps (four per TMEM lane quarter, 8 columns each) read the S
+//     exact FP32 group sums of a chunk with tcgen05.ld, release TMEM, add
+//     the sums with their weights to 64-bit integers (two words above 61 bits),
+//     and after the tile's last chunk round, scale and store.
+// The full form (S = 9) has tiles of at most 24 columns, so that its 9 groups of
+// 48 columns (and the magnitudes' 32, if guarded) fit into TMEM; the magnitudes are
+// slice S of A and one more B tile, summed over all chunks of a tile.
 // Every wait is bounded; on a timeout the kernel sets an error bit, drains
 // what it issued (bounded) and frees its TMEM.
 constexpr int TC_BM = 128;                      // rows of C per CTA (TMEM lanes)
 constexpr int TC_BN = 32;                       // complex columns of C per tile, at most (BN of the kernel: 32, 16 or 8)
 constexpr int TC_BK = 64;                       // BF16 per K block: one 128-byte swizzle row
 constexpr int TC_MAXS = 8;                      // S groups x 64 TMEM columns <= 512
+constexpr int TC_BN_FULL = 24;                 // widest tile of the full form: 9 x 48 + 32 TMEM columns
+// columns of the magnitude product (N of an MMA with M = 128 is a multiple of 16)
+__host__ __device__ constexpr int tc_mag_cols(int bn) { return (bn + 15) / 16 * 16; }
 constexpr int TC_ARING = 6;                     // A-slice stages (S <= 6: one K block of A in flight)
-constexpr int TC_EPI_WARPS = 16;                // epilogue warps 2-17: four per TMEM lane quarter, BN / 4 columns each
-constexpr int TC_THREADS = 32 * (2 + TC_EPI_WARPS);   // warp 0 TMA, warp 1 MMA (and TMEM allocation)
+// epilogue warps, from 2 on: four per TMEM lane quarter, BN / 4 columns each; three of 8
+// columns at BN = 24 (with 16 warps of 6 a thread has 96 registers and spills)
+__host__ __device__ constexpr int tc_epi_warps(int bn) { return bn == 24 ? 12 : 16; }
+__host__ __device__ constexpr int tc_threads(int bn) { return 32 * (2 + tc_epi_warps(bn)); }   // warp 0 TMA, warp 1 MMA
 constexpr int TC_A_TILE = TC_BM * TC_BK * 2;    // 16 KB
 __host__ __device__ constexpr int tc_b_half(int bn) { return bn * TC_BK * 2; }   // 4 KB at BN = 32: BN rows of B'_re or of B'_im
 // MMA instruction descriptor (kind::f16): D F32 (bits 4-5 = 1), A BF16 (bits
@@ -288,11 +383,14 @@ __host__ __device__ constexpr uint32_t tc_idesc(int n) {
 // arithmetic.
 __host__ __device__ constexpr int tc_nstack(int bn) { return 128 / bn; }
 
-__host__ __device__ constexpr size_t tc_smem_bytes(int S, int bn) {
-  return 1024 + (size_t)4 * S * tc_b_half(bn) + (size_t)TC_ARING * TC_A_TILE + 256;
+// B slices of one K block (and the magnitudes, mag columns of them)
+__host__ __device__ constexpr int tc_b_bytes(int S, int bn, int mag) { return 2 * S * tc_b_half(bn) + mag * TC_BK * 2; }
+__host__ __device__ constexpr size_t tc_smem_bytes(int S, int bn, int mag) {
+  return 1024 + (size_t)2 * tc_b_bytes(S, bn, mag) + (size_t)TC_ARING * TC_A_TILE + 256;
 }
-__host__ __device__ constexpr uint32_t tc_tmem_cols(int S, int bn) {   // S groups of 2 bn columns, a power of two
-  return S * bn <= 16 ? 32u : (S * bn <= 32 ? 64u : (S * bn <= 64 ? 128u : (S * bn <= 128 ? 256u : 512u)));
+static_assert(tc_smem_bytes(9, TC_BN_FULL, tc_mag_cols(TC_BN_FULL)) <= 227 * 1024, "shared memory of a CTA");
+__host__ __device__ constexpr uint32_t tc_tmem_cols(int cols) {   // a power of two
+  return cols <= 32 ? 32u : (cols <= 64 ? 64u : (cols <= 128 ? 128u : (cols <= 256 ? 256u : 512u)));
 }
 
 // Shared-memory matrix descriptor of a K-major operand tile written by TMA
@@ -392,21 +490,23 @@ __device__ __forceinline__ void tc_ld(uint32_t taddr, uint32_t (&r)[W]) {
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 struct TcMaps {
-  CUtensorMap a, bre, bim;   // (Kp, rows, S) BF16 slices, box (64, 128 | 32, 1), 128-byte swizzle
+  CUtensorMap a, bre, bim;   // (Kp, rows, S) BF16 slices, box (64, 128 | BN, 1), 128-byte swizzle
+  CUtensorMap bmag;          // guarded: (Kp, n, 1) magnitudes of B, box (64, 32 | 16, 1)
 };
 
-template <bool WIDE, int BITS, int BN>   // BITS: slice width, 0 = a.bits
-__global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_constant__ TcMaps maps, OzArgs a,
+template <bool WIDE, int BITS, int BN, bool FULL = false, bool GUARD = false>   // BITS: slice width, 0 = a.bits
+__global__ void __launch_bounds__(tc_threads(BN), 1) k_oz_gemm_tc(const __grid_constant__ TcMaps maps, OzArgs a,
                                                              int* err) {
-  constexpr int TC_B_HALF = tc_b_half(BN), TC_B_TILE = 2 * TC_B_HALF, NSTACK = tc_nstack(BN), CPW = BN / 4, PC = CPW < 4 ? CPW : 4;
+  constexpr int TC_B_HALF = tc_b_half(BN), TC_B_TILE = 2 * TC_B_HALF, NSTACK = tc_nstack(BN), CPW = 4 * BN / tc_epi_warps(BN);
+  constexpr int PC = CPW < 4 ? CPW : 4, MAG = GUARD ? tc_mag_cols(BN) : 0;
   if (a.active && *a.active == 0) return;   // flush with nothing pending (uniform over the grid)
   extern __shared__ uint8_t tc_smem_raw[];
   const uint32_t raw = smem_u32(tc_smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* basep = tc_smem_raw + (base - raw);
-  const int S = a.S;
-  const uint32_t sB = base;                                     // [2][S] B tiles
-  const uint32_t sA = base + 2u * S * TC_B_TILE;                // [TC_ARING] A tiles of 16 KB
+  const int S = FULL ? OZ_FP64_S : a.S, SA = S + (GUARD ? 1 : 0);   // A slices per K block
+  const uint32_t sB = base, strideB = (uint32_t)tc_b_bytes(S, BN, MAG);   // [2] S B tiles (and the magnitudes)
+  const uint32_t sA = base + 2u * strideB;                      // [TC_ARING] A tiles of 16 KB
   const uint32_t sBar = sA + TC_ARING * TC_A_TILE;              // barriers
   uint64_t* bars = reinterpret_cast<uint64_t*>(basep + (sBar - base));
   // barrier slots: full_b 0-1, empty_b 2-3, full_a FA.., empty_a EA.., a chunk's
@@ -431,13 +531,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
     i0 = (t / tiles_x) * TC_BM;
     j0 = (t % tiles_x) * BN;
   };
-  const uint32_t ncols = tc_tmem_cols(S, BN);
+  const uint32_t ncols = tc_tmem_cols(S * 2 * BN + MAG);
 
   if (threadIdx.x == 0) {
     for (int k = 0; k < 2; ++k) { mbar_init(bar(k), 1); mbar_init(bar(2 + k), 1); }
     for (int k = 0; k < TC_ARING; ++k) { mbar_init(bar(FA + k), 1); mbar_init(bar(EA + k), 1); }
     mbar_init(bar(ACC), 1);
-    mbar_init(bar(TE), TC_EPI_WARPS);
+    mbar_init(bar(TE), tc_epi_warps(BN));
     mbar_init(bar(DONE), 1);
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -469,9 +569,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
         int i0, j0;
         tile_of(u / nkb, i0, j0);
         const int kb = kb0 + u % nkb;
-        mbar_expect_tx(bar(bb), (uint32_t)(S * TC_B_TILE));
+        mbar_expect_tx(bar(bb), strideB);
+        if constexpr (GUARD)
+          tma_load3(sB + (uint32_t)bb * strideB + (uint32_t)S * TC_B_TILE, &maps.bmag, bar(bb), kb * TC_BK, j0, 0);
         for (int q = 0; q < S; ++q) {
-          const uint32_t dst = sB + (uint32_t)(bb * S + q) * TC_B_TILE;
+          const uint32_t dst = sB + (uint32_t)bb * strideB + (uint32_t)q * TC_B_TILE;
           tma_load3(dst, &maps.bre, bar(bb), kb * TC_BK, j0, q);
           tma_load3(dst + TC_B_HALF, &maps.bim, bar(bb), kb * TC_BK, j0, q);
         }
@@ -485,7 +587,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
         int i0, j0;
         tile_of(u / nkb, i0, j0);
         const int kb = kb0 + u % nkb;
-        for (int p = 0; p < S; ++p, ++a_use) {
+        for (int p = 0; p < SA; ++p, ++a_use) {
           // the next block's B as early as its buffer is free (without waiting)
           if (b_next == u + 1 && u + 1 < U && issue_b(u + 1, false)) ++b_next;
           const int slot = a_use % TC_ARING;
@@ -512,15 +614,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
         if (!mbar_wait(bar(bb), (u >> 1) & 1, err, s_abort)) break;
         tc_fence_after();
         bool ok = true;
-        for (int p = 0; p < S; ++p, ++a_use) {
+        for (int p = 0; p < SA; ++p, ++a_use) {
           const int slot = a_use % TC_ARING;
           if (!mbar_wait(bar(FA + slot), (a_use / TC_ARING) & 1, err, s_abort)) { ok = false; break; }
           tc_fence_after();
           const uint64_t ad = tc_desc(sA + (uint32_t)slot * TC_A_TILE);
+          if (GUARD && p == S) {   // the magnitudes, summed over the whole tile
+            const uint64_t bd = tc_desc(sB + (uint32_t)bb * strideB + (uint32_t)S * TC_B_TILE);
+#pragma unroll
+            for (int kk = 0; kk < TC_BK / 16; ++kk)
+              tc_mma(tmem + (uint32_t)(S * 2 * BN), ad + 2u * kk, bd + 2u * kk, tc_idesc(MAG > 0 ? MAG : 16),
+                     (kbi == 0 && kk == 0) ? 0u : 1u);
+          }
           for (int q = 0; q + p < S; q += NSTACK) {
             // pairs (p + 1, q + 1 ..) belong to groups t = p + q + 2 ..: accumulator columns from (p + q) * 64
             const int cnt = min(NSTACK, S - p - q);
-            const uint64_t bd = tc_desc(sB + (uint32_t)(bb * S + q) * TC_B_TILE);
+            const uint64_t bd = tc_desc(sB + (uint32_t)bb * strideB + (uint32_t)q * TC_B_TILE);
             const uint32_t d = tmem + (uint32_t)(p + q) * (2 * BN);
             const uint32_t idesc = tc_idesc(2 * BN * cnt);
 #pragma unroll
@@ -539,9 +648,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
       tc_commit(bar(DONE));           // every MMA issued has completed (the abort path waits on it)
     }
   } else if (U > 0) {
-    // ---- epilogue: warps 2-17, four per TMEM lane quarter (warp % 4); warp w
-    //      takes the CPW columns of group (w - 2) / 4 of each tile, chunk by chunk
-    //      (chunks after the first are added to the C the same thread stored) ----
+    // ---- epilogue: warps from 2 on, in each TMEM lane quarter (warp % 4); warp w
+    //      takes the CPW columns of group (w - 2) / 4 of each tile, chunk by chunk ----
     const int quarter = warp & 3;
     const int cg = (warp - 2) >> 2;
     const uint32_t tq = tmem + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(CPW * cg);
@@ -551,11 +659,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
     const bool plain = oz_plain(a), neg = a.alpha.x < 0.0;
     const bool simple = plain && !a.rs && !a.cs;   // alpha = +-1, beta in {0, 1}, no extra scalings
     const int nch = (nkb + a.kexact - 1) / a.kexact;
+    long long ar[CPW], ai[CPW], lr[WIDE ? CPW : 1], li[WIDE ? CPW : 1];   // the tile's sums so far
     for (int vt = 0; vt < my_tiles * nch; ++vt) {
       int i0, j0;
       tile_of(vt / nch, i0, j0);
       j0 += CPW * cg;
-      const bool first = vt % nch == 0;
+      // several chunks only in the full form: the mixed form's widths take all of K at once
+      const bool first = !FULL || vt % nch == 0, last = !FULL || vt % nch == nch - 1;
       const int row = i0 + 32 * quarter + lane;
       const bool waited = mbar_wait(bar(ACC), vt & 1, err, s_abort);
       // tcgen05.ld is warp-collective: the decision must be uniform over the warp
@@ -563,11 +673,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
       if (!have) break;
       __syncwarp();
       tc_fence_after();
-      long long ar[CPW], ai[CPW], lr[WIDE ? CPW : 1], li[WIDE ? CPW : 1];
+      if (first) {
 #pragma unroll
-      for (int c = 0; c < CPW; ++c) { ar[c] = 0; ai[c] = 0; }
+        for (int c = 0; c < CPW; ++c) { ar[c] = 0; ai[c] = 0; }
 #pragma unroll
-      for (int c = 0; c < (WIDE ? CPW : 1); ++c) { lr[c] = 0; li[c] = 0; }
+        for (int c = 0; c < (WIDE ? CPW : 1); ++c) { lr[c] = 0; li[c] = 0; }
+      }
 #pragma unroll 1
       for (int g = 0; g < ghi; ++g) {
         uint32_t ur[CPW], ui[CPW];
@@ -576,8 +687,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
         tc_wait_ld();
 #pragma unroll
         for (int c = 0; c < CPW; ++c) {
-          ar[c] = (ar[c] << bits) + (long long)__float2int_rn(__uint_as_float(ur[c]));
-          ai[c] = (ai[c] << bits) + (long long)__float2int_rn(__uint_as_float(ui[c]));
+          ar[c] += (long long)__float2int_rn(__uint_as_float(ur[c])) << (bits * (ghi - 1 - g));
+          ai[c] += (long long)__float2int_rn(__uint_as_float(ui[c])) << (bits * (ghi - 1 - g));
         }
       }
       if constexpr (WIDE) {
@@ -589,21 +700,27 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
           tc_wait_ld();
 #pragma unroll
           for (int c = 0; c < CPW; ++c) {
-            lr[c] = (lr[c] << bits) + (long long)__float2int_rn(__uint_as_float(ur[c]));
-            li[c] = (li[c] << bits) + (long long)__float2int_rn(__uint_as_float(ui[c]));
+            lr[c] += (long long)__float2int_rn(__uint_as_float(ur[c])) << (bits * (S - 1 - g));
+            li[c] += (long long)__float2int_rn(__uint_as_float(ui[c])) << (bits * (S - 1 - g));
           }
         }
+      }
+      uint32_t mg[CPW] = {};   // the magnitude sums
+      if (GUARD && last) {
+        tc_ld<CPW>(tq + (uint32_t)(S * 2 * BN), mg);
+        tc_wait_ld();
       }
       // this chunk's accumulators are all in registers: TMEM may take the next chunk
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(TE));
-      if (row >= a.m) continue;
+      if (!last || (!FULL && row >= a.m)) continue;
       if (a.acc) {
 #pragma unroll
         for (int c = 0; c < CPW; ++c) {
-          if (j0 + c >= a.n) continue;
-          unsigned long long* qa = a.acc + (WIDE ? 4 : 2) * ((size_t)(j0 + c) * a.m + row);
+          if (j0 + c >= a.n || row >= a.m) continue;
+          unsigned long long* qa = a.acc + (GUARD ? 5 : WIDE ? 4 : 2) * ((size_t)(j0 + c) * a.m + row);
+          if constexpr (GUARD) atomicAdd(qa + 4, __float2ull_ru(__uint_as_float(mg[c]) * 0x1p40f));
           atomicAdd(qa, (unsigned long long)ar[c]);
           if constexpr (WIDE) {
             atomicAdd(qa + 1, (unsigned long long)lr[c]);
@@ -615,15 +732,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
         }
         continue;
       }
-      const cplx beta = first ? a.beta : cmake(1.0, 0.0);
+      const cplx beta = a.beta;
       const bool rd = beta.x != 0.0 || beta.y != 0.0;
+      const bool rowin = !FULL || row < a.m;
+      unsigned need = 0;   // full form: columns that the slices do not carry
       // the scale sA sB 2^-bits(S+1) is a power of two: the value is the exact
       // integer rounded once with that exponent on the integer units (GB300
       // issues FP64 at a small fraction of its integer rate); the FP64
       // operations left are the extra scalings and the addition of the old C.
       // Passes of 4 columns (2 at BN = 8), the loads (scales, old C) of a pass
       // issued before its first store.
-      const int e_row = oz_expo(a.sA[row]) + e0;
+      const int e_row = rowin ? oz_expo(a.sA[row]) + e0 : 0;
 #pragma unroll
       for (int hh = 0; hh < CPW; hh += PC) {
         cplx cold[PC];
@@ -632,7 +751,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
 #pragma unroll
         for (int c = 0; c < PC; ++c) {
           const int col = j0 + hh + c;
-          const bool in = col < a.n;
+          const bool in = col < a.n && rowin;
           cold[c] = rd && in ? a.C[(size_t)col * a.ldc + row] : cmake(0.0, 0.0);
           e_col[c] = in ? oz_expo(a.sB[col]) + e_row : 0;
           window = window && oz_window(e_col[c]);
@@ -640,25 +759,40 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_gemm_tc(const __grid_const
         if (window && simple) {
 #pragma unroll
           for (int c = 0; c < PC; ++c) {
-            if (j0 + hh + c >= a.n) continue;
+            if (j0 + hh + c >= a.n || !rowin) continue;
             cplx v = cmake(oz_value<WIDE>(ar[hh + c], lr[WIDE ? hh + c : 0], sh, e_col[c], true),
                            oz_value<WIDE>(ai[hh + c], li[WIDE ? hh + c : 0], sh, e_col[c], true));
             if (neg) v = cmake(-v.x, -v.y);
             if (rd) v = cadd(cold[c], v);
+            if (FULL && a.A && !oz_carried<GUARD>(a, __uint_as_float(mg[hh + c]), e_col[c] - e0, v, rd)) {
+              need |= 1u << (hh + c);
+              continue;
+            }
             a.C[(size_t)(j0 + hh + c) * a.ldc + row] = v;
           }
         } else {
 #pragma unroll
           for (int c = 0; c < PC; ++c) {
             const int col = j0 + hh + c;
-            if (col >= a.n) continue;
+            if (col >= a.n || !rowin) continue;
             cplx v = cmake(oz_value<WIDE>(ar[hh + c], lr[WIDE ? hh + c : 0], sh, e_col[c], window),
                            oz_value<WIDE>(ai[hh + c], li[WIDE ? hh + c : 0], sh, e_col[c], window));
             if (e_col[c] > OZ_EXPO_NAN / 2) v = cmake(nan(""), nan(""));
-            if (a.rs || a.cs) v = cscale(v, (a.rs ? a.rs[row] : 1.0) * (a.cs ? a.cs[col] : 1.0));
-            a.C[(size_t)col * a.ldc + row] = oz_combine(a, beta, v, cold[c], plain);
+            if constexpr (FULL) v = oz_scale2(a, v, row, col);
+            else if (a.rs || a.cs) v = cscale(v, (a.rs ? a.rs[row] : 1.0) * (a.cs ? a.cs[col] : 1.0));
+            v = oz_combine(a, beta, v, cold[c], plain);
+            if (FULL && a.A && !oz_carried<GUARD>(a, __uint_as_float(mg[hh + c]), e_col[c] - e0, v, false)) {
+              need |= 1u << (hh + c);
+              continue;
+            }
+            a.C[(size_t)col * a.ldc + row] = v;
           }
         }
+      }
+      if constexpr (FULL) {
+        if (__any_sync(0xffffffffu, need != 0u))
+#pragma unroll 1
+          for (int c = 0; c < CPW; ++c) oz_dot(a, row, j0 + c, (need >> c & 1u) != 0u);
       }
     }
   }
@@ -710,24 +844,29 @@ static int oz_chunk_blocks(int S, int bits) {
   return (int)((1ll << (24 - 2 * bits + 2)) / (S + 2) / TC_BK);
 }
 
-OzSlices ozaki_slices(void* scratch, int m, int n, int K, int S, int bits) {
+static bool oz_full(int S) { return S == OZ_FP64_S; }
+
+OzSlices ozaki_slices(void* scratch, int m, int n, int K, int S, int bits, bool guard) {
   const int Kpad = (K + 15) / 16 * 16;
   const size_t Kp = 2 * (size_t)Kpad;
   OzSlices o;
   o.As = reinterpret_cast<__nv_bfloat16*>(scratch);
-  o.Bre = o.As + (size_t)S * m * Kp;
+  o.Bre = o.As + (size_t)(S + (guard ? 1 : 0)) * m * Kp;
   o.Bim = o.Bre + (size_t)S * n * Kp;
-  o.sA = reinterpret_cast<double*>(o.Bim + (size_t)S * n * Kp);
+  __nv_bfloat16* end = o.Bim + (size_t)S * n * Kp;
+  o.Bmag = guard ? end : nullptr;
+  o.sA = reinterpret_cast<double*>(end + (guard ? (size_t)n * Kp : 0));
   o.sB = o.sA + m;
   o.m = m; o.n = n; o.Kpad = Kpad; o.S = S; o.bits = bits;
   return o;
 }
 
-// Scratch: As S*m*Kp, Bre/Bim S*n*Kp bf16, scales m + n doubles.
+// Scratch: As S*m*Kp, Bre/Bim S*n*Kp bf16 (full form: (m + n)*Kp more for the magnitudes), scales m + n doubles.
 size_t ozaki_scratch_bytes(int m, int n, int K, int S) {
   const size_t Kpad = ((size_t)K + 15) / 16 * 16;
   const size_t Kp = 2 * Kpad;
-  return (size_t)S * Kp * ((size_t)m + 2 * (size_t)n) * sizeof(__nv_bfloat16) + ((size_t)m + n) * sizeof(double) + 256;
+  return (S * ((size_t)m + 2 * (size_t)n) + (oz_full(S) ? (size_t)m + n : 0)) * Kp * sizeof(__nv_bfloat16) +
+         ((size_t)m + n) * sizeof(double) + 256;
 }
 
 // cuTensorMapEncodeTiled from the driver, looked up once (no link against libcuda).
@@ -779,37 +918,56 @@ static cudaError_t launch_tc(int which, dim3 grid, int S, cudaStream_t st, const
   void (*const kernels_tc[6])(TcMaps, OzArgs, int*) = {k_oz_gemm_tc<false, 5, BN>, k_oz_gemm_tc<false, 6, BN>,
                                                        k_oz_gemm_tc<false, 7, BN>, k_oz_gemm_tc<false, 0, BN>,
                                                        k_oz_gemm_tc<true, 7, BN>,  k_oz_gemm_tc<true, 0, BN>};
-  if (cudaError_t e = limits[which].raise((const void*)kernels_tc[which], (int)tc_smem_bytes(TC_MAXS, BN));
+  if (cudaError_t e = limits[which].raise((const void*)kernels_tc[which], (int)tc_smem_bytes(TC_MAXS, BN, 0));
       e != cudaSuccess)
     return e;
-  kernels_tc[which]<<<grid, TC_THREADS, tc_smem_bytes(S, BN), st>>>(maps, a, err);
+  kernels_tc[which]<<<grid, tc_threads(BN), tc_smem_bytes(S, BN, 0), st>>>(maps, a, err);
   return cudaSuccess;
+}
+template <int BN, bool GUARD>
+static cudaError_t launch_tc_full(dim3 grid, cudaStream_t st, const TcMaps& maps, const OzArgs& a, int* err) {
+  static SmemLimit limit;
+  constexpr size_t smem = tc_smem_bytes(OZ_FP64_S, BN, GUARD ? tc_mag_cols(BN) : 0);
+  void (*const fn)(TcMaps, OzArgs, int*) = k_oz_gemm_tc<true, OZ_FP64_BITS, BN, true, GUARD>;
+  if (cudaError_t e = limit.raise((const void*)fn, (int)smem); e != cudaSuccess) return e;
+  fn<<<grid, tc_threads(BN), smem, st>>>(maps, a, err);
+  return cudaSuccess;
+}
+template <bool GUARD>
+static cudaError_t launch_tc_full(int bn, dim3 grid, cudaStream_t st, const TcMaps& maps, const OzArgs& a, int* err) {
+  return bn == 8    ? launch_tc_full<8, GUARD>(grid, st, maps, a, err)
+         : bn == 16 ? launch_tc_full<16, GUARD>(grid, st, maps, a, err)
+                    : launch_tc_full<TC_BN_FULL, GUARD>(grid, st, maps, a, err);
 }
 
 // Complex columns BN of a tile: as narrow as keeps all tiles (times the layers of
 // split K) in one wave.  A tile's time is 3 us until its first MMA, the MMAs and
 // 8 us of epilogue at BN = 32, and the last two shrink with BN; A, in
 // exchange, is read by more CTAs, which a long K does not repay beyond one wave.
-// Flush of 16 sites, us, BN = 32 / 16 / 8: n = 256 23 / 19 / 17, n = 400 (56 bits)
-// 27 / 22 / 24, n = 576 20 / 19 / 21, n = 1024 31 / 34 / 44; product of n = 256
+// Flush of 16 sites, us, BN = 32 / 16 / 8: n = 256 23 / 19 / 17, n = 400 (8 slices of
+// 7 bits) 27 / 22 / 24, n = 576 20 / 19 / 21, n = 1024 31 / 34 / 44; product of n = 256
 // 35 / 31 / 39, of n = 576 105 / 131 / 178.
-static int tc_width(int m, int nn, int layers, int ksteps, int sms) {
+static int tc_width(int m, int nn, int layers, int ksteps, int sms, int widest) {
   const int rows = (m + TC_BM - 1) / TC_BM, most = ksteps <= 4 ? sms + sms / 4 : sms;
-  for (int bn = 8; bn < TC_BN; bn *= 2)
+  for (int bn = 8; bn < widest; bn *= 2)
     if (rows * ((nn + bn - 1) / bn) * layers <= most) return bn;
-  return TC_BN;
+  return widest;
 }
 
 cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                                const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rowscale,
                                const double* colscale, int S, int bits, void* scratch, size_t scratch_bytes,
                                unsigned long long* acc, size_t acc_bytes, cudaStream_t st, const int* active,
-                               int splitk, int* kernels, int* err, bool persistent, bool presliced) {
-  if (S < 1 || S > TC_MAXS || bits < 1 || bits > 8 || !err) return cudaErrorInvalidValue;
+                               int splitk, int* kernels, int* err, bool persistent, bool presliced, bool guard) {
+  const bool full = oz_full(S);
+  if (S < 1 || (S > TC_MAXS && !full) || bits < 1 || bits > 8 || !err) return cudaErrorInvalidValue;
+  if (full && bits != OZ_FP64_BITS) return cudaErrorInvalidValue;
+  guard = guard && full;
+  if (guard && presliced) return cudaErrorInvalidValue;
   const int Kpad = (k + 15) / 16 * 16;
   const size_t Kp = 2 * (size_t)Kpad;
   if (ozaki_scratch_bytes(m, nn, k, S) > scratch_bytes) return cudaErrorInvalidValue;
-  const OzSlices sl = ozaki_slices(scratch, m, nn, k, S, bits);
+  const OzSlices sl = ozaki_slices(scratch, m, nn, k, S, bits, guard);
   if (!presliced) {   // otherwise the slices are already in scratch (cut by the delayed local-update kernel)
     const size_t smem = (size_t)SPLIT_V * (k + 1) * sizeof(cplx);
     static SmemLimit limit_split;
@@ -821,6 +979,9 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
                                                                                    active);
   }
   OzArgs a;
+  a.A = presliced ? nullptr : A; a.B = B; a.lda = lda; a.ldb = ldb; a.k = k; a.opA = opA; a.opB = opB;
+  a.theta = guard ? (float)std::ldexp(std::sqrt(2.0 * k), -8) : 0.0f;
+  a.theta_e = guard ? (int)std::ceil(std::log2((double)a.theta)) : 0;
   a.sA = sl.sA; a.sB = sl.sB;
   a.m = m; a.n = nn; a.Kp = (int)Kp; a.S = S; a.bits = bits;
   a.alpha = alpha; a.beta = beta; a.C = C; a.ldc = ldc; a.rs = rowscale; a.cs = colscale; a.active = active;
@@ -829,16 +990,16 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
   a.kexact = oz_chunk_blocks(S, bits);
   a.kchunk = 0;
   a.acc = nullptr;
-  if (a.kexact < 1) return cudaErrorInvalidValue;
   // persistent CTAs: one per SM (each holds the whole TMEM), every CTA takes
   // tiles x, x + grid, ... and overlaps a tile's epilogue with the next tile's
   // MMAs; otherwise one CTA per tile (chains sharing the GPU: short CTAs let
   // the other chains' kernels in between)
   const int sms = sm_count_of_current_device();
   const int ksteps = (int)((Kp + TC_BK - 1) / TC_BK);
+  if (a.kexact < (full ? 1 : ksteps)) return cudaErrorInvalidValue;
   int layers = 1;
   if (splitk > 1 && !active && ksteps > 1 && acc &&
-      (size_t)m * nn * (wide ? 4 : 2) * sizeof(unsigned long long) <= acc_bytes) {
+      (size_t)m * nn * (guard ? 5 : wide ? 4 : 2) * sizeof(unsigned long long) <= acc_bytes) {
     // split K over blockIdx.z: exact 64-bit integer partial sums in acc, which
     // is zero between products (zeroed at allocation, re-zeroed by the finaliser)
     if (splitk > ksteps) splitk = ksteps;
@@ -846,18 +1007,22 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
     layers = (ksteps + a.kchunk - 1) / a.kchunk;
     a.acc = acc;
   }
-  const int bn = persistent ? tc_width(m, nn, layers, ksteps, sms) : TC_BN;
+  const int widest = full ? TC_BN_FULL : TC_BN;
+  const int bn = persistent ? tc_width(m, nn, layers, ksteps, sms, widest) : widest;
   const int ntiles = ((nn + bn - 1) / bn) * ((m + TC_BM - 1) / TC_BM);
   const dim3 grid(persistent && ntiles > sms ? sms : ntiles, 1, layers);
   if (kernels) *kernels = (a.acc ? 3 : 2) - (presliced ? 1 : 0);
   {
     TcMaps maps;
-    if (!encode_slices(&maps.a, sl.As, Kp, m, S, TC_BM) || !encode_slices(&maps.bre, sl.Bre, Kp, nn, S, bn) ||
-        !encode_slices(&maps.bim, sl.Bim, Kp, nn, S, bn))
+    if (!encode_slices(&maps.a, sl.As, Kp, m, S + (guard ? 1 : 0), TC_BM) ||
+        !encode_slices(&maps.bre, sl.Bre, Kp, nn, S, bn) || !encode_slices(&maps.bim, sl.Bim, Kp, nn, S, bn))
       return cudaErrorInvalidValue;
+    if (guard && !encode_slices(&maps.bmag, sl.Bmag, Kp, nn, 1, tc_mag_cols(bn))) return cudaErrorInvalidValue;
     // the widths of the default targets are compiled in: 5, 6, 7 (40 bits, by K), 7 in two words (56 bits)
     const int which = wide ? (bits == 7 ? 4 : 5) : bits == 5 ? 0 : bits == 6 ? 1 : bits == 7 ? 2 : 3;
-    const cudaError_t e = bn == 32 ? launch_tc<32>(which, grid, S, st, maps, a, err)
+    const cudaError_t e = full      ? (guard ? launch_tc_full<true>(bn, grid, st, maps, a, err)
+                                             : launch_tc_full<false>(bn, grid, st, maps, a, err))
+                        : bn == 32 ? launch_tc<32>(which, grid, S, st, maps, a, err)
                         : bn == 16 ? launch_tc<16>(which, grid, S, st, maps, a, err)
                                    : launch_tc<8>(which, grid, S, st, maps, a, err);
     if (e != cudaSuccess) return e;
@@ -865,7 +1030,9 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
   if (a.acc) {
     const size_t total = (size_t)m * nn;
     const int blocks = (int)((total + 255) / 256 < 4096 ? (total + 255) / 256 : 4096);
-    if (wide) k_oz_finalize<true><<<blocks, 256, 0, st>>>(a);
+    if (guard) k_oz_finalize<true, true, true><<<blocks, 256, 0, st>>>(a);
+    else if (full) k_oz_finalize<true, true><<<blocks, 256, 0, st>>>(a);
+    else if (wide) k_oz_finalize<true><<<blocks, 256, 0, st>>>(a);
     else k_oz_finalize<false><<<blocks, 256, 0, st>>>(a);
   }
   return cudaGetLastError();

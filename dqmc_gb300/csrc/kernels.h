@@ -62,9 +62,10 @@ struct SitePrep {
 cudaError_t launch_local_prepare(const LocalUpdateArgs& a, SitePrep* prep, int* state, int* wflag, cudaStream_t st);
 // BF16 slices of the operands of an m x n x K split-BF16 product in its
 // scratch block: As S x (m x Kp), Bre / Bim S x (n x Kp) (K contiguous, Kp =
-// 2 Kpad), row scales sA (m), column scales sB (n)
+// 2 Kpad), row scales sA (m), column scales sB (n).  Guarded products: magnitudes of
+// A as slice S of As, of B in Bmag (n x Kp); else Bmag is null.
 struct OzSlices {
-  __nv_bfloat16 *As, *Bre, *Bim;
+  __nv_bfloat16 *As, *Bre, *Bim, *Bmag;
   double *sA, *sB;
   int m, n, Kpad, S, bits;
 };
@@ -81,7 +82,7 @@ struct DelayedArgs {
   cplx* wrow;              // (WIN_MAX, 4, 4 WIN_MAX) their rows of the window's block (k_local_window)
   int* wflag;              // (WIN_MAX + 1) acceptances published to the follower clusters
   int* arrive;             // (2) followers that have read the state, clusters started (zero between launches)
-  OzSlices sl;             // the flush's slices, cut by launch_local_factors
+  OzSlices sl;             // the flush's slices, cut where the factors are formed
                            // (sl.As null: X and Y are stored and the flush slices them itself)
 };
 // Decides the next window of the slice on one cluster of 16 CTAs, 8 when other
@@ -214,16 +215,17 @@ cudaError_t measure_peak_fp64(int device, double* tflops);
 
 // ---- split-precision complex GEMM (k_ozaki.cu) ----
 bool ozaki_plan(int K, int target_bits, int* S, int* bits);
-constexpr int OZ_FP64_S = 8, OZ_FP64_BITS = 7;   // slices of the FP64 form's products: 56 mantissa bits at any K
+constexpr int OZ_FP64_S = 9, OZ_FP64_BITS = 7;   // slices of the FP64 form's products: 63 bits at any K
 size_t ozaki_scratch_bytes(int m, int n, int K, int S);
 // where launch_ozaki_zgemm keeps the slices of an m x n x K product in scratch
-OzSlices ozaki_slices(void* scratch, int m, int n, int K, int S, int bits);
+OzSlices ozaki_slices(void* scratch, int m, int n, int K, int S, int bits, bool guard = false);
 cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                                const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rowscale,
                                const double* colscale, int S, int bits, void* scratch, size_t scratch_bytes,
                                unsigned long long* acc, size_t acc_bytes, cudaStream_t st,
                                const int* active = nullptr, int splitk = 1, int* kernels = nullptr,
-                               int* err = nullptr, bool persistent = true, bool presliced = false);
+                               int* err = nullptr, bool persistent = true, bool presliced = false,
+                               bool guard = false);
 
 // ---- adjoint force (k_force.cu) ----
 // grad[:, :, slice0] = d log|det M| / d phi[:, :, slice0] from G of that slice

@@ -29,7 +29,8 @@ __device__ __forceinline__ long long fixed62(double x, int E) {
 
 // Cuts the next signed digit off a 62-bit fixed-point integer: X / 2^s rounded
 // half to even, X <- X - digit 2^s (so |digit| <= 2^bits for the first and
-// 2^(bits - 1) for the later ones).  s < 0 only for the last of 8 slices of 8 bits.
+// 2^(bits - 1) for the later ones).  s < 0 only for the last of 8 slices of 8 bits
+// and of 9 of 7.
 __device__ __forceinline__ int oz_next_digit(long long& X, int s) {
   if (s <= 0) {
     const long long d = X * (1ll << -s);
@@ -56,9 +57,19 @@ __device__ __forceinline__ uint32_t oz_pack2(int a, int b) {   // two digits as 
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// |x| 2^-E (< 1) as BF16, truncated; 0 only for x = 0 (below 2^-60: 2^-60).
+__device__ __forceinline__ uint32_t oz_mag(double x, int E) {
+  const long long b = __double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll;
+  if (b == 0) return 0u;
+  const int f = (int)(b >> 52) - 1023 - E + 127;
+  return f < 67 ? 67u << 7 : (uint32_t)f << 7 | ((uint32_t)(b >> 45) & 0x7Fu);
+}
+
 // Digits of the entries k, k + 1 (k even) of vector vec of one side of a
 // product into o: side 0 a row of op(A) (As: Re digits in k, Im digits in
 // Kpad + k), side 1 a column of op(B) (B'_re = [Re; -Im], B'_im = [Im; Re]).
+// With Bmag the magnitudes as well (side 0 |Re|, |Im| as slice S of As; side 1
+// the larger of the two in both halves).
 __device__ __forceinline__ void oz_store_pair(const OzSlices& o, int side, int vec, int k, cplx x0, cplx x1, int E) {
   const size_t Kp = 2 * (size_t)o.Kpad;
   long long r0 = fixed62(x0.x, E), i0 = fixed62(x0.y, E), r1 = fixed62(x1.x, E), i1 = fixed62(x1.y, E);
@@ -78,6 +89,13 @@ __device__ __forceinline__ void oz_store_pair(const OzSlices& o, int side, int v
       *reinterpret_cast<uint32_t*>(o.Bim + base + k) = im;
       *reinterpret_cast<uint32_t*>(o.Bim + base + o.Kpad + k) = re;
     }
+  }
+  if (o.Bmag) {
+    const uint32_t re = oz_mag(x0.x, E) | oz_mag(x1.x, E) << 16, im = oz_mag(x0.y, E) | oz_mag(x1.y, E) << 16;
+    __nv_bfloat16* v = side == 0 ? o.As + (size_t)o.S * o.m * Kp + (size_t)vec * Kp : o.Bmag + (size_t)vec * Kp;
+    const uint32_t mx = __vmaxu2(re, im);   // BF16 of non-negative values order like integers
+    *reinterpret_cast<uint32_t*>(v + k) = side == 0 ? re : mx;
+    *reinterpret_cast<uint32_t*>(v + o.Kpad + k) = side == 0 ? im : mx;
   }
 }
 

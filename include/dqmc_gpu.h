@@ -321,8 +321,9 @@ DQMC_API int dqmc_measure_zfccc(dqmc_handle* h, const double* greens, const doub
 DQMC_API int dqmc_get_timing(dqmc_handle* h, dqmc_timing* t);
 DQMC_API int dqmc_reset_timing(dqmc_handle* h, int32_t enable);
 /* Diagnostic: C = A * B for n x n complex matrices (column-major, interleaved)
- * with the handle's FP64 GEMM kernel (mode 0) or its split-BF16 tensor-core
- * GEMM (mode 1).  No counterpart in the reference. */
+ * with the handle's FP64 GEMM kernel (mode 0) or the split-BF16 tensor-core
+ * GEMM of its own products (mode 1: ozaki_bits per operand in the mixed form,
+ * FP64 accuracy per element in the FP64 form).  No counterpart in the reference. */
 DQMC_API int dqmc_gemm_check(dqmc_handle* h, int32_t mode, const double* A, const double* B, double* C);
 /* Measures the FP64 FMA throughput of `device` (TFLOP/s, 2 flops per FMA) with
  * a register-resident DFMA kernel: the roofline denominator of the FP64
