@@ -148,7 +148,7 @@ class ModelParams:
     device: int = -1
     precision: str = "fp64"        # "fp64" or "mixed"
     ozaki_bits: int = 0            # mantissa bits per GEMM operand in the mixed form (0 = default 40)
-    delay: int = 0                 # delayed-update depth (0/1 = immediate rank-4)
+    delay: int = 0                 # delayed-update depth (0/1: FP64 rank-4 updates, 16 sites at a time)
     greens_method: str = "scales"  # calculate_greens: "scales" (D-scale separation + LU) or "two_qr" (reference)
     inflight: int = 0              # batches: chains swept at the same time (0 = min(count, 8))
 

@@ -69,7 +69,10 @@ struct dqmc_handle {
   double* action_d = nullptr;
   int* nacc_d = nullptr;
   // delayed updates: pending factors and {next site, pending count}
-  int delay = 1;
+  int delay = 16;             // most acceptances of a round
+  // the flush has the FP64 form's slices: FP64 form, and mixed form at depths 0 and 1
+  // (whose updates are FP64 ones) or where ozaki_bits cannot be had at its inner dimension
+  bool flush_full = true;
   cplx* Xd = nullptr;
   cplx* Yd = nullptr;
   int* dstate = nullptr;
@@ -335,9 +338,10 @@ double ozaki_tensor_flops(double m, double nn, double k, int S) {
   const double kp = 2.0 * std::ceil(k / 16.0) * 16.0;
   return S * (S + 1) / 2.0 * 2.0 * 2.0 * m * nn * kp;
 }
-// slices of a product of this handle: by K and the target in the mixed form
-bool oz_plan(const dqmc_handle* h, int k, int* S, int* bits) {
-  if (h->p.precision == DQMC_PREC_MIXED) return ozaki_plan(k, h->oz_target, S, bits);
+// slices of a product of this handle: by K and the target in the mixed form (full:
+// those of the FP64 form in either)
+bool oz_plan(const dqmc_handle* h, int k, int* S, int* bits, bool full = false) {
+  if (h->p.precision == DQMC_PREC_MIXED && !full) return ozaki_plan(k, h->oz_target, S, bits);
   *S = OZ_FP64_S;
   *bits = OZ_FP64_BITS;
   return true;
@@ -345,10 +349,10 @@ bool oz_plan(const dqmc_handle* h, int k, int* S, int* bits) {
 int zgemm_general(dqmc_handle* h, int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                   const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rs, const double* cs,
                   bool allow_split, int kind = -1, const int* active = nullptr, bool presliced = false,
-                  bool guard = false) {
+                  bool guard = false, bool full = false) {
   if (allow_split) {
     int S = 0, bits = 0;
-    if (!oz_plan(h, k, &S, &bits)) return set_err(h, DQMC_ERR_ARG, "no exact slicing for this K");
+    if (!oz_plan(h, k, &S, &bits, full)) return set_err(h, DQMC_ERR_ARG, "no exact slicing for this K");
     // few output tiles and a long K: split K over more CTAs (exact integer partial sums)
     const int tiles = ((m + 63) / 64) * ((nn + 63) / 64);
     int splitk = 1;
@@ -888,8 +892,9 @@ int capture_round_loop(dqmc_handle* h, int max_rounds, Round&& round) {
 // cluster, factors of its acceptances, flush G += X Y (split-BF16 GEMM)]; the
 // number of rounds is bounded and rounds with nothing left return at once on
 // a device-side flag, so the host never waits.  A depth of 0 or 1 takes the
-// same path with windows of 16 (the update is the same rank-4 update per
-// acceptance; n = 1024: 8.7 ms per slice with one pass over G per acceptance).
+// same path with windows of 16 and, in the mixed form too, a flush with the FP64
+// form's slices (the update is the same rank-4 update per acceptance in 64 bits;
+// n = 1024: 8.7 ms per slice with one pass over G per acceptance).
 // side: the preparation (fields, proposals; not G) only waits for side_fork
 int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* unif_dev, uint8_t* acc_dev,
                       cplx* det_dev, double* pacc_dev, bool side = false) {
@@ -913,7 +918,7 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
   DelayedArgs d{h->Xd, h->Yd, h->dstate, k, h->prep, h->wsite, h->wk, h->wexp, h->wrow, h->wflag, h->wflag + WIN_MAX + 1, {}};
   // the factor kernel cuts the flush's slices
   int S = 0, bits = 0;
-  const bool presliced = oz_plan(h, 4 * k, &S, &bits) && ozaki_scratch_bytes(n, n, 4 * k, S) <= h->oz_bytes;
+  const bool presliced = oz_plan(h, 4 * k, &S, &bits, h->flush_full) && ozaki_scratch_bytes(n, n, 4 * k, S) <= h->oz_bytes;
   if (presliced) d.sl = ozaki_slices(h->oz_scratch, n, n, 4 * k, S, bits);
   if (side) CU(cudaStreamWaitEvent(h->st_side, h->side_fork, 0));
   LAUNCH(DQMC_K_LOCAL, 0.0, 0.0,
@@ -932,7 +937,7 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
     if (!follow) LAUNCH(DQMC_K_FLUSH, 0.0, 0.0, launch_local_factors(a, d, h->st));
     // flush G += X Y over the 4p new columns (p read on the device; no work when p = 0)
     return zgemm_general(h, n, n, 4 * k, 'N', 'T', cmake(1, 0), h->Xd, n, h->Yd, n, cmake(1, 0), h->G, n, nullptr,
-                         nullptr, true, DQMC_K_FLUSH, h->dstate + 1, presliced);
+                         nullptr, true, DQMC_K_FLUSH, h->dstate + 1, presliced, false, h->flush_full);
   };
   // the WHILE node only for a chain that has the GPU to itself: with chains
   // in flight together (coop_cap > 0) it cost a batch of 64 chains 28% of its
@@ -1367,8 +1372,9 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
     int S = 0, bits = 0;
     if (!oz_plan(h, (int)n, &S, &bits)) return fail(DQMC_ERR_ARG);
     h->oz_bytes = ozaki_scratch_bytes((int)n, (int)n, (int)n, S);
-    if (oz_plan(h, 4 * h->delay, &S, &bits))
-      h->oz_bytes = std::max(h->oz_bytes, ozaki_scratch_bytes((int)n, (int)n, 4 * h->delay, S));
+    h->flush_full = p->delay <= 1 || !oz_plan(h, 4 * h->delay, &S, &bits);
+    if (!oz_plan(h, 4 * h->delay, &S, &bits, h->flush_full)) return fail(DQMC_ERR_ARG);
+    h->oz_bytes = std::max(h->oz_bytes, ozaki_scratch_bytes((int)n, (int)n, 4 * h->delay, S));
     A(&h->oz_scratch, h->oz_bytes);
     // split K is taken for fewer than sm_count / 2 output tiles of 64 x 64; two words per real sum above 42
     // bits, and one for the magnitudes
