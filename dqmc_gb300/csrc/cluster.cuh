@@ -2,7 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
-constexpr int kClusterPolls = 1 << 22;   // bound of every wait on another CTA (about 0.1 s)
+constexpr int kClusterPolls = 1 << 22;   // bound of every wait on another CTA: about 0.1 s in shared memory, 3 s in global memory
 
 __device__ __forceinline__ void st_cluster(void* p, unsigned long long v) {   // p: generic address of cluster shared memory
   asm volatile("st.relaxed.cluster.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");

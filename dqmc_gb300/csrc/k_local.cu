@@ -345,7 +345,9 @@ __global__ void __launch_bounds__(128) k_local_prepare(LocalUpdateArgs a, SitePr
   const int i = blockIdx.x * 4 + (threadIdx.x >> 5);
   // delayed rounds of this slice start from site 0 with nothing pending
   if (blockIdx.x == 0 && threadIdx.x == 0) { state[0] = 0; state[1] = 0; state[2] = 0; }
-  if (blockIdx.x == 0 && threadIdx.x <= WIN_MAX) wflag[threadIdx.x] = 0;   // flags carry the window's first site
+  // flags carry the window's first site; the last two are the arrivals, which a
+  // window that timed out leaves behind (no window is in flight here)
+  if (blockIdx.x == 0 && threadIdx.x < WIN_MAX + 3) wflag[threadIdx.x] = 0;
   if (i >= N) return;
   const double* po = &a.phi[((size_t)N * l + i) * 3];
   const double old[3] = {po[0], po[1], po[2]};
@@ -780,7 +782,12 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
   int ticket = 0;
   if (followers > 0) {
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    if (rank == 0 && tid == 0) ticket = atomicAdd(d.arrive + 1, 1);
+    if (rank == 0 && tid == 0) {
+      ticket = atomicAdd(d.arrive + 1, 1);
+      // after a timeout the arrivals are those of the window that timed out, until
+      // the next preparation: nobody starts (decided once for the cluster)
+      if (__ldcg(a.err) & DQMC_KERR_BARRIER_TIMEOUT) ticket = -1;
+    }
   }
   const int we = min(W, N - first);                       // sites of this window
   const int owned = rank < we ? (we - rank + C - 1) / C : 0;   // sites rank + t C
@@ -817,6 +824,10 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
     if (rank == 0 && tid < C) *cl.map_shared_rank(&s_ticket, tid) = __shfl_sync((1u << C) - 1, ticket, 0);
   }
   cl.sync();   // also: every CTA of the cluster runs before its shared memory is written remotely
+  if (followers > 0 && s_ticket < 0) {
+    if (blockIdx.x == 0 && tid == 0) d.state[1] = 0;
+    return;
+  }
   if (followers > 0 && s_ticket > 0) {
     if (tid == 0) {   // the state has been read: the window may advance it
       __threadfence();
@@ -1099,15 +1110,25 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
   // ---- the round's state ----
   if (rank == 0 && wid == 0) {
     if (lane < p) d.wsite[lane] = s_acc[lane];
+    int late = __ldcg(a.err) & DQMC_KERR_BARRIER_TIMEOUT;   // of any CTA: before the barriers above
     if (lane == 0 && followers > 0) {
       // the followers have read the state (bounded wait)
       bool here = false;
       for (int it = 0; it < kClusterPolls && !here; ++it) here = *(volatile int*)d.arrive == followers;
-      if (!here) atomicOr(a.err, DQMC_KERR_BARRIER_TIMEOUT);
-      d.arrive[0] = 0;
-      d.arrive[1] = 0;
+      if (!here) {
+        atomicOr(a.err, DQMC_KERR_BARRIER_TIMEOUT);
+        late = 1;
+      }
+      if (!late) {
+        d.arrive[0] = 0;
+        d.arrive[1] = 0;
+      }
     }
-    __syncwarp();
+    late = __shfl_sync(0xffffffffu, late, 0);
+    if (late) {   // a follower may still arrive or read the state: both stay as they are, and the flush has nothing to do
+      if (lane == 0) d.state[1] = 0;
+      return;
+    }
     // the tracked action: -log(exp(-dS)) of the accepted sites, added in order
     const double lg = lane < p ? -log(__ldcg(&d.wexp[lane])) : 0.0;
     double act = lane == 0 ? *a.action : 0.0;
