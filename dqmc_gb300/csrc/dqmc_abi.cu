@@ -2298,16 +2298,15 @@ int dqmc_measure_equal_time(dqmc_handle* h, const double* greens, double* etpc_p
     for (int q = 0; q < 4; ++q)
       if (outs[q])
         CU(cudaMemcpyAsync(outs[q], h->etc_d + off[q], cnt[q] * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
-    CHK(sync(h));
-    return wait_scalars(h);
+    return sync(h);
   }
   // one copy for the four arrays: a copy to pageable memory costs 8 us whatever its size
   std::vector<double> host((size_t)6 * N);
   CU(cudaMemcpyAsync(host.data(), h->etc_d, host.size() * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-  CHK(wait_scalars(h));   // waits for the stream
+  const int rc = sync(h);   // the arrays are filled also where it finds an error
   for (int q = 0; q < 4; ++q)
     if (outs[q]) std::memcpy(outs[q], host.data() + off[q], cnt[q] * sizeof(double));
-  return DQMC_OK;
+  return rc;
 }
 
 int dqmc_measure(dqmc_handle* h, double* greens_out, double* occupation, double* e_kin) {
