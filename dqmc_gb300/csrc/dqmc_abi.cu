@@ -1464,10 +1464,11 @@ static int local_updates_host(dqmc_handle* h, const double* delta, const double*
   if (detratio) CU(cudaMemcpyAsync(det, h->det_d, N * sizeof(cplx), cudaMemcpyDeviceToHost, h->st));
   if (p_acc) CU(cudaMemcpyAsync(pac, h->pacc_d, N * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   if (accepted) CU(cudaMemcpyAsync(acc, h->acc_d, N, cudaMemcpyDeviceToHost, h->st));
-  CHK(sync(h));
+  const int rc = sync(h);   // the outputs show which ratio was not finite
   if (detratio) std::memcpy(detratio, det, N * sizeof(cplx));
   if (p_acc) std::memcpy(p_acc, pac, N * sizeof(double));
   if (accepted) std::memcpy(accepted, acc, N);
+  CHK(rc);
   if (acc_rate) {
     int before = 0, after = 0;
     std::memcpy(&before, h->pin + kPinCount, sizeof(int));

@@ -34,3 +34,25 @@ def test_equal_time_correlators_report_it(where):
                                            1 if where == "device" else 0)
     assert rc == code
     chain.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("call", ["dqmc_local_updates", "dqmc_update"])
+def test_local_updates_return_the_ratios_beside_the_error(call):
+    """A ratio that is not finite is an error; the per-site outputs say where it is."""
+    from dqmc_gb300 import api
+    chain = api.DQMC(api.ModelParams(L=4, slices=20, safe_mult=20), np.random.default_rng(1).uniform(-1, 1, (3, 16, 20)))
+    chain.init()
+    G = np.array(chain.greens)
+    G[9, 9] = np.nan
+    chain.greens = G
+    delta, unif = np.zeros((3, 16), order="F"), np.full(16, 2.0)   # no acceptance: the NaN stays at its site
+    acc, det, pac = np.full(16, 7, np.uint8), np.full(16, 7.0 + 0j), np.full(16, 7.0)
+    D = lambda a: a.ctypes.data_as(api._D)
+    rate = ctypes.c_double(-1.0)
+    rc = getattr(chain.lib, call)(chain.h, D(delta), D(unif), acc.ctypes.data_as(ctypes.c_void_p), D(det), D(pac),
+                                  ctypes.byref(rate))
+    assert rc != 0
+    assert not (acc == 7).any() and not (det == 7.0).any() and not (pac == 7.0).any()
+    assert np.isnan(det[9]) and (call == "dqmc_update" or np.isfinite(np.delete(det, 9)).all())
+    chain.close()
