@@ -193,14 +193,15 @@ __global__ void __launch_bounds__(LU_THREADS) k_lu_panel(cplx* __restrict__ A, c
     const int ps = pkw >> 16, o = pkw & 0xFFFF;
     if (wid == 0) {
       const cplx pv = pvw;
-      const bool zero = pv.x == 0.0 && pv.y == 0.0;
+      bool zero = pv.x == 0.0 && pv.y == 0.0;
       cplx ri;
       if (UNBLOCKED) {
         ri = zero ? cmake(0.0, 0.0) : cdiv(cmake(1.0, 0.0), pv);
       } else {
         // 1 / pivot = conj(pv) / |pv|^2 (the D-scale separated matrix has no large scales)
         const double d2 = pv.x * pv.x + pv.y * pv.y;
-        const double rd = d2 == 0.0 ? 0.0 : 1.0 / d2;
+        zero = d2 == 0.0;   // also a pivot below 1e-162, which has no reciprocal here
+        const double rd = zero ? 0.0 : 1.0 / d2;
         ri = cmake(pv.x * rd, -pv.y * rd);
       }
       if (lane == 0) {
