@@ -509,10 +509,12 @@ __device__ __forceinline__ double win_adj(const cplx* m, const cplx* mn, int lan
 constexpr unsigned long long kWinEmpty = 0x7FF8DEADBEEF0001ull;
 // 1 / x by Newton's iteration from a single-precision seed (2^-23, 2^-46,
 // then FP64 round-off): four dependent FMAs where the division takes twice
-// that; outside the single-precision range the division.
-__device__ __forceinline__ double recip_newton(double x) {
+// that; within the single-precision range (recip_range).
+__device__ __forceinline__ bool recip_range(double x) {
   const int e = (__double2hiint(x) >> 20) & 0x7FF;
-  if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / x;
+  return e >= 1023 - 100 && e <= 1023 + 100;
+}
+__device__ __forceinline__ double recip_newton(double x) {
   double y = (double)__frcp_rn((float)x);
   y = fma(fma(-x, y, 1.0), y, y);
   return fma(fma(-x, y, 1.0), y, y);
@@ -921,8 +923,13 @@ __global__ void __launch_bounds__(WIN_THREADS) k_local_window(LocalUpdateArgs a,
       named_bar(4, 64);
       if (lane == 0) {
         const double dx = s_det[0], dy = s_det[1];
-        const double rd = recip_newton(fma(dx, dx, dy * dy));
-        s_inv = cmake(dx * rd, flip_sign(dy * rd, true));
+        const double d2 = fma(dx, dx, dy * dy);
+        if (recip_range(d2)) {
+          const double rd = recip_newton(d2);
+          s_inv = cmake(dx * rd, flip_sign(dy * rd, true));
+        } else {   // also where the square leaves the range of double
+          s_inv = cdiv(cmake(1.0, 0.0), cmake(dx, dy));
+        }
       }
       __syncwarp();
       named_arrive(5, 64);
