@@ -410,34 +410,26 @@ int permute(dqmc_handle* h, const cplx* src, cplx* dst, const int* order, bool b
 // I - V_j T_j V_j^H, T_j^-1 = diag(1/tau) + striu(V_j^H V_j)), the products as
 // split-BF16 GEMMs.  Before step j, W differs from I only in rows and columns
 // >= (j+1) b, so every product acts on W[jb:, jb:].
-// FP64 form: the unit diagonals of V_j stay out of the products (k_wy_prep), and
-// the blocks are smaller, since U's error grows with them.  |U - U_exact| at
-// n = 64 / 144 in units of 1e-16: reflectors one by one 3.3 / 4.8; units in the
-// products, blocks of 128 6.9 / 12.5; units apart, blocks of 128 4.6 / 5.9, 64
-// 4.6 / 4.5, 32 3.7 / 3.8.
+// The FP64 form's 63 bits leave no error of the products in U, whatever the block:
+// |U - U_exact| / sqrt(n) of matrices of normal entries in units of 1e-16,
+// reflectors one by one / blocks of 64 / of 128: n = 64 11.0 / 10.9 / 10.9, 144
+// 17.6 / 17.0 / 17.3, 400 32.6 / 31.6 / 32.0, 784 (graded) 48.1 / 46.6 / 46.9.
 constexpr int kWyMax = 128;   // largest compact-WY block (buffer sizes; k_trsm_diag_block limit)
 int form_q_wy(dqmc_handle* h, cplx* W) {
-  const int n = h->n;
-  const bool units = h->p.precision != DQMC_PREC_MIXED;   // kept apart
-  const int b = units ? std::min(h->wy_block, n < 144 ? 32 : 64) : h->wy_block;
-  const cplx beta = cmake(units ? 1.0 : 0.0, 0.0);
+  const int n = h->n, b = h->wy_block;
   CHK(set_identity(h, W));
   for (int jb = ((n - 1) / b) * b; jb >= 0; jb -= b) {
     const int m = n - jb, bs = m < b ? m : b;
-    LAUNCH(DQMC_K_APPLYQ, 0.0, 32.0 * m * bs, launch_wy_prep(h->qr.V, h->qr.tau, n, jb, bs, h->wy_v, h->wy_t, units ? h->wy_s : nullptr,
-                          units ? h->wy_z : nullptr, h->st));
+    LAUNCH(DQMC_K_APPLYQ, 0.0, 32.0 * m * bs, launch_wy_prep(h->qr.V, h->qr.tau, n, jb, bs, h->wy_v, h->wy_t, h->st));
     // S = Vb^H Vb, Z = Vb^H W[jb:, jb:]
-    CHK(zgemm_general(h, bs, bs, m, 'C', 'N', cmake(1, 0), h->wy_v, m, h->wy_v, m, beta, h->wy_s, bs, nullptr,
+    CHK(zgemm_general(h, bs, bs, m, 'C', 'N', cmake(1, 0), h->wy_v, m, h->wy_v, m, cmake(0, 0), h->wy_s, bs, nullptr,
                       nullptr, true, DQMC_K_APPLYQ));
-    CHK(zgemm_general(h, bs, m, m, 'C', 'N', cmake(1, 0), h->wy_v, m, W + (size_t)jb * n + jb, n, beta,
+    CHK(zgemm_general(h, bs, m, m, 'C', 'N', cmake(1, 0), h->wy_v, m, W + (size_t)jb * n + jb, n, cmake(0, 0),
                       h->wy_z, bs, nullptr, nullptr, true, DQMC_K_APPLYQ));
     // Z <- T Z: solve T^-1 Y = Z (upper: strict part S, diagonal 1/tau)
     LAUNCH(DQMC_K_APPLYQ, 4.0 * bs * bs * m, 32.0 * bs * m,
            launch_trsm_diag_block(h->wy_s, bs, h->wy_t, h->wy_z, bs, 0, bs, m, false, h->st));
     // W[jb:, jb:] -= Vb Z
-    if (units)
-      LAUNCH(DQMC_K_APPLYQ, 0.0, 48.0 * bs * m,
-             launch_wy_units(W + (size_t)jb * n + jb, n, h->wy_z, bs, m, h->st));
     CHK(zgemm_general(h, m, m, bs, 'N', 'N', cmake(-1, 0), h->wy_v, m, h->wy_z, bs, cmake(1, 0),
                       W + (size_t)jb * n + jb, n, nullptr, nullptr, true, DQMC_K_APPLYQ));
   }

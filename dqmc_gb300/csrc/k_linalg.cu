@@ -510,41 +510,16 @@ __global__ void __launch_bounds__(QR_THREADS, 1) k_qrp(cplx* __restrict__ A, int
 // leading dimension m) = rows jb.. of reflector columns jb..jb+b; a reflector
 // with tau = 0 is the identity and is stored as v = 0 with tau' = 1, so that
 // T^-1 = diag(1/tau') + striu(Vb^H Vb) stays valid.  trd = tau'.
-// With Z (b x m): Vb = E + V', E the unit diagonals, and V' is written to Vb.
-// S (b x b) and Z then hold what the products V'^H V' and V'^H W are added to:
-// striu(V'^H E + E^H V') = striu of the adjoint of V''s top rows, and E^H W (W is
-// the identity in these rows).  The units are the largest entries of their
-// columns by about sqrt(n), and the split products' error goes by the largest
-// entry: without them it is that of the reflectors applied one by one.
 __global__ void k_wy_prep(const cplx* __restrict__ V, const cplx* __restrict__ tau, int n, int jb, int b,
-                          cplx* __restrict__ Vb, cplx* __restrict__ trd, cplx* __restrict__ S, cplx* __restrict__ Z) {
+                          cplx* __restrict__ Vb, cplx* __restrict__ trd) {
   const int m = n - jb;
   const size_t total = (size_t)m * b;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
     const int c = (int)(e / m), r = (int)(e - (size_t)c * m);
     const cplx t = tau[jb + c];
     const bool ident = t.x == 0.0 && t.y == 0.0;
-    const cplx v = ident ? cmake(0.0, 0.0) : V[(size_t)(jb + c) * n + jb + r];
-    Vb[e] = Z && r == c ? cmake(0.0, 0.0) : v;
-    if (Z) {
-      Z[(size_t)r * b + c] = cmake(r == c && !ident ? 1.0 : 0.0, 0.0);
-      if (r < b) {   // S[c, r] takes column c's entry under reflector r's unit
-        const cplx tr = tau[jb + r];
-        const bool none = r <= c || (tr.x == 0.0 && tr.y == 0.0);
-        S[(size_t)r * b + c] = none ? cmake(0.0, 0.0) : cmake(v.x, -v.y);
-      }
-    }
+    Vb[e] = ident ? cmake(0.0, 0.0) : V[(size_t)(jb + c) * n + jb + r];
     if (r == 0) trd[c] = ident ? cmake(1.0, 0.0) : t;
-  }
-}
-
-// W[0:b, 0:m] -= Z (b x m): the unit diagonals' part of W -= Vb Z
-__global__ void k_wy_units(cplx* __restrict__ W, int ldw, const cplx* __restrict__ Z, int b, int m) {
-  const size_t total = (size_t)m * b;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const int c = (int)(e / b), r = (int)(e - (size_t)c * b);
-    cplx* w = &W[(size_t)c * ldw + r];
-    *w = csub(*w, Z[e]);
   }
 }
 
@@ -1521,14 +1496,9 @@ cudaError_t launch_trsm_diag_block(const cplx* T, int ldT, const cplx* rdiag, cp
   return cudaGetLastError();
 }
 
-cudaError_t launch_wy_prep(const cplx* V, const cplx* tau, int n, int jb, int b, cplx* Vb, cplx* trd, cplx* S,
-                           cplx* Z, cudaStream_t st) {
-  k_wy_prep<<<grid_for((size_t)(n - jb) * b), 256, 0, st>>>(V, tau, n, jb, b, Vb, trd, S, Z);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_wy_units(cplx* W, int ldw, const cplx* Z, int b, int m, cudaStream_t st) {
-  k_wy_units<<<grid_for((size_t)m * b), 256, 0, st>>>(W, ldw, Z, b, m);
+cudaError_t launch_wy_prep(const cplx* V, const cplx* tau, int n, int jb, int b, cplx* Vb, cplx* trd,
+                           cudaStream_t st) {
+  k_wy_prep<<<grid_for((size_t)(n - jb) * b), 256, 0, st>>>(V, tau, n, jb, b, Vb, trd);
   return cudaGetLastError();
 }
 

@@ -158,10 +158,8 @@ struct LUWork {
   cplx* rdiag;       // (n) 1 / diagonal of U
 };
 // compact-WY block jb..jb+b of the reflectors in V/tau: Vb ((n-jb) x b), trd (b) (tau, 1 for identity reflectors)
-// (Z null: S and Z are left alone, Vb keeps its unit diagonals)
-cudaError_t launch_wy_prep(const cplx* V, const cplx* tau, int n, int jb, int b, cplx* Vb, cplx* trd, cplx* S,
-                           cplx* Z, cudaStream_t st);
-cudaError_t launch_wy_units(cplx* W, int ldw, const cplx* Z, int b, int m, cudaStream_t st);
+cudaError_t launch_wy_prep(const cplx* V, const cplx* tau, int n, int jb, int b, cplx* Vb, cplx* trd,
+                           cudaStream_t st);
 // LU panels of LU_PB columns on one cluster (k_lu.cu)
 constexpr int LU_PB = 64;
 struct LUPanel {
