@@ -68,13 +68,11 @@ struct dqmc_handle {
   int out_cap = 0;
   double* action_d = nullptr;
   int* nacc_d = nullptr;
-  // delayed updates: pending factors and {next site, pending count}
+  // delayed updates: {next site, pending count}
   int delay = 16;             // most acceptances of a round
   // the flush has the FP64 form's slices: FP64 form, and mixed form at depths 0 and 1
   // (whose updates are FP64 ones) or where ozaki_bits cannot be had at its inner dimension
   bool flush_full = true;
-  cplx* Xd = nullptr;
-  cplx* Yd = nullptr;
   int* dstate = nullptr;
   SitePrep* prep = nullptr;   // (N) per-site constants of the slice being updated
   int* wsite = nullptr;       // (WIN_MAX) accepted sites of the window
@@ -369,7 +367,7 @@ int zgemm_general(dqmc_handle* h, int m, int nn, int k, char opA, char opB, cplx
     return DQMC_OK;
   }
   LAUNCH(kind >= 0 ? kind : DQMC_K_GEMM, gemm_flops(m, nn, k), gemm_bytes(m, nn, k),
-         launch_zgemm(m, nn, k, opA, opB, alpha, A, lda, B, ldb, beta, C, ldc, rs, cs, h->st, active));
+         launch_zgemm(m, nn, k, opA, opB, alpha, A, lda, B, ldb, beta, C, ldc, rs, cs, h->st));
   return DQMC_OK;
 }
 // n x n x n product of the stabilisation (split-BF16 in the mixed form)
@@ -393,7 +391,7 @@ int apply_q(dqmc_handle* h, cplx* X) {
   return DQMC_OK;
 }
 int trsm_left(dqmc_handle* h, const cplx* T, const int* order, cplx* Y) {
-  LAUNCH(DQMC_K_TRSM, 4.0 * n3(h), 40.0 * n2(h), launch_trsm_left_upper(T, order, nullptr, Y, h->n, h->n, h->st));
+  LAUNCH(DQMC_K_TRSM, 4.0 * n3(h), 40.0 * n2(h), launch_trsm_left_upper(T, order, Y, h->n, h->n, h->st));
   return DQMC_OK;
 }
 int trsm_right(dqmc_handle* h, const cplx* T, const int* order, cplx* Y) {
@@ -907,11 +905,11 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
   a.err = h->err_d;
   a.mc = h->mc;
   const int n = h->n, k = h->delay;
-  DelayedArgs d{h->Xd, h->Yd, h->dstate, k, h->prep, h->wsite, h->wk, h->wexp, h->wrow, h->wflag, h->wflag + WIN_MAX + 1, {}};
-  // the factor kernel cuts the flush's slices
+  DelayedArgs d{h->dstate, k, h->prep, h->wsite, h->wk, h->wexp, h->wrow, h->wflag, h->wflag + WIN_MAX + 1, {}};
+  // the flush's slices are cut where the factors are formed (dqmc_create has room for them)
   int S = 0, bits = 0;
-  const bool presliced = oz_plan(h, 4 * k, &S, &bits, h->flush_full) && ozaki_scratch_bytes(n, n, 4 * k, S) <= h->oz_bytes;
-  if (presliced) d.sl = ozaki_slices(h->oz_scratch, n, n, 4 * k, S, bits);
+  if (!oz_plan(h, 4 * k, &S, &bits, h->flush_full)) return set_err(h, DQMC_ERR_ARG, "no exact slicing for this K");
+  d.sl = ozaki_slices(h->oz_scratch, n, n, 4 * k, S, bits);
   if (side) CU(cudaStreamWaitEvent(h->st_side, h->side_fork, 0));
   LAUNCH(DQMC_K_LOCAL, 0.0, 0.0,
          launch_local_prepare(a, h->prep, h->dstate, h->wflag, side ? h->st_side : h->st));
@@ -928,8 +926,8 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
     LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_window(a, d, h->st, h->coop_cap > 0, follow));
     if (!follow) LAUNCH(DQMC_K_FLUSH, 0.0, 0.0, launch_local_factors(a, d, h->st));
     // flush G += X Y over the 4p new columns (p read on the device; no work when p = 0)
-    return zgemm_general(h, n, n, 4 * k, 'N', 'T', cmake(1, 0), h->Xd, n, h->Yd, n, cmake(1, 0), h->G, n, nullptr,
-                         nullptr, true, DQMC_K_FLUSH, h->dstate + 1, presliced, false, h->flush_full);
+    return zgemm_general(h, n, n, 4 * k, 'N', 'T', cmake(1, 0), nullptr, n, nullptr, n, cmake(1, 0), h->G, n, nullptr,
+                         nullptr, true, DQMC_K_FLUSH, h->dstate + 1, true, false, h->flush_full);
   };
   // the WHILE node only for a chain that has the GPU to itself: with chains
   // in flight together (coop_cap > 0) it cost a batch of 64 chains 28% of its
@@ -951,7 +949,7 @@ void free_all(dqmc_handle* h) {
                   h->Tr, h->Dl, h->Dr, h->W1, h->W2, h->W3, h->W4, h->D1, h->d2, h->ord1, h->qr.vn1,
                   h->qr.vn2, h->qr.order, h->qr.tau, h->qr.beta, h->qr.V, h->qr.bar, h->qr.cand_v, h->qr.cand_q, h->qr.refl, h->qr.slots, h->qr.cols, h->qr.run, h->delta_d, h->unif_d,
                   h->acc_d, h->det_d, h->pacc_d, h->action_d,
-                  h->scal_d, h->oz_scratch, h->oz_acc, h->Xd, h->Yd, h->dstate, h->prep, h->wsite, h->wk, h->wrow, h->wflag, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
+                  h->scal_d, h->oz_scratch, h->oz_acc, h->dstate, h->prep, h->wsite, h->wk, h->wrow, h->wflag, h->wexp, h->lu.perm, h->lu.udiag, h->lu.rdiag, h->lup.piv, h->lup.src, h->lu_L, h->lu_scales, h->wy_v, h->wy_s, h->wy_z, h->wy_t, h->force_d, h->etc_d, h->tdgf_ws, h->tdgf_a, h->tdgf_b, h->gb_u, h->gb_t, h->gb_G, h->gb_d, h->gb_phi, h->gb_evtab};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (h->pin) cudaFreeHost(h->pin);
@@ -1343,8 +1341,6 @@ int dqmc_create(const dqmc_params* p, dqmc_handle** out) {
   h->lup.err = h->err_d;
   h->delay = p->delay > 1 ? p->delay : 16;
   {
-    A((void**)&h->Xd, (size_t)4 * h->delay * n * sizeof(cplx));
-    A((void**)&h->Yd, (size_t)4 * h->delay * n * sizeof(cplx));
     A((void**)&h->dstate, 8 * sizeof(int));   // [0] next site, [1] pending, [2] rounds, [4..5] u64 rounds run
     A((void**)&h->prep, (size_t)h->N * sizeof(SitePrep));
     A((void**)&h->wsite, WIN_MAX * sizeof(int));

@@ -32,13 +32,7 @@ __device__ __forceinline__ cplx load_op(const cplx* X, int ld, int r, int c, int
 __global__ void __launch_bounds__(256) k_zgemm(int m, int nn, int k, char opA, char opB, cplx alpha,
                                               const cplx* __restrict__ A, int lda, const cplx* __restrict__ B,
                                               int ldb, cplx beta, cplx* __restrict__ C, int ldc,
-                                              const double* __restrict__ rs, const double* __restrict__ cs,
-                                              const int* __restrict__ active) {
-  if (active) {
-    const int kk = 4 * *active;
-    if (kk == 0) return;
-    if (kk < k) k = kk;
-  }
+                                              const double* __restrict__ rs, const double* __restrict__ cs) {
   __shared__ cplx sA[GB_K][GB_M + 1];
   __shared__ cplx sB[GB_K][GB_N + 1];
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
@@ -1096,8 +1090,7 @@ __global__ void __launch_bounds__(128) k_apply_q_right(cplx* __restrict__ X, int
 // Y <- That^-1 Y, That[r, q] = T[r, order[q]] upper triangular (logical order).
 // One warp per column of Y (column staged in shared memory).
 __global__ void __launch_bounds__(128) k_trsm_left_upper(const cplx* __restrict__ T, const int* __restrict__ order,
-                                                        const cplx* __restrict__ rdiag, cplx* __restrict__ Y, int n,
-                                                        int m) {
+                                                        cplx* __restrict__ Y, int n, int m) {
   extern __shared__ double smem_t[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int col = blockIdx.x * (blockDim.x / 32) + wid;
@@ -1107,15 +1100,10 @@ __global__ void __launch_bounds__(128) k_trsm_left_upper(const cplx* __restrict_
   for (int r = lane; r < n; r += 32) y[r] = yg[r];
   __syncwarp();
   for (int q = n - 1; q >= 0; --q) {
-    const cplx* tq = T + (size_t)(order ? __ldg(&order[q]) : q) * n;
-    cplx yq;
-    if (rdiag) {
-      yq = cmul(y[q], __ldg(&rdiag[q]));
-    } else {
-      // the unit-scaled factor of a QR has diagonal beta/|beta| = +-1: a sign, not a division
-      const cplx d = __ldg(&tq[q]);
-      yq = (d.y == 0.0 && fabs(d.x) == 1.0) ? cscale(y[q], d.x) : cdiv(y[q], d);
-    }
+    const cplx* tq = T + (size_t)__ldg(&order[q]) * n;
+    // the unit-scaled factor of a QR has diagonal beta/|beta| = +-1: a sign, not a division
+    const cplx d = __ldg(&tq[q]);
+    const cplx yq = (d.y == 0.0 && fabs(d.x) == 1.0) ? cscale(y[q], d.x) : cdiv(y[q], d);
     __syncwarp();
     if (lane == 0) y[q] = yq;
     for (int r = lane; r < q; r += 32) {
@@ -1387,10 +1375,9 @@ static inline int grid_for(size_t total, int threads = 256, int cap = 4096) {
 
 cudaError_t launch_zgemm(int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                          const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rowscale,
-                         const double* colscale, cudaStream_t st, const int* active) {
+                         const double* colscale, cudaStream_t st) {
   dim3 grid((nn + GB_N - 1) / GB_N, (m + GB_M - 1) / GB_M);
-  k_zgemm<<<grid, 256, 0, st>>>(m, nn, k, opA, opB, alpha, A, lda, B, ldb, beta, C, ldc, rowscale, colscale,
-                                active);
+  k_zgemm<<<grid, 256, 0, st>>>(m, nn, k, opA, opB, alpha, A, lda, B, ldb, beta, C, ldc, rowscale, colscale);
   return cudaGetLastError();
 }
 
@@ -1461,12 +1448,11 @@ cudaError_t launch_apply_q_right(cplx* X, int m, int n, const QRWork& w, bool co
   return cudaGetLastError();
 }
 
-cudaError_t launch_trsm_left_upper(const cplx* T, const int* order, const cplx* rdiag, cplx* Y, int n, int m,
-                                   cudaStream_t st) {
+cudaError_t launch_trsm_left_upper(const cplx* T, const int* order, cplx* Y, int n, int m, cudaStream_t st) {
   size_t smem = (size_t)4 * n * sizeof(cplx);
   static SmemLimit smem_limit;
   if (cudaError_t ea = smem_limit.raise((const void*)k_trsm_left_upper, 200 * 1024); ea != cudaSuccess) return ea;
-  k_trsm_left_upper<<<(m + 3) / 4, 128, smem, st>>>(T, order, rdiag, Y, n, m);
+  k_trsm_left_upper<<<(m + 3) / 4, 128, smem, st>>>(T, order, Y, n, m);
   return cudaGetLastError();
 }
 

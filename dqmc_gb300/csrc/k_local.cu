@@ -542,8 +542,7 @@ __device__ __forceinline__ void named_arrive(int id, int threads) {
 // (rows of the accepted sites from k_local_window): every row of X and every
 // column of Y is an independent recurrence of p steps, taken by 8 SPLIT lanes of a
 // warp: 4 components x {real, imaginary} x SPLIT shares of the sum over i.  At
-// the end each vector is cut into the BF16 slices of the flush (or stored in
-// FP64 when the product slices it itself).
+// the end each vector is cut into the BF16 slices of the flush.
 // Bound: FP64 issue, 8 (4p)^2 / 2 multiply-adds per vector.
 struct FacLane {
   int part, q, sp, v;   // this lane's component, share of the sum and vector of its warp
@@ -607,18 +606,12 @@ __device__ __forceinline__ cplx fac_entry(const LocalUpdateArgs& a, int side, in
 }
 // a warp's VPW finished vectors from v0 on
 template <int VPW>
-__device__ __forceinline__ void fac_finish(const LocalUpdateArgs& a, const DelayedArgs& d, int side, int v0, int p,
-                                           const cplx* xs, int ldx) {
-  const int lane = threadIdx.x & 31, n = a.mc.n;
+__device__ __forceinline__ void fac_finish(const DelayedArgs& d, int side, int v0, int p, const cplx* xs, int ldx) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int u = 0; u < VPW; ++u) {
     const cplx* xv = xs + u * ldx;
-    if (d.sl.As) {
-      oz_slice_vec(d.sl, side, v0 + u, 4 * p, [&](int k) { return xv[k]; }, lane);
-    } else {
-      cplx* out = side == 0 ? d.X : d.Y;
-      for (int jq = lane; jq < 4 * p; jq += 32) out[(size_t)jq * n + v0 + u] = xv[jq];
-    }
+    oz_slice_vec(d.sl, side, v0 + u, 4 * p, [&](int k) { return xv[k]; }, lane);
   }
 }
 
@@ -665,7 +658,7 @@ __global__ void __launch_bounds__(FAC_THREADS) k_local_factors(LocalUpdateArgs a
   const int v = wid * VPW + f.v;
   for (int j = 0; j < p; ++j)
     fac_step<SPLIT>(f, xs + v * ldx, j, coef + (size_t)8 * j * (j - 1), side == 0 ? kk + 16 * j : nullptr, s_t[v]);
-  fac_finish<VPW>(a, d, side, v0 + wid * VPW, p, xs + wid * VPW * ldx, ldx);
+  fac_finish<VPW>(d, side, v0 + wid * VPW, p, xs + wid * VPW * ldx, ldx);
 }
 
 // The factors beside the window (a chain that has the GPU to itself): a CTA of
@@ -718,7 +711,7 @@ __device__ void fac_follow(const LocalUpdateArgs& a, const DelayedArgs& d, int f
     named_bar(1, T);
     if (wid * VPW < nv) fac_step<SPLIT>(f, xs + v * ldx, j, cj, side == 0 ? kj : nullptr, ts + 4 * v);
   }
-  if (j > 0 && wid * VPW < nv) fac_finish<VPW>(a, d, side, v0 + wid * VPW, j, xs + wid * VPW * ldx, ldx);
+  if (j > 0 && wid * VPW < nv) fac_finish<VPW>(d, side, v0 + wid * VPW, j, xs + wid * VPW * ldx, ldx);
 }
 
 // Vectors of a follower CTA: the fewest that keep the followers within 7

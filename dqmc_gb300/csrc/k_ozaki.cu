@@ -75,7 +75,7 @@ namespace {
 constexpr int SPLIT_V = 4;
 __global__ void __launch_bounds__(64 * SPLIT_V) k_oz_split(const cplx* __restrict__ A, int lda, char opA,
                                                            const cplx* __restrict__ B, int ldb, char opB, int K,
-                                                           OzSlices o, const int* __restrict__ active) {
+                                                           OzSlices o) {
   extern __shared__ double4_16a smem_split[];
   cplx* tile = reinterpret_cast<cplx*>(smem_split);   // (SPLIT_V, K + 1)
   __shared__ int s_me[2 * SPLIT_V];
@@ -85,11 +85,6 @@ __global__ void __launch_bounds__(64 * SPLIT_V) k_oz_split(const cplx* __restric
   const char op = side ? opB : opA;
   const int v0 = blockIdx.x * SPLIT_V;
   if (v0 >= cnt) return;
-  if (active) {   // only the first 4p inner indices are live (delayed-update flush)
-    const int kk = 4 * *active;
-    if (kk == 0) return;
-    if (kk < K) K = kk;
-  }
   const int ldt = K + 1;
   const bool across = side ? op != 'N' : op == 'N';   // X contiguous across the vectors
   const bool conj = op == 'C';
@@ -256,7 +251,7 @@ __device__ __forceinline__ cplx oz_scale2(const OzArgs& a, cplx v, int row, int 
 // still holds its old value there).  Bound: FP64 issue, 4 multiply-adds per term,
 // as for k_zgemm; rows of A are read 16 bytes per sector.
 __device__ __forceinline__ void oz_dot(const OzArgs& a, int row, int col, bool need) {
-  const int lane = threadIdx.x & 31, K = a.active ? min(a.k, 4 * *a.active) : a.k;
+  const int lane = threadIdx.x & 31, K = a.k;
   unsigned todo = __ballot_sync(0xffffffffu, need);
   while (todo) {
     const int src = __ffs(todo) - 1;
@@ -963,20 +958,19 @@ cudaError_t launch_ozaki_zgemm(int m, int nn, int k, char opA, char opB, cplx al
   if (S < 1 || (S > TC_MAXS && !full) || bits < 1 || bits > 8 || !err) return cudaErrorInvalidValue;
   if (full && bits != OZ_FP64_BITS) return cudaErrorInvalidValue;
   guard = guard && full;
-  if (guard && presliced) return cudaErrorInvalidValue;
+  if ((guard && presliced) || (active && !presliced)) return cudaErrorInvalidValue;
   const int Kpad = (k + 15) / 16 * 16;
   const size_t Kp = 2 * (size_t)Kpad;
   if (ozaki_scratch_bytes(m, nn, k, S) > scratch_bytes) return cudaErrorInvalidValue;
   const OzSlices sl = ozaki_slices(scratch, m, nn, k, S, bits, guard);
-  if (!presliced) {   // otherwise the slices are already in scratch (cut by the delayed local-update kernel)
+  if (!presliced) {   // otherwise the slices are already in scratch (cut by the local updates; A and B are null)
     const size_t smem = (size_t)SPLIT_V * (k + 1) * sizeof(cplx);
     static SmemLimit limit_split;
     if (cudaError_t e = limit_split.raise((const void*)k_oz_split, SPLIT_V * (1024 + 1) * (int)sizeof(cplx));
         e != cudaSuccess)
       return e;
     const int vecs = m > nn ? m : nn;
-    k_oz_split<<<dim3((vecs + SPLIT_V - 1) / SPLIT_V, 2), 64 * SPLIT_V, smem, st>>>(A, lda, opA, B, ldb, opB, k, sl,
-                                                                                   active);
+    k_oz_split<<<dim3((vecs + SPLIT_V - 1) / SPLIT_V, 2), 64 * SPLIT_V, smem, st>>>(A, lda, opA, B, ldb, opB, k, sl);
   }
   OzArgs a;
   a.A = presliced ? nullptr : A; a.B = B; a.lda = lda; a.ldb = ldb; a.k = k; a.opA = opA; a.opB = opB;

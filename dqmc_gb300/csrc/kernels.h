@@ -71,8 +71,6 @@ struct OzSlices {
 };
 constexpr int WIN_MAX = 32;   // most sites of a window (a window takes min(k, 32))
 struct DelayedArgs {
-  cplx* X;
-  cplx* Y;
   int* state;
   int k;                   // most acceptances of a round
   const SitePrep* prep;    // (N) from launch_local_prepare for this slice
@@ -83,7 +81,6 @@ struct DelayedArgs {
   int* wflag;              // (WIN_MAX + 1) acceptances published to the follower clusters
   int* arrive;             // (2) followers that have read the state, clusters started (zero between launches)
   OzSlices sl;             // the flush's slices, cut where the factors are formed
-                           // (sl.As null: X and Y are stored and the flush slices them itself)
 };
 // Decides the next window of the slice on one cluster of 16 CTAs, 8 when other
 // chains share the GPU.
@@ -91,7 +88,7 @@ cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, 
                                 bool follow);
 // whether the window can have follower clusters that form its factors (else launch_local_factors)
 bool local_window_follows(int n, int k);
-// The factors X (n x 4p, column-major) and Y (4p x n, row j at Y + j n) of the window's p acceptances.
+// The slices of the factors X (n x 4p) and Y (4p x n) of the window's p acceptances.
 cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st);
 int local_window_sites(int k);
 // Sets the WHILE condition of a captured round loop (see local_updates_dev):
@@ -103,12 +100,9 @@ cudaError_t launch_round_cond(cudaGraphConditionalHandle hc, int* state, int N, 
 // ---- dense linear algebra (k_linalg.cu) ----
 // C = alpha * op(A) * op(B) + beta * C, all n x n column-major; op: 'N', 'C' (conjugate transpose)
 // optional diagonal scalings: rowscale (applied to rows of op(A)), colscale (to columns of op(B)).
-// active: optional device count p of pending rank-4 factors; when given, the
-// product uses only the first 4p columns of op(A) / rows of op(B), and does
-// nothing when p == 0 (the delayed-update flush).
 cudaError_t launch_zgemm(int m, int nn, int k, char opA, char opB, cplx alpha, const cplx* A, int lda,
                          const cplx* B, int ldb, cplx beta, cplx* C, int ldc, const double* rowscale,
-                         const double* colscale, cudaStream_t st, const int* active = nullptr);
+                         const double* colscale, cudaStream_t st);
 
 struct QRWork {
   double* vn1;       // (2n) partial column norms, reciprocals at [n + j]
@@ -144,8 +138,7 @@ cudaError_t launch_apply_q_right(cplx* X, int m, int n, const QRWork& w, bool co
 //   right: Y <- Y That^-1       (Y is m x n)
 // Row/column permutation by the pivot order is applied by the caller with
 // launch_permute.
-// order == nullptr: T itself is upper triangular; rdiag != nullptr: 1 / diagonal (else the diagonal of T)
-cudaError_t launch_trsm_left_upper(const cplx* T, const int* order, const cplx* rdiag, cplx* Y, int n, int m,
+cudaError_t launch_trsm_left_upper(const cplx* T, const int* order, cplx* Y, int n, int m,
                                    cudaStream_t st);
 // rows j0..j0+b of the m columns of Y <- (b x b diagonal block of T at j0)^-1 (.) (b <= 128):
 // lower: unit lower triangular; else upper with reciprocal diagonal rdiag
