@@ -924,7 +924,7 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
     // followers only where the chain has the GPU to itself
     const bool follow = h->follow && h->coop_cap == 0;
     LAUNCH(DQMC_K_LOCAL, 0.0, 0.0, launch_local_window(a, d, h->st, h->coop_cap > 0, follow));
-    if (!follow) LAUNCH(DQMC_K_FLUSH, 0.0, 0.0, launch_local_factors(a, d, h->st));
+    if (!follow) LAUNCH(DQMC_K_FLUSH, 0.0, 0.0, launch_local_factors(a, d, h->sm_count, h->st));
     // flush G += X Y over the 4p new columns (p read on the device; no work when p = 0)
     return zgemm_general(h, n, n, 4 * k, 'N', 'T', cmake(1, 0), nullptr, n, nullptr, n, cmake(1, 0), h->G, n, nullptr,
                          nullptr, true, DQMC_K_FLUSH, h->dstate + 1, true, false, h->flush_full);

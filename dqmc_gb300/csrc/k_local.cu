@@ -1281,10 +1281,10 @@ bool local_window_follows(int n, int k) {
   return clusters >= 1 + follower_clusters(n, C);
 }
 
-cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st) {
+cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, int sm_count, cudaStream_t st) {
   const int n = a.mc.n, W = local_window_sites(d.k);
-  // lanes per vector: 2 n vectors on about 600 sub-partitions, one warp each
-  const int split = n <= 304 ? 4 : n <= 608 ? 2 : 1;
+  // lanes per vector: 2 n vectors of 8 split lanes on 4 sub-partitions per SM, one warp each
+  const int split = n <= 2 * sm_count ? 4 : n <= 4 * sm_count ? 2 : 1;
   const int vpc = 16 / split;   // n = 4 L^2 with L even: a multiple of 16
   const size_t smem = ((size_t)8 * W * (W - 1) + 16 * W + (size_t)vpc * (4 * d.k + 1)) * sizeof(cplx);
   static SmemLimit limits[3];

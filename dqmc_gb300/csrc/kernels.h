@@ -89,7 +89,7 @@ cudaError_t launch_local_window(const LocalUpdateArgs& a, const DelayedArgs& d, 
 // whether the window can have follower clusters that form its factors (else launch_local_factors)
 bool local_window_follows(int n, int k);
 // The slices of the factors X (n x 4p) and Y (4p x n) of the window's p acceptances.
-cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, cudaStream_t st);
+cudaError_t launch_local_factors(const LocalUpdateArgs& a, const DelayedArgs& d, int sm_count, cudaStream_t st);
 int local_window_sites(int k);
 // Sets the WHILE condition of a captured round loop (see local_updates_dev):
 // another round while state[0] < N, state[2] < max_rounds and *err == 0.
