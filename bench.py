@@ -176,11 +176,18 @@ def flops_model(kind, t, n, accepted, real_flushes):
 
 def real_flush_count(acc_flags, M, N, delay):
     """Flushes with work in one sweep: a round decides a window of
-    min(delay, 32) sites (16 for depths 0 and 1) and flushes with work when it
-    accepted any of them."""
-    w = min(delay, 32) if delay > 1 else 16
-    a = np.asarray(acc_flags, dtype=np.int64).reshape(M, N)
-    return int(sum(a[:, i:i + w].any(axis=1).sum() for i in range(0, N, w)))
+    min(delay, 32) sites (16 for depths 0 and 1; 2 delay below 8, up to `delay`
+    acceptances) and flushes with work when it accepted any of them."""
+    k = delay if delay > 1 else 16
+    w = 2 * k if k < 8 else min(k, 32)
+    flushes = 0
+    for a in np.asarray(acc_flags, dtype=bool).reshape(M, N):
+        i = 0
+        while i < N:
+            hits = np.flatnonzero(a[i:i + w])
+            flushes += hits.size > 0
+            i += hits[k - 1] + 1 if hits.size >= k else w
+    return flushes
 
 
 def cpu_baseline(p, phi, n_calls, seed, threads):

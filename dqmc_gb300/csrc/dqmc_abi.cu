@@ -918,7 +918,7 @@ int local_updates_dev(dqmc_handle* h, const double* delta_dev, const double* uni
     CU(cudaStreamWaitEvent(h->st, h->side_join, 0));
   }
   // a round consumes a whole window of sites or k acceptances
-  const int w = local_window_sites(k);
+  const int w = std::min(local_window_sites(k), k);
   const int rounds = (h->N + w - 1) / w + 1;
   auto round = [&]() -> int {
     // followers only where the chain has the GPU to itself

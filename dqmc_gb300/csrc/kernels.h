@@ -69,7 +69,7 @@ struct OzSlices {
   double *sA, *sB;
   int m, n, Kpad, S, bits;
 };
-constexpr int WIN_MAX = 32;   // most sites of a window (a window takes min(k, 32))
+constexpr int WIN_MAX = 32;   // most sites of a window
 struct DelayedArgs {
   int* state;
   int k;                   // most acceptances of a round

@@ -65,9 +65,9 @@ typedef struct dqmc_params {
   int32_t device;      /* CUDA device ordinal; -1 = the calling thread's current device */
   int32_t ozaki_bits;  /* mixed form: mantissa bits kept per GEMM operand (0 = default 40); at most what
                           8 slices reach at the product's inner dimension (40 bits at K = 1024) */
-  int32_t delay;       /* delayed-update depth k, at most 64: rounds of min(k, 32) sites, whose accepted rank-4
-                          updates are applied to G together.  0 or 1: FP64 rank-4 updates in either form,
-                          16 sites at a time */
+  int32_t delay;       /* delayed-update depth k, at most 64: at most k accepted rank-4 updates are applied to G
+                          together, of a window of k sites (2k below 8, 32 above 32).  0 or 1: FP64 rank-4
+                          updates in either form, 16 sites at a time */
   int32_t greens_method; /* DQMC_GREENS_SCALES (default) or DQMC_GREENS_TWO_QR */
   int32_t inflight;    /* dqmc_batch_create: chains swept at the same time (0 = min(count, 8)); first chain's value.
                           dqmc_create: > 1 caps the cooperative grids as for one of that many batch chains */
