@@ -321,8 +321,10 @@ int wrap_greens(dqmc_handle* h, cplx* gf, int slice, int direction) {
 // is at most 0.01 of an FMA chain's, unless the large entries of its row meet the
 // small ones of its column; guard makes such elements FP64 dot products.  Guarded
 // are the updates of the LU and of the triangular solves, which divide by what
-// they leave (few elements: solves 4.71 -> 4.93 ms, LU 8.00 -> 8.13 ms in two
-// stabilisations at L = 16), and every product of operands that the caller gave.
+// they leave (two stabilisations at L = 16, beta = 20: solves 4.71 -> 4.91 ms, LU
+// 8.00 -> 8.04; at beta = 2, where G is short-ranged and up to 18% of the elements
+// are of that kind, solves 4.7 -> 9.3), and every product of operands that the
+// caller gave.
 // In the others (T and U of the stack, Q, the flush) up to half of the elements
 // are of that kind, and guarded they would cost what the FMA kernel does (sweep
 // at L = 16 193 instead of 89 ms); there the rounding of entries of order one in

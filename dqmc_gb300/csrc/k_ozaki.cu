@@ -246,38 +246,53 @@ __device__ __forceinline__ cplx oz_scale2(const OzArgs& a, cplx v, int row, int 
   if (a.cs) v = cscale(v, a.cs[col]);
   return v;
 }
-// the elements C[row of this lane, col] for which need is set, one warp each: dot
-// products in FP64 multiply-adds over the operands (called by whole warps; C
-// still holds its old value there).  Bound: FP64 issue, 4 multiply-adds per term,
-// as for k_zgemm; rows of A are read 16 bytes per sector.
+// the elements C[row of this lane, col] for which need is set, 8 lanes each: dot
+// products in FP64 multiply-adds over the operands, in four sums per lane (called
+// by whole warps; C still holds its old value there).  Bound: FP64 issue, 4
+// multiply-adds per term as for k_zgemm, and as much again for the sums of the
+// lanes at K = 64 (a whole warp per element has three times that).
 __device__ __forceinline__ void oz_dot(const OzArgs& a, int row, int col, bool need) {
-  const int lane = threadIdx.x & 31, K = a.k;
+  const int lane = threadIdx.x & 31, sub = lane & 7, K = a.k;
+  const size_t sa = a.opA == 'N' ? a.lda : 1, sb = a.opB == 'N' ? 1 : a.ldb;
+  const bool ca = a.opA == 'C', cb = a.opB == 'C';
   unsigned todo = __ballot_sync(0xffffffffu, need);
   while (todo) {
-    const int src = __ffs(todo) - 1;
-    todo &= todo - 1;
-    const int r = __shfl_sync(0xffffffffu, row, src), c = __shfl_sync(0xffffffffu, col, src);
+    int src = -1;   // lane group q takes the q-th element left
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (todo && lane >> 3 == q) src = __ffs(todo) - 1;
+      todo &= todo - 1;
+    }
+    const int r = __shfl_sync(0xffffffffu, row, max(src, 0)), c = __shfl_sync(0xffffffffu, col, max(src, 0));
     const cplx* pa = a.opA == 'N' ? a.A + r : a.A + (size_t)r * a.lda;
     const cplx* pb = a.opB == 'N' ? a.B + (size_t)c * a.ldb : a.B + c;
-    const size_t sa = a.opA == 'N' ? a.lda : 1, sb = a.opB == 'N' ? 1 : a.ldb;
-    cplx s = cmake(0.0, 0.0);
-#pragma unroll 4
-    for (int k = lane; k < K; k += 32) {
-      cplx x = pa[k * sa], y = pb[k * sb];
-      if (a.opA == 'C') x = cconj(x);
-      if (a.opB == 'C') y = cconj(y);
-      s = cfma(x, y, s);
-    }
+    cplx s[4];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    for (int q = 0; q < 4; ++q) s[q] = cmake(0.0, 0.0);
+    if (src >= 0) {
+      for (int k0 = sub; k0 < K; k0 += 32) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int k = k0 + 8 * q;
+          if (k >= K) continue;
+          cplx x = pa[k * sa], y = pb[k * sb];
+          if (ca) x = cconj(x);
+          if (cb) y = cconj(y);
+          s[q] = cfma(x, y, s[q]);
+        }
+      }
     }
-    if (lane == 0) {
+    cplx t = cadd(cadd(s[0], s[1]), cadd(s[2], s[3]));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    }
+    if (src >= 0 && sub == 0) {
       cplx* cp = &a.C[(size_t)c * a.ldc + r];
-      s = cmul(a.alpha, oz_scale2(a, s, r, c));   // as k_zgemm, also for what is not finite
-      if (a.beta.x != 0.0 || a.beta.y != 0.0) s = cfma(a.beta, *cp, s);
-      *cp = s;
+      t = cmul(a.alpha, oz_scale2(a, t, r, c));   // as k_zgemm, also for what is not finite
+      if (a.beta.x != 0.0 || a.beta.y != 0.0) t = cfma(a.beta, *cp, t);
+      *cp = t;
     }
     __syncwarp();
   }
