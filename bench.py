@@ -57,10 +57,10 @@ METRIC = "O(3) L=16 sweeps/s: mixed vs FP64 at G err≤1e-8; batched chain-sweep
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the
 # roofline kernels at L=16 (n = 1024), one ncu capture of this bench's L=16
 # mixed profiling workload (--profile-calls 12): k_oz_gemm_tc (one n x n x n
-# product: 170.9 + 14.0 MB).  None: the kind is several kernels per algorithmic
+# product, tiles of 32 columns, 16 epilogue warps, MMAs of N = 256: 167.2 + 13.6 MB).  None: the kind is several kernels per algorithmic
 # unit (QR, blocked LU, blocked triangular solves, compact-WY Q formation, flush)
 TRAFFIC = {"qrp": None, "lu": None, "apply_q": None, "trsm": None, "flush": None,
-           "ozaki_gemm": 184.852e6}
+           "ozaki_gemm": 180.792e6}
 
 
 def model_params(L, M):

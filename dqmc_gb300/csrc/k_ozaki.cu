@@ -2,9 +2,9 @@
 //
 //   C = alpha * diag(rs) * op(A) * op(B) * diag(cs) + beta * C     (complex FP64)
 //
-// GB300 runs FP64 at ~1/1500 of its BF16 tensor rate, so the mixed-precision
-// form computes the dense products of the UDT stabilisation and of the
-// delayed local-update flush as sums of exact BF16 x BF16 -> FP32 products:
+// GB300 runs FP64 at ~1/1500 of its BF16 tensor rate, so both forms compute the
+// dense products of the UDT stabilisation and of the local updates' flush as
+// sums of exact BF16 x BF16 -> FP32 products:
 //
 //  * every row i of op(A) gets a power-of-two scale sigma_i > max_k |op(A)_ik|
 //    (real and imaginary parts together), every column j of op(B) a scale
@@ -362,7 +362,9 @@ __global__ void k_oz_finalize(OzArgs a) {
 //     and after the tile's last chunk round, scale and store.
 // The full form (S = 9) has tiles of at most 24 columns, so that its 9 groups of
 // 48 columns (and the magnitudes' 32, if guarded) fit into TMEM; the magnitudes are
-// slice S of A and one more B tile, summed over all chunks of a tile.
+// slice S of A and one more B tile, summed over all chunks of a tile.  At n = 1024,
+// slicing included, 8 slices of 7 bits at 32 columns -> this: product 0.36 -> 0.48 ms,
+// flush of 16 sites 36 -> 44 us on average.
 // Every wait is bounded; on a timeout the kernel sets an error bit, drains
 // what it issued (bounded) and frees its TMEM.
 constexpr int TC_BM = 128;                      // rows of C per CTA (TMEM lanes)
