@@ -323,7 +323,7 @@ int wrap_greens(dqmc_handle* h, cplx* gf, int slice, int direction) {
 // are the updates of the LU and of the triangular solves, which divide by what
 // they leave (two stabilisations at L = 16, beta = 20: solves 4.71 -> 4.91 ms, LU
 // 8.00 -> 8.04; at beta = 2, where G is short-ranged and up to 18% of the elements
-// are of that kind, solves 4.7 -> 9.3), and every product of operands that the
+// are of that kind, solves 4.7 -> 7.9), and every product of operands that the
 // caller gave.
 // In the others (T and U of the stack, Q, the flush) up to half of the elements
 // are of that kind, and guarded they would cost what the FMA kernel does (sweep

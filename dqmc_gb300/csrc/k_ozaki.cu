@@ -246,54 +246,81 @@ __device__ __forceinline__ cplx oz_scale2(const OzArgs& a, cplx v, int row, int 
   if (a.cs) v = cscale(v, a.cs[col]);
   return v;
 }
-// the elements C[row of this lane, col] for which need is set, 8 lanes each: dot
-// products in FP64 multiply-adds over the operands, in four sums per lane (called
-// by whole warps; C still holds its old value there).  Bound: FP64 issue, 4
-// multiply-adds per term as for k_zgemm, and as much again for the sums of the
-// lanes at K = 64 (a whole warp per element has three times that).
+// t = op(A)[row, :] op(B)[:, col] into C[row, col], as k_zgemm does (also for what is not finite)
+__device__ __forceinline__ void oz_put(const OzArgs& a, int row, int col, cplx t) {
+  cplx* cp = &a.C[(size_t)col * a.ldc + row];
+  t = cmul(a.alpha, oz_scale2(a, t, row, col));
+  if (a.beta.x != 0.0 || a.beta.y != 0.0) t = cfma(a.beta, *cp, t);
+  *cp = t;
+}
+// The elements C[row of this lane, col] for which need is set: dot products in
+// FP64 multiply-adds over the operands (called by whole warps; C still holds its
+// old value there).  8 lanes per element, or one where most lanes have one; every
+// lane adds four sums and reads four terms ahead.  Bound: FP64 issue, 4 multiply-
+// adds per term as for k_zgemm, and with 8 lanes as much again for the sums of the
+// lanes at K = 64.  All elements of n = 1024: not read ahead 17.1 ms, so 10.1
+// (k_zgemm 8.3).
 __device__ __forceinline__ void oz_dot(const OzArgs& a, int row, int col, bool need) {
-  const int lane = threadIdx.x & 31, sub = lane & 7, K = a.k;
+  const int lane = threadIdx.x & 31, K = a.k;
   const size_t sa = a.opA == 'N' ? a.lda : 1, sb = a.opB == 'N' ? 1 : a.ldb;
-  const bool ca = a.opA == 'C', cb = a.opB == 'C';
+  const int fa = a.opA == 'C' ? (int)0x80000000 : 0, fb = a.opB == 'C' ? (int)0x80000000 : 0;
+  auto conj_if = [](cplx v, int f) { return cmake(v.x, __hiloint2double(__double2hiint(v.y) ^ f, __double2loint(v.y))); };
   unsigned todo = __ballot_sync(0xffffffffu, need);
+  const bool lanes = __popc(todo) >= 20;   // one lane per element
   while (todo) {
-    int src = -1;   // lane group q takes the q-th element left
+    int r = row, c = col, k0 = 0, step = 1;
+    bool on = need;
+    if (lanes) {
+      todo = 0u;
+    } else {
+      int src = -1;   // lane group q takes the q-th element left
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (todo && lane >> 3 == q) src = __ffs(todo) - 1;
-      todo &= todo - 1;
+      for (int q = 0; q < 4; ++q) {
+        if (todo && lane >> 3 == q) src = __ffs(todo) - 1;
+        todo &= todo - 1;
+      }
+      on = src >= 0;
+      r = __shfl_sync(0xffffffffu, row, max(src, 0));
+      c = __shfl_sync(0xffffffffu, col, max(src, 0));
+      k0 = lane & 7;
+      step = 8;
     }
-    const int r = __shfl_sync(0xffffffffu, row, max(src, 0)), c = __shfl_sync(0xffffffffu, col, max(src, 0));
-    const cplx* pa = a.opA == 'N' ? a.A + r : a.A + (size_t)r * a.lda;
-    const cplx* pb = a.opB == 'N' ? a.B + (size_t)c * a.ldb : a.B + c;
     cplx s[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) s[q] = cmake(0.0, 0.0);
-    if (src >= 0) {
-      for (int k0 = sub; k0 < K; k0 += 32) {
+    if (on) {
+      const cplx* pa = a.opA == 'N' ? a.A + r : a.A + (size_t)r * a.lda;
+      const cplx* pb = a.opB == 'N' ? a.B + (size_t)c * a.ldb : a.B + c;
+      cplx x[4], y[4], xn[4], yn[4];
+      auto read = [&](int k, cplx(&u)[4], cplx(&v)[4]) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int k = k0 + 8 * q;
-          if (k >= K) continue;
-          cplx x = pa[k * sa], y = pb[k * sb];
-          if (ca) x = cconj(x);
-          if (cb) y = cconj(y);
-          s[q] = cfma(x, y, s[q]);
+          const int kk = k + q * step;
+          u[q] = kk < K ? pa[kk * sa] : cmake(0.0, 0.0);
+          v[q] = kk < K ? pb[kk * sb] : cmake(0.0, 0.0);
+        }
+      };
+      read(k0, x, y);
+#pragma unroll 1
+      for (int k = k0; k < K; k += 4 * step) {
+        read(k + 4 * step, xn, yn);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          s[q] = cfma(conj_if(x[q], fa), conj_if(y[q], fb), s[q]);
+          x[q] = xn[q];
+          y[q] = yn[q];
         }
       }
     }
     cplx t = cadd(cadd(s[0], s[1]), cadd(s[2], s[3]));
+    if (!lanes) {
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
-      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+      for (int o = 4; o > 0; o >>= 1) {
+        t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+        t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+      }
     }
-    if (src >= 0 && sub == 0) {
-      cplx* cp = &a.C[(size_t)c * a.ldc + r];
-      t = cmul(a.alpha, oz_scale2(a, t, r, c));   // as k_zgemm, also for what is not finite
-      if (a.beta.x != 0.0 || a.beta.y != 0.0) t = cfma(a.beta, *cp, t);
-      *cp = t;
-    }
+    if (on && (lanes || (lane & 7) == 0)) oz_put(a, r, c, t);
     __syncwarp();
   }
 }
@@ -671,62 +698,63 @@ __global__ void __launch_bounds__(tc_threads(BN), 1) k_oz_gemm_tc(const __grid_c
     const bool plain = oz_plain(a), neg = a.alpha.x < 0.0;
     const bool simple = plain && !a.rs && !a.cs;   // alpha = +-1, beta in {0, 1}, no extra scalings
     const int nch = (nkb + a.kexact - 1) / a.kexact;
-    long long ar[CPW], ai[CPW], lr[WIDE ? CPW : 1], li[WIDE ? CPW : 1];   // the tile's sums so far
-    for (int vt = 0; vt < my_tiles * nch; ++vt) {
+    for (int tt = 0; tt < my_tiles; ++tt) {
       int i0, j0;
-      tile_of(vt / nch, i0, j0);
+      tile_of(tt, i0, j0);
       j0 += CPW * cg;
-      // several chunks only in the full form: the mixed form's widths take all of K at once
-      const bool first = !FULL || vt % nch == 0, last = !FULL || vt % nch == nch - 1;
       const int row = i0 + 32 * quarter + lane;
-      const bool waited = mbar_wait(bar(ACC), vt & 1, err, s_abort);
-      // tcgen05.ld is warp-collective: the decision must be uniform over the warp
-      const bool have = __all_sync(0xffffffffu, waited && !*s_abort);
-      if (!have) break;
-      __syncwarp();
-      tc_fence_after();
-      if (first) {
+      long long ar[CPW], ai[CPW], lr[WIDE ? CPW : 1], li[WIDE ? CPW : 1];   // the tile's sums
 #pragma unroll
-        for (int c = 0; c < CPW; ++c) { ar[c] = 0; ai[c] = 0; }
+      for (int c = 0; c < CPW; ++c) { ar[c] = 0; ai[c] = 0; }
 #pragma unroll
-        for (int c = 0; c < (WIDE ? CPW : 1); ++c) { lr[c] = 0; li[c] = 0; }
-      }
+      for (int c = 0; c < (WIDE ? CPW : 1); ++c) { lr[c] = 0; li[c] = 0; }
+      uint32_t mg[CPW] = {};   // the magnitude sums
+      bool have = true;
+      // several chunks only in the full form: the mixed form's widths take all of K at once
+      for (int ch = 0; ch < (FULL ? nch : 1); ++ch) {
+        const bool waited = mbar_wait(bar(ACC), (FULL ? tt * nch + ch : tt) & 1, err, s_abort);
+        // tcgen05.ld is warp-collective: the decision must be uniform over the warp
+        have = __all_sync(0xffffffffu, waited && !*s_abort);
+        if (!have) break;
+        __syncwarp();
+        tc_fence_after();
 #pragma unroll 1
-      for (int g = 0; g < ghi; ++g) {
-        uint32_t ur[CPW], ui[CPW];
-        tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN), ur);
-        tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN + BN), ui);
-        tc_wait_ld();
-#pragma unroll
-        for (int c = 0; c < CPW; ++c) {
-          ar[c] += (long long)__float2int_rn(__uint_as_float(ur[c])) << (bits * (ghi - 1 - g));
-          ai[c] += (long long)__float2int_rn(__uint_as_float(ui[c])) << (bits * (ghi - 1 - g));
-        }
-      }
-      if constexpr (WIDE) {
-#pragma unroll 1
-        for (int g = ghi; g < S; ++g) {
+        for (int g = 0; g < ghi; ++g) {
           uint32_t ur[CPW], ui[CPW];
           tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN), ur);
           tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN + BN), ui);
           tc_wait_ld();
 #pragma unroll
           for (int c = 0; c < CPW; ++c) {
-            lr[c] += (long long)__float2int_rn(__uint_as_float(ur[c])) << (bits * (S - 1 - g));
-            li[c] += (long long)__float2int_rn(__uint_as_float(ui[c])) << (bits * (S - 1 - g));
+            ar[c] += (long long)__float2int_rn(__uint_as_float(ur[c])) << (bits * (ghi - 1 - g));
+            ai[c] += (long long)__float2int_rn(__uint_as_float(ui[c])) << (bits * (ghi - 1 - g));
           }
         }
+        if constexpr (WIDE) {
+#pragma unroll 1
+          for (int g = ghi; g < S; ++g) {
+            uint32_t ur[CPW], ui[CPW];
+            tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN), ur);
+            tc_ld<CPW>(tq + (uint32_t)(g * 2 * BN + BN), ui);
+            tc_wait_ld();
+#pragma unroll
+            for (int c = 0; c < CPW; ++c) {
+              lr[c] += (long long)__float2int_rn(__uint_as_float(ur[c])) << (bits * (S - 1 - g));
+              li[c] += (long long)__float2int_rn(__uint_as_float(ui[c])) << (bits * (S - 1 - g));
+            }
+          }
+        }
+        if (GUARD && ch == nch - 1) {
+          tc_ld<CPW>(tq + (uint32_t)(S * 2 * BN), mg);
+          tc_wait_ld();
+        }
+        // this chunk's accumulators are all in registers: TMEM may take the next chunk
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(TE));
       }
-      uint32_t mg[CPW] = {};   // the magnitude sums
-      if (GUARD && last) {
-        tc_ld<CPW>(tq + (uint32_t)(S * 2 * BN), mg);
-        tc_wait_ld();
-      }
-      // this chunk's accumulators are all in registers: TMEM may take the next chunk
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(TE));
-      if (!last || (!FULL && row >= a.m)) continue;
+      if (!have) break;
+      if (!FULL && row >= a.m) continue;
       if (a.acc) {
 #pragma unroll
         for (int c = 0; c < CPW; ++c) {
